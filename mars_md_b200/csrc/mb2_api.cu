@@ -60,7 +60,7 @@ struct mb2_context {
 	// pair tables
 	PairTables pt;
 	DevBuf<PairTableRef> refs;
-	DevBuf<int> table_offsets;  // per type pair: offset of its table's bins, -1 none
+	FastTableBufs fast;
 	DevBuf<float> bin_force;
 	DevBuf<float2> bin_energy;
 
@@ -803,20 +803,10 @@ int mb2_set_pair_tables(mb2_context* ctx, int num_types, const uint32_t* term_ma
 							cudaMemcpyHostToDevice));
 		MB2_CUDA(cudaMemcpy(ctx->bin_energy.ptr, be.data(), be.size() * sizeof(float2),
 							cudaMemcpyHostToDevice));
-		// Tables of one start, bin width and length for every type pair that
-		// has one (compared bit for bit): the kernel reads 4-byte offsets.
-		std::vector<int> offs;
-		PairTableRef u;
-		const bool uniform = uniform_tables(refs, offs, u);
-		ctx->table_offsets.ensure(tt);
-		MB2_CUDA(cudaMemcpy(ctx->table_offsets.ptr, offs.data(), tt * sizeof(int),
-							cudaMemcpyHostToDevice));
+		ctx->fast.set(refs, bf, be, ctx->pt);
 		ctx->pt.num_types = num_types;
 		ctx->pt.total_bins = static_cast<uint32_t>(total);
 		ctx->pt.refs = ctx->refs.ptr;
-		ctx->pt.offsets = ctx->table_offsets.ptr;
-		ctx->pt.uniform = uniform;
-		ctx->pt.uniform_ref = u;
 		ctx->pt.bin_force = ctx->bin_force.ptr;
 		ctx->pt.bin_energy = ctx->bin_energy.ptr;
 		ctx->term_matrix_h.assign(term_matrix, term_matrix + tt);
@@ -1310,7 +1300,8 @@ std::vector<uint64_t> run_graph_key(const mb2_context* ctx, const float4* pos, c
 		P(ctx->inv.ptr), P(ctx->force_sorted.ptr), P(ctx->energy.ptr), P(ctx->step_d.ptr),
 		P(ctx->bonded_tables[0].ptr), P(ctx->bonded_tables[1].ptr), P(ctx->bonded_tables[2].ptr),
 		static_cast<uint64_t>(ctx->pt.num_types), ctx->pt.total_bins, P(ctx->pt.refs),
-		P(ctx->pt.offsets), static_cast<uint64_t>(ctx->pt.uniform), fbits(ctx->pt.uniform_ref.start),
+		P(ctx->pt.fast_force), P(ctx->pt.fast_energy), P(ctx->pt.fast_offsets),
+		fbits(ctx->pt.reach_force), fbits(ctx->pt.reach_energy), fbits(ctx->pt.uniform_ref.start),
 		fbits(ctx->pt.uniform_ref.step_inv), static_cast<uint64_t>(ctx->pt.uniform_ref.last),
 		P(ctx->pt.bin_force), P(ctx->pt.bin_energy), P(ctx->pt.terms),
 		static_cast<uint64_t>(ctx->types.num_types), P(ctx->types.charge), P(ctx->types.diffusion),

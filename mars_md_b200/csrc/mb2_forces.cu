@@ -75,18 +75,6 @@ __device__ __forceinline__ float wrap1(float x, float l, float inv, float half) 
 	return x >= half ? __fsub_rn(x, l) : x;
 }
 
-// wrap1 for a component known to lie in [-l/2, l/2] (rows inside the box,
-// below): the reference's image floor(RN(x / l)) is 0 for x >= 0 and -1 for
-// x < 0, so its result is x, or RN(RN(x + l) - l) (which is >= l/2 before the
-// second rounding, so the reference takes that branch too), picked by the
-// sign bit. -0 takes the second form: RN(RN(-0 + l) - l) = +0, as the
-// reference's floor(-0) = -0 gives. (A negative x so small that x / l
-// underflows, |x| < 2^-149 l, would keep x where this gives +0.)
-__device__ __forceinline__ float wrap_inner(float x, float l, float negl) {
-	const float w = __fadd_rn(__fadd_rn(x, l), negl);
-	return __float_as_int(x) < 0 ? w : x;
-}
-
 // math::sinh_minus_x / x_cosh_minus_sinh (src/Types/Math.h:199-216): the
 // reference's series below |x| = 1, the direct difference above.
 __device__ __forceinline__ float sinh_minus_x(float x) {
@@ -185,56 +173,35 @@ __device__ __forceinline__ void analytic_terms(uint32_t terms, const PairTermRef
 	}
 }
 
-// The table references of one row's type: the full 16-byte reference per j
-// type, or (kUniform) the shared start / step_inv / last with a 4-byte offset
-// per j type, one broadcast shared-memory word for the warp instead of a
-// 128-bit load.
-template <bool kUniform>
+// The table references of one row's type.
 struct TableRow {
 	const PairTableRef* row;
-	const int* off;
-	PairTableRef u;
-	__device__ __forceinline__ PairTableRef operator()(int tj) const {
-		if (kUniform) {
-			PairTableRef t = u;
-			t.offset = off[tj];
-			return t;
-		}
-		return row[tj];
-	}
+	__device__ __forceinline__ PairTableRef operator()(int tj) const { return row[tj]; }
 };
 
-// One pair of the half list, rounded as the reference rounds it. flip
-// (bit 31 of the entry): the reference orients the pair j -> i. With kTerms,
-// the analytical terms of the type pair come first, then the table.
-//
-// The x and y components go through sm_100's packed FP32 instructions
-// (__fadd2_rn / __fmul2_rn: two IEEE round-to-nearest operations each, so
-// every value is the scalar one bit for bit), z stays scalar. npi = (-pi.x,
-// -pi.y); a - b is computed as a + (-b) and b * l as -(b * (-l)), both exact
-// rewrites. The i-force is accumulated negated (nxy, nz): -(a - h) = (-a) + h
-// in round-to-nearest, so the caller's negation at the end gives the same sum.
-template <bool kEnergy, bool kAllPeriodic, bool kTerms, bool kInner, class TRow>
-__device__ __forceinline__ void pair_scalar(const float4& pi, float2 npi, const float4& pj,
-											uint32_t j, uint32_t flip,
-											const TRow& trow, const float* bin_f,
-											const float2* bin_e, const PairTermRef* arow,
-											const PairSolvent& sv, const Box& box,
-											const DistWindow& win, float4* force, float2& nxy, float& nz,
-											float& fe, double& e_acc, double& w_acc) {
-	// r = wrap_diff(pos[second] - pos[first])
-	// (pi - pj is exactly -(pj - pi) in round-to-nearest, so a sign flip
-	// suffices; a multiply by -1 is that flip, on the FMA pipe)
-	const float sgn = __uint_as_float(flip | 0x3F800000u);  // +1, or -1 when flipped
-	float2 dxy = __fmul2_rn(__fadd2_rn(make_float2(pj.x, pj.y), npi), make_float2(sgn, sgn));
-	float dz = __fmul_rn(__fsub_rn(pj.z, pi.z), sgn);
+// r = wrap_diff(pos[second] - pos[first]) as the reference rounds it: sgn is -1
+// when the pair is stored second to first (pi - pj is exactly -(pj - pi) in
+// round-to-nearest, so the multiply is the flip, on the FMA pipe). npi =
+// (-pi.x, -pi.y). kInner: the caller knows that every component lies in
+// [-l/2, l/2] of an all-periodic box.
+template <bool kAllPeriodic, bool kInner>
+__device__ __forceinline__ void oriented_image(const float4& pi, const float2& npi,
+											   const float4& pj, float sgn, const Box& box,
+											   float2& dxy, float& dz) {
+	dxy = __fmul2_rn(__fadd2_rn(make_float2(pj.x, pj.y), npi), make_float2(sgn, sgn));
+	dz = __fmul_rn(__fsub_rn(pj.z, pi.z), sgn);
 	if (kInner) {
-		// the row lies inside the box: |d| <= l/2 on every axis
+		// The reference's image floor(RN(x / l)) is 0 for x >= 0 and -1 for
+		// x < 0, so its result is x, or RN(RN(x + l) - l) (RN(x + l) is >= l/2,
+		// so the reference takes its second branch too; for -0 it is +0). Both
+		// are RN(RN(x + m) - m) with m = 0 or l, chosen on the FMA pipe: the ALU
+		// pipe is the busier one.
 		const float2 l = make_float2(box.size[0], box.size[1]);
-		const float2 w = __fadd2_rn(__fadd2_rn(dxy, l), make_float2(-l.x, -l.y));
-		dxy.x = __float_as_int(dxy.x) < 0 ? w.x : dxy.x;
-		dxy.y = __float_as_int(dxy.y) < 0 ? w.y : dxy.y;
-		dz = wrap_inner(dz, box.size[2], -box.size[2]);
+		const float2 up = make_float2(__saturatef(dxy.x * 0x1p126f), __saturatef(dxy.y * 0x1p126f));
+		const float2 m = __ffma2_rn(up, make_float2(-l.x, -l.y), l);
+		dxy = __fadd2_rn(__fadd2_rn(dxy, m), make_float2(-m.x, -m.y));
+		const float mz = __fmaf_rn(__saturatef(dz * 0x1p126f), -box.size[2], box.size[2]);
+		dz = __fsub_rn(__fadd_rn(dz, mz), mz);
 	} else if (kAllPeriodic) {
 		// wrap1 on x and y: image = floor(d / l); d -= image * l; d >= l/2 -> d - l.
 		const float2 negl = make_float2(-box.size[0], -box.size[1]);
@@ -251,6 +218,30 @@ __device__ __forceinline__ void pair_scalar(const float4& pi, float2 npi, const 
 		dxy = make_float2(r.x, r.y);
 		dz = r.z;
 	}
+}
+
+// One pair of the half list, rounded as the reference rounds it. flip
+// (bit 31 of the entry): the reference orients the pair j -> i. With kTerms,
+// the analytical terms of the type pair come first, then the table.
+//
+// The x and y components go through sm_100's packed FP32 instructions
+// (__fadd2_rn / __fmul2_rn: two IEEE round-to-nearest operations each, so
+// every value is the scalar one bit for bit), z stays scalar. npi = (-pi.x,
+// -pi.y); a - b is computed as a + (-b) and b * l as -(b * (-l)), both exact
+// rewrites. The i-force is accumulated negated (nxy, nz): -(a - h) = (-a) + h
+// in round-to-nearest, so the caller's negation at the end gives the same sum.
+template <bool kEnergy, bool kAllPeriodic, bool kTerms, class TRow>
+__device__ __forceinline__ void pair_scalar(const float4& pi, float2 npi, const float4& pj,
+											uint32_t j, uint32_t flip,
+											const TRow& trow, const float* bin_f,
+											const float2* bin_e, const PairTermRef* arow,
+											const PairSolvent& sv, const Box& box,
+											const DistWindow& win, float4* force, float2& nxy, float& nz,
+											float& fe, double& e_acc, double& w_acc) {
+	const float sgn = __uint_as_float(flip | 0x3F800000u);  // +1, or -1 when flipped
+	float2 dxy;
+	float dz;
+	oriented_image<kAllPeriodic, false>(pi, npi, pj, sgn, box, dxy, dz);
 	const float dx = dxy.x, dy = dxy.y;
 	const float2 sq = __fmul2_rn(dxy, dxy);
 	const float d2v = __fadd_rn(__fadd_rn(sq.x, sq.y), __fmul_rn(dz, dz));
@@ -308,6 +299,38 @@ __device__ __forceinline__ void pair_scalar(const float4& pi, float2 npi, const 
 	fe += half;
 }
 
+// The lanes' sums of minus the i-force over a row, negated (exact) and added.
+template <int G, bool kEnergy>
+__device__ __forceinline__ void reduce_row(const float2& nxy, float nz, float fe, bool any, int sub,
+										   float4* out) {
+	float fx = nxy.x, fy = nxy.y, fz = nz;
+	if (G > 1) {
+#pragma unroll
+		for (int o = G / 2; o > 0; o >>= 1) {
+			fx += __shfl_xor_sync(0xFFFFFFFFu, fx, o, G);
+			fy += __shfl_xor_sync(0xFFFFFFFFu, fy, o, G);
+			fz += __shfl_xor_sync(0xFFFFFFFFu, fz, o, G);
+			if (kEnergy) fe += __shfl_xor_sync(0xFFFFFFFFu, fe, o, G);
+		}
+	}
+	if (any && sub == 0) red_add_v4(out, -fx, -fy, -fz, fe);
+}
+
+// fast_pair_kernel's tables and constants: the uniform tables' start, step
+// inverse and last bin, the first bins (null: type pair (a, b)'s at
+// (a T + b) stride), and the squared distances above which a pair adds nothing
+// (loose), below which it takes the reference's tests (close2) and below which
+// the reference skips it (lo).
+struct FastArgs {
+	const float* bin_force;
+	const float2* bin_energy;
+	const int* offsets;
+	const PairTableRef* refs;  // offset < 0: no table (a NaN then adds nothing)
+	int T, stride, last;
+	float start, step_inv;
+	float loose, close2, lo;
+};
+
 // Box of a row: one box for the whole list, or the box of the row's system
 // (batched replicas: system id in the top bits of the sorted key).
 struct OneBox {
@@ -327,26 +350,20 @@ struct SystemBoxes {
 	__device__ __forceinline__ Box row(uint32_t i) const { return boxes[keys[i] >> sys_shift]; }
 };
 
-// Resident 256-thread blocks per SM each pair-kernel variant is compiled for.
-// The force-only tabulated kernel is bound by issue and gather latency: 8
-// blocks (32 registers, full occupancy) ran it 6 % faster than the 40
-// registers it takes unbounded, in spite of a few bytes of spill (none in the
-// uniform-table variant); the energy and analytical variants need their
-// registers. The batched variant (box per row) runs best at 6 blocks (40
-// registers, a few bytes of spill): 1.06 -> 1.02 ms per batched step against
-// 48 registers, and 1.08 at 8 blocks, where it spills 60 bytes.
+// Resident 256-thread blocks per SM the general pair kernel is compiled for.
 template <bool kEnergy, bool kTerms, bool kOneBox>
 constexpr int pair_min_blocks() {
 	return !kOneBox ? 6 : (kTerms ? 3 : (kEnergy ? 5 : 8));
 }
 
-template <int G, bool kEnergy, bool kAllPeriodic, bool kTerms, bool kUniform, class BoxSrc>
+// The general pair kernel: tables of different starts or bin widths, and the
+// analytical terms. Every pair in the reference's own operations.
+template <int G, bool kEnergy, bool kAllPeriodic, bool kTerms, class BoxSrc>
 __global__ void __launch_bounds__(
 	256, pair_min_blocks<kEnergy, kTerms, std::is_same<BoxSrc, OneBox>::value>()) pair_force_kernel(
 	const float4* __restrict__ sorted_pos, const uint32_t* __restrict__ nbr,
 	const uint32_t* __restrict__ row_len, uint32_t n, uint32_t cap, int T,
-	const PairTableRef* __restrict__ refs_g, const int* __restrict__ offs_g, PairTableRef uref,
-	const float* __restrict__ force_g,
+	const PairTableRef* __restrict__ refs_g, const float* __restrict__ force_g,
 	const float2* __restrict__ energy_g, uint32_t total_bins,
 	const PairTermRef* __restrict__ terms_g, PairSolvent sv, BoxSrc boxes, DistWindow win,
 	float4* force, double* __restrict__ ev) {
@@ -354,19 +371,13 @@ __global__ void __launch_bounds__(
 	// The per-type-pair references (T*T, 16 B each) are staged in shared
 	// memory. On the one-box path the per-bin force (and energy) tables are
 	// read through L1 (a few KB, hot in every SM's L1) instead of a copy per
-	// block: that leaves the L1 to the neighbour-position gathers, whose
-	// latency bounds this kernel (1.63 -> 1.51 ms per 2 M-bead launch; asking
-	// the driver for the largest L1 carve-out on top made it slower, 1.80 ms).
-	// The batched path (many small systems, short rows, fewer resident warps)
-	// is faster with the tables in shared memory.
+	// block: that leaves the L1 to the neighbour-position gathers. The batched
+	// path (many small systems, short rows, fewer resident warps) is faster
+	// with the tables in shared memory.
 	constexpr bool kStage = !std::is_same<BoxSrc, OneBox>::value;
 	extern __shared__ float4 smem4[];
 	PairTableRef* refs = reinterpret_cast<PairTableRef*>(smem4);
-	int* soff = reinterpret_cast<int*>(smem4);
-	for (int k = threadIdx.x; k < T * T; k += blockDim.x) {
-		if (kUniform) soff[k] = offs_g[k];
-		else refs[k] = refs_g[k];
-	}
+	for (int k = threadIdx.x; k < T * T; k += blockDim.x) refs[k] = refs_g[k];
 	const float* __restrict__ bin_f = force_g;
 	const float2* __restrict__ bin_e = energy_g;
 	if (kStage) {
@@ -386,10 +397,7 @@ __global__ void __launch_bounds__(
 	const bool valid = i < n;
 	const Box& box = boxes.row(valid ? i : 0u);
 	const float4 pi = valid ? sorted_pos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-	TableRow<kUniform> trow;
-	trow.row = refs + (valid ? type_of(pi) : 0) * T;
-	trow.off = soff + (valid ? type_of(pi) : 0) * T;
-	trow.u = uref;
+	const TableRow trow{refs + (valid ? type_of(pi) : 0) * T};
 	const PairTermRef* arow = kTerms ? terms_g + (valid ? type_of(pi) : 0) * T : nullptr;
 	const uint32_t cnt = valid ? row_len[i] : 0u;
 	// Entry k of row i: ((i / H) * cap + k) * H + i % H.
@@ -398,13 +406,159 @@ __global__ void __launch_bounds__(
 	float2 nxy = make_float2(0.0f, 0.0f);  // minus the i-force, x and y
 	float nz = 0.0f, fe = 0.0f;
 	double e_acc = 0.0, w_acc = 0.0;
-	// A row inside the box (all-periodic box, displacement tracked): every
-	// neighbour's minimum image is its plain difference, |d| <= list radius +
-	// twice the largest displacement since the build < l/2, so the pairs take
-	// wrap_inner's shorter sequence (same result). Decided per warp.
-	constexpr bool kCanInner = kAllPeriodic && std::is_same<BoxSrc, OneBox>::value;
+	// Two entries per lane per iteration: both neighbour gathers are in flight
+	// before either pair's arithmetic.
+	uint32_t t = sub;
+	for (; t + G < cnt; t += 2 * G) {
+		const uint32_t e0 = __ldcs(col + static_cast<size_t>(t) * H);
+		const uint32_t e1 = __ldcs(col + static_cast<size_t>(t + G) * H);
+		const uint32_t j0 = e0 & ~kOrientBit, j1 = e1 & ~kOrientBit;
+		const float4 p0 = sorted_pos[j0];
+		const float4 p1 = sorted_pos[j1];
+		pair_scalar<kEnergy, kAllPeriodic, kTerms>(pi, npi, p0, j0, e0 & kOrientBit, trow, bin_f,
+												   bin_e, arow, sv, box, win, force, nxy, nz, fe,
+												   e_acc, w_acc);
+		pair_scalar<kEnergy, kAllPeriodic, kTerms>(pi, npi, p1, j1, e1 & kOrientBit, trow, bin_f,
+												   bin_e, arow, sv, box, win, force, nxy, nz, fe,
+												   e_acc, w_acc);
+	}
+	if (t < cnt) {
+		const uint32_t entry = __ldcs(col + static_cast<size_t>(t) * H);
+		const uint32_t j = entry & ~kOrientBit;
+		pair_scalar<kEnergy, kAllPeriodic, kTerms>(pi, npi, sorted_pos[j], j, entry & kOrientBit,
+												   trow, bin_f, bin_e, arow, sv, box, win, force,
+												   nxy, nz, fe, e_acc, w_acc);
+	}
+	reduce_row<G, kEnergy>(nxy, nz, fe, valid && cnt != 0u, sub, &force[i]);
+	if (kEnergy) block_add_f64(e_acc, w_acc, ev);
+}
+
+// Pair forces through tables of one start and bin width. The list, its layout,
+// the sums and every pair's value, bit for bit, are the general kernel's; a
+// pair takes fewer instructions to it (the general kernel is bound by issuing
+// them, 76 thread instructions a pair and 82 % issue active at 2,097,152
+// beads, with the L1's data pipe at 80 % close behind):
+//  * one hardware 1 / sqrt (PTX rsqrt.approx) serves the root and the
+//    reciprocal, each by one Newton-Raphson correction (Markstein, see
+//    sqrt_rn_nr): root and reciprocal are the correctly rounded ones, but for
+//    one reciprocal in some 10^7 that is an ulp off;
+//  * the bin comes from one addition rounded down, with the first bin of the
+//    row's types in the addend, and is read at (type pair) * stride + bin: no
+//    conversion, no clamp, no lookup of the table;
+//  * the minimum image of rows inside the box picks its form on the FMA pipe
+//    (oriented_image): the ALU pipe is the busier one;
+//  * pairs beyond the last bin that holds a force are dropped before the root
+//    whatever the cutoff: they add nothing.
+// Below close2 (where the reference skips the pair, and below the tables'
+// start), and for a NaN, a branch restores the reference's tests and clamps.
+//
+// One gather is in flight ahead of the pair at hand and the entry after it is
+// read, which fits 32 registers (8 blocks an SM) without spill; two pairs in
+// flight together spill 60 bytes there and at 40 registers lose the warps
+// (run of 20 steps at 2,097,152 beads, with a first form of this arithmetic:
+// 32.5 ms with the general kernel, 37.1 and 34.7 ms for those two, 31.0 ms
+// pipelined). What bounds it is then the L1's data pipe (81 % of its
+// wavefronts, half of them the j-forces' reductions) with issue (78 %) close
+// behind; the tables in shared memory instead of L1 took 34.5 ms.
+template <bool kEnergy, bool kOneBox>
+constexpr int fast_min_blocks() {
+	return kEnergy ? 5 : (kOneBox ? 8 : 6);
+}
+template <int G, bool kEnergy, bool kDirect, class BoxSrc>
+__global__ void __launch_bounds__(256, fast_min_blocks<kEnergy, std::is_same<BoxSrc, OneBox>::value>())
+	fast_pair_kernel(
+	const float4* __restrict__ sorted_pos, const uint32_t* __restrict__ nbr,
+	const uint32_t* __restrict__ row_len, uint32_t n, uint32_t cap, FastArgs fa, BoxSrc boxes,
+	float4* force, double* __restrict__ ev) {
+	constexpr int H = 32 / G;
+	const int sub = threadIdx.x & (G - 1);  // lane within the row's group
+	const uint32_t i = blockIdx.x * (blockDim.x / G) + threadIdx.x / G;
+	const bool valid = i < n;
+	const Box& box = boxes.row(valid ? i : 0u);
+	const float4 pi = valid ? sorted_pos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+	const int trow = (valid ? type_of(pi) : 0) * fa.T;
+	const uint32_t cnt = valid ? row_len[i] : 0u;
+	// Entry k of row i: ((i / H) * cap + k) * H + i % H.
+	const uint32_t* col = nbr + (static_cast<size_t>(i / H) * cap) * H + (i % H);
+	const float2 npi = make_float2(-pi.x, -pi.y);
+	float2 nxy = make_float2(0.0f, 0.0f);  // minus the i-force, x and y
+	float nz = 0.0f, fe = 0.0f;
+	double e_acc = 0.0, w_acc = 0.0;
+	// 2^23 plus the first bin of the row's types: added to a bin coordinate and
+	// rounded down, the sum holds the bin's index in its low bits.
+	constexpr uint32_t kBits = 0x4B000000u;  // 2^23 as float bits
+	const float magic = 8388608.0f + (kDirect ? static_cast<float>(trow * fa.stride) : 0.0f);
+	auto pair = [&](uint32_t entry, const float4& pj, auto inner_tag) {
+		constexpr bool kInner = decltype(inner_tag)::value;
+		const float sgn = __uint_as_float((entry & kOrientBit) | 0x3F800000u);
+		float2 dxy;
+		float dz;
+		oriented_image<true, kInner>(pi, npi, pj, sgn, box, dxy, dz);
+		const float2 sq = __fmul2_rn(dxy, dxy);
+		const float d2 = __fadd_rn(__fadd_rn(sq.x, sq.y), __fmul_rn(dz, dz));
+		if (d2 > fa.loose) return;
+		float y;
+		asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d2));
+		const float g = __fmul_rn(d2, y);
+		const float dist = __fmaf_rn(__fmaf_rn(-g, g, d2), __fmul_rn(0.5f, y), g);
+		const float inv = __fmaf_rn(y, __fmaf_rn(-dist, y, 1.0f), y);
+		const float w = __fmul_rn(__fsub_rn(dist, fa.start), fa.step_inv);
+		const float t = __fadd_rd(w, magic);
+		uint32_t home = __float_as_uint(t);
+		if (kEnergy) home = min(home, __float_as_uint(magic) + static_cast<uint32_t>(fa.last));
+		if (!(d2 >= fa.close2)) {  // (or NaN)
+			if (d2 < fa.lo || fa.refs[trow + type_of(pj)].offset < 0) return;
+			home = __float_as_uint(magic) + static_cast<uint32_t>(min(max(__float2int_rd(w), 0), fa.last));
+		}
+		const uint32_t bin = home - kBits +
+							 (kDirect ? static_cast<uint32_t>(type_of(pj)) * static_cast<uint32_t>(fa.stride)
+									  : static_cast<uint32_t>(__ldg(fa.offsets + trow + type_of(pj))));
+		const float fm = __ldg(fa.bin_force + bin);
+		// f = unit * F acts on the pair's second particle: j, unless flipped.
+		const float2 uxy = __fmul2_rn(make_float2(inv, inv), dxy);
+		const float uz = __fmul_rn(inv, dz);
+		const float fs = __fmul_rn(fm, sgn);
+		const float2 hxy = __fmul2_rn(uxy, make_float2(fs, fs));
+		const float hz = __fmul_rn(uz, fs);
+		float half = 0.0f;
+		if (kEnergy) {
+			const float2 ue = __ldg(fa.bin_energy + bin);
+			const float e = __fadd_rn(__fmul_rn(ue.y, __fsub_rn(w, floorf(w))), ue.x);
+			half = __fmul_rn(e, 0.5f);
+			e_acc += static_cast<double>(e);
+			w_acc += (static_cast<double>(hxy.x) * dxy.x + static_cast<double>(hxy.y) * dxy.y +
+					  static_cast<double>(hz) * dz) * static_cast<double>(sgn);
+		}
+		red_add_v4(&force[entry & ~kOrientBit], hxy.x, hxy.y, hz, half);
+		nxy = __fadd2_rn(nxy, hxy);
+		nz = __fadd_rn(nz, hz);
+		fe += half;
+	};
+	auto walk = [&](auto inner_tag) {
+		if (sub < static_cast<int>(cnt)) {
+			const uint32_t* p = col + sub * H;
+			int left = static_cast<int>(cnt) - sub;  // entries from p on, this lane's every G-th
+			uint32_t e0 = __ldcs(p);
+			uint32_t e1 = left > G ? __ldcs(p + G * H) : e0;
+			float4 p0 = sorted_pos[e0 & ~kOrientBit];
+			while (left > G) {
+				const float4 p1 = sorted_pos[e1 & ~kOrientBit];
+				const uint32_t e2 = left > 2 * G ? __ldcs(p + 2 * G * H) : e1;
+				pair(e0, p0, inner_tag);
+				p0 = p1;
+				e0 = e1;
+				e1 = e2;
+				p += G * H;
+				left -= G;
+			}
+			pair(e0, p0, inner_tag);
+		}
+	};
+	// A row inside the box (displacement tracked): every neighbour's minimum
+	// image is its plain difference, since |d| <= list radius + twice the
+	// largest displacement since the build < l/2. Decided per warp.
 	bool inner = false;
-	if constexpr (kCanInner) {
+	if constexpr (std::is_same<BoxSrc, OneBox>::value) {
 		if (boxes.d2max != nullptr) {
 			const float m = boxes.margin + 2.0f * sqrtf(__uint_as_float(__ldg(boxes.d2max)));
 			const float c[3] = {pi.x, pi.y, pi.z};
@@ -416,52 +570,12 @@ __global__ void __launch_bounds__(
 			inner = inner || !valid;
 		}
 		inner = __all_sync(0xFFFFFFFFu, inner);
-	}
-	// Two entries per lane per iteration: both neighbour gathers are in flight
-	// before either pair's arithmetic (the kernel is bound by gather latency).
-	auto walk = [&](auto inner_tag) {
-		constexpr bool kIn = decltype(inner_tag)::value;
-		uint32_t t = sub;
-		for (; t + G < cnt; t += 2 * G) {
-			const uint32_t e0 = __ldcs(col + static_cast<size_t>(t) * H);
-			const uint32_t e1 = __ldcs(col + static_cast<size_t>(t + G) * H);
-			const uint32_t j0 = e0 & ~kOrientBit, j1 = e1 & ~kOrientBit;
-			const float4 p0 = sorted_pos[j0];
-			const float4 p1 = sorted_pos[j1];
-			pair_scalar<kEnergy, kAllPeriodic, kTerms, kIn>(pi, npi, p0, j0, e0 & kOrientBit,
-															trow, bin_f, bin_e, arow, sv, box,
-															win, force, nxy, nz, fe, e_acc, w_acc);
-			pair_scalar<kEnergy, kAllPeriodic, kTerms, kIn>(pi, npi, p1, j1, e1 & kOrientBit,
-															trow, bin_f, bin_e, arow, sv, box,
-															win, force, nxy, nz, fe, e_acc, w_acc);
-		}
-		if (t < cnt) {
-			const uint32_t entry = __ldcs(col + static_cast<size_t>(t) * H);
-			const uint32_t j = entry & ~kOrientBit;
-			pair_scalar<kEnergy, kAllPeriodic, kTerms, kIn>(pi, npi, sorted_pos[j], j,
-															entry & kOrientBit, trow, bin_f,
-															bin_e, arow, sv, box, win, force, nxy,
-															nz, fe, e_acc, w_acc);
-		}
-	};
-	if constexpr (kCanInner) {
 		if (inner) walk(std::true_type{});
 		else walk(std::false_type{});
 	} else {
 		walk(std::false_type{});
 	}
-	// The lanes' sums of minus the i-force, then negated (exact).
-	float fx = nxy.x, fy = nxy.y, fz = nz;
-	if (G > 1) {
-#pragma unroll
-		for (int o = G / 2; o > 0; o >>= 1) {
-			fx += __shfl_xor_sync(0xFFFFFFFFu, fx, o, G);
-			fy += __shfl_xor_sync(0xFFFFFFFFu, fy, o, G);
-			fz += __shfl_xor_sync(0xFFFFFFFFu, fz, o, G);
-			if (kEnergy) fe += __shfl_xor_sync(0xFFFFFFFFu, fe, o, G);
-		}
-	}
-	if (valid && sub == 0 && cnt != 0u) red_add_v4(&force[i], -fx, -fy, -fz, fe);
+	reduce_row<G, kEnergy>(nxy, nz, fe, valid && cnt != 0u, sub, &force[i]);
 	if (kEnergy) block_add_f64(e_acc, w_acc, ev);
 }
 
@@ -720,13 +834,60 @@ __global__ void __launch_bounds__(256) restraint_kernel(const int* __restrict__ 
 	if (get_energy) block_add_f64(e_acc, 0.0, energy);
 }
 
-template <int G, bool kEnergy, bool kAllPeriodic, bool kTerms, class BoxSrc, bool kUniform = false>
+// fast_pair_kernel's arguments. loose: the reference's window, or, where the
+// tables end before it, the distance at which the last bin that holds
+// something ends (a little more: the bins there hold nothing). close2: above
+// the window's lower end, and where the tables start above 0, a little above
+// their start.
+FastArgs fast_args(const PairTables& t, float cutoff_sq, int get_energy) {
+	const PairTableRef& u = t.uniform_ref;
+	FastArgs fa;
+	fa.bin_force = t.fast_force;
+	fa.bin_energy = t.fast_energy;
+	fa.offsets = t.fast_offsets;
+	fa.refs = t.refs;
+	fa.T = t.num_types;
+	fa.last = u.last;
+	fa.stride = u.last + 1;
+	fa.start = u.start;
+	fa.step_inv = u.step_inv;
+	const DistWindow win = dist_window(cutoff_sq);
+	const double end = (get_energy ? t.reach_energy : t.reach_force) * (1.0 + 1e-6);
+	fa.loose = std::min(win.hi, static_cast<float>(end * end * (1.0 + 1e-6)));
+	fa.lo = win.lo;
+	const double close = std::max(1e-5, u.start > 0.0f ? u.start * (1.0 + 1e-6) : 0.0);
+	fa.close2 = static_cast<float>(close * close * (1.0 + 1e-6));
+	return fa;
+}
+
+// The tables for which the bin arithmetic holds: uniform ones whose largest
+// bin coordinate, at the end of the launch's reach, is a small number.
+bool fast_ok(const PairTables& t, float cutoff_sq, int get_energy) {
+	if (!t.fast_force || t.terms) return false;
+	const double cut = cutoff_sq > 0.0f ? std::sqrt(static_cast<double>(cutoff_sq)) : INFINITY;
+	const double end = std::min<double>(cut, get_energy ? t.reach_energy : t.reach_force);
+	const double from = std::max(0.0, -static_cast<double>(t.uniform_ref.start));
+	return (end + from) * t.uniform_ref.step_inv < 65536.0;
+}
+
+template <int G, bool kEnergy, class BoxSrc>
+void launch_fast(const float4* sorted_pos, const uint32_t* nbr, const uint32_t* row_len,
+				 uint32_t n, uint32_t cap, const FastArgs& fa, const BoxSrc& boxes,
+				 float4* force_sorted, double* ev, cudaStream_t st) {
+	const uint32_t blocks = (n + 256 / G - 1) / (256 / G);
+	auto kern = fa.offsets ? fast_pair_kernel<G, kEnergy, false, BoxSrc>
+						   : fast_pair_kernel<G, kEnergy, true, BoxSrc>;
+	MB2_LAUNCH kern<<<blocks, 256, 0, st>>>(sorted_pos, nbr, row_len, n, cap, fa, boxes,
+											force_sorted, ev);
+}
+
+template <int G, bool kEnergy, bool kAllPeriodic, bool kTerms, class BoxSrc>
 void launch_pair(const float4* sorted_pos, const uint32_t* nbr, const uint32_t* row_len,
 				 uint32_t n, uint32_t cap, const PairTables& t, const BoxSrc& boxes,
 				 float cutoff_sq, float4* force_sorted, double* ev, cudaStream_t st) {
 	const uint32_t rows = 256 / G;
 	const uint32_t blocks = (n + rows - 1) / rows;
-	auto kern = pair_force_kernel<G, kEnergy, kAllPeriodic, kTerms, kUniform, BoxSrc>;
+	auto kern = pair_force_kernel<G, kEnergy, kAllPeriodic, kTerms, BoxSrc>;
 	constexpr bool kStage = !std::is_same<BoxSrc, OneBox>::value;
 	const size_t smem =
 		static_cast<size_t>(t.num_types * t.num_types) * sizeof(PairTableRef) +
@@ -737,57 +898,52 @@ void launch_pair(const float4* sorted_pos, const uint32_t* nbr, const uint32_t* 
 		MB2_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
 									  static_cast<int>(smem)));
 	MB2_LAUNCH kern<<<blocks, 256, smem, st>>>(sorted_pos, nbr, row_len, n, cap, t.num_types,
-											   t.refs, t.offsets, t.uniform_ref, t.bin_force,
-											   t.bin_energy, t.total_bins,
+											   t.refs, t.bin_force, t.bin_energy, t.total_bins,
 											   t.terms, t.solvent, boxes, dist_window(cutoff_sq),
 											   force_sorted, ev);
 }
 
-template <int G, bool kEnergy, bool kAllPeriodic, class BoxSrc>
-void launch_pair_t(const float4* sorted_pos, const uint32_t* nbr, const uint32_t* row_len,
-				   uint32_t n, uint32_t cap, const PairTables& t, const BoxSrc& boxes,
-				   float cutoff_sq, float4* force_sorted, double* ev, cudaStream_t st) {
-	// Analytical terms only on the one-box path (batched replicas are tabulated).
+template <int G, bool kEnergy, class BoxSrc>
+void launch_pair_e(const float4* sorted_pos, const uint32_t* nbr, const uint32_t* row_len,
+				   uint32_t n, uint32_t cap, const PairTables& t, const FastArgs* fa,
+				   const BoxSrc& boxes, bool all_periodic, float cutoff_sq, float4* force_sorted,
+				   double* ev, cudaStream_t st) {
+	if (fa) {  // uniform tables, every axis periodic
+		launch_fast<G, kEnergy>(sorted_pos, nbr, row_len, n, cap, *fa, boxes, force_sorted, ev, st);
+		return;
+	}
 	if constexpr (std::is_same<BoxSrc, OneBox>::value) {
+		// Analytical terms only on the one-box path (batched replicas are tabulated).
 		if (t.terms) {
-			launch_pair<G, kEnergy, kAllPeriodic, true>(sorted_pos, nbr, row_len, n, cap, t, boxes,
-														cutoff_sq, force_sorted, ev, st);
+			if (all_periodic) launch_pair<G, kEnergy, true, true>(sorted_pos, nbr, row_len, n, cap, t, boxes, cutoff_sq, force_sorted, ev, st);
+			else launch_pair<G, kEnergy, false, true>(sorted_pos, nbr, row_len, n, cap, t, boxes, cutoff_sq, force_sorted, ev, st);
 			return;
 		}
 	}
-	if (t.uniform && t.offsets) {
-		launch_pair<G, kEnergy, kAllPeriodic, false, BoxSrc, true>(
-			sorted_pos, nbr, row_len, n, cap, t, boxes, cutoff_sq, force_sorted, ev, st);
-		return;
-	}
-	launch_pair<G, kEnergy, kAllPeriodic, false>(sorted_pos, nbr, row_len, n, cap, t, boxes,
-												 cutoff_sq, force_sorted, ev, st);
+	if (all_periodic) launch_pair<G, kEnergy, true, false>(sorted_pos, nbr, row_len, n, cap, t, boxes, cutoff_sq, force_sorted, ev, st);
+	else launch_pair<G, kEnergy, false, false>(sorted_pos, nbr, row_len, n, cap, t, boxes, cutoff_sq, force_sorted, ev, st);
 }
 
 template <int G, class BoxSrc>
 void launch_pair_g(const float4* sorted_pos, const uint32_t* nbr, const uint32_t* row_len,
-				   uint32_t n, uint32_t cap, const PairTables& t, const BoxSrc& boxes,
-				   bool all_periodic, float cutoff_sq, int get_energy, float4* force_sorted,
-				   double* ev, cudaStream_t st) {
-	if (get_energy) {
-		if (all_periodic) launch_pair_t<G, true, true>(sorted_pos, nbr, row_len, n, cap, t, boxes, cutoff_sq, force_sorted, ev, st);
-		else launch_pair_t<G, true, false>(sorted_pos, nbr, row_len, n, cap, t, boxes, cutoff_sq, force_sorted, ev, st);
-	} else {
-		if (all_periodic) launch_pair_t<G, false, true>(sorted_pos, nbr, row_len, n, cap, t, boxes, cutoff_sq, force_sorted, ev, st);
-		else launch_pair_t<G, false, false>(sorted_pos, nbr, row_len, n, cap, t, boxes, cutoff_sq, force_sorted, ev, st);
-	}
+				   uint32_t n, uint32_t cap, const PairTables& t, const FastArgs* fa,
+				   const BoxSrc& boxes, bool all_periodic, float cutoff_sq, int get_energy,
+				   float4* force_sorted, double* ev, cudaStream_t st) {
+	if (get_energy) launch_pair_e<G, true>(sorted_pos, nbr, row_len, n, cap, t, fa, boxes, all_periodic, cutoff_sq, force_sorted, ev, st);
+	else launch_pair_e<G, false>(sorted_pos, nbr, row_len, n, cap, t, fa, boxes, all_periodic, cutoff_sq, force_sorted, ev, st);
 }
 
 template <class BoxSrc>
 void launch_pair_lanes(const float4* sorted_pos, const uint32_t* nbr, const uint32_t* row_len,
 					   uint32_t n, uint32_t cap, int lanes_per_row, const PairTables& t,
-					   const BoxSrc& boxes, bool all_periodic, float cutoff_sq, int get_energy,
-					   float4* force_sorted, double* ev, cudaStream_t st) {
+					   const FastArgs* fa, const BoxSrc& boxes, bool all_periodic,
+					   float cutoff_sq, int get_energy, float4* force_sorted, double* ev,
+					   cudaStream_t st) {
 	switch (lanes_per_row) {
-	case 4: launch_pair_g<4>(sorted_pos, nbr, row_len, n, cap, t, boxes, all_periodic, cutoff_sq, get_energy, force_sorted, ev, st); break;
-	case 8: launch_pair_g<8>(sorted_pos, nbr, row_len, n, cap, t, boxes, all_periodic, cutoff_sq, get_energy, force_sorted, ev, st); break;
-	case 16: launch_pair_g<16>(sorted_pos, nbr, row_len, n, cap, t, boxes, all_periodic, cutoff_sq, get_energy, force_sorted, ev, st); break;
-	default: launch_pair_g<32>(sorted_pos, nbr, row_len, n, cap, t, boxes, all_periodic, cutoff_sq, get_energy, force_sorted, ev, st); break;
+	case 4: launch_pair_g<4>(sorted_pos, nbr, row_len, n, cap, t, fa, boxes, all_periodic, cutoff_sq, get_energy, force_sorted, ev, st); break;
+	case 8: launch_pair_g<8>(sorted_pos, nbr, row_len, n, cap, t, fa, boxes, all_periodic, cutoff_sq, get_energy, force_sorted, ev, st); break;
+	case 16: launch_pair_g<16>(sorted_pos, nbr, row_len, n, cap, t, fa, boxes, all_periodic, cutoff_sq, get_energy, force_sorted, ev, st); break;
+	default: launch_pair_g<32>(sorted_pos, nbr, row_len, n, cap, t, fa, boxes, all_periodic, cutoff_sq, get_energy, force_sorted, ev, st); break;
 	}
 }
 
@@ -894,25 +1050,89 @@ size_t pair_table_arrays(int num_types, const uint32_t* term_matrix, int num_tab
 	return total;
 }
 
-bool uniform_tables(const std::vector<PairTableRef>& refs, std::vector<int>& offsets,
-					PairTableRef& u) {
-	bool uniform = false, any = false;
+bool fast_pair_tables(const std::vector<PairTableRef>& refs, const std::vector<float>& bf,
+					  const std::vector<float2>& be, PairTableRef& u, std::vector<int>& first,
+					  std::vector<float>& ff, std::vector<float2>& fe, float& reach_force,
+					  float& reach_energy) {
+	bool any = false;
 	u = PairTableRef{0.0f, 0.0f, 0, -1};
-	offsets.assign(refs.size(), -1);
-	for (size_t k = 0; k < refs.size(); ++k) {
-		offsets[k] = refs[k].offset;
-		if (refs[k].offset < 0) continue;
+	for (const PairTableRef& r : refs) {
+		if (r.offset < 0) continue;
 		if (!any) {
-			u = refs[k];
-			any = uniform = true;
-		} else if (std::memcmp(&u.start, &refs[k].start, sizeof(float)) != 0 ||
-				   std::memcmp(&u.step_inv, &refs[k].step_inv, sizeof(float)) != 0 ||
-				   u.last != refs[k].last) {
-			uniform = false;
+			u = r;
+			any = true;
+		} else if (std::memcmp(&u.start, &r.start, sizeof(float)) != 0 ||
+				   std::memcmp(&u.step_inv, &r.step_inv, sizeof(float)) != 0 || u.last != r.last) {
+			return false;
 		}
 	}
+	if (!any || !(u.step_inv > 0.0f)) return false;
+	const size_t stride = static_cast<size_t>(u.last) + 1;
+	// The last bin with a force, and with a force or an energy, over all tables.
+	int last_f = -1, last_e = -1;
+	for (const PairTableRef& r : refs) {
+		if (r.offset < 0) continue;
+		for (int k = 0; k <= u.last; ++k) {
+			const bool f = !(bf[r.offset + k] == 0.0f);
+			const bool e = f || !(be[r.offset + k].x == 0.0f) || !(be[r.offset + k].y == 0.0f);
+			if (f) last_f = std::max(last_f, k);
+			if (e) last_e = std::max(last_e, k);
+		}
+	}
+	auto edge = [&](int bin) {
+		const double d = static_cast<double>(u.start) + (bin + 1.0) / u.step_inv;
+		return std::nextafter(static_cast<float>(std::max(d, 0.0)), INFINITY);
+	};
+	reach_force = edge(last_f);
+	// The last bin's energy holds for every distance beyond the table.
+	reach_energy = last_e == u.last ? INFINITY : edge(last_e);
 	u.offset = -1;
-	return uniform;
+	first.clear();
+	if (refs.size() * stride <= 32768) {
+		// Every type pair's bins side by side (zeros where it has no table).
+		ff.assign(refs.size() * stride, 0.0f);
+		fe.assign(refs.size() * stride, make_float2(0.0f, 0.0f));
+		for (size_t k = 0; k < refs.size(); ++k) {
+			if (refs[k].offset < 0) continue;
+			std::copy_n(bf.begin() + refs[k].offset, stride, ff.begin() + k * stride);
+			std::copy_n(be.begin() + refs[k].offset, stride, fe.begin() + k * stride);
+		}
+		return true;
+	}
+	// Many types: each table once, then a table of zeros, and each type
+	// pair's first bin.
+	ff = bf;
+	fe = be;
+	const int zeros = static_cast<int>(bf.size());
+	ff.resize(bf.size() + stride, 0.0f);
+	fe.resize(be.size() + stride, make_float2(0.0f, 0.0f));
+	for (const PairTableRef& r : refs) first.push_back(r.offset < 0 ? zeros : r.offset);
+	return true;
+}
+
+void FastTableBufs::set(const std::vector<PairTableRef>& refs, const std::vector<float>& bf,
+						const std::vector<float2>& be, PairTables& t) {
+	std::vector<int> first_h;
+	std::vector<float> ff;
+	std::vector<float2> fe;
+	t.fast_force = nullptr;
+	t.fast_energy = nullptr;
+	t.fast_offsets = nullptr;
+	if (!fast_pair_tables(refs, bf, be, t.uniform_ref, first_h, ff, fe, t.reach_force,
+						  t.reach_energy))
+		return;
+	force.ensure(ff.size());
+	energy.ensure(fe.size());
+	MB2_CUDA(cudaMemcpy(force.ptr, ff.data(), ff.size() * sizeof(float), cudaMemcpyHostToDevice));
+	MB2_CUDA(cudaMemcpy(energy.ptr, fe.data(), fe.size() * sizeof(float2), cudaMemcpyHostToDevice));
+	if (!first_h.empty()) {
+		first.ensure(first_h.size());
+		MB2_CUDA(cudaMemcpy(first.ptr, first_h.data(), first_h.size() * sizeof(int),
+							cudaMemcpyHostToDevice));
+		t.fast_offsets = first.ptr;
+	}
+	t.fast_force = force.ptr;
+	t.fast_energy = energy.ptr;
 }
 
 void pair_forces(const float4* sorted_pos, const uint32_t* nbr, const uint32_t* row_len,
@@ -921,11 +1141,13 @@ void pair_forces(const float4* sorted_pos, const uint32_t* nbr, const uint32_t* 
 				 cudaStream_t st, const unsigned int* d2max, float list_rc) {
 	if (n == 0) return;
 	const bool all_periodic = box.periodic[0] && box.periodic[1] && box.periodic[2];
+	const bool fast = all_periodic && fast_ok(t, cutoff_sq, get_energy);
 	const bool track = d2max != nullptr && list_rc > 0.0f && std::isfinite(list_rc);
 	const OneBox one{box, track ? d2max : nullptr,
 					 track ? list_rc * (1.0f + 0x1p-20f) + kInnerSafety : 0.0f};
-	launch_pair_lanes(sorted_pos, nbr, row_len, n, cap, lanes_per_row, t, one, all_periodic,
-					  cutoff_sq, get_energy, force_sorted, ev, st);
+	const FastArgs fa = fast ? fast_args(t, cutoff_sq, get_energy) : FastArgs{};
+	launch_pair_lanes(sorted_pos, nbr, row_len, n, cap, lanes_per_row, t, fast ? &fa : nullptr,
+					  one, all_periodic, cutoff_sq, get_energy, force_sorted, ev, st);
 }
 
 void pair_forces_systems(const float4* sorted_pos, const uint32_t* nbr, const uint32_t* row_len,
@@ -934,7 +1156,9 @@ void pair_forces_systems(const float4* sorted_pos, const uint32_t* nbr, const ui
 						 bool all_periodic, float cutoff_sq, int get_energy, float4* force_sorted,
 						 double* ev, cudaStream_t st) {
 	if (n == 0) return;
-	launch_pair_lanes(sorted_pos, nbr, row_len, n, cap, lanes_per_row, t,
+	const bool fast = all_periodic && fast_ok(t, cutoff_sq, get_energy);
+	const FastArgs fa = fast ? fast_args(t, cutoff_sq, get_energy) : FastArgs{};
+	launch_pair_lanes(sorted_pos, nbr, row_len, n, cap, lanes_per_row, t, fast ? &fa : nullptr,
 					  SystemBoxes{boxes, sorted_keys, sys_shift}, all_periodic, cutoff_sq,
 					  get_energy, force_sorted, ev, st);
 }

@@ -237,17 +237,20 @@ struct PairTables {
 	const float2* bin_energy = nullptr;   // device: (U[k], U[k+1]-U[k]), (U[size-1], 0) last
 	const PairTermRef* terms = nullptr;   // device [T*T], or null: tabulated terms only
 	PairSolvent solvent{};
-	// Every type pair with a table uses tables of one start, bin width and
-	// length (uniform.start / step_inv / last): the kernel then reads only
-	// each type pair's offset (device [T*T], -1: no table).
-	const int* offsets = nullptr;
-	bool uniform = false;
+	// Set when every type pair with a table uses tables of one start, (positive)
+	// bin width and length, uniform_ref's: the bins of each type pair (a, b) at
+	// (a * num_types + b) * (last + 1), or from fast_offsets[a * num_types + b]
+	// when that is not null; zeros for a type pair without a table. Beyond
+	// reach_force no bin holds a force, beyond reach_energy none anything.
+	const float* fast_force = nullptr;
+	const float2* fast_energy = nullptr;
+	const int* fast_offsets = nullptr;
+	float reach_force = 0.0f, reach_energy = 0.0f;
 	PairTableRef uniform_ref{0.0f, 0.0f, 0, -1};
 };
 // d2max / list_rc (optional): the displacement track of the list's build and
-// its list radius. With them, rows of an all-periodic box that lie deeper
-// inside the box than list_rc + 2 * sqrt(*d2max) (plus a safety band) take a
-// shorter minimum-image sequence with the same result.
+// its list radius. With them, rows that lie deeper inside the box than
+// list_rc + 2 * sqrt(*d2max) (plus a safety band) take no minimum image.
 void pair_forces(const float4* sorted_pos, const uint32_t* nbr, const uint32_t* row_len,
 				 uint32_t n, uint32_t cap, int lanes_per_row, const PairTables& t, const Box& box,
 				 float cutoff_sq, int get_energy, float4* force_sorted, double* energy_virial,
@@ -258,11 +261,21 @@ size_t pair_table_arrays(int num_types, const uint32_t* term_matrix, int num_tab
 						 const float* values, const uint32_t* sizes, const float* starts,
 						 const float* step_invs, std::vector<PairTableRef>& refs,
 						 std::vector<float>& bf, std::vector<float2>& be);
-// Host: per-type-pair table offsets (-1: no table) and whether every type
-// pair with a table uses one start, step inverse and length (compared bit for
-// bit), which *u then holds (offset -1).
-bool uniform_tables(const std::vector<PairTableRef>& refs, std::vector<int>& offsets,
-					PairTableRef& u);
+// Host: whether the tables are uniform (compared bit for bit), and then *u
+// (offset -1), the bins as PairTables::fast_force / fast_energy lay them out,
+// first (empty: side by side) and the reaches.
+bool fast_pair_tables(const std::vector<PairTableRef>& refs, const std::vector<float>& bf,
+					  const std::vector<float2>& be, PairTableRef& u, std::vector<int>& first,
+					  std::vector<float>& ff, std::vector<float2>& fe, float& reach_force,
+					  float& reach_energy);
+// Device copies of those, and the PairTables fields that name them.
+struct FastTableBufs {
+	DevBuf<float> force;
+	DevBuf<float2> energy;
+	DevBuf<int> first;
+	void set(const std::vector<PairTableRef>& refs, const std::vector<float>& bf,
+			 const std::vector<float2>& be, PairTables& t);
+};
 // Batched replicas: row i's box is boxes[sorted_keys[i] >> sys_shift].
 void pair_forces_systems(const float4* sorted_pos, const uint32_t* nbr, const uint32_t* row_len,
 						 uint32_t n, uint32_t cap, int lanes_per_row, const PairTables& t,
