@@ -36,6 +36,7 @@ struct mb2_context {
 	DevBuf<float4> ref_sorted;
 	DevBuf<unsigned int> d2max;
 	float track_rc = 0.0f;
+	float split = 0.0f;  // distance of the last build's near / far split (0: none)
 	DevBuf<StencilEntry> stencil;
 	DevBuf<float> bbox;  // 6 floats, ordered-int min/max
 	DevBuf<unsigned int> disp;
@@ -276,7 +277,7 @@ void sort_particles(mb2_context* ctx, const float4* pos, const int* type_ids, ui
 // (0, rc_list), rows are split near / far (below); otherwise rows keep the
 // walk's candidate order.
 void build(mb2_context* ctx, const float4* pos, const int* type_ids, uint32_t n, float rc_list,
-		   float cutoff, cudaStream_t st) {
+		   float cutoff, cudaStream_t st, bool whole_rows = false) {
 	require(ctx->box_set, MB2_ERR_STATE, "mb2_build_pairlist: call mb2_set_box first");
 	require(n <= ctx->max_particles, MB2_ERR_CAPACITY,
 			"mb2_build_pairlist: more particles than the context was created for");
@@ -330,16 +331,7 @@ void build(mb2_context* ctx, const float4* pos, const int* type_ids, uint32_t n,
 	}
 	wg.lim = g.lim;
 	wg.rc2 = rc2;
-	// Rows put the pairs that are likely to come within the interaction cutoff
-	// before the next rebuild first (d <= cutoff + 25 % of the skin at build
-	// time) and the rest after them: in a row's tail the whole warp's pairs are
-	// beyond the cutoff for most iterations of the force kernel, which then
-	// skips the force part. The split moves no pair in or out of the list.
-	// Measured on the 2,097,152-bead workload (fused step, rebuild every 20
-	// steps): 1.94 ms without the split; 1.87 ms at 25 % of the skin, 1.89 at
-	// 10 % and at 40 %, 1.92 at 70 %.
-	const float split =
-		(cutoff > 0.0f && cutoff < rc_list) ? cutoff + 0.25f * (rc_list - cutoff) : 0.0f;
+	const float split = row_split(ctx->pt, ctx->box, rc_list, cutoff);
 	wg.split2 = split > 0.0f ? split * split : INFINITY;
 	for (int a = 0; a < 3; ++a) {
 		// Morton coordinate q = trunc((x - bmin) / range * 1023) on 0..1023, a cell
@@ -376,8 +368,18 @@ void build(mb2_context* ctx, const float4* pos, const int* type_ids, uint32_t n,
 	// step than 8 or 4 at 4,096 (21.3 against 23.3 us), 32,768 (54.9 / 58.5)
 	// and 65,536 beads (polymers, 52.9 / 55.5); at 2,097,152 beads 8 lanes are
 	// the fastest.
+	// Rows whose far entries are mostly not read (ends_early) count as their
+	// near part, unless the caller's kernels read all of them (the adjoint's).
+	// Below some 16,000 particles a step is launches and latency: a 4,096-bead
+	// run lost 12 % to the tracking pack, 12,012 beads were level and 65,536
+	// gained 12 %.
+	const bool ends_early = split > 0.0f && split < 0.8f * cutoff && n > 16384u;
 	auto choose_lanes = [&](double mean) {
 		if (ctx->lanes_request) return ctx->lanes_request;
+		if (ends_early && !whole_rows) {
+			const double f = split / rc_list;
+			return mean * f * f * f >= 8.0 ? 8 : 4;
+		}
 		if (n <= kRowWalkMaxN) return mean >= 16.0 ? 16 : 8;
 		if (mean >= 256.0) return 16;
 		if (mean >= 48.0) return 8;
@@ -417,12 +419,14 @@ void build(mb2_context* ctx, const float4* pos, const int* type_ids, uint32_t n,
 	ctx->ref_pos.ensure(n);
 	MB2_CUDA(cudaMemcpyAsync(ctx->ref_pos.ptr, pos, static_cast<size_t>(n) * sizeof(float4),
 							 cudaMemcpyDeviceToDevice, st));
-	// and, in Z order, the origin of the displacement the packs track. Only
-	// above kRowWalkMaxN particles: the inner rows save the pair kernel
-	// 2.6 % at 2,097,152 beads, while on a 65,536-bead step the pack's extra
-	// read and reduction cost more (1-2 us) than they save.
+	// and, in Z order, the origin of the displacement the packs track: where
+	// it saves the pair kernel the rows' far part, and above kRowWalkMaxN
+	// particles, where the inner rows save it 2.6 % at 2,097,152 beads (on a
+	// 65,536-bead step the pack's extra read and reduction cost more for
+	// those alone, 1-2 us).
 	ctx->track_rc = 0.0f;
-	if (n > kRowWalkMaxN) {
+	ctx->split = split;
+	if (n > kRowWalkMaxN || ends_early) {
 		ctx->ref_sorted.ensure(n);
 		ctx->d2max.ensure(1);
 		MB2_CUDA(cudaMemcpyAsync(ctx->ref_sorted.ptr, ctx->sorted_pos.ptr,
@@ -478,7 +482,8 @@ void pair_kernel(mb2_context* ctx, uint32_t n, float cutoff, int get_energy, cud
 	// covers the positions the kernel reads.
 	pair_forces(ctx->sorted_pos.ptr, ctx->nbr.ptr, ctx->row_len.ptr, n, ctx->cap, ctx->lanes, ctx->pt,
 				ctx->box, cutoff_sq, get_energy, ctx->force_sorted.ptr, ctx->energy.ptr, st,
-				ctx->track_rc > 0.0f ? ctx->d2max.ptr : nullptr, ctx->track_rc);
+				ctx->track_rc > 0.0f ? ctx->d2max.ptr : nullptr, ctx->track_rc, ctx->row_far.ptr,
+				ctx->split);
 }
 
 void pair_forces_impl(mb2_context* ctx, const float4* pos, const int* type_ids, float4* fe,
@@ -1308,7 +1313,7 @@ std::vector<uint64_t> run_graph_key(const mb2_context* ctx, const float4* pos, c
 		P(ctx->types.pmf_offset), P(ctx->types.pmf_count), P(ctx->types.terms),
 		P(ctx->types.force_grid_id), P(ctx->types.force_grid_scale), P(ctx->types.grids),
 		static_cast<uint64_t>(ctx->types.num_grids), P(ctx->ref_sorted.ptr), P(ctx->d2max.ptr),
-		fbits(ctx->track_rc)};
+		fbits(ctx->track_rc), P(ctx->row_far.ptr), fbits(ctx->split)};
 	push_words(k, ctx->pt.solvent);
 	push_words(k, ctx->box);
 	return k;
@@ -1417,7 +1422,7 @@ int mb2_window_forward(mb2_context* ctx, float* pos4, float* force_energy4, cons
 			const uint32_t k0 = sgi * checkpoint_every;
 			const uint32_t k1 = std::min(num_steps, k0 + checkpoint_every);
 			copy4(ctx->ckpt.ptr + static_cast<size_t>(sgi) * n, pos, n, st);
-			build(ctx, pos, type_ids, n, prm->pairlist_cutoff, prm->cutoff, st);
+			build(ctx, pos, type_ids, n, prm->pairlist_cutoff, prm->cutoff, st, true);
 			for (uint32_t k = k0; k < k1; ++k)
 				window_step(ctx, pos, fe, type_ids, n, first_step + k, prm, st);
 		}
@@ -1503,7 +1508,7 @@ int mb2_window_backward(mb2_context* ctx, const float* grad_final4, float* grad_
 			const uint32_t k1 = std::min(w.num_steps, k0 + C);
 			// Recompute the segment from its checkpoint, keeping every state.
 			copy4(ctx->wpos.ptr, ctx->ckpt.ptr + static_cast<size_t>(sgi) * n, n, st);
-			build(ctx, ctx->wpos.ptr, w.type_ids, n, prm->pairlist_cutoff, prm->cutoff, st);
+			build(ctx, ctx->wpos.ptr, w.type_ids, n, prm->pairlist_cutoff, prm->cutoff, st, true);
 			for (uint32_t k = k0; k < k1; ++k) {
 				copy4(ctx->states.ptr + static_cast<size_t>(k - k0) * n, ctx->wpos.ptr, n, st);
 				if (k + 1 < k1)

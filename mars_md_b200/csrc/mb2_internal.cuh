@@ -251,10 +251,17 @@ struct PairTables {
 // d2max / list_rc (optional): the displacement track of the list's build and
 // its list radius. With them, rows that lie deeper inside the box than
 // list_rc + 2 * sqrt(*d2max) (plus a safety band) take no minimum image.
+// row_far / split (optional, with d2max): the far entries at the end of each
+// row and the distance beyond which all of them were at the build (0: unknown).
+// They are left out of a launch while the displacements since the build cannot
+// have brought one within reach of the tables.
 void pair_forces(const float4* sorted_pos, const uint32_t* nbr, const uint32_t* row_len,
 				 uint32_t n, uint32_t cap, int lanes_per_row, const PairTables& t, const Box& box,
 				 float cutoff_sq, int get_energy, float4* force_sorted, double* energy_virial,
-				 cudaStream_t st, const unsigned int* d2max = nullptr, float list_rc = 0.0f);
+				 cudaStream_t st, const unsigned int* d2max = nullptr, float list_rc = 0.0f,
+				 const uint32_t* row_far = nullptr, float split = 0.0f);
+// Where a build for these tables splits its rows near / far (0: it does not).
+float row_split(const PairTables& t, const Box& box, float rc_list, float cutoff);
 // Host: per-type-pair lookup constants and per-bin force / (U0, dU) arrays of
 // a set of tabulated pair tables; returns the total number of bins.
 size_t pair_table_arrays(int num_types, const uint32_t* term_matrix, int num_tables,
