@@ -17,6 +17,8 @@ unsigned long long g_launches = 0;
 // FP64 reduction slots: pair energy, pair virial, bond, angle, dihedral and
 // restraint energy.
 constexpr int kEnergySlots = 6;
+// Words of a build's statistics (see build).
+constexpr int kBuildStats = 6;
 
 struct mb2_context {
 	int device = 0;
@@ -291,9 +293,11 @@ void build(mb2_context* ctx, const float4* pos, const int* type_ids, uint32_t n,
 	for (int a = 0; a < 3; ++a) extent[a] = bmax[a] - bmin[a];
 	// stats: [0] pairs, [1] longest row (both set by each walk), [2] particles
 	// with a non-finite coordinate (counted while packing, read with the
-	// walk's statistics, so no extra synchronisation).
-	ctx->stats.ensure(3);
-	MB2_CUDA(cudaMemsetAsync(ctx->stats.ptr + 2, 0, sizeof(unsigned long long), st));
+	// walk's statistics, so no extra synchronisation), [3] set by a sort that
+	// gave up waiting.
+	ctx->stats.ensure(kBuildStats);
+	MB2_CUDA(cudaMemsetAsync(ctx->stats.ptr + 2, 0, (kBuildStats - 2) * sizeof(unsigned long long), st));
+	ctx->scratch.sort_error = reinterpret_cast<uint32_t*>(ctx->stats.ptr + 3);
 	sort_particles(ctx, pos, type_ids, n, bmin, bmax, st, ctx->stats.ptr + 2);
 
 	const float rc2 = rc_list * rc_list;
@@ -351,9 +355,10 @@ void build(mb2_context* ctx, const float4* pos, const int* type_ids, uint32_t n,
 				   ctx->cell_end.ptr, ctx->stencil.ptr, g.num_stencil, wg, n, ctx->box, ctx->excl,
 				   ctx->nbr.ptr, cap, hshift, ctx->row_len.ptr, ctx->row_far.ptr, ctx->stats.ptr,
 				   st);
-		MB2_CUDA(cudaMemcpyAsync(ctx->pinned, ctx->stats.ptr, 3 * sizeof(uint64_t),
+		MB2_CUDA(cudaMemcpyAsync(ctx->pinned, ctx->stats.ptr, 4 * sizeof(uint64_t),
 								 cudaMemcpyDeviceToHost, st));
 		MB2_CUDA(cudaStreamSynchronize(st));
+		require(ctx->pinned[3] == 0, MB2_ERR_CUDA, "mb2_build_pairlist: the sort did not finish");
 		// The walk runs on such particles without harm (cell indices come from
 		// the clamped Morton keys, and a NaN fails every distance test), but
 		// the list is not the reference's meaning of one: refuse it.

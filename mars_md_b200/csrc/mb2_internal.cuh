@@ -60,23 +60,12 @@ struct DevBuf {
 
 // Context-owned scratch for sorting and scanning.
 struct Scratch {
-	DevBuf<uint32_t> keys_alt, vals_alt, hist, scan_blocks;
-	uint32_t* sort_keys_alt = nullptr;
-	uint32_t* sort_vals_alt = nullptr;
-	uint32_t* sort_hist = nullptr;
-	void ensure_sort(size_t n, size_t hist_n) {
+	DevBuf<uint32_t> keys_alt, vals_alt, work, scan_blocks;
+	uint32_t* sort_error = nullptr;  // set by a sort that gave up (null: only in its work)
+	void ensure_sort(size_t n, size_t work_words) {
 		keys_alt.ensure(n);
 		vals_alt.ensure(n);
-		hist.ensure(hist_n);
-		sort_keys_alt = keys_alt.ptr;
-		sort_vals_alt = vals_alt.ptr;
-		sort_hist = hist.ptr;
-	}
-	void release() {
-		keys_alt.release();
-		vals_alt.release();
-		hist.release();
-		scan_blocks.release();
+		work.ensure(work_words);
 	}
 };
 
@@ -97,14 +86,13 @@ void permute_gather(const void* in, const uint32_t* s2o, uint32_t n, int elem_by
 					cudaStream_t st);
 // idx[i] = inv[idx[i]] where 0 <= idx[i] < n (others unchanged).
 void remap_indices(int* idx, size_t count, const uint32_t* inv, uint32_t n, cudaStream_t st);
-// Elements per radix-sort tile; the digit histogram holds 256 words per tile.
-constexpr uint32_t kSortTile = 2048;
-// Radix sort with caller-supplied scratch: keys_alt and vals_alt of n words,
-// hist of 256 * ceil(n / kSortTile) words, block_sums of
-// scan_blocks_needed(that) words. Nothing there needs to start at zero.
+// The sort with caller-supplied scratch: keys_alt and vals_alt of n words,
+// work of sort_work_words(n) words (8-byte aligned). Nothing there needs to
+// start at zero.
+size_t sort_work_words(uint32_t n);
 void radix_sort_pairs_into(uint32_t* keys, uint32_t* vals, uint32_t n, uint32_t* keys_alt,
-						   uint32_t* vals_alt, uint32_t* hist, uint32_t* block_sums,
-						   cudaStream_t st);
+						   uint32_t* vals_alt, uint32_t* work, cudaStream_t st,
+						   uint32_t* error = nullptr);
 // noalloc.cu: the same sort over the library's static scratch (no allocation).
 void radix_sort_pairs_static(uint32_t* keys, uint32_t* vals, uint32_t n, cudaStream_t st);
 
@@ -112,9 +100,6 @@ void radix_sort_pairs_static(uint32_t* keys, uint32_t* vals, uint32_t n, cudaStr
 // total is non-null the grand total is stored there (device pointer).
 void exclusive_scan_u32(Scratch& s, const uint32_t* in, uint32_t* out, size_t n, uint32_t* total,
 						cudaStream_t st);
-size_t scan_blocks_needed(size_t n);
-void exclusive_scan_u32_into(const uint32_t* in, uint32_t* out, size_t n, uint32_t* block_sums,
-							 cudaStream_t st);
 
 // Exclusion view (src/Interactions/DeviceExclusions.h:22-75), device pointers.
 struct Exclusions {

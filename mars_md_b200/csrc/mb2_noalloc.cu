@@ -35,18 +35,15 @@ namespace mb2 {
 namespace {
 
 constexpr uint32_t kMaxPairs = MB2_SORT_STATIC_MAX;
-static_assert(kMaxPairs % kSortTile == 0, "the maximum is a whole number of tiles");
 constexpr size_t kAlignWords = 64;  // 256-byte sub-buffer alignment
 constexpr size_t round_up(size_t w) { return (w + kAlignWords - 1) / kAlignWords * kAlignWords; }
-constexpr size_t kHistWords = static_cast<size_t>(kMaxPairs / kSortTile) * 256u;
-constexpr size_t kBlockSumWords = (kHistWords + 1023) / 1024;  // scan blocks of 1024 elements
+constexpr size_t kWorkWords = 256 * 256 * 2 + 1032;  // sort_work_words of any n up to the maximum (checked per call)
 constexpr size_t kKeysOff = 0;
 constexpr size_t kValsOff = kKeysOff + round_up(kMaxPairs);
-constexpr size_t kHistOff = kValsOff + round_up(kMaxPairs);
-constexpr size_t kSumsOff = kHistOff + round_up(kHistWords);
-constexpr size_t kWords = kSumsOff + round_up(kBlockSumWords);
+constexpr size_t kWorkOff = kValsOff + round_up(kMaxPairs);
+constexpr size_t kWords = kWorkOff + round_up(kWorkWords);
 
-// keys_alt | vals_alt | digit histogram | scan block sums (~8.6 MB).
+// keys_alt | vals_alt | histograms, tickets and look-back words (~8.6 MB).
 static __device__ __align__(256) uint32_t g_sort_scratch[kWords];
 
 // Device address of the array on the current device. In host code the
@@ -71,11 +68,9 @@ void radix_sort_pairs_static(uint32_t* keys, uint32_t* vals, uint32_t n, cudaStr
 						"; use mb2_radix_sort_pairs"};
 	uint32_t* base = scratch_on_current_device();
 	if (n <= 1) return;
-	const size_t hist_words = static_cast<size_t>((n + kSortTile - 1) / kSortTile) * 256u;
-	if (hist_words > kHistWords || scan_blocks_needed(hist_words) > kBlockSumWords)
+	if (sort_work_words(n) > kWorkWords)
 		throw Error{MB2_ERR_CAPACITY, "mb2_radix_sort_pairs_static: scratch layout too small"};
-	radix_sort_pairs_into(keys, vals, n, base + kKeysOff, base + kValsOff, base + kHistOff,
-						  base + kSumsOff, st);
+	radix_sort_pairs_into(keys, vals, n, base + kKeysOff, base + kValsOff, base + kWorkOff, st);
 }
 
 }  // namespace mb2

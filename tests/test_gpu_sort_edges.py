@@ -1,0 +1,28 @@
+"""The sort at the sizes where its launch changes (the counting sort's last size,
+the small and the large tiles' first and last, whole tiles and one element
+more), with many equal keys and with all 32 bits in use, against a stable host
+sort: integers, so equal."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [1, 2, 33, 8191, 8192, 8193, 9216, 9217, 262144, 262145, 266240, 266241,
+                               1000003])
+@pytest.mark.parametrize("bits", [3, 9, 32])
+def test_sort_is_the_stable_sort(ctx_factory, n, bits):
+    rng = np.random.default_rng(n + bits)
+    keys_np = rng.integers(0, 1 << bits, n, dtype=np.uint64).astype(np.uint32)
+    if bits == 32 and n > 2:
+        keys_np[n // 2:n // 2 + n // 8] = 0xFFFFFFFF   # as the padding of a last tile
+    vals_np = rng.permutation(n).astype(np.int32)
+    keys = torch.from_numpy(keys_np.view(np.int32).copy()).cuda()
+    vals = torch.from_numpy(vals_np.copy()).cuda()
+    ctx = ctx_factory(n)
+    ctx.radix_sort_pairs(keys, vals)
+    torch.cuda.synchronize()
+    order = np.argsort(keys_np, kind="stable")
+    assert np.array_equal(keys.cpu().numpy().view(np.uint32), keys_np[order])
+    assert np.array_equal(vals.cpu().numpy(), vals_np[order])
