@@ -117,11 +117,14 @@ struct mb2_context {
 
 	// Optional per-stage CUDA-event timing on the launching stream.
 	bool profiling = false;
-	// mb2_run: the replayed graph of one step body between rebuild checks, the
-	// values it bakes in, its kernel launches and the device step counter.
-	cudaGraphExec_t run_graph = nullptr;
-	std::vector<uint64_t> run_key;
-	unsigned long long run_launches = 0;
+	// mb2_run: the replayed graphs of the step bodies between rebuild checks,
+	// one of a single step and one of all the steps of an interval, the values
+	// each bakes in, its kernel launches, and the device step counter.
+	struct RunGraph {
+		cudaGraphExec_t exec = nullptr;
+		std::vector<uint64_t> key;
+		unsigned long long launches = 0;
+	} run_one, run_many;
 	DevBuf<unsigned long long> step_d;
 	std::vector<std::pair<cudaEvent_t, cudaEvent_t>> prof[MB2_NUM_STAGES];
 };
@@ -661,7 +664,8 @@ int mb2_destroy(mb2_context* ctx) {
 			cudaEventDestroy(be.second);
 		}
 	if (ctx->pinned) cudaFreeHost(ctx->pinned);
-	if (ctx->run_graph) cudaGraphExecDestroy(ctx->run_graph);
+	for (auto* g : {&ctx->run_one, &ctx->run_many})
+		if (g->exec) cudaGraphExecDestroy(g->exec);
 	delete ctx;  // device buffers free themselves
 	return MB2_OK;
 }
@@ -1262,21 +1266,27 @@ void step_once(mb2_context* ctx, float4* pos, float4* fe, const int* type_ids,
 						ctx->types, ctx->box, p, bonded ? 1 : 0, st);
 }
 
-// A BD step that is not a rebuild check, with the step number taken from
-// ctx->step_d and advanced by one at the end: the body mb2_run captures.
+// A step that is not a rebuild check, its number *ctx->step_d + offset: the
+// body mb2_run captures.
 void step_body_replayable(mb2_context* ctx, float4* pos, float4* fe, const int* type_ids,
 						  const uint32_t* flags, uint32_t n, const mb2_step_params* prm,
-						  cudaStream_t st) {
+						  uint64_t offset, cudaStream_t st) {
 	const bool bonded = step_has_bonded(prm);
 	pack_sorted_positions(pos, type_ids, ctx->s2o.ptr, n, ctx->sorted_pos.ptr, st, nullptr,
 						  sorted_forces(ctx, n), bonded ? fe : nullptr, track_of(ctx));
 	pair_kernel(ctx, n, prm->cutoff, prm->get_energy, st, true);
 	bonded_stage(ctx, pos, fe, prm, prm->get_energy, st);
+	const StepClock clock{ctx->step_d.ptr, offset, prm->seed, prm->patch_id};
+	if (prm->integrator == 1) {
+		baoab_integrate_gather(pos, reinterpret_cast<float4*>(prm->mom4), fe,
+							   ctx->force_sorted.ptr, ctx->inv.ptr, bonded ? 1 : 0, type_ids, flags,
+							   n, ctx->types, ctx->box, prm->dt, prm->kT, 0u, 0u, 0u, prm->efield,
+							   prm->deferred_kick_pending ? 1 : 0, st, clock);
+		return;
+	}
 	BdParams p{prm->dt, prm->kT, 0u, 0u, 0u, {prm->efield[0], prm->efield[1], prm->efield[2]}};
 	bd_integrate_gather(pos, fe, ctx->force_sorted.ptr, ctx->inv.ptr, type_ids, flags, n,
-						ctx->types, ctx->box, p, bonded ? 1 : 0, st, ctx->step_d.ptr, prm->seed,
-						prm->patch_id);
-	step_counter_add(ctx->step_d.ptr, 1, st);
+						ctx->types, ctx->box, p, bonded ? 1 : 0, st, clock);
 }
 
 uint64_t fbits(float f) {
@@ -1300,7 +1310,9 @@ std::vector<uint64_t> run_graph_key(const mb2_context* ctx, const float4* pos, c
 	auto P = [](const void* p) { return static_cast<uint64_t>(reinterpret_cast<uintptr_t>(p)); };
 	std::vector<uint64_t> k = {
 		P(pos), P(fe), P(type_ids), P(flags), n, fbits(prm->cutoff), fbits(prm->dt),
-		fbits(prm->kT), prm->seed, prm->patch_id, fbits(prm->efield[0]), fbits(prm->efield[1]),
+		fbits(prm->kT), prm->seed, prm->patch_id, static_cast<uint64_t>(prm->integrator),
+		P(prm->mom4), static_cast<uint64_t>(prm->deferred_kick_pending != 0), P(ctx->types.mass),
+		P(ctx->types.damping), fbits(prm->efield[0]), fbits(prm->efield[1]),
 		fbits(prm->efield[2]), static_cast<uint64_t>(prm->get_energy), P(prm->bonds2),
 		P(prm->bond_table_idx), prm->num_bonds, P(prm->angles4), P(prm->angle_table_idx),
 		prm->num_angles, P(prm->dihedrals4), P(prm->dihedral_table_idx), prm->num_dihedrals,
@@ -1322,6 +1334,44 @@ std::vector<uint64_t> run_graph_key(const mb2_context* ctx, const float4* pos, c
 	push_words(k, ctx->pt.solvent);
 	push_words(k, ctx->box);
 	return k;
+}
+
+// Captures `steps` step bodies into g unless it already holds them for this key.
+template <class Body>
+void capture_steps(mb2_context::RunGraph& g, std::vector<uint64_t> key, uint32_t steps, Body body) {
+	key.push_back(steps);
+	if (g.exec && key == g.key) return;
+	if (g.exec) {
+		MB2_CUDA(cudaGraphExecDestroy(g.exec));
+		g.exec = nullptr;
+	}
+	cudaStream_t cs;
+	MB2_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
+	cudaGraph_t graph = nullptr;
+	const unsigned long long l0 = g_launches;
+	cudaError_t ec = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
+	if (ec != cudaSuccess) {
+		cudaStreamDestroy(cs);
+		MB2_CUDA(ec);
+	}
+	try {
+		for (uint32_t k = 0; k < steps; ++k) body(k, cs);
+	} catch (...) {
+		cudaStreamEndCapture(cs, &graph);
+		if (graph) cudaGraphDestroy(graph);
+		cudaStreamDestroy(cs);
+		g_launches = l0;
+		throw;
+	}
+	ec = cudaStreamEndCapture(cs, &graph);
+	g.launches = g_launches - l0;
+	g_launches = l0;  // counted at each replay instead
+	cudaStreamDestroy(cs);
+	MB2_CUDA(ec);
+	const cudaError_t ei = cudaGraphInstantiate(&g.exec, graph, 0);
+	cudaGraphDestroy(graph);
+	MB2_CUDA(ei);
+	g.key = std::move(key);
 }
 
 }  // namespace
@@ -1346,56 +1396,38 @@ int mb2_run(mb2_context* ctx, float* pos4, float* force_energy4, const int* type
 		const cudaStream_t st = S(stream);
 		float4* pos = reinterpret_cast<float4*>(pos4);
 		float4* fe = reinterpret_cast<float4*>(force_energy4);
-		// Graph replay serves BD steps that are not rebuild checks; the rest (and
-		// every step while per-stage profiling is on) run as mb2_step does.
-		const bool replayable = prm->integrator == 0 && prm->rebuild_period != 0 && n > 0;
+		// Graph replay serves the steps that are not rebuild checks; the rest (and
+		// every step while per-stage profiling is on) run as mb2_step does. The
+		// steps from one check to the next are one graph where the call has them
+		// all (up to kRunSteps of them), so that no launch gap is left between
+		// them; what is left over is replayed step by step.
+		constexpr uint32_t kRunSteps = 32;
+		const uint32_t period = prm->rebuild_period;
+		const bool replayable = period != 0 && n > 0;
 		ctx->step_d.ensure(1);
-		bool counter_set = false;
-		for (uint32_t k = 0; k < num_steps; ++k) {
+		for (uint32_t k = 0; k < num_steps;) {
 			const uint64_t step = first_step + k;
-			const bool check = (step - 1) % (prm->rebuild_period ? prm->rebuild_period : 1) == 0;
+			const bool check = (step - 1) % (period ? period : 1) == 0;
 			if (!replayable || check || ctx->profiling || !ctx->built || ctx->built_n != n) {
 				step_once(ctx, pos, fe, type_ids, flags, n, step, prm, st);
-				counter_set = false;
+				++k;
 				continue;
 			}
 			ctx->force_sorted.ensure(n);  // no allocation inside the capture
 			const std::vector<uint64_t> key = run_graph_key(ctx, pos, fe, type_ids, flags, n, prm);
-			if (!ctx->run_graph || key != ctx->run_key) {
-				if (ctx->run_graph) {
-					MB2_CUDA(cudaGraphExecDestroy(ctx->run_graph));
-					ctx->run_graph = nullptr;
-				}
-				cudaStream_t cs;
-				MB2_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
-				cudaGraph_t g = nullptr;
-				const unsigned long long l0 = g_launches;
-				MB2_CUDA(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
-				try {
-					step_body_replayable(ctx, pos, fe, type_ids, flags, n, prm, cs);
-				} catch (...) {
-					cudaStreamEndCapture(cs, &g);
-					if (g) cudaGraphDestroy(g);
-					cudaStreamDestroy(cs);
-					g_launches = l0;
-					throw;
-				}
-				const cudaError_t ec = cudaStreamEndCapture(cs, &g);
-				ctx->run_launches = g_launches - l0;
-				g_launches = l0;  // counted at each replay instead
-				cudaStreamDestroy(cs);
-				MB2_CUDA(ec);
-				const cudaError_t ei = cudaGraphInstantiate(&ctx->run_graph, g, 0);
-				cudaGraphDestroy(g);
-				MB2_CUDA(ei);
-				ctx->run_key = key;
-			}
-			if (!counter_set) {
-				step_counter_set(ctx->step_d.ptr, step, st);
-				counter_set = true;
-			}
-			MB2_CUDA(cudaGraphLaunch(ctx->run_graph, st));
-			g_launches += ctx->run_launches;
+			const uint32_t many = std::min(period - 1u, kRunSteps);
+			const uint64_t to_check = period - (step - 1) % period;
+			const uint64_t ahead = std::min<uint64_t>(num_steps - k, to_check);
+			const bool use_many = many > 1u && ahead >= many;
+			auto& g = use_many ? ctx->run_many : ctx->run_one;
+			const uint32_t steps = use_many ? many : 1u;
+			capture_steps(g, key, steps, [&](uint32_t offset, cudaStream_t cs) {
+				step_body_replayable(ctx, pos, fe, type_ids, flags, n, prm, offset, cs);
+			});
+			step_counter_set(ctx->step_d.ptr, step, st);
+			MB2_CUDA(cudaGraphLaunch(g.exec, st));
+			g_launches += g.launches;
+			k += steps;
 		}
 	});
 }

@@ -218,24 +218,28 @@ __device__ __forceinline__ uint64_t mix_seed(uint64_t seed, uint64_t patch, uint
 // writes), added to what the bonded kernels left in ForceEnergy when any ran
 // (read_fe), and the result stored to ForceEnergy as the reference leaves it
 // after integrate_motion; then the grid force, noise and update as bd_kernel.
-// step_ptr (graph replay): the step number comes from device memory and the
+// clock (graph replay): the step number comes from device memory and the
 // Philox key is mixed here from (seed, patch_id, step), as the host does for
-// bp.base_seed otherwise. kGrids false (no grid loaded): without the grid
+// bp.base_seed otherwise; the noise, which needs nothing else, is drawn before
+// the wait for the force kernels (its base is set by a launch before the
+// graph, so it is readable by then). kGrids false (no grid loaded): without the grid
 // code the kernel takes fewer registers and more warps fit on an SM.
 template <bool kGrids>
 __global__ void __launch_bounds__(256) bd_gather_kernel(
 	float4* __restrict__ pos, float4* __restrict__ fe, const float4* __restrict__ fs,
 	const uint32_t* __restrict__ inv, const int* __restrict__ type_ids,
 	const uint32_t* __restrict__ flags, uint32_t n, TypeTable ty, Box box, BdParams bp,
-	int read_fe, const unsigned long long* __restrict__ step_ptr, uint64_t seed,
-	uint64_t patch_id) {
+	int read_fe, StepClock clock) {
+	chain_begin();
 	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-	if (i >= n) return;
-	if (step_ptr) {
-		const uint64_t step = *step_ptr;
+	if (clock.ptr) {
+		const uint64_t step = *clock.ptr + clock.offset;
 		bp.step = static_cast<uint32_t>(step);
-		bp.base_seed = mix_seed(seed, patch_id, step);
+		bp.base_seed = mix_seed(clock.seed, clock.patch_id, step);
 	}
+	const float3 xi = bd_noise(bp.base_seed, bp.base_ctr + i, bp.step);
+	chain_wait();
+	if (i >= n) return;
 	float4 f = fs[inv[i]];
 	if (read_fe) {
 		const float4 ext = fe[i];
@@ -251,7 +255,6 @@ __global__ void __launch_bounds__(256) bd_gather_kernel(
 	const float4 p = pos[i];
 	const int type = type_ids[i];
 	const float4 pmf = position_force<kGrids>(ty, type, p.x, p.y, p.z, bp.efield);
-	const float3 xi = bd_noise(bp.base_seed, bp.base_ctr + i, bp.step);
 	if (pmf.w != 0.0f) f.w = __fadd_rn(f.w, pmf.w);
 	fe[i] = f;
 	pos[i] = bd_update(p, __fadd_rn(f.x, pmf.x), __fadd_rn(f.y, pmf.y), __fadd_rn(f.z, pmf.z),
@@ -282,8 +285,16 @@ __global__ void __launch_bounds__(256) baoab_kernel(
 	const float4* __restrict__ fs, const uint32_t* __restrict__ inv, int read_fe,
 	const int* __restrict__ type_ids, const uint32_t* __restrict__ flags, uint32_t n,
 	TypeTable ty, Box box, float dt, float kT, uint32_t step, uint64_t seed, uint32_t base_ctr,
-	float3 efield, int pending) {
+	float3 efield, int pending, StepClock clock) {
+	chain_begin();
 	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+	if (clock.ptr) {  // as bd_gather_kernel
+		const uint64_t now = *clock.ptr + clock.offset;
+		step = static_cast<uint32_t>(now);
+		seed = mix_seed(clock.seed, clock.patch_id, now);
+	}
+	const float3 xi = bd_noise(seed, base_ctr + i, step, kBaoabStream);
+	chain_wait();
 	if (i >= n) return;
 	float4 p = pos[i];
 	float4 f;
@@ -330,7 +341,6 @@ __global__ void __launch_bounds__(256) baoab_kernel(
 	p.y = drift(p.y, m.y);
 	p.z = drift(p.z, m.z);
 	const float4 g = ty.damping[type];
-	const float3 xi = bd_noise(seed, base_ctr + i, step, kBaoabStream);
 	auto ou = [&](float mv, float gamma, float r) {  // O
 		const float c = expf(__fmul_rn(-gamma, dt));
 		const float ns = __fmul_rn(
@@ -378,6 +388,8 @@ __global__ void __launch_bounds__(256) bd_systems_kernel(
 	const uint32_t* __restrict__ sys_of, const uint32_t* __restrict__ offsets,
 	const Box* __restrict__ boxes, uint32_t n, TypeTable ty, float dt, float kT, uint64_t seed,
 	uint64_t patch_id, const unsigned long long* __restrict__ step_ptr) {
+	chain_begin();
+	chain_wait();
 	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
 	if (i >= n) return;
 	const uint64_t step = *step_ptr;
@@ -419,16 +431,21 @@ void bd_integrate(float4* pos, float4* fe, const int* type_ids, const uint32_t* 
 	MB2_LAUNCH bd_kernel<<<(n + 255) / 256, 256, 0, st>>>(pos, fe, type_ids, flags, n, types, box, p);
 }
 
+namespace {
+// Threads per block of the integrators: a small system's blocks are kept small,
+// so that its few warps, each a chain of dependent arithmetic, spread over SMs.
+uint32_t integrate_threads(uint32_t n) { return n <= 148u * 256u ? 64u : 256u; }
+}  // namespace
+
 void bd_integrate_gather(float4* pos, float4* fe, const float4* force_sorted, const uint32_t* inv,
 						 const int* type_ids, const uint32_t* flags, uint32_t n,
 						 const TypeTable& types, const Box& box, const BdParams& p, int read_fe,
-						 cudaStream_t st, const unsigned long long* step_ptr, uint64_t seed,
-						 uint64_t patch_id) {
+						 cudaStream_t st, const StepClock& clock) {
 	if (n == 0) return;
 	auto kern = types.num_grids == 0 ? bd_gather_kernel<false> : bd_gather_kernel<true>;
-	MB2_LAUNCH kern<<<(n + 255) / 256, 256, 0, st>>>(pos, fe, force_sorted, inv, type_ids, flags, n,
-													 types, box, p, read_fe, step_ptr, seed,
-													 patch_id);
+	const uint32_t threads = integrate_threads(n);
+	launch_chained(kern, (n + threads - 1) / threads, threads, 0, st, pos, fe, force_sorted, inv,
+				   type_ids, flags, n, types, box, p, read_fe, clock);
 }
 
 void baoab_integrate(float4* pos, float4* mom, float4* fe, const int* type_ids,
@@ -438,18 +455,21 @@ void baoab_integrate(float4* pos, float4* mom, float4* fe, const int* type_ids,
 	if (n == 0) return;
 	MB2_LAUNCH baoab_kernel<false><<<(n + 255) / 256, 256, 0, st>>>(
 		pos, mom, fe, nullptr, nullptr, 0, type_ids, flags, n, types, box, dt, kT, step, base_seed,
-		base_ctr, make_float3(efield[0], efield[1], efield[2]), pending);
+		base_ctr, make_float3(efield[0], efield[1], efield[2]), pending, StepClock{});
 }
 
 void baoab_integrate_gather(float4* pos, float4* mom, float4* fe, const float4* force_sorted,
 							const uint32_t* inv, int read_fe, const int* type_ids,
 							const uint32_t* flags, uint32_t n, const TypeTable& types,
 							const Box& box, float dt, float kT, uint32_t step, uint64_t base_seed,
-							uint32_t base_ctr, const float* efield, int pending, cudaStream_t st) {
+							uint32_t base_ctr, const float* efield, int pending, cudaStream_t st,
+							const StepClock& clock) {
 	if (n == 0) return;
-	MB2_LAUNCH baoab_kernel<true><<<(n + 255) / 256, 256, 0, st>>>(
-		pos, mom, fe, force_sorted, inv, read_fe, type_ids, flags, n, types, box, dt, kT, step,
-		base_seed, base_ctr, make_float3(efield[0], efield[1], efield[2]), pending);
+	const uint32_t threads = integrate_threads(n);
+	launch_chained(baoab_kernel<true>, (n + threads - 1) / threads, threads, 0, st, pos, mom, fe,
+				   force_sorted, inv, read_fe, type_ids, flags, n, types, box, dt, kT, step,
+				   base_seed, base_ctr, make_float3(efield[0], efield[1], efield[2]), pending,
+				   clock);
 }
 
 void baoab_last_update(float4* mom, const float4* fe, const uint32_t* flags, uint32_t n,
@@ -465,9 +485,8 @@ void bd_integrate_systems(float4* pos, float4* fe, const float4* force_sorted,
 						  uint64_t patch_id, const unsigned long long* step_ptr, cudaStream_t st) {
 	if (n == 0) return;
 	auto kern = types.num_grids == 0 ? bd_systems_kernel<false> : bd_systems_kernel<true>;
-	MB2_LAUNCH kern<<<(n + 255) / 256, 256, 0, st>>>(pos, fe, force_sorted, inv, type_ids, sys_of,
-													 offsets, boxes, n, types, dt, kT, seed,
-													 patch_id, step_ptr);
+	launch_chained(kern, (n + 255) / 256, 256u, 0, st, pos, fe, force_sorted, inv, type_ids, sys_of,
+				   offsets, boxes, n, types, dt, kT, seed, patch_id, step_ptr);
 }
 
 void step_counter_set(unsigned long long* ptr, uint64_t value, cudaStream_t st) {

@@ -387,6 +387,7 @@ __global__ void __launch_bounds__(
 	constexpr bool kStage = !std::is_same<BoxSrc, OneBox>::value;
 	extern __shared__ float4 smem4[];
 	PairTableRef* refs = reinterpret_cast<PairTableRef*>(smem4);
+	chain_begin();
 	for (int k = threadIdx.x; k < T * T; k += blockDim.x) refs[k] = refs_g[k];
 	const float* __restrict__ bin_f = force_g;
 	const float2* __restrict__ bin_e = energy_g;
@@ -401,6 +402,7 @@ __global__ void __launch_bounds__(
 		bin_e = se;
 	}
 	__syncthreads();
+	chain_wait();
 
 	const int sub = threadIdx.x & (G - 1);  // lane within the row's group
 	const uint32_t i = blockIdx.x * (blockDim.x / G) + threadIdx.x / G;
@@ -481,6 +483,8 @@ __global__ void __launch_bounds__(256, fast_min_blocks<kEnergy, std::is_same<Box
 	const uint32_t* __restrict__ row_len, uint32_t n, uint32_t cap, FastArgs fa, BoxSrc boxes,
 	float4* force, double* __restrict__ ev) {
 	constexpr int H = 32 / G;
+	chain_begin();
+	chain_wait();
 	const int sub = threadIdx.x & (G - 1);  // lane within the row's group
 	const uint32_t i = blockIdx.x * (blockDim.x / G) + threadIdx.x / G;
 	const bool valid = i < n;
@@ -736,6 +740,8 @@ __global__ void __launch_bounds__(256) bond_angle_kernel(
 	const int* __restrict__ angle_idx, uint32_t na, const Table* __restrict__ angle_tables,
 	const float4* __restrict__ pos, float4* fe, Box box, int get_energy, double* bond_energy,
 	double* angle_energy) {
+	chain_begin();
+	chain_wait();
 	const uint32_t bond_blocks = (nb + blockDim.x - 1) / blockDim.x;
 	if (blockIdx.x < bond_blocks) {
 		const double e = bond_term(blockIdx.x * blockDim.x + threadIdx.x, bonds, bond_idx, nb, pos,
@@ -911,8 +917,8 @@ void launch_fast(const float4* sorted_pos, const uint32_t* nbr, const uint32_t* 
 								  : fast_pair_kernel<G, kEnergy, true, true, BoxSrc>)
 					: (fa.offsets ? fast_pair_kernel<G, kEnergy, false, false, BoxSrc>
 								  : fast_pair_kernel<G, kEnergy, true, false, BoxSrc>);
-	MB2_LAUNCH kern<<<blocks, 256, 0, st>>>(sorted_pos, nbr, row_len, n, cap, fa, boxes,
-											force_sorted, ev);
+	launch_chained(kern, blocks, 256u, 0, st, sorted_pos, nbr, row_len, n, cap, fa, boxes, force_sorted,
+				   ev);
 }
 
 template <int G, bool kEnergy, bool kAllPeriodic, bool kTerms, class BoxSrc>
@@ -931,10 +937,9 @@ void launch_pair(const float4* sorted_pos, const uint32_t* nbr, const uint32_t* 
 	if (smem > 48 * 1024)
 		MB2_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
 									  static_cast<int>(smem)));
-	MB2_LAUNCH kern<<<blocks, 256, smem, st>>>(sorted_pos, nbr, row_len, n, cap, t.num_types,
-											   t.refs, t.bin_force, t.bin_energy, t.total_bins,
-											   t.terms, t.solvent, boxes, dist_window(cutoff_sq),
-											   force_sorted, ev);
+	launch_chained(kern, blocks, 256u, smem, st, sorted_pos, nbr, row_len, n, cap, t.num_types,
+				   t.refs, t.bin_force, t.bin_energy, t.total_bins, t.terms, t.solvent, boxes,
+				   dist_window(cutoff_sq), force_sorted, ev);
 }
 
 template <int G, bool kEnergy, class BoxSrc>
@@ -1277,9 +1282,8 @@ void bond_angle_forces(const int2* bonds, const int* bond_idx, uint32_t nb, cons
 					   int get_energy, double* bond_energy, double* angle_energy, cudaStream_t st) {
 	const uint32_t blocks = (nb + 255) / 256 + (na + 255) / 256;
 	if (blocks == 0) return;
-	MB2_LAUNCH bond_angle_kernel<<<blocks, 256, 0, st>>>(bonds, bond_idx, nb, bond_tables, angles,
-														 angle_idx, na, angle_tables, pos, fe, box,
-														 get_energy, bond_energy, angle_energy);
+	launch_chained(bond_angle_kernel, blocks, 256u, 0, st, bonds, bond_idx, nb, bond_tables, angles,
+				   angle_idx, na, angle_tables, pos, fe, box, get_energy, bond_energy, angle_energy);
 }
 
 void dihedral_forces(const int4* dihedrals, const int* table_idx, uint32_t nd, const float4* pos,

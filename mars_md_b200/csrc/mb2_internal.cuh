@@ -28,6 +28,35 @@ struct Error {
 			throw ::mb2::Error{2, std::string(#call) + ": " + cudaGetErrorString(e_)};   \
 	} while (0)
 
+// Launches a kernel of the step's chain (pack, pair, bonded, integrate): it may
+// be scheduled while the kernel before it in the stream still runs, and itself
+// waits for that kernel's end in chain_wait(). Hides the launch latency between
+// the kernels of a small system's step, about 1 us each.
+template <class... P, class... A>
+void launch_chained(void (*kernel)(P...), uint32_t blocks, uint32_t threads, size_t smem,
+					cudaStream_t st, A... args) {
+	cudaLaunchAttribute attr{};
+	attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+	attr.val.programmaticStreamSerializationAllowed = 1;
+	cudaLaunchConfig_t c{};
+	c.gridDim = dim3(blocks);
+	c.blockDim = dim3(threads);
+	c.dynamicSmemBytes = smem;
+	c.stream = st;
+	c.attrs = &attr;
+	c.numAttrs = 1;
+	++g_launches;
+	MB2_CUDA(cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...));
+}
+
+// First thing in every kernel that launch_chained launches: lets the next
+// kernel of the chain be scheduled, then waits until the kernels before this
+// one have ended and their writes are visible (nothing to wait for in an
+// ordinary launch). Each kernel of a chain waits before it touches memory, so
+// a kernel's end implies the end of all before it.
+__device__ __forceinline__ void chain_begin() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Throws Error{code, msg} unless cond holds.
 inline void expect_arg(bool cond, int code, const char* msg) {
 	if (!cond) throw Error{code, msg};
@@ -336,14 +365,19 @@ struct BdParams {
 void bd_integrate(float4* pos, float4* fe, const int* type_ids, const uint32_t* flags, uint32_t n,
 				  const TypeTable& types, const Box& box, const BdParams& p, cudaStream_t st);
 // The fused step's integrate: force = force_sorted[inv[i]] (+ fe[i] if read_fe).
-// step_ptr non-null: the step number is read from device memory at run time
-// (a replayed graph) and the Philox key mixed on the device from seed and
-// patch_id; p.step and p.base_seed are then unused.
+// clock.ptr non-null: the step number is *clock.ptr + clock.offset at run time
+// (a replayed graph, whose base a step_counter_set launched before it sets) and
+// the Philox key is mixed on the device from seed and patch_id; p.step and
+// p.base_seed are then unused.
+struct StepClock {
+	const unsigned long long* ptr = nullptr;
+	unsigned long long offset = 0;
+	uint64_t seed = 0, patch_id = 0;
+};
 void bd_integrate_gather(float4* pos, float4* fe, const float4* force_sorted, const uint32_t* inv,
 						 const int* type_ids, const uint32_t* flags, uint32_t n,
 						 const TypeTable& types, const Box& box, const BdParams& p, int read_fe,
-						 cudaStream_t st, const unsigned long long* step_ptr = nullptr,
-						 uint64_t seed = 0, uint64_t patch_id = 0);
+						 cudaStream_t st, const StepClock& clock = StepClock{});
 // Langevin BAOAB (Integrator/BAOAB.h): with grids, ForceEnergy += position
 // force for every particle; `pending` applies the deferred closing half-kick
 // first; then B-A-O-A and wrap. Noise key (seed, base_ctr + i, step, stream 0x1356914).
@@ -357,7 +391,8 @@ void baoab_integrate_gather(float4* pos, float4* mom, float4* fe, const float4* 
 							const uint32_t* inv, int read_fe, const int* type_ids,
 							const uint32_t* flags, uint32_t n, const TypeTable& types,
 							const Box& box, float dt, float kT, uint32_t step, uint64_t base_seed,
-							uint32_t base_ctr, const float* efield, int pending, cudaStream_t st);
+							uint32_t base_ctr, const float* efield, int pending, cudaStream_t st,
+							const StepClock& clock = StepClock{});
 // BAOAB_LastUpdate: mom += 0.5 dt F (closing half-kick) for non-frozen particles.
 void baoab_last_update(float4* mom, const float4* fe, const uint32_t* flags, uint32_t n,
 					   float dt, cudaStream_t st);

@@ -492,6 +492,8 @@ __global__ void __launch_bounds__(256) pack_kernel(const float4* __restrict__ po
 												   float4* __restrict__ clear_a,
 												   float4* __restrict__ clear_b,
 												   DisplacementTrack track) {
+	chain_begin();
+	chain_wait();
 	const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
 	// The tracked word so far, read before the loads (see displacement_kernel).
 	const unsigned int seen = track.d2max && (threadIdx.x & 31) == 0
@@ -615,8 +617,8 @@ void pack_sorted_positions(const float4* pos, const int* type_ids, const uint32_
 						   unsigned long long* nonfinite, float4* clear_a, float4* clear_b,
 						   const DisplacementTrack& track) {
 	if (n == 0) return;
-	MB2_LAUNCH pack_kernel<<<(n + 255) / 256, 256, 0, st>>>(pos, type_ids, s2o, n, sorted_pos,
-															 nonfinite, clear_a, clear_b, track);
+	launch_chained(pack_kernel, (n + 255) / 256, 256, 0, st, pos, type_ids, s2o, n, sorted_pos,
+				   nonfinite, clear_a, clear_b, track);
 }
 
 }  // namespace mb2
