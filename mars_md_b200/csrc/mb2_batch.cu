@@ -18,6 +18,7 @@
 // step counter) in a CUDA graph and replays it; pairlist rebuilds run eagerly
 // at the rebuild period (the list is re-sized from the walk's counts).
 #include <algorithm>
+#include <cfloat>
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -144,12 +145,74 @@ __global__ void __launch_bounds__(256) batch_row_stats_kernel(const uint32_t* __
 // every system), from which their displacements are measured.
 __global__ void __launch_bounds__(256) batch_snapshot_kernel(const float4* __restrict__ pos,
 															 const uint32_t* __restrict__ sys_of,
+															 const uint32_t* __restrict__ offsets,
 															 const uint32_t* __restrict__ flags,
-															 uint32_t n, float4* __restrict__ ref) {
+															 uint32_t n, float4* __restrict__ ref,
+															 unsigned int* __restrict__ moved) {
 	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
 	if (i >= n) return;
-	if (flags && !flags[sys_of[i]]) return;
+	const uint32_t s = sys_of[i];
+	if (flags && !flags[s]) return;
 	ref[i] = pos[i];
+	if (i == offsets[s]) moved[s] = 0u;
+}
+
+// The step's pack: Z-ordered positions, the pair-force accumulator cleared,
+// and (moved not null) the largest squared displacement of each system since
+// its own list build raised in moved[system] (float bits, which order as the
+// non-negative floats do; not finite: +inf). A warp reads the word first and
+// only raises it when its own maximum is larger. Sixteen bytes more to read a
+// particle than without, against the rows' far part that the pair kernel then
+// need not read (see set_far).
+__global__ void __launch_bounds__(256) batch_pack_kernel(
+	const float4* __restrict__ pos, const int* __restrict__ type_ids,
+	const uint32_t* __restrict__ s2o, const uint32_t* __restrict__ keys,
+	const Box* __restrict__ boxes, const float4* __restrict__ ref, uint32_t n,
+	float4* __restrict__ sorted_pos, float4* __restrict__ clear, unsigned int* moved) {
+	chain_begin();
+	chain_wait();
+	const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+	unsigned int bits = 0u;
+	uint32_t sys = 0xFFFFFFFFu;
+	if (k < n) {
+		const uint32_t o = s2o[k];
+		float4 p = pos[o];
+		clear[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+		if (moved) {
+			sys = keys[k] >> kSysShift;
+			const float4 r = ref[o];
+			const float3 d = wrap_diff(boxes[sys], __fsub_rn(p.x, r.x), __fsub_rn(p.y, r.y),
+									   __fsub_rn(p.z, r.z));
+			const float d2 = len2(d.x, d.y, d.z);
+			bits = d2 <= FLT_MAX ? __float_as_uint(d2) : 0x7F800000u;
+		}
+		p.w = __int_as_float(type_ids[o]);
+		sorted_pos[k] = p;
+	}
+	if (!moved) return;
+	const uint32_t s0 = __shfl_sync(0xFFFFFFFFu, sys, 0);
+	if (__all_sync(0xFFFFFFFFu, sys == s0 || k >= n)) {
+		const unsigned int most = __reduce_max_sync(0xFFFFFFFFu, bits);
+		if ((threadIdx.x & 31) == 0 && s0 != 0xFFFFFFFFu &&
+			most > *reinterpret_cast<volatile unsigned int*>(moved + s0))
+			atomicMax(moved + s0, most);
+	} else if (k < n) {
+		atomicMax(moved + sys, bits);
+	}
+}
+
+// A build's far entries moved behind the near ones, as join_far_kernel does it,
+// in the rows of the systems that were rebuilt (flags null: all).
+__global__ void __launch_bounds__(256) batch_join_far_kernel(
+	uint32_t* __restrict__ nbr, const uint32_t* __restrict__ row_len,
+	const uint32_t* __restrict__ row_far, const uint32_t* __restrict__ keys,
+	const uint32_t* __restrict__ flags, uint32_t n, uint32_t cap, int hshift) {
+	const uint32_t slice = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+	const uint32_t slices = (n + (1u << hshift) - 1u) >> hshift;
+	if (slice >= slices) return;  // whole warp
+	const uint32_t i = (slice << hshift) + (threadIdx.x & ((1u << hshift) - 1u));
+	const bool mine = i < n && (!flags || flags[keys[i] >> kSysShift]);
+	join_far_slice(nbr, mine ? row_len[i] : 0u, mine ? row_far[i] : 0u, slice, cap, hshift);
 }
 
 __global__ void __launch_bounds__(256) batch_cell_ranges_kernel(const uint32_t* __restrict__ keys,
@@ -175,22 +238,23 @@ __global__ void __launch_bounds__(256) batch_cell_ranges_kernel(const uint32_t* 
 // particles of the system and are skipped), lay their candidate ranges end to
 // end by a warp scan, and test 32 consecutive candidates a round with the
 // reference's exact test, each lane finding its candidate's cell by a binary
-// search over the running totals held one per lane. Hits are appended in
-// candidate order. Six resident blocks per SM (40 registers): 1 % faster per
+// search over the running totals held one per lane. Hits are appended with
+// two ballots, near entries from the front of the row, far ones from the back. Six resident blocks per SM (40 registers): 1 % faster per
 // build than 48 registers at five, and than 32 at eight.
 __device__ __forceinline__ uint32_t batch_row(
 	uint32_t i, uint32_t lane, const float4* __restrict__ sorted_pos,
 	const uint32_t* __restrict__ keys, const uint32_t* __restrict__ s2o,
 	const uint32_t* __restrict__ begin, const uint32_t* __restrict__ end,
 	const SysGrid* __restrict__ grids, const Box* __restrict__ boxes,
-	const uint4* __restrict__ stencil, uint32_t* __restrict__ nbr, uint32_t cap, int hshift) {
+	const uint4* __restrict__ stencil, uint32_t* __restrict__ nbr, uint32_t cap, int hshift,
+	uint32_t& far) {
 	const uint32_t lt = (1u << lane) - 1u;
 	const uint32_t key = keys[i];
 	const uint32_t sys = key >> kSysShift;
 	const SysGrid* g = grids + sys;
 	const int m = g->wg.m;
 	const uint32_t c = (key & kLocalMask) >> g->wg.shift;
-	const float rc2 = g->wg.rc2;
+	const float rc2 = g->wg.rc2, split2 = g->wg.split2;
 	const uint32_t cell_base = g->cell_base;
 	const uint4* st = stencil + g->stencil_off;
 	const int ns = static_cast<int>(g->stencil_n);
@@ -210,6 +274,7 @@ __device__ __forceinline__ uint32_t batch_row(
 	const uint32_t h = 1u << hshift;
 	uint32_t* base = nbr + (static_cast<size_t>(i >> hshift) * cap << hshift) + (i & (h - 1u));
 	uint32_t len = 0;
+	far = 0;
 	for (int k0 = 0; k0 < ns; k0 += 32) {
 		uint32_t jb = 0, je = 0;
 		const int k = k0 + static_cast<int>(lane);
@@ -246,7 +311,7 @@ __device__ __forceinline__ uint32_t batch_row(
 			}
 			const uint32_t ob = __shfl_sync(0xFFFFFFFFu, jb, owner & 31);
 			const uint32_t oe = __shfl_sync(0xFFFFFFFFu, excl, owner & 31);
-			bool hit = false;
+			bool hit = false, near = false;
 			uint32_t entry = 0;
 			if (t < total) {
 				const uint32_t j = ob + (t - oe);
@@ -254,20 +319,26 @@ __device__ __forceinline__ uint32_t batch_row(
 				const float dx = wrap_diff_scalar(__fsub_rn(pj.x, pi.x), lx, ix, hx);
 				const float dy = wrap_diff_scalar(__fsub_rn(pj.y, pi.y), ly, iy, hy);
 				const float dz = wrap_diff_scalar(__fsub_rn(pj.z, pi.z), lz, iz, hz);
-				if (len2(dx, dy, dz) <= rc2) {
+				const float d2 = len2(dx, dy, dz);
+				if (d2 <= rc2) {
 					hit = true;
+					near = d2 <= split2;
 					entry = j | (static_cast<int>(s2o[j]) < a ? kOrientBit : 0u);
 				}
 			}
-			const uint32_t hm = __ballot_sync(0xFFFFFFFFu, hit);
+			const uint32_t nm = __ballot_sync(0xFFFFFFFFu, hit && near);
+			const uint32_t fm = __ballot_sync(0xFFFFFFFFu, hit && !near);
 			if (hit) {
-				const uint32_t p = len + static_cast<uint32_t>(__popc(hm & lt));
-				if (p < cap) base[static_cast<size_t>(p) * h] = entry;
+				const uint32_t p = len + far + static_cast<uint32_t>(__popc((nm | fm) & lt));
+				const uint32_t slot = near ? len + static_cast<uint32_t>(__popc(nm & lt))
+										   : cap - 1u - (far + static_cast<uint32_t>(__popc(fm & lt)));
+				if (p < cap) base[static_cast<size_t>(slot) * h] = entry;
 			}
-			len += static_cast<uint32_t>(__popc(hm));
+			len += static_cast<uint32_t>(__popc(nm));
+			far += static_cast<uint32_t>(__popc(fm));
 		}
 	}
-	return len;
+	return len + far;
 }
 
 // One warp per group of 32 consecutive sorted particles: a group whose
@@ -285,7 +356,7 @@ __global__ void __launch_bounds__(256, 7) batch_group_kernel(
 	const uint32_t* __restrict__ end, const SysGrid* __restrict__ grids,
 	const Box* __restrict__ boxes, const uint4* __restrict__ stencil,
 	const uint32_t* __restrict__ flags, uint32_t n, uint32_t* __restrict__ nbr, uint32_t cap,
-	int hshift, uint32_t* __restrict__ row_len) {
+	int hshift, uint32_t* __restrict__ row_len, uint32_t* __restrict__ row_far) {
 	__shared__ uint32_t split_tab[1 << kLocalBits];
 	__shared__ uint4 cell_buf[8 * kCellBuf];  // per warp: kept cells (jlo, end, image code, offset)
 	__shared__ float4 cand_buf[8 * 32];       // per warp: candidates that pass the group test
@@ -315,7 +386,7 @@ __global__ void __launch_bounds__(256, 7) batch_group_kernel(
 	const int z0 = warp_min(valid ? cz : INT_MAX), z1 = warp_max(valid ? cz : INT_MIN);
 	const bool coherent = one_system && (x1 - x0) <= wg.emax && (y1 - y0) <= wg.emax &&
 						  (z1 - z0) <= wg.emax;
-	uint32_t len = 0;
+	uint32_t len = 0, far = 0;
 	if (coherent) {
 		const float4 pi = valid ? sorted_pos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
 		const int a = valid ? static_cast<int>(s2o[i]) : 0;
@@ -332,18 +403,26 @@ __global__ void __launch_bounds__(256, 7) batch_group_kernel(
 										 valid, pi, a, 0, 0, -1, c_first, x0, x1, y0, y1, z0, z1,
 										 gxlo, gxhi, gylo, gyhi, gzlo, gzhi, row);
 		len = row.total();
+		far = row.far;
 	} else {
 		uint32_t todo = __ballot_sync(0xFFFFFFFFu, walked);
 		while (todo) {
 			const int l = __ffs(todo) - 1;
 			todo &= todo - 1u;
+			uint32_t far_l;
 			const uint32_t len_l = batch_row(i_first + static_cast<uint32_t>(l), lane, sorted_pos,
 											 keys, s2o, begin, end, grids, boxes, stencil, nbr,
-											 cap, hshift);
-			if (static_cast<int>(lane) == l) len = len_l;
+											 cap, hshift, far_l);
+			if (static_cast<int>(lane) == l) {
+				len = len_l;
+				far = far_l;
+			}
 		}
 	}
-	if (walked) row_len[i] = len;
+	if (walked) {
+		row_len[i] = len;
+		row_far[i] = far;
+	}
 }
 
 // Largest squared displacement of each system's particles since their
@@ -428,6 +507,12 @@ struct mb2_batch {
 	unsigned long long system_rebuilds = 0;  // systems rebuilt, summed over those builds
 	DevBuf<unsigned long long> stats, step_d;
 	DevBuf<unsigned int> disp;
+	// Rows' far entries, the near / far split of the lists (0: none), and each
+	// system's largest squared displacement since its build (the packs keep it).
+	DevBuf<uint32_t> row_far;
+	float split = 0.0f;
+	DevBuf<unsigned int> moved;
+	float longest_edge = 0.0f;
 	DevBuf<double> energy;
 	unsigned long long* pinned = nullptr;
 	unsigned int* pinned_sys = nullptr;  // per system: displacement readback, then rebuild flags
@@ -518,7 +603,7 @@ void choose_grids(mb2_batch* b, float rc) {
 		wg.lim = g.lim;
 		wg.rc2 = rc * rc;
 		fast_test_band(bx, rc, &wg.fast_lo, &wg.fast_hi);
-		wg.split2 = INFINITY;
+		wg.split2 = b->split > 0.0f ? b->split * b->split : INFINITY;
 		// Cell c of level m spans Morton coordinates [c, c + 1) * 2^(7 - m) of
 		// the 7-bit scale over the box, L / 2^m wide; the margin covers the
 		// rounding of that mapping, as on the plain path.
@@ -558,8 +643,8 @@ void choose_grids(mb2_batch* b, float rc) {
 // list would if it ran alone (a patch of the reference rebuilds on its own
 // skin check). A change of grid, or a row longer than the list's row
 // capacity, rebuilds every system.
-void batch_build(mb2_batch* b, const float4* pos, const int* type_ids, float rc, cudaStream_t st,
-				 const unsigned int* flags_h = nullptr) {
+void batch_build(mb2_batch* b, const float4* pos, const int* type_ids, float rc, float cutoff,
+				 cudaStream_t st, const unsigned int* flags_h = nullptr) {
 	expect_arg(rc > 0.0f && std::isfinite(rc), MB2_ERR_ARG,
 			   "mb2_batch_build: pairlist cutoff must be positive and finite");
 	for (uint32_t s = 0; s < b->num_systems; ++s)
@@ -567,7 +652,18 @@ void batch_build(mb2_batch* b, const float4* pos, const int* type_ids, float rc,
 			expect_arg(2.0f * rc < b->boxes_h[s].size[a], MB2_ERR_ARG,
 					   "mb2_batch_build: every box edge must exceed twice the list radius");
 	const uint32_t n = b->n;
-	if (b->grid_rc != rc) {
+	// Rows are split near / far only where the tables end well short of the
+	// cutoff (every batched box is periodic): the far entries are then mostly
+	// not read. A split at the cutoff, as the plain path's, gained nothing here.
+	// A rebuild of some systems, and a build without a cutoff, keep the split in
+	// force.
+	float split = b->split;
+	if (!flags_h && cutoff > 0.0f) {
+		split = row_split(b->pt, b->boxes_h[0], rc, cutoff);
+		if (!(split < 0.8f * cutoff)) split = 0.0f;
+	}
+	if (b->grid_rc != rc || b->split != split) {
+		b->split = split;
 		choose_grids(b, rc);
 		flags_h = nullptr;
 	}
@@ -624,6 +720,7 @@ void batch_build(mb2_batch* b, const float4* pos, const int* type_ids, float rc,
 		MB2_LAUNCH batch_cell_ranges_kernel<<<(n + 255) / 256, 256, 0, st>>>(
 			b->keys.ptr, n, b->grids.ptr, b->cell_begin.ptr, b->cell_end.ptr);
 	b->row_len.ensure(n);
+	b->row_far.ensure(n);
 	b->stats.ensure(2);
 	auto walk = [&](uint32_t cap, const uint32_t* fl) {
 		MB2_CUDA(cudaMemsetAsync(b->stats.ptr, 0, 2 * sizeof(unsigned long long), st));
@@ -632,7 +729,7 @@ void batch_build(mb2_batch* b, const float4* pos, const int* type_ids, float rc,
 			MB2_LAUNCH batch_group_kernel<<<(n + 255) / 256, 256, 0, st>>>(
 				b->sorted_pos.ptr, b->keys.ptr, b->s2o.ptr, b->cell_begin.ptr, b->cell_end.ptr,
 				b->grids.ptr, b->boxes.ptr, b->stencil.ptr, fl, n, b->nbr.ptr, cap, hshift,
-				b->row_len.ptr);
+				b->row_len.ptr, b->row_far.ptr);
 			MB2_LAUNCH batch_row_stats_kernel<<<std::min<uint32_t>((n + 255) / 256, 1184), 256, 0,
 												 st>>>(b->row_len.ptr, n, b->stats.ptr);
 		}
@@ -658,8 +755,11 @@ void batch_build(mb2_batch* b, const float4* pos, const int* type_ids, float rc,
 		b->lanes = 4;
 		const auto counted = walk(0u, nullptr);
 		const double mean = n ? static_cast<double>(counted.first) / n : 0.0;
+		// Split rows count as their near part.
+		const double f = b->split > 0.0f ? b->split / rc : 1.0;
+		const double read = mean * f * f * f;
 		b->lanes = b->lanes_request ? b->lanes_request
-									: (mean >= 256.0 ? 16 : (mean >= 48.0 ? 8 : 4));
+									: (read >= 256.0 ? 16 : (read >= 48.0 ? 8 : 4));
 		size_list(counted.second);
 	}
 	ensure_list();
@@ -670,15 +770,22 @@ void batch_build(mb2_batch* b, const float4* pos, const int* type_ids, float rc,
 		size_list(stats.second);
 		ensure_list();
 		if (dflags) {
-			batch_build(b, pos, type_ids, rc, st, nullptr);
+			batch_build(b, pos, type_ids, rc, cutoff, st, nullptr);
 			return;
 		}
 		stats = walk(b->cap, nullptr);
 	}
+	if (n && b->split > 0.0f) {
+		const int hshift = __builtin_ctz(32 / b->lanes);
+		const uint32_t slices = (n + (1u << hshift) - 1u) >> hshift;
+		MB2_LAUNCH batch_join_far_kernel<<<(slices + 7) / 8, 256, 0, st>>>(
+			b->nbr.ptr, b->row_len.ptr, b->row_far.ptr, b->keys.ptr, dflags, n, b->cap, hshift);
+	}
 	b->ref_pos.ensure(n);
+	b->moved.ensure(b->num_systems);
 	if (n)
-		MB2_LAUNCH batch_snapshot_kernel<<<(n + 255) / 256, 256, 0, st>>>(pos, b->sys_of.ptr, dflags,
-																		  n, b->ref_pos.ptr);
+		MB2_LAUNCH batch_snapshot_kernel<<<(n + 255) / 256, 256, 0, st>>>(
+			pos, b->sys_of.ptr, b->offsets_d.ptr, dflags, n, b->ref_pos.ptr, b->moved.ptr);
 	b->num_pairs = stats.first;
 	b->built = true;
 	b->system_rebuilds += rebuilt;
@@ -716,12 +823,14 @@ void step_body(mb2_batch* b, float4* pos, float4* fe, const int* type_ids,
 			   const mb2_step_params* prm, cudaStream_t st) {
 	const uint32_t n = b->n;
 	if (n == 0) return;
-	pack_sorted_positions(pos, type_ids, b->s2o.ptr, n, b->sorted_pos.ptr, st);
-	MB2_CUDA(cudaMemsetAsync(b->force_sorted.ptr, 0, static_cast<size_t>(n) * sizeof(float4), st));
+	launch_chained(batch_pack_kernel, (n + 255) / 256, 256u, 0, st, pos, type_ids, b->s2o.ptr,
+				   b->keys.ptr, b->boxes.ptr, b->ref_pos.ptr, n, b->sorted_pos.ptr,
+				   b->force_sorted.ptr, b->split > 0.0f ? b->moved.ptr : nullptr);
 	const float cutoff_sq = prm->cutoff > 0.0f ? prm->cutoff * prm->cutoff : 0.0f;
 	pair_forces_systems(b->sorted_pos.ptr, b->nbr.ptr, b->row_len.ptr, n, b->cap, b->lanes, b->pt,
 						b->boxes.ptr, b->keys.ptr, kSysShift, true, cutoff_sq, 0,
-						b->force_sorted.ptr, b->energy.ptr, st);
+						b->force_sorted.ptr, b->energy.ptr, st, b->moved.ptr, b->row_far.ptr, b->split,
+						b->longest_edge);
 	bd_integrate_systems(pos, fe, b->force_sorted.ptr, b->inv.ptr, type_ids, b->sys_of.ptr,
 						 b->offsets_d.ptr, b->boxes.ptr, n, b->types, prm->dt, prm->kT, prm->seed,
 						 prm->patch_id, b->step_d.ptr, st);
@@ -752,7 +861,7 @@ void maybe_rebuild(mb2_batch* b, const float4* pos, const int* type_ids, uint64_
 	const bool at_period = period == 0 || (step - 1) % period == 0;
 	const float skin = prm->pairlist_cutoff - prm->cutoff;
 	if (!b->built || (at_period && (period == 0 || skin <= 0.0f))) {
-		batch_build(b, pos, type_ids, prm->pairlist_cutoff, st);
+		batch_build(b, pos, type_ids, prm->pairlist_cutoff, prm->cutoff, st);
 		++b->rebuilds;
 	} else if (at_period) {
 		batch_sys_disp(b, pos, st);
@@ -765,7 +874,7 @@ void maybe_rebuild(mb2_batch* b, const float4* pos, const int* type_ids, uint64_
 			due += r ? 1u : 0u;
 		}
 		if (due) {
-			batch_build(b, pos, type_ids, prm->pairlist_cutoff, st,
+			batch_build(b, pos, type_ids, prm->pairlist_cutoff, prm->cutoff, st,
 						due == b->num_systems ? nullptr : b->pinned_sys);
 			++b->rebuilds;
 		}
@@ -816,7 +925,8 @@ int mb2_batch_create(int device, uint32_t num_systems, const uint32_t* counts,
 				bx.size[a] = l;
 				bx.inv[a] = 1.0f / l;
 				bx.half[a] = 0.5f * l;
-				bx.periodic[a] = 1;
+					bx.periodic[a] = 1;
+				b->longest_edge = std::max(b->longest_edge, l);
 			}
 			for (uint32_t i = b->offsets[s]; i < b->offsets[s + 1]; ++i) sys_of[i] = s;
 		}
@@ -930,7 +1040,7 @@ int mb2_batch_build(mb2_batch* b, const float* pos4, const int* type_ids, float 
 					void* stream, uint64_t* num_pairs) {
 	return bguard(b, [&] {
 		expect_arg(b->n == 0 || (pos4 && type_ids), MB2_ERR_ARG, "mb2_batch_build: null argument");
-		batch_build(b, reinterpret_cast<const float4*>(pos4), type_ids, pairlist_cutoff,
+		batch_build(b, reinterpret_cast<const float4*>(pos4), type_ids, pairlist_cutoff, 0.0f,
 					S(stream));
 		if (num_pairs) *num_pairs = b->num_pairs;
 	});
@@ -983,6 +1093,8 @@ int mb2_batch_run(mb2_batch* b, float* pos4, float* force_energy4, const int* ty
 				reinterpret_cast<uint64_t>(pos), reinterpret_cast<uint64_t>(fe),
 				reinterpret_cast<uint64_t>(type_ids), reinterpret_cast<uint64_t>(b->nbr.ptr),
 				reinterpret_cast<uint64_t>(b->force_sorted.ptr), b->cap,
+				reinterpret_cast<uint64_t>(b->row_far.ptr), reinterpret_cast<uint64_t>(b->moved.ptr),
+				reinterpret_cast<uint64_t>(b->ref_pos.ptr), f2u(b->split),
 				static_cast<uint64_t>(b->lanes), b->n, f2u(prm->cutoff), f2u(prm->dt),
 				f2u(prm->kT), prm->seed, prm->patch_id,
 				// tables and types (pointers, sizes, the uniform-table constants)
@@ -1088,9 +1200,9 @@ int mb2_batch_autotune(mb2_batch* b, const float* pos4, const int* type_ids,
 				reset_tuning(b, levels[li], lanes_c[gi]);
 				MB2_CUDA(cudaMemcpyAsync(tpos.ptr, pos4, static_cast<size_t>(n) * 16,
 										 cudaMemcpyDeviceToDevice, st));
-				batch_build(b, tpos.ptr, type_ids, prm->pairlist_cutoff, st);  // sizes the list
+				batch_build(b, tpos.ptr, type_ids, prm->pairlist_cutoff, prm->cutoff, st);  // sizes the list
 				MB2_CUDA(cudaEventRecord(e0, st));
-				batch_build(b, tpos.ptr, type_ids, prm->pairlist_cutoff, st);
+				batch_build(b, tpos.ptr, type_ids, prm->pairlist_cutoff, prm->cutoff, st);
 				MB2_CUDA(cudaEventRecord(e1, st));
 				b->force_sorted.ensure(n);
 				step_counter_set(b->step_d.ptr, 1, st);
@@ -1123,13 +1235,13 @@ int mb2_batch_autotune(mb2_batch* b, const float* pos4, const int* type_ids,
 								 cudaMemcpyDeviceToDevice, st));
 		b->force_sorted.ensure(n);
 		step_counter_set(b->step_d.ptr, 1, st);
-		batch_build(b, tpos.ptr, type_ids, prm->pairlist_cutoff, st);
+		batch_build(b, tpos.ptr, type_ids, prm->pairlist_cutoff, prm->cutoff, st);
 		for (uint32_t k = 0; k < period; ++k) step_body(b, tpos.ptr, tfe.ptr, type_ids, prm, st);
 		const float skin = prm->pairlist_cutoff - prm->cutoff;
 		uint32_t cadence = period;
 		float disp_at_period = 0.0f;
 		for (int rep = 0; rep < 2; ++rep) {
-			batch_build(b, tpos.ptr, type_ids, prm->pairlist_cutoff, st);
+			batch_build(b, tpos.ptr, type_ids, prm->pairlist_cutoff, prm->cutoff, st);
 			bool exceeded = false;
 			for (uint32_t k = 1; k <= period; ++k) {
 				step_body(b, tpos.ptr, tfe.ptr, type_ids, prm, st);

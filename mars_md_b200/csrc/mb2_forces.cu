@@ -1214,12 +1214,14 @@ void pair_forces_systems(const float4* sorted_pos, const uint32_t* nbr, const ui
 						 uint32_t n, uint32_t cap, int lanes_per_row, const PairTables& t,
 						 const Box* boxes, const uint32_t* sorted_keys, int sys_shift,
 						 bool all_periodic, float cutoff_sq, int get_energy, float4* force_sorted,
-						 double* ev, cudaStream_t st) {
+						 double* ev, cudaStream_t st, const unsigned int* moved,
+						 const uint32_t* row_far, float split, float longest_edge) {
 	if (n == 0) return;
 	const bool fast = all_periodic && fast_ok(t, cutoff_sq, get_energy);
-	const FastArgs fa = fast ? fast_args(t, cutoff_sq, get_energy) : FastArgs{};
+	FastArgs fa = fast ? fast_args(t, cutoff_sq, get_energy) : FastArgs{};
+	if (fast && moved) set_far(fa, row_far, split, longest_edge);
 	launch_pair_lanes(sorted_pos, nbr, row_len, n, cap, lanes_per_row, t, fast ? &fa : nullptr,
-					  SystemBoxes{boxes, sorted_keys, sys_shift, nullptr}, all_periodic, cutoff_sq,
+					  SystemBoxes{boxes, sorted_keys, sys_shift, moved}, all_periodic, cutoff_sq,
 					  get_energy, force_sorted, ev, st);
 }
 

@@ -297,12 +297,14 @@ struct FastTableBufs {
 	void set(const std::vector<PairTableRef>& refs, const std::vector<float>& bf,
 			 const std::vector<float2>& be, PairTables& t);
 };
-// Batched replicas: row i's box is boxes[sorted_keys[i] >> sys_shift].
+// Batched replicas: row i's box is boxes[sorted_keys[i] >> sys_shift]; moved,
+// row_far and split as d2max, row_far and split above, moved per system.
 void pair_forces_systems(const float4* sorted_pos, const uint32_t* nbr, const uint32_t* row_len,
 						 uint32_t n, uint32_t cap, int lanes_per_row, const PairTables& t,
 						 const Box* boxes, const uint32_t* sorted_keys, int sys_shift,
 						 bool all_periodic, float cutoff_sq, int get_energy, float4* force_sorted,
-						 double* ev, cudaStream_t st);
+						 double* ev, cudaStream_t st, const unsigned int* moved,
+						 const uint32_t* row_far, float split, float longest_edge);
 void scatter_add_forces(const float4* force_sorted, const uint32_t* s2o, uint32_t n,
 						float4* force_energy, int get_energy, cudaStream_t st);
 // Exhaustive device check of sqrt_rn_nr against __fsqrt_rn on [2^-60,

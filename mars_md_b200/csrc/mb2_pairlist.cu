@@ -417,38 +417,16 @@ __global__ void __launch_bounds__(256) build_rows_kernel(
 	}
 }
 
-// Moves each row's far entries (stored backwards from the end of its cap
-// slots) to follow its near entries, so that a row is one contiguous run:
-// near entries in candidate order, then the far ones. One warp per slice of
-// H rows: lane l copies entries l / H, l / H + 32 / H, ... of row l % H, so
-// each load and store instruction touches neighbouring words. Destinations
-// precede sources (near + far <= cap) and every batch is loaded before it is
-// stored, so the in-place copy is safe.
+// After a storing walk: each slice's far entries joined to its near ones.
 __global__ void __launch_bounds__(256) join_far_kernel(uint32_t* __restrict__ nbr,
 													   const uint32_t* __restrict__ row_len,
 													   const uint32_t* __restrict__ row_far,
 													   uint32_t n, uint32_t cap, int hshift) {
 	const uint32_t slice = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-	const uint32_t lane = threadIdx.x & 31u;
-	const uint32_t h = 1u << hshift;
-	const uint32_t slices = (n + h - 1u) >> hshift;
+	const uint32_t slices = (n + (1u << hshift) - 1u) >> hshift;
 	if (slice >= slices) return;  // whole warp
-	const uint32_t r = lane & (h - 1u), kk = lane >> hshift, step = 32u >> hshift;
-	const uint32_t i = (slice << hshift) + r;
-	const uint32_t far = i < n ? row_far[i] : 0u;
-	const uint32_t near = i < n ? row_len[i] - far : 0u;
-	uint32_t most = far;
-#pragma unroll
-	for (int o = 16; o > 0; o >>= 1) most = max(most, __shfl_xor_sync(0xFFFFFFFFu, most, o));
-	uint32_t* base = nbr + static_cast<size_t>(slice) * cap * h + r;
-	for (uint32_t k0 = 0; k0 < most; k0 += step) {
-		const uint32_t k = k0 + kk;
-		uint32_t v = 0u;
-		if (k < far) v = base[static_cast<size_t>(cap - far + k) * h];
-		__syncwarp();
-		if (k < far) base[static_cast<size_t>(near + k) * h] = v;
-		__syncwarp();
-	}
+	const uint32_t i = (slice << hshift) + (threadIdx.x & ((1u << hshift) - 1u));
+	join_far_slice(nbr, i < n ? row_len[i] : 0u, i < n ? row_far[i] : 0u, slice, cap, hshift);
 }
 
 // DisplacementKernel::min_image (AdaptiveKernels.h:56-65). Both inputs are

@@ -98,6 +98,33 @@ struct RowWriter {
 	__device__ __forceinline__ uint32_t total() const { return len + far; }
 };
 
+// Moves a slice's far entries (stored backwards from the end of each row's cap
+// slots) to follow its near entries, so that a row is one contiguous run: near
+// entries in candidate order, then the far ones. One warp per slice of H rows;
+// len, far: of row (lane mod H). Lane l copies entries l / H, l / H + 32 / H,
+// ... of that row, so each load and store instruction touches neighbouring
+// words. Destinations precede sources (near + far <= cap) and every batch is
+// loaded before it is stored, so the in-place copy is safe.
+__device__ __forceinline__ void join_far_slice(uint32_t* __restrict__ nbr, uint32_t len, uint32_t far,
+											   uint32_t slice, uint32_t cap, int hshift) {
+	const uint32_t lane = threadIdx.x & 31u;
+	const uint32_t h = 1u << hshift;
+	const uint32_t r = lane & (h - 1u), kk = lane >> hshift, step = 32u >> hshift;
+	const uint32_t near = len - far;
+	uint32_t most = far;
+#pragma unroll
+	for (int o = 16; o > 0; o >>= 1) most = max(most, __shfl_xor_sync(0xFFFFFFFFu, most, o));
+	uint32_t* base = nbr + static_cast<size_t>(slice) * cap * h + r;
+	for (uint32_t k0 = 0; k0 < most; k0 += step) {
+		const uint32_t k = k0 + kk;
+		uint32_t v = 0u;
+		if (k < far) v = base[static_cast<size_t>(cap - far + k) * h];
+		__syncwarp();
+		if (k < far) base[static_cast<size_t>(near + k) * h] = v;
+		__syncwarp();
+	}
+}
+
 // The walk of a coherent group (its particles' cells within emax of each
 // other on every axis): candidate cells are the group's cell box widened by
 // the stencil radius (or every cell on an axis the stencil spans); the lanes
