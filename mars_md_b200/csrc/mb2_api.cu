@@ -267,7 +267,7 @@ void morton_domain(mb2_context* ctx, const float4* pos, uint32_t n, cudaStream_t
 
 void sort_particles(mb2_context* ctx, const float4* pos, const int* type_ids, uint32_t n,
 					const float* bmin, const float* bmax, cudaStream_t st,
-					unsigned long long* nonfinite = nullptr) {
+					unsigned long long* odd) {
 	ctx->keys.ensure(n);
 	ctx->s2o.ensure(n);
 	ctx->inv.ensure(n);
@@ -275,7 +275,7 @@ void sort_particles(mb2_context* ctx, const float4* pos, const int* type_ids, ui
 	morton_encode(pos, n, bmin, bmax, ctx->keys.ptr, ctx->s2o.ptr, st);
 	radix_sort_pairs(ctx->scratch, ctx->keys.ptr, ctx->s2o.ptr, n, st);
 	inverse_and_gather(ctx->s2o.ptr, n, pos, ctx->inv.ptr, nullptr, st);
-	pack_sorted_positions(pos, type_ids, ctx->s2o.ptr, n, ctx->sorted_pos.ptr, st, nonfinite);
+	pack_sorted_positions(pos, type_ids, ctx->s2o.ptr, n, ctx->sorted_pos.ptr, st, odd, &ctx->box);
 }
 
 // cutoff: the interaction cutoff the list will serve. When it lies in
@@ -297,7 +297,7 @@ void build(mb2_context* ctx, const float4* pos, const int* type_ids, uint32_t n,
 	// stats: [0] pairs, [1] longest row (both set by each walk), [2] particles
 	// with a non-finite coordinate (counted while packing, read with the
 	// walk's statistics, so no extra synchronisation), [3] set by a sort that
-	// gave up waiting.
+	// gave up waiting, [4] set when a particle lies far outside the box.
 	ctx->stats.ensure(kBuildStats);
 	MB2_CUDA(cudaMemsetAsync(ctx->stats.ptr + 2, 0, (kBuildStats - 2) * sizeof(unsigned long long), st));
 	ctx->scratch.sort_error = reinterpret_cast<uint32_t*>(ctx->stats.ptr + 3);
@@ -306,10 +306,11 @@ void build(mb2_context* ctx, const float4* pos, const int* type_ids, uint32_t n,
 	const float rc2 = rc_list * rc_list;
 	if (!ctx->grid_valid || ctx->grid_rc != rc_list || ctx->grid_n != n ||
 		std::memcmp(ctx->grid_extent, extent, sizeof(extent)) != 0) {
-		ctx->grid = choose_cell_grid(extent, ctx->box.periodic, std::sqrt(rc2), n);
+		ctx->grid = choose_cell_grid(extent, ctx->box.periodic, std::sqrt(rc2), n, walk_rows(n));
 		if (ctx->level_offset != 0) {
 			const int m = std::min(8, std::max(0, ctx->grid.m + ctx->level_offset));
-			ctx->grid = choose_cell_grid(extent, ctx->box.periodic, std::sqrt(rc2), n, m, m);
+			ctx->grid =
+				choose_cell_grid(extent, ctx->box.periodic, std::sqrt(rc2), n, walk_rows(n), m, m);
 		}
 		ctx->stencil.ensure(ctx->grid.stencil.size());
 		MB2_CUDA(cudaMemcpyAsync(ctx->stencil.ptr, ctx->grid.stencil.data(),
@@ -329,35 +330,29 @@ void build(mb2_context* ctx, const float4* pos, const int* type_ids, uint32_t n,
 	WalkGrid wg{};
 	wg.m = g.m;
 	wg.shift = g.shift;
-	wg.emax = 3;
-	for (int a = 0; a < 3; ++a) {
-		wg.radius[a] = g.radius[a];
-		wg.wmin[a] = g.wmin[a];
-		wg.full[a] = ctx->box.periodic[a] && g.m > 0 && (2 * g.radius[a] + 1 >= (1 << g.m));
-		if (g.m == 0) wg.full[a] = ctx->box.periodic[a];
-	}
-	wg.lim = g.lim;
 	wg.rc2 = rc2;
 	const float split = row_split(ctx->pt, ctx->box, rc_list, cutoff);
 	wg.split2 = split > 0.0f ? split * split : INFINITY;
+	// Coordinates the walk's cheap distances round: the box, or on an open axis
+	// the particles' extent.
+	Box around = ctx->box;
 	for (int a = 0; a < 3; ++a) {
-		// Morton coordinate q = trunc((x - bmin) / range * 1023) on 0..1023, a cell
-		// of level m spanning 2^(10-m) of them; the margin covers the rounding of
-		// that mapping (a few ulp of the coordinates) with room to spare.
-		const double range = std::max(static_cast<double>(bmax[a]) - bmin[a], 1e-6);
-		wg.dom_lo[a] = bmin[a];
-		wg.cell_w[a] = static_cast<float>(std::ldexp(1.0, 10 - g.m) * range / 1023.0);
-		wg.eps[a] = static_cast<float>(1e-5 * (std::fabs(static_cast<double>(bmin[a])) + range) + 1e-6);
+		if (!around.periodic[a]) {
+			around.origin[a] = bmin[a];
+			around.size[a] = extent[a];
+		}
+		wg.eps[a] = static_cast<float>(
+			1e-6 * (std::fabs(static_cast<double>(around.origin[a])) + around.size[a]) + 1e-6);
 	}
-	fast_test_band(ctx->box, rc_list, &wg.fast_lo, &wg.fast_hi);
+	fast_test_band(around, rc_list, &wg.fast_lo, &wg.fast_hi);
 	ctx->row_len.ensure(n);
 	ctx->row_far.ensure(n);
 	auto walk = [&](uint32_t cap) {
 		const int hshift = __builtin_ctz(32 / ctx->lanes);
 		build_walk(ctx->sorted_pos.ptr, ctx->keys.ptr, ctx->s2o.ptr, ctx->cell_begin.ptr,
 				   ctx->cell_end.ptr, ctx->stencil.ptr, g.num_stencil, wg, n, ctx->box, ctx->excl,
-				   ctx->nbr.ptr, cap, hshift, ctx->row_len.ptr, ctx->row_far.ptr, ctx->stats.ptr,
-				   st);
+				   ctx->nbr.ptr, cap, hshift, ctx->row_len.ptr, ctx->row_far.ptr, ctx->stats.ptr + 4,
+				   ctx->stats.ptr, st);
 		MB2_CUDA(cudaMemcpyAsync(ctx->pinned, ctx->stats.ptr, 4 * sizeof(uint64_t),
 								 cudaMemcpyDeviceToHost, st));
 		MB2_CUDA(cudaStreamSynchronize(st));
@@ -370,8 +365,8 @@ void build(mb2_context* ctx, const float4* pos, const int* type_ids, uint32_t n,
 					" particle(s) with a NaN or infinite coordinate");
 		return std::make_pair(ctx->pinned[0], ctx->pinned[1]);
 	};
-	// Lanes per row of the force kernels. A system small enough for the row
-	// walk leaves most of the GPU idle, so its rows get more lanes (more
+	// Lanes per row of the force kernels. A small system leaves most of the
+	// GPU idle, so its rows get more lanes (more
 	// threads, shorter per-lane chains): 16 lanes measured 5-9 % faster per
 	// step than 8 or 4 at 4,096 (21.3 against 23.3 us), 32,768 (54.9 / 58.5)
 	// and 65,536 beads (polymers, 52.9 / 55.5); at 2,097,152 beads 8 lanes are
@@ -388,7 +383,7 @@ void build(mb2_context* ctx, const float4* pos, const int* type_ids, uint32_t n,
 			const double f = split / rc_list;
 			return mean * f * f * f >= 8.0 ? 8 : 4;
 		}
-		if (n <= kRowWalkMaxN) return mean >= 16.0 ? 16 : 8;
+		if (n <= kSmallN) return mean >= 16.0 ? 16 : 8;
 		if (mean >= 256.0) return 16;
 		if (mean >= 48.0) return 8;
 		return 4;
@@ -428,13 +423,13 @@ void build(mb2_context* ctx, const float4* pos, const int* type_ids, uint32_t n,
 	MB2_CUDA(cudaMemcpyAsync(ctx->ref_pos.ptr, pos, static_cast<size_t>(n) * sizeof(float4),
 							 cudaMemcpyDeviceToDevice, st));
 	// and, in Z order, the origin of the displacement the packs track: where
-	// it saves the pair kernel the rows' far part, and above kRowWalkMaxN
+	// it saves the pair kernel the rows' far part, and above kSmallN
 	// particles, where the inner rows save it 2.6 % at 2,097,152 beads (on a
 	// 65,536-bead step the pack's extra read and reduction cost more for
 	// those alone, 1-2 us).
 	ctx->track_rc = 0.0f;
 	ctx->split = split;
-	if (n > kRowWalkMaxN || ends_early) {
+	if (n > kSmallN || ends_early) {
 		ctx->ref_sorted.ensure(n);
 		ctx->d2max.ensure(1);
 		MB2_CUDA(cudaMemcpyAsync(ctx->ref_sorted.ptr, ctx->sorted_pos.ptr,
@@ -498,7 +493,7 @@ void pair_forces_impl(mb2_context* ctx, const float4* pos, const int* type_ids, 
 					  uint32_t n, float cutoff, int get_energy, cudaStream_t st) {
 	require(ctx->built, MB2_ERR_STATE, "mb2_pair_forces: no pairlist; call mb2_build_pairlist");
 	if (n == 0) return;
-	pack_sorted_positions(pos, type_ids, ctx->s2o.ptr, n, ctx->sorted_pos.ptr, st, nullptr,
+	pack_sorted_positions(pos, type_ids, ctx->s2o.ptr, n, ctx->sorted_pos.ptr, st, nullptr, nullptr,
 						  sorted_forces(ctx, n), nullptr, track_of(ctx));
 	pair_kernel(ctx, n, cutoff, get_energy, st, true);
 	scatter_add_forces(ctx->force_sorted.ptr, ctx->s2o.ptr, n, fe, get_energy, st);
@@ -607,7 +602,7 @@ bool step_has_bonded(const mb2_step_params* prm) {
 void window_step(mb2_context* ctx, float4* pos, float4* fe, const int* type_ids, uint32_t n,
 				 uint64_t step, const mb2_step_params* prm, cudaStream_t st) {
 	const bool bonded = prm->num_bonds != 0 || prm->num_angles != 0;
-	pack_sorted_positions(pos, type_ids, ctx->s2o.ptr, n, ctx->sorted_pos.ptr, st, nullptr,
+	pack_sorted_positions(pos, type_ids, ctx->s2o.ptr, n, ctx->sorted_pos.ptr, st, nullptr, nullptr,
 						  sorted_forces(ctx, n), bonded ? fe : nullptr, track_of(ctx));
 	pair_kernel(ctx, n, prm->cutoff, 0, st, true);
 	if (bonded)
@@ -1242,7 +1237,7 @@ void step_once(mb2_context* ctx, float4* pos, float4* fe, const int* type_ids,
 	} else if (n) {
 		// The pack also clears the pair-force accumulator and, when bonded
 		// terms run, ForceEnergy.
-		pack_sorted_positions(pos, type_ids, ctx->s2o.ptr, n, ctx->sorted_pos.ptr, st, nullptr,
+		pack_sorted_positions(pos, type_ids, ctx->s2o.ptr, n, ctx->sorted_pos.ptr, st, nullptr, nullptr,
 							  sorted_forces(ctx, n), bonded ? fe : nullptr, track_of(ctx));
 	}
 	if (n == 0) return;
@@ -1272,7 +1267,7 @@ void step_body_replayable(mb2_context* ctx, float4* pos, float4* fe, const int* 
 						  const uint32_t* flags, uint32_t n, const mb2_step_params* prm,
 						  uint64_t offset, cudaStream_t st) {
 	const bool bonded = step_has_bonded(prm);
-	pack_sorted_positions(pos, type_ids, ctx->s2o.ptr, n, ctx->sorted_pos.ptr, st, nullptr,
+	pack_sorted_positions(pos, type_ids, ctx->s2o.ptr, n, ctx->sorted_pos.ptr, st, nullptr, nullptr,
 						  sorted_forces(ctx, n), bonded ? fe : nullptr, track_of(ctx));
 	pair_kernel(ctx, n, prm->cutoff, prm->get_energy, st, true);
 	bonded_stage(ctx, pos, fe, prm, prm->get_energy, st);

@@ -7,8 +7,8 @@
 // radix sort groups the systems and orders each one spatially; cells of
 // system s are the top 3 m_s bits of its 21-bit code, stored after the cells
 // of systems < s. The pairlist is one sliced-ELL half list over all sorted
-// particles (a row's neighbours are always in its own system), walked one
-// warp per row over the row's own system grid, box and stencil.
+// particles (a row's neighbours are always in its own system), walked over
+// the rows' own system grid, box and stencil.
 // Pair forces read each row's box from the system table; the integrator
 // gathers the pair force through the inverse permutation and keys its noise
 // exactly as a plain step of system s with seed (seed + s) would: Philox key
@@ -52,8 +52,14 @@ __device__ __forceinline__ uint32_t morton7(float x, float o, float scale) {
 	return static_cast<uint32_t>(min(max(q, 0), (1 << kLocalBits) - 1));
 }
 
-// Morton key of one particle in its own system's box.
-__device__ __forceinline__ uint32_t batch_key(const float4& p, const Box& b, uint32_t s) {
+// Morton key of one particle in its own system's box; *outside is set when the
+// particle lies more than half a box outside it.
+__device__ __forceinline__ uint32_t batch_key(const float4& p, const Box& b, uint32_t s,
+											  uint32_t* outside) {
+	const float c[3] = {p.x, p.y, p.z};
+#pragma unroll
+	for (int a = 0; a < 3; ++a)
+		if (c[a] < b.origin[a] - b.half[a] || c[a] > b.origin[a] + b.size[a] + b.half[a]) *outside = 1u;
 	const float k = static_cast<float>(1 << kLocalBits);
 	const uint32_t x = morton7(p.x, b.origin[0], __fmul_rn(k, b.inv[0]));
 	const uint32_t y = morton7(p.y, b.origin[1], __fmul_rn(k, b.inv[1]));
@@ -65,11 +71,12 @@ __global__ void __launch_bounds__(256) batch_encode_kernel(const float4* __restr
 														   const uint32_t* __restrict__ sys_of,
 														   const Box* __restrict__ boxes,
 														   uint32_t n, uint32_t* __restrict__ keys,
-														   uint32_t* __restrict__ idx) {
+														   uint32_t* __restrict__ idx,
+														   uint32_t* outside) {
 	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
 	if (i >= n) return;
 	const uint32_t s = sys_of[i];
-	keys[i] = batch_key(pos[i], boxes[s], s);
+	keys[i] = batch_key(pos[i], boxes[s], s, outside);
 	idx[i] = i;
 }
 
@@ -80,13 +87,13 @@ __global__ void __launch_bounds__(256) batch_compact_kernel(
 	const float4* __restrict__ pos, const uint32_t* __restrict__ sys_of,
 	const Box* __restrict__ boxes, const uint32_t* __restrict__ offsets,
 	const uint32_t* __restrict__ flags, const uint32_t* __restrict__ cstart, uint32_t n,
-	uint32_t* __restrict__ ckeys, uint32_t* __restrict__ cidx) {
+	uint32_t* __restrict__ ckeys, uint32_t* __restrict__ cidx, uint32_t* outside) {
 	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
 	if (i >= n) return;
 	const uint32_t s = sys_of[i];
 	if (!flags[s]) return;
 	const uint32_t c = cstart[s] + (i - offsets[s]);
-	ckeys[c] = batch_key(pos[i], boxes[s], s);
+	ckeys[c] = batch_key(pos[i], boxes[s], s, outside);
 	cidx[c] = i;
 }
 
@@ -231,197 +238,45 @@ __global__ void __launch_bounds__(256) batch_cell_ranges_kernel(const uint32_t* 
 	if (i + 1 == n || cell(keys[i + 1]) != c) end[c] = i + 1;
 }
 
-// One warp per particle row, the plain path's row walk (build_rows_kernel)
-// with the row's own system: its cell grid, its box (periodic on every axis)
-// and its pruned stencil. The lanes take the stencil's cells 32 at a time
-// (cells whose Morton code precedes the particle's hold only earlier
-// particles of the system and are skipped), lay their candidate ranges end to
-// end by a warp scan, and test 32 consecutive candidates a round with the
-// reference's exact test, each lane finding its candidate's cell by a binary
-// search over the running totals held one per lane. Hits are appended with
-// two ballots, near entries from the front of the row, far ones from the back. Six resident blocks per SM (40 registers): 1 % faster per
-// build than 48 registers at five, and than 32 at eight.
-__device__ __forceinline__ uint32_t batch_row(
-	uint32_t i, uint32_t lane, const float4* __restrict__ sorted_pos,
-	const uint32_t* __restrict__ keys, const uint32_t* __restrict__ s2o,
-	const uint32_t* __restrict__ begin, const uint32_t* __restrict__ end,
-	const SysGrid* __restrict__ grids, const Box* __restrict__ boxes,
-	const uint4* __restrict__ stencil, uint32_t* __restrict__ nbr, uint32_t cap, int hshift,
-	uint32_t& far) {
-	const uint32_t lt = (1u << lane) - 1u;
-	const uint32_t key = keys[i];
-	const uint32_t sys = key >> kSysShift;
-	const SysGrid* g = grids + sys;
-	const int m = g->wg.m;
-	const uint32_t c = (key & kLocalMask) >> g->wg.shift;
-	const float rc2 = g->wg.rc2, split2 = g->wg.split2;
-	const uint32_t cell_base = g->cell_base;
-	const uint4* st = stencil + g->stencil_off;
-	const int ns = static_cast<int>(g->stencil_n);
-	const Box* bx = boxes + sys;
-	const float lx = bx->size[0], ly = bx->size[1], lz = bx->size[2];
-	const float ix = bx->inv[0], iy = bx->inv[1], iz = bx->inv[2];
-	const float hx = bx->half[0], hy = bx->half[1], hz = bx->half[2];
-	// Interleaved (Morton) cell codes: x bits at 3k + 2, y at 3k + 1, z at 3k.
-	// A neighbour's code is the home code plus the stencil offset on each axis
-	// in interleaved form, carried through the other axes' bits (set to one)
-	// and masked, which wraps every axis modulo 2^m.
-	const uint32_t lvl = (1u << (3 * m)) - 1u;
-	const uint32_t mx = 0x24924924u & lvl, my = 0x12492492u & lvl, mz = 0x09249249u & lvl;
-	const uint32_t cxo = c | ~mx, cyo = c | ~my, czo = c | ~mz;
-	const float4 pi = sorted_pos[i];
-	const int a = static_cast<int>(s2o[i]);
-	const uint32_t h = 1u << hshift;
-	uint32_t* base = nbr + (static_cast<size_t>(i >> hshift) * cap << hshift) + (i & (h - 1u));
-	uint32_t len = 0;
-	far = 0;
-	for (int k0 = 0; k0 < ns; k0 += 32) {
-		uint32_t jb = 0, je = 0;
-		const int k = k0 + static_cast<int>(lane);
-		if (k < ns) {
-			const uint4 se = st[k];  // interleaved offsets, modulo 2^m per axis
-			const uint32_t nc = ((cxo + se.x) & mx) | ((cyo + se.y) & my) | ((czo + se.z) & mz);
-			if (nc >= c) {
-				const uint32_t b = begin[cell_base + nc];
-				jb = b > i + 1u ? b : i + 1u;
-				je = end[cell_base + nc];
-			}
-		}
-		// The chunk's candidate ranges laid end to end (a scan of their
-		// lengths); each round the lanes take the next 32 candidates, lane l
-		// finding the cell that holds candidate t0 + l by a binary search over
-		// the lanes' running totals. An empty cell (begin = end = 0) or one
-		// ending at i has jb >= je.
-		const uint32_t cnt = je > jb ? je - jb : 0u;
-		uint32_t incl = cnt;
-#pragma unroll
-		for (int o = 1; o < 32; o <<= 1) {
-			const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-			if (static_cast<int>(lane) >= o) incl += v;
-		}
-		const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
-		const uint32_t excl = incl - cnt;
-		for (uint32_t t0 = 0; t0 < total; t0 += 32u) {
-			const uint32_t t = t0 + lane;
-			int owner = 0;  // first lane whose running total exceeds t
-#pragma unroll
-			for (int step = 16; step > 0; step >>= 1) {
-				const uint32_t v = __shfl_sync(0xFFFFFFFFu, incl, owner + step - 1);
-				if (v <= t) owner += step;
-			}
-			const uint32_t ob = __shfl_sync(0xFFFFFFFFu, jb, owner & 31);
-			const uint32_t oe = __shfl_sync(0xFFFFFFFFu, excl, owner & 31);
-			bool hit = false, near = false;
-			uint32_t entry = 0;
-			if (t < total) {
-				const uint32_t j = ob + (t - oe);
-				const float4 pj = sorted_pos[j];
-				const float dx = wrap_diff_scalar(__fsub_rn(pj.x, pi.x), lx, ix, hx);
-				const float dy = wrap_diff_scalar(__fsub_rn(pj.y, pi.y), ly, iy, hy);
-				const float dz = wrap_diff_scalar(__fsub_rn(pj.z, pi.z), lz, iz, hz);
-				const float d2 = len2(dx, dy, dz);
-				if (d2 <= rc2) {
-					hit = true;
-					near = d2 <= split2;
-					entry = j | (static_cast<int>(s2o[j]) < a ? kOrientBit : 0u);
-				}
-			}
-			const uint32_t nm = __ballot_sync(0xFFFFFFFFu, hit && near);
-			const uint32_t fm = __ballot_sync(0xFFFFFFFFu, hit && !near);
-			if (hit) {
-				const uint32_t p = len + far + static_cast<uint32_t>(__popc((nm | fm) & lt));
-				const uint32_t slot = near ? len + static_cast<uint32_t>(__popc(nm & lt))
-										   : cap - 1u - (far + static_cast<uint32_t>(__popc(fm & lt)));
-				if (p < cap) base[static_cast<size_t>(slot) * h] = entry;
-			}
-			len += static_cast<uint32_t>(__popc(nm));
-			far += static_cast<uint32_t>(__popc(fm));
-		}
-	}
-	return len + far;
-}
-
-// One warp per group of 32 consecutive sorted particles: a group whose
-// particles all belong to one system and sit in cells within emax of each
-// other walks as the plain group walk does (walk_coherent_group, over the
-// system's grid and box: candidate cells pruned by their real distance from
-// the group's coordinate range, candidates dropped 32 at a time by the group
-// test, each survivor loaded once for all 32 lanes and decided by the cheap
-// test, the exact test behind a warp vote). Any other group (at a system's
-// start or end, or across a Morton discontinuity) walks its rows one at a
-// time with the row walk. Same pair set; rows in candidate order.
-__global__ void __launch_bounds__(256, 7) batch_group_kernel(
-	const float4* __restrict__ sorted_pos, const uint32_t* __restrict__ keys,
-	const uint32_t* __restrict__ s2o, const uint32_t* __restrict__ begin,
-	const uint32_t* __restrict__ end, const SysGrid* __restrict__ grids,
-	const Box* __restrict__ boxes, const uint4* __restrict__ stencil,
-	const uint32_t* __restrict__ flags, uint32_t n, uint32_t* __restrict__ nbr, uint32_t cap,
-	int hshift, uint32_t* __restrict__ row_len, uint32_t* __restrict__ row_far) {
-	__shared__ uint32_t split_tab[1 << kLocalBits];
-	__shared__ uint4 cell_buf[8 * kCellBuf];  // per warp: kept cells (jlo, end, image code, offset)
-	__shared__ float4 cand_buf[8 * 32];       // per warp: candidates that pass the group test
-	for (int k = threadIdx.x; k < (1 << kLocalBits); k += blockDim.x) split_tab[k] = split_by3(k);
-	__syncthreads();
-	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-	const uint32_t i_first = i & ~31u;
-	if (i_first >= n) return;  // whole warp past the end
-	const uint32_t lane = threadIdx.x & 31u;
-	const bool valid = i < n;
-	const uint32_t key = valid ? keys[i] : 0u;
-	const uint32_t sys = key >> kSysShift;
-	const uint32_t sys0 = __shfl_sync(0xFFFFFFFFu, sys, 0);
-	const bool one_system = __all_sync(0xFFFFFFFFu, !valid || sys == sys0);
-	// Only the rows of systems being rebuilt (flags null: all) are walked;
-	// the others keep their rows.
-	const bool walked = valid && (!flags || flags[sys]);
+// The walk, as the plain path's (walk_run), each run with its own system's
+// grid, box and stencil: a warp's rows are walked in runs of one system and
+// cell. Only the rows of systems being rebuilt (flags null: all) are walked;
+// the others keep their rows.
+__global__ void __launch_bounds__(256) batch_walk_kernel(
+	const uint32_t* __restrict__ keys, WalkArrays w, const SysGrid* __restrict__ grids,
+	const Box* __restrict__ boxes, const uint32_t* __restrict__ flags, uint32_t n,
+	const uint32_t* __restrict__ outside) {
+	__shared__ WalkShared shared[8];
+	const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+	const uint32_t i0 = (blockIdx.x * 8u + warp) * kWalkRows;
+	if (i0 >= n) return;
+	const uint32_t rows = min(kWalkRows, n - i0);
+	const uint32_t key = keys[i0 + min(lane, rows - 1u)];
+	const bool walked = !flags || flags[key >> kSysShift];
 	if (!__any_sync(0xFFFFFFFFu, walked)) return;
-	const SysGrid* g = grids + sys0;
-	const WalkGrid& wg = g->wg;
-	const uint32_t c = (key & kLocalMask) >> wg.shift;
-	const int cx = static_cast<int>(compact_by3(c >> 2));
-	const int cy = static_cast<int>(compact_by3(c >> 1));
-	const int cz = static_cast<int>(compact_by3(c));
-	const int x0 = warp_min(valid ? cx : INT_MAX), x1 = warp_max(valid ? cx : INT_MIN);
-	const int y0 = warp_min(valid ? cy : INT_MAX), y1 = warp_max(valid ? cy : INT_MIN);
-	const int z0 = warp_min(valid ? cz : INT_MAX), z1 = warp_max(valid ? cz : INT_MIN);
-	const bool coherent = one_system && (x1 - x0) <= wg.emax && (y1 - y0) <= wg.emax &&
-						  (z1 - z0) <= wg.emax;
-	uint32_t len = 0, far = 0;
-	if (coherent) {
-		const float4 pi = valid ? sorted_pos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-		const int a = valid ? static_cast<int>(s2o[i]) : 0;
-		const float gxlo = warp_minf(valid ? pi.x : INFINITY), gxhi = warp_maxf(valid ? pi.x : -INFINITY);
-		const float gylo = warp_minf(valid ? pi.y : INFINITY), gyhi = warp_maxf(valid ? pi.y : -INFINITY);
-		const float gzlo = warp_minf(valid ? pi.z : INFINITY), gzhi = warp_maxf(valid ? pi.z : -INFINITY);
-		const int h = 1 << hshift;
-		RowWriter row{nbr + (static_cast<size_t>(i >> hshift) * cap << hshift) + (i & (h - 1)), 0u,
-					  0u, cap, h};
-		const uint32_t c_first = __shfl_sync(0xFFFFFFFFu, c, 0);
-		walk_coherent_group<false, true>(sorted_pos, s2o, begin + g->cell_base, end + g->cell_base,
-										 split_tab, cell_buf,
-										 cand_buf, wg, boxes[sys0], Exclusions{}, i, i_first,
-										 valid, pi, a, 0, 0, -1, c_first, x0, x1, y0, y1, z0, z1,
-										 gxlo, gxhi, gylo, gyhi, gzlo, gzhi, row);
-		len = row.total();
-		far = row.far;
-	} else {
-		uint32_t todo = __ballot_sync(0xFFFFFFFFu, walked);
-		while (todo) {
-			const int l = __ffs(todo) - 1;
-			todo &= todo - 1u;
-			uint32_t far_l;
-			const uint32_t len_l = batch_row(i_first + static_cast<uint32_t>(l), lane, sorted_pos,
-											 keys, s2o, begin, end, grids, boxes, stencil, nbr,
-											 cap, hshift, far_l);
-			if (static_cast<int>(lane) == l) {
-				len = len_l;
-				far = far_l;
-			}
+	const bool exact_all = *outside != 0u;
+	const uint32_t cell = key >> grids[key >> kSysShift].wg.shift;  // system and cell
+	const StencilEntry* stencils = w.stencil;
+	const uint32_t *begins = w.begin, *ends = w.end;
+	for (uint32_t r = 0; r < rows;) {
+		const uint32_t c = __shfl_sync(0xFFFFFFFFu, cell, r);
+		const uint32_t sys = __shfl_sync(0xFFFFFFFFu, key, r) >> kSysShift;
+		const uint32_t same = __ballot_sync(0xFFFFFFFFu, (key >> kSysShift) == sys && cell == c &&
+														   lane >= r && lane < rows);
+		const uint32_t run = static_cast<uint32_t>(__popc(same));
+		if (!flags || flags[sys]) {
+			const SysGrid* g = grids + sys;
+			const WalkGrid wg = g->wg;
+			w.begin = begins + g->cell_base;
+			w.end = ends + g->cell_base;
+			w.stencil = stencils + g->stencil_off;
+			w.ns = static_cast<int>(g->stencil_n);
+			uint32_t t, l;
+			walk_run<false>(w, wg, boxes[sys], Exclusions{}, shared[warp], i0 + r, i0 + r + run,
+							c & ((1u << (3 * wg.m)) - 1u), exact_all, &t, &l);
+			__syncwarp();
 		}
-	}
-	if (walked) {
-		row_len[i] = len;
-		row_far[i] = far;
+		r += run;
 	}
 }
 
@@ -496,7 +351,8 @@ struct mb2_batch {
 	DevBuf<float4> sorted_pos, ref_pos, force_sorted;
 	DevBuf<SysGrid> grids;
 	std::vector<SysGrid> grids_h;
-	DevBuf<uint4> stencil;  // every system's pruned cell stencil (interleaved offsets), concatenated
+	DevBuf<StencilEntry> stencil;  // every system's pruned cell stencil, concatenated
+	DevBuf<uint32_t> outside;      // set by a build that meets a particle far outside its box
 	uint32_t total_cells = 0;
 	float grid_rc = -1.0f;
 	int level_offset = 0;
@@ -579,56 +435,34 @@ uint64_t f2u(float f) {
 // the 7-bit Morton scale) shifted by the tuner's level offset.
 void choose_grids(mb2_batch* b, float rc) {
 	b->grids_h.resize(b->num_systems);
-	std::vector<uint4> stencil;
+	std::vector<StencilEntry> stencil;
 	uint32_t base = 0;
 	for (uint32_t s = 0; s < b->num_systems; ++s) {
 		const Box& bx = b->boxes_h[s];
 		const uint32_t ns = b->offsets[s + 1] - b->offsets[s];
-		const CellGrid g0 = choose_cell_grid(bx.size, bx.periodic, rc, ns, 0, kMaxLevel);
+		const CellGrid g0 = choose_cell_grid(bx.size, bx.periodic, rc, ns, kWalkRows, 0, kMaxLevel);
 		const int m = std::min(std::max(g0.m + b->level_offset, 0), kMaxLevel);
-		const CellGrid g = (m == g0.m) ? g0 : choose_cell_grid(bx.size, bx.periodic, rc, ns, m, m);
+		const CellGrid g = (m == g0.m) ? g0 : choose_cell_grid(bx.size, bx.periodic, rc, ns, kWalkRows, m, m);
 		SysGrid sg{};
 		WalkGrid& wg = sg.wg;
 		wg.m = g.m;
 		wg.shift = 3 * (kLocalBits - g.m);
-		// Groups whose cells spread up to 5 apart walk together (coherent);
-		// the rest walk row by row: 5.27 ms per build against 5.33 at 3 and
-		// 5.75 at 7 (wider candidate boxes).
-		wg.emax = 5;
-		for (int a = 0; a < 3; ++a) {
-			wg.radius[a] = g.radius[a];
-			wg.wmin[a] = g.wmin[a];
-			wg.full[a] = g.m == 0 || 2 * g.radius[a] + 1 >= (1 << g.m);
-		}
-		wg.lim = g.lim;
 		wg.rc2 = rc * rc;
 		fast_test_band(bx, rc, &wg.fast_lo, &wg.fast_hi);
 		wg.split2 = b->split > 0.0f ? b->split * b->split : INFINITY;
-		// Cell c of level m spans Morton coordinates [c, c + 1) * 2^(7 - m) of
-		// the 7-bit scale over the box, L / 2^m wide; the margin covers the
-		// rounding of that mapping, as on the plain path.
-		for (int a = 0; a < 3; ++a) {
-			wg.dom_lo[a] = bx.origin[a];
-			wg.cell_w[a] = static_cast<float>(static_cast<double>(bx.size[a]) / (1 << g.m));
+		for (int a = 0; a < 3; ++a)
 			wg.eps[a] = static_cast<float>(
-				1e-5 * (std::fabs(static_cast<double>(bx.origin[a])) + bx.size[a]) + 1e-6);
-		}
+				1e-6 * (std::fabs(static_cast<double>(bx.origin[a])) + bx.size[a]) + 1e-6);
 		sg.cell_base = base;
 		sg.stencil_off = static_cast<uint32_t>(stencil.size());
 		sg.stencil_n = static_cast<uint32_t>(g.stencil.size());
-		// Offsets modulo 2^m per axis (every batched box is periodic), interleaved
-		// into Morton bit positions.
-		const int cells = 1 << g.m;
-		for (const StencilEntry& e : g.stencil) {
-			auto d = [cells](int v) { return split_by3(static_cast<uint32_t>((v % cells + cells) % cells)); };
-			stencil.push_back(make_uint4(d(e.dx) << 2, d(e.dy) << 1, d(e.dz), 0u));
-		}
+		stencil.insert(stencil.end(), g.stencil.begin(), g.stencil.end());
 		base += 1u << (3 * g.m);
 		b->grids_h[s] = sg;
 	}
 	b->stencil.ensure(std::max<size_t>(stencil.size(), 1));
 	if (!stencil.empty())
-		MB2_CUDA(cudaMemcpy(b->stencil.ptr, stencil.data(), stencil.size() * sizeof(uint4),
+		MB2_CUDA(cudaMemcpy(b->stencil.ptr, stencil.data(), stencil.size() * sizeof(StencilEntry),
 							cudaMemcpyHostToDevice));
 	b->total_cells = base;
 	b->grids.ensure(b->num_systems);
@@ -674,6 +508,8 @@ void batch_build(mb2_batch* b, const float4* pos, const int* type_ids, float rc,
 	b->s2o.ensure(n);
 	b->inv.ensure(n);
 	b->sorted_pos.ensure(n);
+	b->outside.ensure(1);
+	MB2_CUDA(cudaMemsetAsync(b->outside.ptr, 0, sizeof(uint32_t), st));
 	if (flags_h) {
 		// Only the rebuilt systems' particles are sorted: the others keep their
 		// sorted slots (keys and order of their own last build).
@@ -698,7 +534,7 @@ void batch_build(mb2_batch* b, const float4* pos, const int* type_ids, float rc,
 		b->cidx.ensure(std::max<uint32_t>(m, 1));
 		MB2_LAUNCH batch_compact_kernel<<<(n + 255) / 256, 256, 0, st>>>(
 			pos, b->sys_of.ptr, b->boxes.ptr, b->offsets_d.ptr, dflags, b->cstart.ptr, n,
-			b->ckeys.ptr, b->cidx.ptr);
+			b->ckeys.ptr, b->cidx.ptr, b->outside.ptr);
 		if (m) radix_sort_pairs(b->scratch, b->ckeys.ptr, b->cidx.ptr, m, st);
 		if (m)
 			MB2_LAUNCH batch_scatter_sorted_kernel<<<(m + 255) / 256, 256, 0, st>>>(
@@ -707,7 +543,7 @@ void batch_build(mb2_batch* b, const float4* pos, const int* type_ids, float rc,
 	} else {
 		if (n)
 			MB2_LAUNCH batch_encode_kernel<<<(n + 255) / 256, 256, 0, st>>>(
-				pos, b->sys_of.ptr, b->boxes.ptr, n, b->keys.ptr, b->s2o.ptr);
+				pos, b->sys_of.ptr, b->boxes.ptr, n, b->keys.ptr, b->s2o.ptr, b->outside.ptr);
 		radix_sort_pairs(b->scratch, b->keys.ptr, b->s2o.ptr, n, st);
 	}
 	inverse_and_gather(b->s2o.ptr, n, pos, b->inv.ptr, nullptr, st);
@@ -726,10 +562,11 @@ void batch_build(mb2_batch* b, const float4* pos, const int* type_ids, float rc,
 		MB2_CUDA(cudaMemsetAsync(b->stats.ptr, 0, 2 * sizeof(unsigned long long), st));
 		if (n) {
 			const int hshift = __builtin_ctz(32 / b->lanes);
-			MB2_LAUNCH batch_group_kernel<<<(n + 255) / 256, 256, 0, st>>>(
-				b->sorted_pos.ptr, b->keys.ptr, b->s2o.ptr, b->cell_begin.ptr, b->cell_end.ptr,
-				b->grids.ptr, b->boxes.ptr, b->stencil.ptr, fl, n, b->nbr.ptr, cap, hshift,
-				b->row_len.ptr, b->row_far.ptr);
+			const WalkArrays w{b->sorted_pos.ptr, b->s2o.ptr, b->cell_begin.ptr, b->cell_end.ptr,
+							   b->stencil.ptr,    0,          b->nbr.ptr,        cap,
+							   hshift,            b->row_len.ptr, b->row_far.ptr};
+			MB2_LAUNCH batch_walk_kernel<<<(n + 8 * kWalkRows - 1) / (8 * kWalkRows), 256, 0, st>>>(
+				b->keys.ptr, w, b->grids.ptr, b->boxes.ptr, fl, n, b->outside.ptr);
 			MB2_LAUNCH batch_row_stats_kernel<<<std::min<uint32_t>((n + 255) / 256, 1184), 256, 0,
 												 st>>>(b->row_len.ptr, n, b->stats.ptr);
 		}

@@ -144,46 +144,41 @@ struct CellGrid {
 	int shift = 30;            // 3 * (10 - m)
 	int num_stencil = 0;
 	std::vector<StencilEntry> stencil;  // one cell's pruned stencil
-	int radius[3] = {0, 0, 0};          // stencil half-width in cells per axis
-	float wmin[3] = {0, 0, 0};          // narrowest cell width per axis
-	float lim = 0.0f;                   // pruning bound on the squared cell gap
 };
-// Up to this many particles the pairlist is walked one warp per particle
-// (build_rows_kernel) instead of one warp per 32 (build_walk_kernel).
-// Measured per build, group walk against row walk: 65,536-bead polymers 0.75
-// vs 0.30 ms; uniform beads at 0.002 A^-3, 32,768: 0.43 vs 0.34 ms (the group
-// walk's best at that size); 131,072: 1.06 vs 0.75 ms; 262,144: 1.36 vs
-// 1.48 ms; 524,288: 1.74 vs 2.30 ms; 2,097,152: 5.45 vs 10.6 ms.
-constexpr uint32_t kRowWalkMaxN = 131072;
+// Up to this many particles a system is small: its rows get more lanes in the
+// pair kernels, and no displacement is tracked for the inner rows alone.
+constexpr uint32_t kSmallN = 131072;
+// Rows a warp walks when a list is built (at most kWalkRows): as many as share
+// the finding of candidates well, fewer where the GPU would be left short of
+// warps.
+inline uint32_t walk_rows(uint32_t n) {
+	return n >= 65536u ? 8u : (n >= 32768u ? 4u : (n >= 12288u ? 2u : 1u));
+}
 
-// Parameters of the group walk (passed by value to the kernel).
+// Parameters of the walk (passed by value to the kernel).
 struct WalkGrid {
-	int m, shift, emax;
-	int full[3];               // periodic axis whose stencil spans every cell
-	int radius[3];
-	float wmin[3];
-	float lim;
+	int m, shift;
 	float rc2;                 // pairlist cutoff squared, as the reference rounds it
 	float fast_lo, fast_hi;    // d^2 band that needs the exact test
 	float split2;              // entries with d^2 above it go to the row's far segment
-	// Real-space extent of cell c on each axis: [lo + c w - eps, lo + (c+1) w + eps)
-	// (Morton domain origin, cell width, rounding margin of the Morton mapping).
-	float dom_lo[3], cell_w[3], eps[3];
+	float eps[3];              // rounding margin of a coordinate box
 };
-// Cell level m in [m_lo, m_hi] minimising candidates plus per-cell cost; the
+// Cell level m in [m_lo, m_hi] minimising the walk's cost at `rows` rows a warp; the
 // widths assume the 10-bit Morton scale (conservative for coarser scales).
 CellGrid choose_cell_grid(const float* extent, const int* periodic, float rc_list, size_t n,
-						  int m_lo = 0, int m_hi = 8);
+						  double rows, int m_lo = 0, int m_hi = 8);
 void fast_test_band(const Box& box, float rc_list, float* fast_lo, float* fast_hi);
 void cell_ranges(const uint32_t* keys, uint32_t n, int shift, uint32_t* begin, uint32_t* end,
 				 size_t num_cells, cudaStream_t st);
-// One walk over all groups: rows appended to the sliced-ELL list (entries past
+// One walk over all rows: rows appended to the sliced-ELL list (entries past
 // `cap` are counted, not stored); stats[0] += pairs, stats[1] = max row length.
+// *outside != 0: a particle lies far outside the box (see pack).
 void build_walk(const float4* sorted_pos, const uint32_t* keys, const uint32_t* s2o,
 				const uint32_t* begin, const uint32_t* end, const StencilEntry* stencil,
 				int num_stencil, const WalkGrid& wg, uint32_t n, const Box& box,
 				const Exclusions& ex, uint32_t* nbr, uint32_t cap, int hshift, uint32_t* row_len,
-				uint32_t* row_far, unsigned long long* stats, cudaStream_t st);
+				uint32_t* row_far, const unsigned long long* outside, unsigned long long* stats,
+				cudaStream_t st);
 // After a storing walk: each row's far entries moved to follow its near ones.
 void join_far(uint32_t* nbr, const uint32_t* row_len, const uint32_t* row_far, uint32_t n,
 			  uint32_t cap, int hshift, cudaStream_t st);
@@ -208,14 +203,15 @@ struct DisplacementTrack {
 };
 DisplacementTrack displacement_track(const Box& box, const float4* ref_sorted,
 									 unsigned int* d2max);
-// nonfinite (optional): incremented once per particle with a NaN or infinite
-// coordinate.
+// odd (optional, with box): odd[0] incremented once per particle with a NaN or
+// infinite coordinate, odd[2] set when one lies more than half a box outside a
+// periodic axis.
 // clear_a / clear_b (may be null): float4[n] arrays zeroed by the same launch.
 // track (optional): raises track.d2max to this step's largest displacement.
 void pack_sorted_positions(const float4* pos, const int* type_ids, const uint32_t* s2o,
 						   uint32_t n, float4* sorted_pos, cudaStream_t st,
-						   unsigned long long* nonfinite = nullptr, float4* clear_a = nullptr,
-						   float4* clear_b = nullptr,
+						   unsigned long long* odd = nullptr, const Box* box = nullptr,
+						   float4* clear_a = nullptr, float4* clear_b = nullptr,
 						   const DisplacementTrack& track = DisplacementTrack{});
 
 // forces.cu

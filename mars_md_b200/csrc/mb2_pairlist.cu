@@ -46,7 +46,7 @@ double ulp_of(double x) {
 }  // namespace
 
 CellGrid choose_cell_grid(const float* extent, const int* periodic, float rc_list, size_t n,
-						  int m_lo, int m_hi) {
+						  double rows, int m_lo, int m_hi) {
 	CellGrid best;
 	double best_cost = -1.0;
 	const double rc = static_cast<double>(rc_list);
@@ -56,7 +56,6 @@ CellGrid choose_cell_grid(const float* extent, const int* periodic, float rc_lis
 		if (m > m_lo && num_cells > 2.0 * static_cast<double>(n)) break;
 		std::vector<int> off[3];
 		std::vector<double> gap[3];
-		int radius[3] = {0, 0, 0};
 		double wmin[3] = {0, 0, 0};
 		for (int a = 0; a < 3; ++a) {
 			if (m == 0) {
@@ -72,7 +71,6 @@ CellGrid choose_cell_grid(const float* extent, const int* periodic, float rc_lis
 			wmin[a] = static_cast<double>(extent[a]) * (std::ldexp(1.0, k) - 1.0) / 1023.0 *
 					  (1.0 - 1e-6);
 			const int r = static_cast<int>(std::floor(rc / wmin[a])) + 1;
-			radius[a] = r;
 			if (periodic[a] && 2 * r + 1 >= cells) {
 				for (int d = 0; d < cells; ++d) {
 					off[a].push_back(d);
@@ -106,18 +104,20 @@ CellGrid choose_cell_grid(const float* extent, const int* periodic, float rc_lis
 					}
 				}
 		const double per_cell = static_cast<double>(n) / num_cells;
-		const double cost = static_cast<double>(st.size()) * (per_cell + 2.0);
+		// What the walk spends on a row: finding the stencil's cells (some 3 warp
+		// instructions each) and loading and placing their candidates (2.4 each, of
+		// the half that follow the rows), shared by the rows of a run; a run is
+		// what a warp's rows have in one cell. (The tests against the rows
+		// themselves hardly depend on the level.) Against counting cells and
+		// candidates alone: 131,071 beads 411 -> 333 us.
+		const double run = std::max(1.0, rows / (1.0 + (rows - 1.0) / std::max(per_cell, 1e-6)));
+		const double cost = static_cast<double>(st.size()) * (3.0 + 1.2 * per_cell) / run;
 		if (best_cost < 0.0 || cost < best_cost) {
 			best_cost = cost;
 			best.m = m;
 			best.shift = 3 * (10 - m);
 			best.num_stencil = static_cast<int>(st.size());
 			best.stencil = st;
-			for (int a = 0; a < 3; ++a) {
-				best.radius[a] = radius[a];
-				best.wmin[a] = static_cast<float>(wmin[a]);
-			}
-			best.lim = static_cast<float>(lim);
 		}
 	}
 	return best;
@@ -152,118 +152,53 @@ __global__ void __launch_bounds__(256) cell_ranges_kernel(const uint32_t* __rest
 }
 
 
-// One warp owns a group of 32 consecutive sorted particles, lane = particle.
-// The group's cells are Morton-adjacent; the warp walks, in lockstep, every
-// cell whose real extent lies within rc of the group's coordinate range (found
-// by the lanes in parallel over the group's cell box widened by the stencil
-// radius), loading each candidate once for all 32 lanes (a broadcast). Cells before the group's first cell in
-// Morton order hold only earlier particles and are skipped without loading
-// their ranges. A group whose cells straddle a Morton discontinuity (wide
-// bounding box) walks each particle's own pruned stencil instead. Each row
-// keeps candidate order (runs of consecutive sorted j), which keeps the force
-// kernel's gathers local.
-// Seven resident blocks per SM (32 registers, a little spill): the walk is
-// bound by instruction issue and the latency of its dependent loads (cell
-// ranges, then candidates), and more warps hide the latency. Measured on the
-// 2,097,152-bead workload when the budget was set: 7.1 ms per build at 7
-// blocks, 7.7 at 6 (40 registers), 7.9 at 5 (48 registers); with the group
-// test and the voted exact test, 6.0 ms at 7 blocks and 6.05 at 6.
-// kFull: some periodic axis is spanned whole by the group's candidate cells
-// (small boxes); without it the candidate test needs no minimum-image wrap.
-template <bool kExcl, bool kFull>
-__global__ void __launch_bounds__(256, 7) build_walk_kernel(
-	const float4* __restrict__ sorted_pos, const uint32_t* __restrict__ keys,
-	const uint32_t* __restrict__ s2o, const uint32_t* __restrict__ begin,
-	const uint32_t* __restrict__ end, const StencilEntry* __restrict__ stencil_g, int ns,
-	WalkGrid wg, uint32_t n, Box box, Exclusions ex, uint32_t* __restrict__ nbr, uint32_t cap,
-	int hshift, uint32_t* __restrict__ row_len, uint32_t* __restrict__ row_far,
+// The walk: each warp owns rows_per_warp consecutive sorted particles and walks
+// them in runs of one cell (walk_run). Bound by issuing the tests: at 8 rows a
+// warp about a quarter of the warp instructions a row of the two walks before
+// it (one warp per particle, which found and loaded every candidate anew for
+// each row; one lane per particle, which ran the appends of 32 rows one
+// candidate at a time). Statistics are added once per block.
+template <bool kExcl>
+__global__ void __launch_bounds__(256) build_walk_kernel(
+	const uint32_t* __restrict__ keys, WalkArrays w, WalkGrid wg, uint32_t n, Box box,
+	Exclusions ex, uint32_t rows_per_warp, const unsigned long long* __restrict__ outside,
 	unsigned long long* __restrict__ stats) {
-	__shared__ uint32_t split_tab[256];
-	__shared__ uint4 cell_buf[8 * kCellBuf];  // per warp: kept cells (jlo, end, image code, offset)
-	__shared__ float4 cand_buf[8 * 32];       // per warp: candidates that pass the group test
-	const int cells = 1 << wg.m;
-	for (int k = threadIdx.x; k < cells; k += blockDim.x) split_tab[k] = split_by3(k);
+	__shared__ WalkShared shared[8];
+	__shared__ uint32_t part[2][8];
+	const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+	const uint32_t i0 = (blockIdx.x * 8u + warp) * rows_per_warp;
+	uint32_t total = 0, longest = 0;
+	if (i0 < n) {
+		const uint32_t rows = min(rows_per_warp, n - i0);
+		const bool exact_all = *outside != 0ull;
+		const uint32_t cell = keys[i0 + min(lane, rows - 1u)] >> wg.shift;
+		for (uint32_t r = 0; r < rows;) {
+			const uint32_t c = __shfl_sync(0xFFFFFFFFu, cell, r);
+			const uint32_t same = __ballot_sync(0xFFFFFFFFu, cell == c && lane >= r && lane < rows);
+			const uint32_t run = static_cast<uint32_t>(__popc(same));
+			uint32_t t, l;
+			walk_run<kExcl>(w, wg, box, ex, shared[warp], i0 + r, i0 + r + run, c, exact_all, &t, &l);
+			total += t;
+			longest = max(longest, l);
+			r += run;
+			__syncwarp();
+		}
+	}
+	if (lane == 0) {
+		part[0][warp] = total;
+		part[1][warp] = longest;
+	}
 	__syncthreads();
-	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-	const uint32_t i_first = i & ~31u;
-	if (i_first >= n) return;  // whole warp past the end
-	const bool valid = i < n;
-	const int h = 1 << hshift;
-	const uint32_t mask = static_cast<uint32_t>(cells - 1);
-	const float4 pi = valid ? sorted_pos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-	const uint32_t c = valid ? keys[i] >> wg.shift : 0u;
-	const int cx = static_cast<int>(compact_by3(c >> 2));
-	const int cy = static_cast<int>(compact_by3(c >> 1));
-	const int cz = static_cast<int>(compact_by3(c));
-	const int a = valid ? static_cast<int>(s2o[i]) : 0;
-	int row_b = 0, row_e = 0, body = -1;
-	if (kExcl && valid) {
-		if (ex.offsets && static_cast<uint32_t>(a) < ex.num_particles) {
-			row_b = ex.offsets[a];
-			row_e = ex.offsets[a + 1];
+	if (threadIdx.x == 0) {
+		unsigned long long sum = 0, most = 0;
+		for (int k = 0; k < 8; ++k) {
+			sum += part[0][k];
+			most = max(most, static_cast<unsigned long long>(part[1][k]));
 		}
-		body = ex.rigid_body_id ? ex.rigid_body_id[a] : -1;
-	}
-	RowWriter row{nbr + (static_cast<size_t>(i >> hshift) * cap << hshift) + (i & (h - 1)), 0u,
-				  0u, cap, h};
-	const uint32_t c_first = keys[i_first] >> wg.shift;
-
-	// Cell bounding box of the group (valid lanes only).
-	const int x0 = warp_min(valid ? cx : INT_MAX), x1 = warp_max(valid ? cx : INT_MIN);
-	const int y0 = warp_min(valid ? cy : INT_MAX), y1 = warp_max(valid ? cy : INT_MIN);
-	const int z0 = warp_min(valid ? cz : INT_MAX), z1 = warp_max(valid ? cz : INT_MIN);
-	const bool coherent = (x1 - x0) <= wg.emax && (y1 - y0) <= wg.emax && (z1 - z0) <= wg.emax;
-	// The group's coordinate range: cells are pruned by their real distance to
-	// it, which is tighter than the cell-index gap.
-	const float gxlo = warp_minf(valid ? pi.x : INFINITY), gxhi = warp_maxf(valid ? pi.x : -INFINITY);
-	const float gylo = warp_minf(valid ? pi.y : INFINITY), gyhi = warp_maxf(valid ? pi.y : -INFINITY);
-	const float gzlo = warp_minf(valid ? pi.z : INFINITY), gzhi = warp_maxf(valid ? pi.z : -INFINITY);
-
-	if (coherent) {
-		walk_coherent_group<kExcl, kFull>(sorted_pos, s2o, begin, end, split_tab, cell_buf,
-										  cand_buf, wg, box, ex, i, i_first, valid, pi, a, row_b,
-										  row_e, body, c_first, x0, x1, y0, y1, z0, z1, gxlo,
-										  gxhi, gylo, gyhi, gzlo, gzhi, row);
-	} else if (valid) {
-		// Wide group: each lane walks its own pruned cell stencil, exact test.
-		for (int k = 0; k < ns; ++k) {
-			const StencilEntry se = stencil_g[k];
-			const int4 s = make_int4(se.dx, se.dy, se.dz, 0);
-			int nx = cx + s.x, ny = cy + s.y, nz = cz + s.z;
-			if (box.periodic[0]) nx = static_cast<int>(static_cast<uint32_t>(nx + cells) & mask);
-			else if (nx < 0 || nx >= cells) continue;
-			if (box.periodic[1]) ny = static_cast<int>(static_cast<uint32_t>(ny + cells) & mask);
-			else if (ny < 0 || ny >= cells) continue;
-			if (box.periodic[2]) nz = static_cast<int>(static_cast<uint32_t>(nz + cells) & mask);
-			else if (nz < 0 || nz >= cells) continue;
-			const uint32_t nc = (split_tab[nx] << 2) | (split_tab[ny] << 1) | split_tab[nz];
-			if (nc < c) continue;  // every particle there precedes i
-			const uint32_t b = begin[nc], e = end[nc];
-			for (uint32_t j = b > i + 1u ? b : i + 1u; j < e; ++j) {
-				const float4 pj = sorted_pos[j];
-				if (exact_hit(box, pi, pj, wg.rc2)) {
-					const int bj = static_cast<int>(s2o[j]);
-					if (kExcl && is_excluded(ex, bj, row_b, row_e, body)) continue;
-					row.append(j | (bj < a ? kOrientBit : 0u));
-				}
-			}
+		if (sum) {
+			atomicAdd(stats, sum);
+			atomicMax(stats + 1, most);
 		}
-	}
-	if (valid) {
-		row_len[i] = row.total();
-		row_far[i] = row.far;
-	}
-	// stats[0] = total pairs, stats[1] = longest row
-	unsigned long long tot = valid ? row.total() : 0u;
-	int mx = valid ? static_cast<int>(min(row.total(), 0x7FFFFFFFu)) : 0;
-#pragma unroll
-	for (int o = 16; o > 0; o >>= 1) {
-		tot += __shfl_xor_sync(0xFFFFFFFFu, tot, o);
-		mx = max(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
-	}
-	if ((threadIdx.x & 31) == 0) {
-		atomicAdd(stats, tot);
-		atomicMax(stats + 1, static_cast<unsigned long long>(mx));
 	}
 }
 
@@ -282,138 +217,6 @@ __global__ void __launch_bounds__(256) export_kernel(const uint32_t* __restrict_
 	for (uint32_t k = 0; k < len; ++k) {
 		const int b = static_cast<int>(s2o[base[static_cast<size_t>(k) * h] & ~kOrientBit]);
 		out[off + k] = make_int2(a < b ? a : b, a < b ? b : a);
-	}
-}
-
-// Small systems: one warp per particle row. The lanes take the row's pruned
-// stencil cells 32 at a time (cells whose Morton code precedes the particle's
-// hold only earlier particles and are skipped). The kept cells' candidate
-// ranges are laid end to end by a warp scan of their lengths, and every round
-// tests 32 consecutive candidates of that stream, one per lane, with the
-// reference's exact test: each lane finds the cell its candidate falls in by a
-// binary search over the running totals, held one per lane and read with warp
-// shuffles. A round's hits are appended with two ballots (near entries from
-// the front of the row, far ones from the back, as the group walk does). The
-// group walk runs one warp per 32 particles and leaves most of the GPU idle
-// below some 10^5 particles; here every particle has a warp. Rows hold the
-// same pairs in another order.
-template <bool kExcl>
-__global__ void __launch_bounds__(256) build_rows_kernel(
-	const float4* __restrict__ sorted_pos, const uint32_t* __restrict__ keys,
-	const uint32_t* __restrict__ s2o, const uint32_t* __restrict__ begin,
-	const uint32_t* __restrict__ end, const StencilEntry* __restrict__ stencil_g, int ns,
-	WalkGrid wg, uint32_t n, Box box, Exclusions ex, uint32_t* __restrict__ nbr, uint32_t cap,
-	int hshift, uint32_t* __restrict__ row_len, uint32_t* __restrict__ row_far,
-	unsigned long long* __restrict__ stats) {
-	const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-	if (i >= n) return;  // whole warp
-	const uint32_t lane = threadIdx.x & 31u;
-	const uint32_t lt = (1u << lane) - 1u;
-	const int cells = 1 << wg.m;
-	const float4 pi = sorted_pos[i];
-	const uint32_t c = keys[i] >> wg.shift;
-	const int cx = static_cast<int>(compact_by3(c >> 2));
-	const int cy = static_cast<int>(compact_by3(c >> 1));
-	const int cz = static_cast<int>(compact_by3(c));
-	// A neighbour's cell code is the home code plus the stencil entry's
-	// interleaved offset on each axis, carried through the other axes' bits
-	// (set to one) and masked: modulo 2^m per axis, so open axes also check
-	// the plain coordinate range.
-	const uint32_t lvl = (1u << (3 * wg.m)) - 1u;
-	const uint32_t mx = 0x24924924u & lvl, my = 0x12492492u & lvl, mz = 0x09249249u & lvl;
-	const uint32_t cxo = c | ~mx, cyo = c | ~my, czo = c | ~mz;
-	const int a = static_cast<int>(s2o[i]);
-	int row_b = 0, row_e = 0, body = -1;
-	if (kExcl) {
-		if (ex.offsets && static_cast<uint32_t>(a) < ex.num_particles) {
-			row_b = ex.offsets[a];
-			row_e = ex.offsets[a + 1];
-		}
-		body = ex.rigid_body_id ? ex.rigid_body_id[a] : -1;
-	}
-	const uint32_t h = 1u << hshift;
-	uint32_t* base = nbr + (static_cast<size_t>(i >> hshift) * cap << hshift) + (i & (h - 1u));
-	uint32_t len = 0, far = 0;
-	for (int k0 = 0; k0 < ns; k0 += 32) {
-		uint32_t jb = 0, je = 0;
-		const int k = k0 + static_cast<int>(lane);
-		if (k < ns) {
-			const StencilEntry se = stencil_g[k];
-			bool in = true;
-			if (!box.periodic[0]) in = in && static_cast<unsigned>(cx + se.dx) < static_cast<unsigned>(cells);
-			if (!box.periodic[1]) in = in && static_cast<unsigned>(cy + se.dy) < static_cast<unsigned>(cells);
-			if (!box.periodic[2]) in = in && static_cast<unsigned>(cz + se.dz) < static_cast<unsigned>(cells);
-			if (in) {
-				const uint32_t d = static_cast<uint32_t>(se.pad);
-				const uint32_t nc = ((cxo + (d & mx)) & mx) | ((cyo + (d & my)) & my) |
-									((czo + (d & mz)) & mz);
-				if (nc >= c) {  // earlier cells hold only earlier particles
-					const uint32_t b = begin[nc];
-					jb = b > i + 1u ? b : i + 1u;
-					je = end[nc];
-				}
-			}
-		}
-		// The batch's candidate ranges laid end to end (a scan of their
-		// lengths); each round the lanes take the next 32 candidates, lane l
-		// finding the cell that holds candidate t0 + l by a binary search over
-		// the lanes' running totals.
-		// An empty cell (begin = end = 0) or one ending at i has jb >= je.
-		const uint32_t cnt = je > jb ? je - jb : 0u;
-		uint32_t incl = cnt;
-#pragma unroll
-		for (int o = 1; o < 32; o <<= 1) {
-			const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-			if (static_cast<int>(lane) >= o) incl += v;
-		}
-		const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
-		const uint32_t excl = incl - cnt;
-		for (uint32_t t0 = 0; t0 < total; t0 += 32u) {
-			const uint32_t t = t0 + lane;
-			int owner = 0;  // first lane whose running total exceeds t
-#pragma unroll
-			for (int step = 16; step > 0; step >>= 1) {
-				const uint32_t v = __shfl_sync(0xFFFFFFFFu, incl, owner + step - 1);
-				if (v <= t) owner += step;
-			}
-			const uint32_t ob = __shfl_sync(0xFFFFFFFFu, jb, owner & 31);
-			const uint32_t oe = __shfl_sync(0xFFFFFFFFu, excl, owner & 31);
-			bool hit = false, near = false;
-			uint32_t entry = 0;
-			if (t < total) {
-				const uint32_t j = ob + (t - oe);
-				const float4 pj = sorted_pos[j];
-				const float3 d = wrap_diff(box, __fsub_rn(pj.x, pi.x), __fsub_rn(pj.y, pi.y),
-										   __fsub_rn(pj.z, pi.z));
-				const float d2 = len2(d.x, d.y, d.z);
-				if (d2 <= wg.rc2) {
-					const int bj = static_cast<int>(s2o[j]);
-					if (!(kExcl && is_excluded(ex, bj, row_b, row_e, body))) {
-						hit = true;
-						near = d2 <= wg.split2;
-						entry = j | (bj < a ? kOrientBit : 0u);
-					}
-				}
-			}
-			const uint32_t nm = __ballot_sync(0xFFFFFFFFu, hit && near);
-			const uint32_t fm = __ballot_sync(0xFFFFFFFFu, hit && !near);
-			if (hit) {
-				// Position among all of the row's entries (for the capacity check)
-				// and the slot: near entries from the front, far from the back.
-				const uint32_t p = len + far + static_cast<uint32_t>(__popc((nm | fm) & lt));
-				const uint32_t slot = near ? len + static_cast<uint32_t>(__popc(nm & lt))
-										   : cap - 1u - (far + static_cast<uint32_t>(__popc(fm & lt)));
-				if (p < cap) base[static_cast<size_t>(slot) * h] = entry;
-			}
-			len += static_cast<uint32_t>(__popc(nm));
-			far += static_cast<uint32_t>(__popc(fm));
-		}
-	}
-	if (lane == 0) {
-		row_len[i] = len + far;
-		row_far[i] = far;
-		atomicAdd(stats, static_cast<unsigned long long>(len + far));
-		atomicMax(stats + 1, static_cast<unsigned long long>(len + far));
 	}
 }
 
@@ -466,8 +269,8 @@ __global__ void __launch_bounds__(256) pack_kernel(const float4* __restrict__ po
 												   const int* __restrict__ type_ids,
 												   const uint32_t* __restrict__ s2o, uint32_t n,
 												   float4* __restrict__ sorted_pos,
-												   unsigned long long* nonfinite,
-												   float4* __restrict__ clear_a,
+												   unsigned long long* odd, float3 far_lo,
+												   float3 far_hi, float4* __restrict__ clear_a,
 												   float4* __restrict__ clear_b,
 												   DisplacementTrack track) {
 	chain_begin();
@@ -485,8 +288,12 @@ __global__ void __launch_bounds__(256) pack_kernel(const float4* __restrict__ po
 		if (clear_b) clear_b[s] = make_float4(0.f, 0.f, 0.f, 0.f);
 		const uint32_t o = s2o[s];
 		float4 p = pos[o];
-		if (nonfinite && !(isfinite(p.x) && isfinite(p.y) && isfinite(p.z)))
-			atomicAdd(nonfinite, 1ull);
+		if (odd) {
+			if (!(isfinite(p.x) && isfinite(p.y) && isfinite(p.z))) atomicAdd(odd, 1ull);
+			if (p.x < far_lo.x || p.x > far_hi.x || p.y < far_lo.y || p.y > far_hi.y ||
+				p.z < far_lo.z || p.z > far_hi.z)
+				odd[2] = 1ull;
+		}
 		if (track.d2max) {
 			const float4 r = track.ref_sorted[s];
 			d2 = len2(min_image(__fsub_rn(p.x, r.x), track.len[0]),
@@ -524,31 +331,17 @@ void build_walk(const float4* sorted_pos, const uint32_t* keys, const uint32_t* 
 				const uint32_t* begin, const uint32_t* end, const StencilEntry* stencil,
 				int num_stencil, const WalkGrid& wg, uint32_t n, const Box& box,
 				const Exclusions& ex, uint32_t* nbr, uint32_t cap, int hshift, uint32_t* row_len,
-				uint32_t* row_far, unsigned long long* stats, cudaStream_t st) {
+				uint32_t* row_far, const unsigned long long* outside, unsigned long long* stats,
+				cudaStream_t st) {
 	MB2_CUDA(cudaMemsetAsync(stats, 0, 2 * sizeof(unsigned long long), st));
 	if (n == 0) return;
 	const bool excl = ex.offsets != nullptr || ex.rigid_body_id != nullptr;
-	// The kernel variant with the minimum-image wrap is needed when a coherent
-	// group's candidate cells can span a whole periodic axis: a cell spread of
-	// up to emax plus the stencil's 2 * radius + 1 reaching the cell count.
-	bool full = false;
-	for (int a = 0; a < 3; ++a)
-		full = full || (box.periodic[a] && wg.emax + 2 * wg.radius[a] + 1 >= (1 << wg.m));
-	if (n <= kRowWalkMaxN) {
-		// One warp per particle (8 particles per 256-thread block).
-		auto rows = excl ? build_rows_kernel<true> : build_rows_kernel<false>;
-		MB2_LAUNCH rows<<<(n + 7) / 8, 256, 0, st>>>(sorted_pos, keys, s2o, begin, end, stencil,
-													 num_stencil, wg, n, box, ex, nbr, cap,
-													 hshift, row_len, row_far, stats);
-		return;
-	}
-	auto kern = excl ? (full ? build_walk_kernel<true, true> : build_walk_kernel<true, false>)
-					 : (full ? build_walk_kernel<false, true> : build_walk_kernel<false, false>);
-	// The stencil (used by the few groups that walk per particle) is read
-	// through L1, leaving shared memory to the cell buffers.
-	MB2_LAUNCH kern<<<(n + 255) / 256, 256, 0, st>>>(sorted_pos, keys, s2o, begin, end,
-														 stencil, num_stencil, wg, n, box, ex,
-														 nbr, cap, hshift, row_len, row_far, stats);
+	const WalkArrays w{sorted_pos, s2o, begin,  end,    stencil, num_stencil,
+					   nbr,        cap, hshift, row_len, row_far};
+	const uint32_t rows = walk_rows(n);
+	auto kern = excl ? build_walk_kernel<true> : build_walk_kernel<false>;
+	MB2_LAUNCH kern<<<(n + 8 * rows - 1) / (8 * rows), 256, 0, st>>>(keys, w, wg, n, box, ex, rows,
+																	 outside, stats);
 }
 
 void join_far(uint32_t* nbr, const uint32_t* row_len, const uint32_t* row_far, uint32_t n,
@@ -592,11 +385,18 @@ DisplacementTrack displacement_track(const Box& box, const float4* ref_sorted,
 
 void pack_sorted_positions(const float4* pos, const int* type_ids, const uint32_t* s2o,
 						   uint32_t n, float4* sorted_pos, cudaStream_t st,
-						   unsigned long long* nonfinite, float4* clear_a, float4* clear_b,
-						   const DisplacementTrack& track) {
+						   unsigned long long* odd, const Box* box, float4* clear_a,
+						   float4* clear_b, const DisplacementTrack& track) {
 	if (n == 0) return;
+	float lo[3] = {-INFINITY, -INFINITY, -INFINITY}, hi[3] = {INFINITY, INFINITY, INFINITY};
+	for (int a = 0; odd && a < 3; ++a) {
+		if (!box->periodic[a]) continue;
+		lo[a] = box->origin[a] - 0.5f * box->size[a];
+		hi[a] = box->origin[a] + 1.5f * box->size[a];
+	}
 	launch_chained(pack_kernel, (n + 255) / 256, 256, 0, st, pos, type_ids, s2o, n, sorted_pos,
-				   nonfinite, clear_a, clear_b, track);
+				   odd, make_float3(lo[0], lo[1], lo[2]), make_float3(hi[0], hi[1], hi[2]), clear_a,
+				   clear_b, track);
 }
 
 }  // namespace mb2

@@ -1,6 +1,6 @@
-// Device pieces of the pairlist walks shared by the plain and the batched
-// builds: the reference's exact pair test, warp reductions, the cell gap of
-// the group walk, the sliced-ELL row writer and the coherent-group walk.
+// Device pieces of the pairlist walk shared by the plain and the batched
+// builds: the reference's exact pair test, the walk of a run of rows, and the
+// join of a slice's far entries.
 #pragma once
 
 #include "mb2_internal.cuh"
@@ -25,78 +25,251 @@ __device__ __forceinline__ bool exact_hit(const Box& box, const float4& pi, cons
 	return len2(d.x, d.y, d.z) <= rc2;
 }
 
-__device__ __forceinline__ int warp_min(int v) {
-#pragma unroll
-	for (int o = 16; o > 0; o >>= 1) v = min(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
-	return v;
-}
-__device__ __forceinline__ float warp_minf(float v) {
-#pragma unroll
-	for (int o = 16; o > 0; o >>= 1) v = fminf(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
-	return v;
-}
-__device__ __forceinline__ float warp_maxf(float v) {
-#pragma unroll
-	for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
-	return v;
-}
-
-// Distance along one axis from the group's coordinate range [glo, ghi] to
-// cell nx (shifted by sh, the periodic image offset): the cell's real extent
-// with the Morton rounding margin; on a periodic axis the edge cells also hold
-// particles that lie outside the box (their Morton coordinate clamps), so
-// they extend outwards without bound.
-__device__ __forceinline__ float cell_gap(const WalkGrid& wg, int ax, int nx, int cells,
-										  bool periodic, float sh, float glo, float ghi) {
-	float lo = wg.dom_lo[ax] + static_cast<float>(nx) * wg.cell_w[ax] + sh - wg.eps[ax];
-	float hi = wg.dom_lo[ax] + static_cast<float>(nx + 1) * wg.cell_w[ax] + sh + wg.eps[ax];
-	if (periodic) {
-		if (nx == 0) lo = -INFINITY;
-		if (nx == cells - 1) hi = INFINITY;
-	}
-	return fmaxf(0.0f, fmaxf(lo - ghi, glo - hi));
-}
-
-// Cells a warp buffers before walking them (32 tested at a time: at most
-// 31 left over plus 32 new).
-constexpr uint32_t kCellBuf = 64;
-
-// Periodic image offset of a buffered cell on axis ax: code bits 2ax..2ax+1
-// hold 1 (-size) or 2 (+size).
-__device__ __forceinline__ float image_shift(uint32_t code, int ax, const Box& box) {
-	const uint32_t c = (code >> (2 * ax)) & 3u;
-	return c == 1u ? -box.size[ax] : (c == 2u ? box.size[ax] : 0.0f);
-}
-
-__device__ __forceinline__ int warp_max(int v) {
-#pragma unroll
-	for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
-	return v;
-}
-
-// Appends one lane's row of the sliced-ELL list: near entries from the front,
-// far entries (beyond the split radius) from the back of the row's cap slots;
-// join_far_kernel then moves the far ones to follow the near ones. Entries
-// past cap are only counted (the host then grows the list and walks again).
-struct RowWriter {
-	uint32_t* base;  // &nbr[entry 0 of this row]
-	uint32_t len;    // near entries
-	uint32_t far;    // far entries
-	uint32_t cap;
-	int h;           // slice height: stride between a row's entries
-	__device__ __forceinline__ void append(uint32_t entry) {
-		if (len + far < cap) base[static_cast<size_t>(len) * h] = entry;
-		++len;
-	}
-	// Near entry to the front, far entry to the back, without a branch.
-	__device__ __forceinline__ void put(uint32_t entry, bool near) {
-		const uint32_t slot = near ? len : cap - 1u - far;
-		if (len + far < cap) base[static_cast<size_t>(slot) * h] = entry;
-		len += near ? 1u : 0u;
-		far += near ? 0u : 1u;
-	}
-	__device__ __forceinline__ uint32_t total() const { return len + far; }
+// Most rows a warp walks, and the shared memory it does so in.
+constexpr uint32_t kWalkRows = 8;
+struct WalkShared {
+	float4 rows[kWalkRows];                // position, original index in .w
+	int4 excl[kWalkRows];                  // exclusion row [x, y), rigid body z
+	unsigned long long base[kWalkRows];    // index of the row's entry 0 in the list
+	float4 cand[64];                       // candidates that passed the run's test, index in .w
 };
+
+// One cell grid's arrays and the list being written.
+struct WalkArrays {
+	const float4* sorted_pos;
+	const uint32_t* s2o;
+	const uint32_t* begin;  // this grid's cells
+	const uint32_t* end;
+	const StencilEntry* stencil;
+	int ns;
+	uint32_t* nbr;
+	uint32_t cap;
+	int hshift;
+	uint32_t* row_len;
+	uint32_t* row_far;
+};
+
+// nearest image of x (a multiple of l away): x - l rint(x / l), one rounding;
+// inv = 0 (an open axis) leaves x.
+__device__ __forceinline__ float nearest(float x, float l, float inv, float* k) {
+	constexpr float kRound = 12582912.0f;  // 1.5 * 2^23: adding it rounds to nearest
+	*k = __fsub_rn(__fmaf_rn(x, inv, kRound), kRound);
+	return __fmaf_rn(*k, -l, x);
+}
+
+// The rows [rb, re) of one cell c (at most kWalkRows), walked by one warp.
+//
+// The lanes take the cell's pruned stencil 32 cells at a time (cells whose
+// Morton code precedes c hold only earlier particles and are skipped), lay
+// their candidate ranges end to end (a warp scan of the lengths) and load 32
+// candidates a round, each lane finding its candidate's cell by a binary
+// search over the running totals held one per lane and read with shuffles. A
+// candidate is moved into the image nearest the rows' coordinate box once for
+// all rows, dropped when its distance from that box is beyond the radius, and
+// otherwise queued in shared memory; each time the queue holds 32, one per
+// lane, they are tested against every row. So the cost of finding, loading
+// and moving a candidate is shared by the run's rows, the test that is left is
+// three differences and a sum of squares, and all lanes hold a candidate.
+//
+// A cheap distance decides all but candidates within rounding of the radius
+// (fast_lo < d^2 <= fast_hi), which take the reference's exact test behind a
+// warp vote, so the pair set is the reference's bit for bit. Where the image
+// nearest the box need not be the one nearest each row (a box edge below twice
+// the radius and the run's extent), each row takes its own; particles far
+// outside the box (exact_all) take the exact test throughout.
+//
+// A row's hits are appended with two ballots: near entries (within split2)
+// from the front of its slots, far ones from the back; join_far_slice then
+// moves the far ones behind the near ones. Entries past cap are only counted
+// (the host then grows the list and walks again). Returns the rows' total and
+// longest lengths in *total and *longest (the same in every lane).
+template <bool kExcl>
+__device__ __forceinline__ void walk_run(const WalkArrays& w, const WalkGrid& wg, const Box& box,
+										 const Exclusions& ex, WalkShared& sh, uint32_t rb,
+										 uint32_t re, uint32_t c, bool exact_all,
+										 uint32_t* total_out, uint32_t* longest_out) {
+	const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
+	const int nr = static_cast<int>(re - rb);
+	const int cells = 1 << wg.m;
+	const float len[3] = {box.size[0], box.size[1], box.size[2]};
+	const float inv[3] = {box.periodic[0] ? box.inv[0] : 0.0f, box.periodic[1] ? box.inv[1] : 0.0f,
+						  box.periodic[2] ? box.inv[2] : 0.0f};
+	// The rows and their coordinate box.
+	const uint32_t mine = rb + min(lane & (kWalkRows - 1u), static_cast<uint32_t>(nr - 1));
+	const float4 q = w.sorted_pos[mine];
+	const int own = static_cast<int>(w.s2o[mine]);
+	float mid[3] = {q.x, q.y, q.z}, half[3] = {q.x, q.y, q.z};
+#pragma unroll
+	for (int a = 0; a < 3; ++a) {
+		float lo = mid[a], hi = mid[a];
+#pragma unroll
+		for (uint32_t o = kWalkRows / 2; o > 0; o >>= 1) {
+			lo = fminf(lo, __shfl_xor_sync(0xFFFFFFFFu, lo, o));
+			hi = fmaxf(hi, __shfl_xor_sync(0xFFFFFFFFu, hi, o));
+		}
+		mid[a] = 0.5f * (lo + hi);
+		half[a] = 0.5f * (hi - lo) + wg.eps[a];
+	}
+	if (lane < static_cast<uint32_t>(nr)) {
+		sh.rows[lane] = make_float4(q.x, q.y, q.z, __int_as_float(own));
+		if (kExcl) {
+			int4 e = make_int4(0, 0, -1, 0);
+			if (ex.offsets && static_cast<uint32_t>(own) < ex.num_particles) {
+				e.x = ex.offsets[own];
+				e.y = ex.offsets[own + 1];
+			}
+			if (ex.rigid_body_id) e.z = ex.rigid_body_id[own];
+			sh.excl[lane] = e;
+		}
+		const uint32_t h = 1u << w.hshift;
+		sh.base[lane] = (static_cast<unsigned long long>(mine >> w.hshift) * w.cap << w.hshift) +
+						(mine & (h - 1u));
+	}
+	__syncwarp();
+	const float gate = wg.fast_hi * 1.00001f, rc = sqrtf(gate);
+	bool per_row = false;
+#pragma unroll
+	for (int a = 0; a < 3; ++a)
+		per_row = per_row || (box.periodic[a] && len[a] <= 2.0f * (rc + half[a] + wg.eps[a]));
+	uint32_t row_len = 0, row_far = 0;  // of row `lane`
+	uint32_t queued = 0;
+	const bool split = wg.split2 < INFINITY;
+
+	auto test = [&](uint32_t m) {
+		const bool there = lane < m;
+		const float4 p = sh.cand[lane];
+		const uint32_t j = __float_as_uint(p.w);
+		const int bj = there ? static_cast<int>(w.s2o[j]) : 0;
+		for (int r = 0; r < nr; ++r) {
+			const float4 row = sh.rows[r];
+			float dx = p.x - row.x, dy = p.y - row.y, dz = p.z - row.z;
+			if (per_row) {
+				float k;
+				dx = nearest(dx, len[0], inv[0], &k);
+				dy = nearest(dy, len[1], inv[1], &k);
+				dz = nearest(dz, len[2], inv[2], &k);
+			}
+			const float d2 = dx * dx + dy * dy + dz * dz;
+			const bool later = there && j > rb + static_cast<uint32_t>(r);
+			bool hit = later && d2 < wg.fast_lo && !exact_all;
+			const bool band = later && !hit && (d2 <= wg.fast_hi || exact_all);
+			if (__any_sync(0xFFFFFFFFu, band)) {
+				if (band) hit = exact_hit(box, w.sorted_pos[rb + r], w.sorted_pos[j], wg.rc2);
+			}
+			if (kExcl && hit) {
+				const int4 e = sh.excl[r];
+				hit = !is_excluded(ex, bj, e.x, e.y, e.z);
+			}
+			const bool near = !split || d2 <= wg.split2;
+			const uint32_t nm = __ballot_sync(0xFFFFFFFFu, hit && near);
+			const uint32_t fm = __ballot_sync(0xFFFFFFFFu, hit && !near);
+			if ((nm | fm) == 0u) continue;
+			const uint32_t all = __shfl_sync(0xFFFFFFFFu, row_len, r);
+			const uint32_t far = __shfl_sync(0xFFFFFFFFu, row_far, r);
+			if (hit) {
+				const uint32_t place = all + static_cast<uint32_t>(__popc((nm | fm) & lt));
+				const uint32_t slot =
+					near ? all - far + static_cast<uint32_t>(__popc(nm & lt))
+						 : w.cap - 1u - (far + static_cast<uint32_t>(__popc(fm & lt)));
+				const uint32_t flip = bj < __float_as_int(row.w) ? kOrientBit : 0u;
+				if (place < w.cap)
+					w.nbr[sh.base[r] + (static_cast<unsigned long long>(slot) << w.hshift)] = j | flip;
+			}
+			if (static_cast<int>(lane) == r) {
+				row_len += static_cast<uint32_t>(__popc(nm | fm));
+				row_far += static_cast<uint32_t>(__popc(fm));
+			}
+		}
+	};
+
+	const uint32_t lvl = (1u << (3 * wg.m)) - 1u;
+	const uint32_t mx = 0x24924924u & lvl, my = 0x12492492u & lvl, mz = 0x09249249u & lvl;
+	// A neighbour's cell code is the home code plus the stencil entry's
+	// interleaved offset on each axis, carried through the other axes' bits
+	// (set to one) and masked: modulo 2^m per axis, so open axes also check
+	// the plain coordinate range.
+	const uint32_t cxo = c | ~mx, cyo = c | ~my, czo = c | ~mz;
+	const int cx = static_cast<int>(compact_by3(c >> 2)), cy = static_cast<int>(compact_by3(c >> 1)),
+			  cz = static_cast<int>(compact_by3(c));
+	for (int k0 = 0; k0 < w.ns; k0 += 32) {
+		uint32_t jb = 0, je = 0;
+		const int k = k0 + static_cast<int>(lane);
+		if (k < w.ns) {
+			const StencilEntry se = w.stencil[k];
+			bool in = true;
+			if (!box.periodic[0]) in = in && static_cast<unsigned>(cx + se.dx) < static_cast<unsigned>(cells);
+			if (!box.periodic[1]) in = in && static_cast<unsigned>(cy + se.dy) < static_cast<unsigned>(cells);
+			if (!box.periodic[2]) in = in && static_cast<unsigned>(cz + se.dz) < static_cast<unsigned>(cells);
+			if (in) {
+				const uint32_t d = static_cast<uint32_t>(se.pad);
+				const uint32_t nc = ((cxo + (d & mx)) & mx) | ((cyo + (d & my)) & my) |
+									((czo + (d & mz)) & mz);
+				if (nc >= c) {  // earlier cells hold only earlier particles
+					const uint32_t b = w.begin[nc];
+					jb = b > rb + 1u ? b : rb + 1u;
+					je = w.end[nc];
+				}
+			}
+		}
+		// An empty cell (begin = end = 0) or one that ends at the rows has jb >= je.
+		const uint32_t cnt = je > jb ? je - jb : 0u;
+		uint32_t incl = cnt;
+#pragma unroll
+		for (int o = 1; o < 32; o <<= 1) {
+			const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+			if (static_cast<int>(lane) >= o) incl += v;
+		}
+		const uint32_t stream = __shfl_sync(0xFFFFFFFFu, incl, 31);
+		const uint32_t off = jb - (incl - cnt);  // candidate t of this cell is off + t
+		for (uint32_t t0 = 0; t0 < stream; t0 += 32u) {
+			const uint32_t t = t0 + lane;
+			int owner = 0;  // first lane whose running total exceeds t
+#pragma unroll
+			for (int step = 16; step > 0; step >>= 1) {
+				const uint32_t v = __shfl_sync(0xFFFFFFFFu, incl, owner + step - 1);
+				if (v <= t) owner += step;
+			}
+			const uint32_t j = __shfl_sync(0xFFFFFFFFu, off, owner & 31) + t;
+			bool pass = false;
+			float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
+			if (t < stream) {
+				p = w.sorted_pos[j];
+				float k0f, k1f, k2f;
+				const float dx = nearest(p.x - mid[0], len[0], inv[0], &k0f);
+				const float dy = nearest(p.y - mid[1], len[1], inv[1], &k1f);
+				const float dz = nearest(p.z - mid[2], len[2], inv[2], &k2f);
+				const float gx = fmaxf(0.0f, fabsf(dx) - half[0]);
+				const float gy = fmaxf(0.0f, fabsf(dy) - half[1]);
+				const float gz = fmaxf(0.0f, fabsf(dz) - half[2]);
+				pass = exact_all || gx * gx + gy * gy + gz * gz <= gate;
+				p.x = __fmaf_rn(k0f, -len[0], p.x);
+				p.y = __fmaf_rn(k1f, -len[1], p.y);
+				p.z = __fmaf_rn(k2f, -len[2], p.z);
+				p.w = __uint_as_float(j);
+			}
+			const uint32_t pm = __ballot_sync(0xFFFFFFFFu, pass);
+			if (pass) sh.cand[queued + static_cast<uint32_t>(__popc(pm & lt))] = p;
+			queued += static_cast<uint32_t>(__popc(pm));
+			__syncwarp();
+			if (queued >= 32u) {
+				test(32u);
+				queued -= 32u;
+				const float4 rest = sh.cand[32u + lane];
+				__syncwarp();
+				sh.cand[lane] = rest;
+				__syncwarp();
+			}
+		}
+	}
+	if (queued) test(queued);
+	__syncwarp();
+	if (lane < static_cast<uint32_t>(nr)) {
+		w.row_len[rb + lane] = row_len;
+		w.row_far[rb + lane] = row_far;
+	}
+	*total_out = __reduce_add_sync(0xFFFFFFFFu, row_len);
+	*longest_out = __reduce_max_sync(0xFFFFFFFFu, row_len);
+}
 
 // Moves a slice's far entries (stored backwards from the end of each row's cap
 // slots) to follow its near entries, so that a row is one contiguous run: near
@@ -123,172 +296,6 @@ __device__ __forceinline__ void join_far_slice(uint32_t* __restrict__ nbr, uint3
 		if (k < far) base[static_cast<size_t>(near + k) * h] = v;
 		__syncwarp();
 	}
-}
-
-// The walk of a coherent group (its particles' cells within emax of each
-// other on every axis): candidate cells are the group's cell box widened by
-// the stencil radius (or every cell on an axis the stencil spans); the lanes
-// test 32 of them at a time in parallel, each against the group's coordinate
-// range, and append the kept ones, in box order, to the warp's buffer; the
-// warp then walks the buffered cells' candidates together, each loaded once
-// for all 32 lanes. begin / end index this grid's cells; c_first is the cell
-// of the group's first particle, whose earlier cells hold only earlier
-// particles. Shared by the plain group walk and the batched one.
-template <bool kExcl, bool kFull>
-__device__ __forceinline__ void walk_coherent_group(
-	const float4* __restrict__ sorted_pos, const uint32_t* __restrict__ s2o,
-	const uint32_t* __restrict__ begin, const uint32_t* __restrict__ end,
-	const uint32_t* split_tab, uint4* cell_buf, float4* cand_buf, const WalkGrid& wg,
-	const Box& box, const Exclusions& ex, uint32_t i, uint32_t i_first, bool valid,
-	const float4& pi, int a, int row_b, int row_e, int body, uint32_t c_first, int x0, int x1,
-	int y0, int y1, int z0, int z1, float gxlo, float gxhi, float gylo, float gyhi, float gzlo,
-	float gzhi, RowWriter& row) {
-	const int cells = 1 << wg.m;
-	// Candidate cells: the group's cell box widened by the stencil radius (or
-	// every cell on an axis the stencil spans). The lanes test 32 of them at
-	// a time in parallel, each against the group's coordinate range, and
-	// append the kept ones, in box order, to the warp's buffer; the warp
-	// then walks the buffered cells' candidates together.
-	const int lo[3] = {x0, y0, z0}, hi[3] = {x1, y1, z1};
-	const float glo[3] = {gxlo, gylo, gzlo}, ghi[3] = {gxhi, gyhi, gzhi};
-	int from[3], span[3];
-	bool full[3];
-#pragma unroll
-	for (int ax = 0; ax < 3; ++ax) {
-		full[ax] = kFull && box.periodic[ax] && (hi[ax] - lo[ax] + 2 * wg.radius[ax] + 1 >= cells);
-		from[ax] = full[ax] ? 0 : lo[ax] - wg.radius[ax];
-		span[ax] = full[ax] ? cells : hi[ax] - lo[ax] + 2 * wg.radius[ax] + 1;
-	}
-	const uint32_t total = static_cast<uint32_t>(span[0] * span[1] * span[2]);
-	const int lane = static_cast<int>(threadIdx.x & 31u);
-	uint4* buf = cell_buf + (threadIdx.x >> 5) * kCellBuf;
-	uint32_t count = 0;
-	float4* cbuf = cand_buf + (threadIdx.x >> 5) * 32;
-	const uint32_t lt_mask = (1u << lane) - 1u;
-	// A candidate whose distance from the group's coordinate range (less
-	// the Morton rounding margin) is above the fast test's upper bound gives
-	// every lane d^2 > fast_hi below, so no lane keeps it; such candidates
-	// are dropped 32 at a time before the lanes test the rest one by one.
-	const float gate = wg.fast_hi;
-	auto walk_buffered = [&](uint32_t m) {
-		// Offsets of the buffered cells' candidate ranges in one stream.
-		const uint32_t l0 = static_cast<uint32_t>(lane) < m ? buf[lane].y - buf[lane].x : 0u;
-		const uint32_t l1 = static_cast<uint32_t>(lane) + 32u < m ? buf[lane + 32].y - buf[lane + 32].x : 0u;
-		uint32_t s0 = l0, s1 = l1;
-#pragma unroll
-		for (int o = 1; o < 32; o <<= 1) {
-			const uint32_t a0 = __shfl_up_sync(0xFFFFFFFFu, s0, o);
-			const uint32_t a1 = __shfl_up_sync(0xFFFFFFFFu, s1, o);
-			if (lane >= o) {
-				s0 += a0;
-				s1 += a1;
-			}
-		}
-		const uint32_t tot0 = __shfl_sync(0xFFFFFFFFu, s0, 31);
-		const uint32_t stream = tot0 + __shfl_sync(0xFFFFFFFFu, s1, 31);
-		if (static_cast<uint32_t>(lane) < m) buf[lane].w = s0 - l0;
-		if (static_cast<uint32_t>(lane) + 32u < m) buf[lane + 32].w = tot0 + s1 - l1;
-		__syncwarp();
-		uint32_t kc = 0;  // this lane's cell in the stream (advances monotonically)
-		for (uint32_t t0 = 0; t0 < stream; t0 += 32u) {
-			const uint32_t t = t0 + static_cast<uint32_t>(lane);
-			bool pass = false;
-			float4 cand = make_float4(0.f, 0.f, 0.f, 0.f);
-			if (t < stream) {
-				while (kc + 1u < m && buf[kc + 1u].w <= t) ++kc;
-				const uint4 cb = buf[kc];
-				const uint32_t j = cb.x + (t - cb.w);
-				const float4 pj = sorted_pos[j];
-				// The candidate moved into the group's image.
-				const float sx = pj.x + image_shift(cb.z, 0, box);
-				const float sy = pj.y + image_shift(cb.z, 1, box);
-				const float sz = pj.z + image_shift(cb.z, 2, box);
-				const float gx = full[0] ? 0.0f : fmaxf(0.0f, fmaxf(gxlo - sx, sx - gxhi) - wg.eps[0]);
-				const float gy = full[1] ? 0.0f : fmaxf(0.0f, fmaxf(gylo - sy, sy - gyhi) - wg.eps[1]);
-				const float gz = full[2] ? 0.0f : fmaxf(0.0f, fmaxf(gzlo - sz, sz - gzhi) - wg.eps[2]);
-				pass = gx * gx + gy * gy + gz * gz <= gate;
-				cand = make_float4(sx, sy, sz, __uint_as_float(j));
-			}
-			const uint32_t pm = __ballot_sync(0xFFFFFFFFu, pass);
-			if (pass) cbuf[__popc(pm & lt_mask)] = cand;
-			__syncwarp();
-			const int np = __popc(pm);
-			for (int q = 0; q < np; ++q) {
-				const float4 c4 = cbuf[q];
-				const uint32_t j = __float_as_uint(c4.w);
-				float dx = c4.x - pi.x, dy = c4.y - pi.y, dz = c4.z - pi.z;
-				if (kFull) {
-					if (full[0]) dx -= box.size[0] * rintf(dx * box.inv[0]);
-					if (full[1]) dy -= box.size[1] * rintf(dy * box.inv[1]);
-					if (full[2]) dz -= box.size[2] * rintf(dz * box.inv[2]);
-				}
-				const float d2 = dx * dx + dy * dy + dz * dz;
-				bool hit = valid && j > i && d2 < wg.fast_lo;
-				// The exact test for the few lanes within rounding of the radius,
-				// behind a warp vote so that the other candidates skip it.
-				const bool band = valid && j > i && !hit && d2 <= wg.fast_hi;
-				if (__any_sync(0xFFFFFFFFu, band)) {
-					if (band) hit = exact_hit(box, pi, sorted_pos[j], wg.rc2);
-				}
-				if (hit) {
-					const int bj = static_cast<int>(s2o[j]);
-					if (kExcl && is_excluded(ex, bj, row_b, row_e, body)) continue;
-					row.put(j | (bj < a ? kOrientBit : 0u), d2 <= wg.split2);
-				}
-			}
-			__syncwarp();
-		}
-	};
-	for (uint32_t base = 0; base < total; base += 32u) {
-		const uint32_t idx = base + static_cast<uint32_t>(lane);
-		bool keep = false;
-		uint4 rec = make_uint4(0u, 0u, 0u, 0u);
-		if (idx < total) {
-			const uint32_t iz = idx % static_cast<uint32_t>(span[2]);
-			const uint32_t t = idx / static_cast<uint32_t>(span[2]);
-			const int u[3] = {from[0] + static_cast<int>(t / static_cast<uint32_t>(span[1])),
-							  from[1] + static_cast<int>(t % static_cast<uint32_t>(span[1])),
-							  from[2] + static_cast<int>(iz)};
-			bool in_range = true;
-			float g2 = 0.0f;
-			uint32_t code = 0, nc = 0;
-#pragma unroll
-			for (int ax = 0; ax < 3; ++ax) {
-				int nn = u[ax];
-				float sh = 0.0f;
-				if (!full[ax]) {
-					if (box.periodic[ax]) {
-						if (nn < 0) { nn += cells; sh = -box.size[ax]; code |= 1u << (2 * ax); }
-						else if (nn >= cells) { nn -= cells; sh = box.size[ax]; code |= 2u << (2 * ax); }
-					} else if (nn < 0 || nn >= cells) {
-						in_range = false;
-						nn = 0;
-					}
-					const float g = cell_gap(wg, ax, nn, cells, box.periodic[ax], sh, glo[ax], ghi[ax]);
-					g2 += g * g;
-				}
-				nc |= split_tab[nn] << (2 - ax);
-			}
-			if (in_range && g2 <= wg.lim && nc >= c_first) {
-				const uint32_t b = begin[nc], e = end[nc];
-				const uint32_t jlo = b > i_first + 1u ? b : i_first + 1u;
-				if (jlo < e) {
-					keep = true;
-					rec = make_uint4(jlo, e, code, 0u);
-				}
-			}
-		}
-		const uint32_t kept = __ballot_sync(0xFFFFFFFFu, keep);
-		if (keep) buf[count + __popc(kept & ((1u << lane) - 1u))] = rec;
-		count += static_cast<uint32_t>(__popc(kept));
-		__syncwarp();
-		if (count >= 32u) {
-			walk_buffered(count);
-			count = 0;
-			__syncwarp();
-		}
-	}
-	walk_buffered(count);
 }
 
 }  // namespace mb2
