@@ -70,6 +70,8 @@ __global__ void __launch_bounds__(256) adj_mu_kernel(const float4* __restrict__ 
 													 float4* __restrict__ mu_sorted,
 													 double4* __restrict__ tan,
 													 double4* __restrict__ tan_sorted) {
+	chain_begin();
+	chain_wait();
 	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
 	if (i >= n) return;
 	// The tangent accumulators of this step start at zero.
@@ -100,6 +102,7 @@ __global__ void __launch_bounds__(256) adj_pair_kernel(
 	const float* __restrict__ force_g, uint32_t total_bins, Box box, float cutoff_sq,
 	double* tan_sorted, double* __restrict__ grad_bins) {
 	constexpr int H = 32 / G;
+	chain_begin();
 	extern __shared__ double sg[];
 	PairTableRef* refs = reinterpret_cast<PairTableRef*>(sg + total_bins);
 	float* bin_f = reinterpret_cast<float*>(refs + T * T);
@@ -109,6 +112,7 @@ __global__ void __launch_bounds__(256) adj_pair_kernel(
 	}
 	for (int k = threadIdx.x; k < T * T; k += blockDim.x) refs[k] = refs_g[k];
 	__syncthreads();
+	chain_wait();
 	const int sub = threadIdx.x & (G - 1);
 	const uint32_t rows_per_block = blockDim.x / G;
 	for (uint32_t row0 = blockIdx.x * rows_per_block; row0 < n; row0 += gridDim.x * rows_per_block) {
@@ -148,15 +152,18 @@ __global__ void __launch_bounds__(256) adj_pair_kernel(
 			const float ud = ux * dvx + uy * dvy + uz * dvz;
 			const float k = F / d;
 			const float gx = k * (dvx - ux * ud), gy = k * (dvy - uy * ud), gz = k * (dvz - uz * ud);
-			add_d3(tan_sorted + 4 * static_cast<size_t>(j), gx, gy, gz);
-			tx -= gx;
-			ty -= gy;
-			tz -= gz;
-			if (home < tr.last) {
-				const double gb = static_cast<double>(tr.step_inv) * ud;
-				atomicAdd(&sg[tr.offset + home], gb);
-				atomicAdd(&sg[tr.offset + home + 1], -gb);
+			// Most bins of a table that ends short of the cutoff hold no force:
+			// their pairs' tangents are zeros and add nothing (but for a NaN).
+			if (k != 0.0f || !(ud - ud == 0.0f)) {
+				add_d3(tan_sorted + 4 * static_cast<size_t>(j), gx, gy, gz);
+				tx -= gx;
+				ty -= gy;
+				tz -= gz;
 			}
+			// dF/dU[home] = step_inv and dF/dU[home + 1] = -step_inv: summed once
+			// a bin here, spread over the two table values by the flush.
+			if (home < tr.last)
+				atomicAdd(&sg[tr.offset + home], static_cast<double>(tr.step_inv) * ud);
 		}
 #pragma unroll
 		for (int o = G / 2; o > 0; o >>= 1) {
@@ -166,7 +173,11 @@ __global__ void __launch_bounds__(256) adj_pair_kernel(
 		}
 		if (valid && sub == 0 && cnt != 0u) add_d3(tan_sorted + 4 * static_cast<size_t>(i), tx, ty, tz);
 	}
-	flush_bins(sg, grad_bins, total_bins);
+	__syncthreads();
+	for (uint32_t k = threadIdx.x; k < total_bins; k += blockDim.x) {
+		const double g = sg[k] - (k > 0u ? sg[k - 1u] : 0.0);
+		if (g != 0.0) atomicAdd(&grad_bins[k], g);
+	}
 }
 
 // Bond term (original order) over blocks [0, nblocks) of the launch
@@ -283,6 +294,8 @@ __global__ void __launch_bounds__(256) adj_bond_angle_kernel(
 	uint32_t total_bins, double* __restrict__ grad_bins, const int4* __restrict__ angles,
 	const int* __restrict__ angle_idx, uint32_t na, const Table* __restrict__ angle_tables,
 	const float4* __restrict__ pos, const float4* __restrict__ mu, Box box, double* tan) {
+	chain_begin();
+	chain_wait();
 	extern __shared__ double sg[];
 	if (blockIdx.x < bond_blocks)
 		adj_bonds(blockIdx.x, bond_blocks, bonds, bond_idx, nb, pos, mu, bond_tables, values_base,
@@ -298,6 +311,8 @@ __global__ void __launch_bounds__(256) adj_combine_kernel(float4* __restrict__ l
 														  const double4* __restrict__ tan_sorted,
 														  const uint32_t* __restrict__ inv,
 														  uint32_t n) {
+	chain_begin();
+	chain_wait();
 	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
 	if (i >= n) return;
 	const double4 a = tan[i], b = tan_sorted[inv[i]];
@@ -413,11 +428,10 @@ void launch_adj_pair(const AdjointStepArgs& a, cudaStream_t st) {
 	if (smem > 48 * 1024)
 		MB2_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
 									  static_cast<int>(smem)));
-	MB2_LAUNCH kern<<<grid_for_rows(a.n, G), 256, smem, st>>>(
-		a.sorted_pos, a.mu_sorted, a.nbr, a.row_len, a.n, a.cap, a.tables.num_types,
-		a.tables.refs, a.tables.bin_force, a.tables.total_bins, a.box, a.cutoff_sq,
-		reinterpret_cast<double*>(a.tan_sorted),
-		a.grad_pair);
+	launch_chained(kern, grid_for_rows(a.n, G), 256u, smem, st, a.sorted_pos, a.mu_sorted, a.nbr,
+				   a.row_len, a.n, a.cap, a.tables.num_types, a.tables.refs, a.tables.bin_force,
+				   a.tables.total_bins, a.box, a.cutoff_sq, reinterpret_cast<double*>(a.tan_sorted),
+				   a.grad_pair);
 }
 
 template <int G>
@@ -444,9 +458,8 @@ void launch_rdf(const float4* sorted_pos, const uint32_t* nbr, const uint32_t* r
 void adjoint_step(const AdjointStepArgs& a, cudaStream_t st) {
 	const uint32_t n = a.n;
 	if (n == 0) return;
-	MB2_LAUNCH adj_mu_kernel<<<(n + 255) / 256, 256, 0, st>>>(a.lam, a.type_ids, a.diffusion, a.inv,
-															  n, a.dt_over_kT, a.mu, a.mu_sorted,
-															  a.tan, a.tan_sorted);
+	launch_chained(adj_mu_kernel, (n + 255) / 256, 256u, 0, st, a.lam, a.type_ids, a.diffusion, a.inv,
+				   n, a.dt_over_kT, a.mu, a.mu_sorted, a.tan, a.tan_sorted);
 	switch (a.lanes) {
 	case 4: launch_adj_pair_g<4>(a, st); break;
 	case 8: launch_adj_pair_g<8>(a, st); break;
@@ -458,13 +471,13 @@ void adjoint_step(const AdjointStepArgs& a, cudaStream_t st) {
 			a.num_bonds ? std::min<uint32_t>((a.num_bonds + 255) / 256, kPersistentBlocks) : 0u;
 		const uint32_t angle_blocks = (a.num_angles + 255) / 256;
 		const size_t smem = a.num_bonds ? static_cast<size_t>(a.bond_bins) * 8 : 0;
-		MB2_LAUNCH adj_bond_angle_kernel<<<bond_blocks + angle_blocks, 256, smem, st>>>(
-			bond_blocks, a.bonds, a.bond_table_idx, a.num_bonds, a.bond_tables, a.bond_values_base,
-			a.bond_bins, a.grad_bond, a.angles, a.angle_table_idx, a.num_angles, a.angle_tables,
-			a.pos, a.mu, a.box, reinterpret_cast<double*>(a.tan));
+		launch_chained(adj_bond_angle_kernel, bond_blocks + angle_blocks, 256u, smem, st, bond_blocks,
+					   a.bonds, a.bond_table_idx, a.num_bonds, a.bond_tables, a.bond_values_base,
+					   a.bond_bins, a.grad_bond, a.angles, a.angle_table_idx, a.num_angles,
+					   a.angle_tables, a.pos, a.mu, a.box, reinterpret_cast<double*>(a.tan));
 	}
-	MB2_LAUNCH adj_combine_kernel<<<(n + 255) / 256, 256, 0, st>>>(a.lam, a.tan, a.tan_sorted, a.inv,
-																   n);
+	launch_chained(adj_combine_kernel, (n + 255) / 256, 256u, 0, st, a.lam, a.tan, a.tan_sorted, a.inv,
+				   n);
 }
 
 void rdf_pairs(const float4* sorted_pos, const uint32_t* nbr, const uint32_t* row_len, uint32_t n,
