@@ -14,8 +14,8 @@
 // exactly as a plain step of system s with seed (seed + s) would: Philox key
 // mixed from (seed + s, patch_id, step), counter = index within the system.
 //
-// mb2_batch_run captures the non-rebuild step (pack, clear, pair, integrate,
-// step counter) in a CUDA graph and replays it; pairlist rebuilds run eagerly
+// mb2_batch_run captures the non-rebuild step (pack, pair, integrate, step
+// counter) in a CUDA graph and replays it; pairlist rebuilds run eagerly
 // at the rebuild period (the list is re-sized from the walk's counts).
 #include <algorithm>
 #include <cfloat>
@@ -654,7 +654,7 @@ float batch_max_disp(mb2_batch* b, const float4* pos, cudaStream_t st) {
 	return batch_sys_disp(b, pos, st);
 }
 
-// The per-step work after any rebuild: pack, clear, pair forces, integrate,
+// The per-step work after any rebuild: pack, pair forces, integrate,
 // advance the device step counter.
 void step_body(mb2_batch* b, float4* pos, float4* fe, const int* type_ids,
 			   const mb2_step_params* prm, cudaStream_t st) {

@@ -356,7 +356,7 @@ class Context:
     def run(self, pos, fe, type_ids, flags, first_step, num_steps, params: "L.StepParams",
             stream=None):
         """Steps first_step .. first_step + num_steps - 1 as ``step`` would, the
-        steps between rebuild checks replayed from one captured CUDA graph."""
+        steps between rebuild checks replayed from captured CUDA graphs."""
         self.check(self.lib.mb2_run(self.h, _p(pos), _p(fe), _p(type_ids), _p(flags),
                                     pos.shape[0], int(first_step), int(num_steps),
                                     C.byref(params), _stream(stream)))
