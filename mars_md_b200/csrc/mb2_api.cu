@@ -30,7 +30,7 @@ struct mb2_context {
 	Scratch scratch;
 
 	// Z-order state of the last build
-	DevBuf<uint32_t> keys, s2o, inv, row_len, row_off, nbr, cell_begin, cell_end, row_far;
+	DevBuf<uint32_t> keys, s2o, inv, row_len, row_off, nbr, cell_begin, cell_end, row_back;
 	DevBuf<float4> sorted_pos, ref_pos, force_sorted;
 	// Displacement since the last build, tracked by the step's pack (the
 	// pair kernel's inner rows): the build's Z-ordered positions, the squared
@@ -38,7 +38,7 @@ struct mb2_context {
 	DevBuf<float4> ref_sorted;
 	DevBuf<unsigned int> d2max;
 	float track_rc = 0.0f;
-	float split = 0.0f;  // distance of the last build's near / far split (0: none)
+	float split = 0.0f;  // the last build's near / far split, where its rows end with the near part
 	DevBuf<StencilEntry> stencil;
 	DevBuf<float> bbox;  // 6 floats, ordered-int min/max
 	DevBuf<unsigned int> disp;
@@ -333,6 +333,7 @@ void build(mb2_context* ctx, const float4* pos, const int* type_ids, uint32_t n,
 	wg.rc2 = rc2;
 	const float split = row_split(ctx->pt, ctx->box, rc_list, cutoff);
 	wg.split2 = split > 0.0f ? split * split : INFINITY;
+	wg.near_last = split_ends_early(split, cutoff) ? 1 : 0;
 	// Coordinates the walk's cheap distances round: the box, or on an open axis
 	// the particles' extent.
 	Box around = ctx->box;
@@ -346,12 +347,12 @@ void build(mb2_context* ctx, const float4* pos, const int* type_ids, uint32_t n,
 	}
 	fast_test_band(around, rc_list, &wg.fast_lo, &wg.fast_hi);
 	ctx->row_len.ensure(n);
-	ctx->row_far.ensure(n);
+	ctx->row_back.ensure(n);
 	auto walk = [&](uint32_t cap) {
 		const int hshift = __builtin_ctz(32 / ctx->lanes);
 		build_walk(ctx->sorted_pos.ptr, ctx->keys.ptr, ctx->s2o.ptr, ctx->cell_begin.ptr,
 				   ctx->cell_end.ptr, ctx->stencil.ptr, g.num_stencil, wg, n, ctx->box, ctx->excl,
-				   ctx->nbr.ptr, cap, hshift, ctx->row_len.ptr, ctx->row_far.ptr, ctx->stats.ptr + 4,
+				   ctx->nbr.ptr, cap, hshift, ctx->row_len.ptr, ctx->row_back.ptr, ctx->stats.ptr + 4,
 				   ctx->stats.ptr, st);
 		MB2_CUDA(cudaMemcpyAsync(ctx->pinned, ctx->stats.ptr, 4 * sizeof(uint64_t),
 								 cudaMemcpyDeviceToHost, st));
@@ -376,7 +377,7 @@ void build(mb2_context* ctx, const float4* pos, const int* type_ids, uint32_t n,
 	// Below some 16,000 particles a step is launches and latency: a 4,096-bead
 	// run lost 12 % to the tracking pack, 12,012 beads were level and 65,536
 	// gained 12 %.
-	const bool ends_early = split > 0.0f && split < 0.8f * cutoff && n > 16384u;
+	const bool ends_early = wg.near_last && n > 16384u;
 	auto choose_lanes = [&](double mean) {
 		if (ctx->lanes_request) return ctx->lanes_request;
 		if (ends_early && !whole_rows) {
@@ -416,7 +417,7 @@ void build(mb2_context* ctx, const float4* pos, const int* type_ids, uint32_t n,
 		stats = walk(ctx->cap);
 	}
 	if (split > 0.0f)
-		join_far(ctx->nbr.ptr, ctx->row_len.ptr, ctx->row_far.ptr, n, ctx->cap,
+		join_back(ctx->nbr.ptr, ctx->row_len.ptr, ctx->row_back.ptr, n, ctx->cap,
 				 __builtin_ctz(32 / ctx->lanes), st);
 	// Snapshot for the skin check (ZOrderPairlist.cpp:172-173).
 	ctx->ref_pos.ensure(n);
@@ -428,7 +429,7 @@ void build(mb2_context* ctx, const float4* pos, const int* type_ids, uint32_t n,
 	// 65,536-bead step the pack's extra read and reduction cost more for
 	// those alone, 1-2 us).
 	ctx->track_rc = 0.0f;
-	ctx->split = split;
+	ctx->split = wg.near_last ? split : 0.0f;
 	if (n > kSmallN || ends_early) {
 		ctx->ref_sorted.ensure(n);
 		ctx->d2max.ensure(1);
@@ -485,7 +486,7 @@ void pair_kernel(mb2_context* ctx, uint32_t n, float cutoff, int get_energy, cud
 	// covers the positions the kernel reads.
 	pair_forces(ctx->sorted_pos.ptr, ctx->nbr.ptr, ctx->row_len.ptr, n, ctx->cap, ctx->lanes, ctx->pt,
 				ctx->box, cutoff_sq, get_energy, ctx->force_sorted.ptr, ctx->energy.ptr, st,
-				ctx->track_rc > 0.0f ? ctx->d2max.ptr : nullptr, ctx->track_rc, ctx->row_far.ptr,
+				ctx->track_rc > 0.0f ? ctx->d2max.ptr : nullptr, ctx->track_rc, ctx->row_back.ptr,
 				ctx->split);
 }
 
@@ -1325,7 +1326,7 @@ std::vector<uint64_t> run_graph_key(const mb2_context* ctx, const float4* pos, c
 		P(ctx->types.pmf_offset), P(ctx->types.pmf_count), P(ctx->types.terms),
 		P(ctx->types.force_grid_id), P(ctx->types.force_grid_scale), P(ctx->types.grids),
 		static_cast<uint64_t>(ctx->types.num_grids), P(ctx->ref_sorted.ptr), P(ctx->d2max.ptr),
-		fbits(ctx->track_rc), P(ctx->row_far.ptr), fbits(ctx->split)};
+		fbits(ctx->track_rc), P(ctx->row_back.ptr), fbits(ctx->split)};
 	push_words(k, ctx->pt.solvent);
 	push_words(k, ctx->box);
 	return k;

@@ -208,18 +208,18 @@ __global__ void __launch_bounds__(256) batch_pack_kernel(
 	}
 }
 
-// A build's far entries moved behind the near ones, as join_far_kernel does it,
+// A build's far entries moved behind the near ones, as join_back_kernel does it,
 // in the rows of the systems that were rebuilt (flags null: all).
-__global__ void __launch_bounds__(256) batch_join_far_kernel(
+__global__ void __launch_bounds__(256) batch_join_back_kernel(
 	uint32_t* __restrict__ nbr, const uint32_t* __restrict__ row_len,
-	const uint32_t* __restrict__ row_far, const uint32_t* __restrict__ keys,
+	const uint32_t* __restrict__ row_back, const uint32_t* __restrict__ keys,
 	const uint32_t* __restrict__ flags, uint32_t n, uint32_t cap, int hshift) {
 	const uint32_t slice = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
 	const uint32_t slices = (n + (1u << hshift) - 1u) >> hshift;
 	if (slice >= slices) return;  // whole warp
 	const uint32_t i = (slice << hshift) + (threadIdx.x & ((1u << hshift) - 1u));
 	const bool mine = i < n && (!flags || flags[keys[i] >> kSysShift]);
-	join_far_slice(nbr, mine ? row_len[i] : 0u, mine ? row_far[i] : 0u, slice, cap, hshift);
+	join_back_slice(nbr, mine ? row_len[i] : 0u, mine ? row_back[i] : 0u, slice, cap, hshift);
 }
 
 __global__ void __launch_bounds__(256) batch_cell_ranges_kernel(const uint32_t* __restrict__ keys,
@@ -365,7 +365,7 @@ struct mb2_batch {
 	DevBuf<unsigned int> disp;
 	// Rows' far entries, the near / far split of the lists (0: none), and each
 	// system's largest squared displacement since its build (the packs keep it).
-	DevBuf<uint32_t> row_far;
+	DevBuf<uint32_t> row_back;
 	float split = 0.0f;
 	DevBuf<unsigned int> moved;
 	float longest_edge = 0.0f;
@@ -450,6 +450,7 @@ void choose_grids(mb2_batch* b, float rc) {
 		wg.rc2 = rc * rc;
 		fast_test_band(bx, rc, &wg.fast_lo, &wg.fast_hi);
 		wg.split2 = b->split > 0.0f ? b->split * b->split : INFINITY;
+		wg.near_last = 1;
 		for (int a = 0; a < 3; ++a)
 			wg.eps[a] = static_cast<float>(
 				1e-6 * (std::fabs(static_cast<double>(bx.origin[a])) + bx.size[a]) + 1e-6);
@@ -494,7 +495,7 @@ void batch_build(mb2_batch* b, const float4* pos, const int* type_ids, float rc,
 	float split = b->split;
 	if (!flags_h && cutoff > 0.0f) {
 		split = row_split(b->pt, b->boxes_h[0], rc, cutoff);
-		if (!(split < 0.8f * cutoff)) split = 0.0f;
+		if (!split_ends_early(split, cutoff)) split = 0.0f;
 	}
 	if (b->grid_rc != rc || b->split != split) {
 		b->split = split;
@@ -556,7 +557,7 @@ void batch_build(mb2_batch* b, const float4* pos, const int* type_ids, float rc,
 		MB2_LAUNCH batch_cell_ranges_kernel<<<(n + 255) / 256, 256, 0, st>>>(
 			b->keys.ptr, n, b->grids.ptr, b->cell_begin.ptr, b->cell_end.ptr);
 	b->row_len.ensure(n);
-	b->row_far.ensure(n);
+	b->row_back.ensure(n);
 	b->stats.ensure(2);
 	auto walk = [&](uint32_t cap, const uint32_t* fl) {
 		MB2_CUDA(cudaMemsetAsync(b->stats.ptr, 0, 2 * sizeof(unsigned long long), st));
@@ -564,7 +565,7 @@ void batch_build(mb2_batch* b, const float4* pos, const int* type_ids, float rc,
 			const int hshift = __builtin_ctz(32 / b->lanes);
 			const WalkArrays w{b->sorted_pos.ptr, b->s2o.ptr, b->cell_begin.ptr, b->cell_end.ptr,
 							   b->stencil.ptr,    0,          b->nbr.ptr,        cap,
-							   hshift,            b->row_len.ptr, b->row_far.ptr};
+							   hshift,            b->row_len.ptr, b->row_back.ptr};
 			MB2_LAUNCH batch_walk_kernel<<<(n + 8 * kWalkRows - 1) / (8 * kWalkRows), 256, 0, st>>>(
 				b->keys.ptr, w, b->grids.ptr, b->boxes.ptr, fl, n, b->outside.ptr);
 			MB2_LAUNCH batch_row_stats_kernel<<<std::min<uint32_t>((n + 255) / 256, 1184), 256, 0,
@@ -615,8 +616,8 @@ void batch_build(mb2_batch* b, const float4* pos, const int* type_ids, float rc,
 	if (n && b->split > 0.0f) {
 		const int hshift = __builtin_ctz(32 / b->lanes);
 		const uint32_t slices = (n + (1u << hshift) - 1u) >> hshift;
-		MB2_LAUNCH batch_join_far_kernel<<<(slices + 7) / 8, 256, 0, st>>>(
-			b->nbr.ptr, b->row_len.ptr, b->row_far.ptr, b->keys.ptr, dflags, n, b->cap, hshift);
+		MB2_LAUNCH batch_join_back_kernel<<<(slices + 7) / 8, 256, 0, st>>>(
+			b->nbr.ptr, b->row_len.ptr, b->row_back.ptr, b->keys.ptr, dflags, n, b->cap, hshift);
 	}
 	b->ref_pos.ensure(n);
 	b->moved.ensure(b->num_systems);
@@ -666,7 +667,7 @@ void step_body(mb2_batch* b, float4* pos, float4* fe, const int* type_ids,
 	const float cutoff_sq = prm->cutoff > 0.0f ? prm->cutoff * prm->cutoff : 0.0f;
 	pair_forces_systems(b->sorted_pos.ptr, b->nbr.ptr, b->row_len.ptr, n, b->cap, b->lanes, b->pt,
 						b->boxes.ptr, b->keys.ptr, kSysShift, true, cutoff_sq, 0,
-						b->force_sorted.ptr, b->energy.ptr, st, b->moved.ptr, b->row_far.ptr, b->split,
+						b->force_sorted.ptr, b->energy.ptr, st, b->moved.ptr, b->row_back.ptr, b->split,
 						b->longest_edge);
 	bd_integrate_systems(pos, fe, b->force_sorted.ptr, b->inv.ptr, type_ids, b->sys_of.ptr,
 						 b->offsets_d.ptr, b->boxes.ptr, n, b->types, prm->dt, prm->kT, prm->seed,
@@ -930,7 +931,7 @@ int mb2_batch_run(mb2_batch* b, float* pos4, float* force_energy4, const int* ty
 				reinterpret_cast<uint64_t>(pos), reinterpret_cast<uint64_t>(fe),
 				reinterpret_cast<uint64_t>(type_ids), reinterpret_cast<uint64_t>(b->nbr.ptr),
 				reinterpret_cast<uint64_t>(b->force_sorted.ptr), b->cap,
-				reinterpret_cast<uint64_t>(b->row_far.ptr), reinterpret_cast<uint64_t>(b->moved.ptr),
+				reinterpret_cast<uint64_t>(b->row_back.ptr), reinterpret_cast<uint64_t>(b->moved.ptr),
 				reinterpret_cast<uint64_t>(b->ref_pos.ptr), f2u(b->split),
 				static_cast<uint64_t>(b->lanes), b->n, f2u(prm->cutoff), f2u(prm->dt),
 				f2u(prm->kT), prm->seed, prm->patch_id,

@@ -329,9 +329,10 @@ struct FastArgs {
 	int T, stride, last;
 	float start, step_inv;
 	float loose, close2, lo;
-	// Far entries of each row, and twice the displacement up to which none of
-	// them can be within `loose` (0: the rows are walked whole).
-	const uint32_t* row_far;
+	// Near entries at the end of each row, and twice the displacement up to which
+	// none of the far ones before them can be within `loose` (0: the rows are
+	// walked whole).
+	const uint32_t* row_back;
 	float far_gap;
 };
 
@@ -495,12 +496,16 @@ __global__ void __launch_bounds__(256, fast_min_blocks<kEnergy, std::is_same<Box
 	// A pair apart by more than the split at the build is apart by more than
 	// the split less both displacements now: while that is beyond every bin
 	// that holds a force, the far entries add nothing and are not read.
+	uint32_t first = 0u;
 	if (kFar && valid) {
 		const unsigned int d2 = boxes.moved(i);
-		if (2.0f * sqrtf(__uint_as_float(d2)) < fa.far_gap) cnt -= fa.row_far[i];
+		if (2.0f * sqrtf(__uint_as_float(d2)) < fa.far_gap) {
+			first = cnt - fa.row_back[i];
+			cnt -= first;
+		}
 	}
 	// Entry k of row i: ((i / H) * cap + k) * H + i % H.
-	const uint32_t* col = nbr + (static_cast<size_t>(i / H) * cap) * H + (i % H);
+	const uint32_t* col = nbr + (static_cast<size_t>(i / H) * cap + first) * H + (i % H);
 	const float2 npi = make_float2(-pi.x, -pi.y);
 	float2 nxy = make_float2(0.0f, 0.0f);  // minus the i-force, x and y
 	float nz = 0.0f, fe = 0.0f;
@@ -880,20 +885,20 @@ FastArgs fast_args(const PairTables& t, float cutoff_sq, int get_energy) {
 	fa.lo = win.lo;
 	const double close = std::max(1e-5, u.start > 0.0f ? u.start * (1.0 + 1e-6) : 0.0);
 	fa.close2 = static_cast<float>(close * close * (1.0 + 1e-6));
-	fa.row_far = nullptr;
+	fa.row_back = nullptr;
 	fa.far_gap = 0.0f;
 	return fa;
 }
 
 // The split's far entries may be left out while 2 D < far_gap: the slack
 // covers the rounding of the build's distances and of the displacements.
-void set_far(FastArgs& fa, const uint32_t* row_far, float split, float longest_edge) {
-	if (!row_far || !(split > 0.0f)) return;
+void set_far(FastArgs& fa, const uint32_t* row_back, float split, float longest_edge) {
+	if (!row_back || !(split > 0.0f)) return;
 	const float gap = split - std::sqrt(fa.loose) - 0.02f - 1e-6f * longest_edge;
 	// A gap that a step or two closes (a split at the cutoff) is not worth its
 	// test: 2 % of the 2,097,152-bead run.
 	if (!(gap > 0.2f * split)) return;
-	fa.row_far = row_far;
+	fa.row_back = row_back;
 	fa.far_gap = gap;
 }
 
@@ -1196,7 +1201,7 @@ void pair_forces(const float4* sorted_pos, const uint32_t* nbr, const uint32_t* 
 				 uint32_t n, uint32_t cap, int lanes_per_row, const PairTables& t, const Box& box,
 				 float cutoff_sq, int get_energy, float4* force_sorted, double* ev,
 				 cudaStream_t st, const unsigned int* d2max, float list_rc,
-				 const uint32_t* row_far, float split) {
+				 const uint32_t* row_back, float split) {
 	if (n == 0) return;
 	const bool all_periodic = box.periodic[0] && box.periodic[1] && box.periodic[2];
 	const bool fast = all_periodic && fast_ok(t, cutoff_sq, get_energy);
@@ -1205,7 +1210,7 @@ void pair_forces(const float4* sorted_pos, const uint32_t* nbr, const uint32_t* 
 					 track ? list_rc * (1.0f + 0x1p-20f) + kInnerSafety : 0.0f};
 	FastArgs fa = fast ? fast_args(t, cutoff_sq, get_energy) : FastArgs{};
 	if (fast && track)
-		set_far(fa, row_far, split, std::max(box.size[0], std::max(box.size[1], box.size[2])));
+		set_far(fa, row_back, split, std::max(box.size[0], std::max(box.size[1], box.size[2])));
 	launch_pair_lanes(sorted_pos, nbr, row_len, n, cap, lanes_per_row, t, fast ? &fa : nullptr,
 					  one, all_periodic, cutoff_sq, get_energy, force_sorted, ev, st);
 }
@@ -1215,11 +1220,11 @@ void pair_forces_systems(const float4* sorted_pos, const uint32_t* nbr, const ui
 						 const Box* boxes, const uint32_t* sorted_keys, int sys_shift,
 						 bool all_periodic, float cutoff_sq, int get_energy, float4* force_sorted,
 						 double* ev, cudaStream_t st, const unsigned int* moved,
-						 const uint32_t* row_far, float split, float longest_edge) {
+						 const uint32_t* row_back, float split, float longest_edge) {
 	if (n == 0) return;
 	const bool fast = all_periodic && fast_ok(t, cutoff_sq, get_energy);
 	FastArgs fa = fast ? fast_args(t, cutoff_sq, get_energy) : FastArgs{};
-	if (fast && moved) set_far(fa, row_far, split, longest_edge);
+	if (fast && moved) set_far(fa, row_back, split, longest_edge);
 	launch_pair_lanes(sorted_pos, nbr, row_len, n, cap, lanes_per_row, t, fast ? &fa : nullptr,
 					  SystemBoxes{boxes, sorted_keys, sys_shift, moved}, all_periodic, cutoff_sq,
 					  get_energy, force_sorted, ev, st);

@@ -160,7 +160,8 @@ struct WalkGrid {
 	int m, shift;
 	float rc2;                 // pairlist cutoff squared, as the reference rounds it
 	float fast_lo, fast_hi;    // d^2 band that needs the exact test
-	float split2;              // entries with d^2 above it go to the row's far segment
+	float split2;              // d^2 that parts a row's entries, near and far
+	int near_last;             // the near part follows the far one (else precedes it)
 	float eps[3];              // rounding margin of a coordinate box
 };
 // Cell level m in [m_lo, m_hi] minimising the walk's cost at `rows` rows a warp; the
@@ -177,10 +178,10 @@ void build_walk(const float4* sorted_pos, const uint32_t* keys, const uint32_t* 
 				const uint32_t* begin, const uint32_t* end, const StencilEntry* stencil,
 				int num_stencil, const WalkGrid& wg, uint32_t n, const Box& box,
 				const Exclusions& ex, uint32_t* nbr, uint32_t cap, int hshift, uint32_t* row_len,
-				uint32_t* row_far, const unsigned long long* outside, unsigned long long* stats,
+				uint32_t* row_back, const unsigned long long* outside, unsigned long long* stats,
 				cudaStream_t st);
-// After a storing walk: each row's far entries moved to follow its near ones.
-void join_far(uint32_t* nbr, const uint32_t* row_len, const uint32_t* row_far, uint32_t n,
+// After a storing walk: each row's back part moved to follow its front part.
+void join_back(uint32_t* nbr, const uint32_t* row_len, const uint32_t* row_back, uint32_t n,
 			  uint32_t cap, int hshift, cudaStream_t st);
 void export_pairs(const uint32_t* nbr, const uint32_t* row_len, const uint32_t* row_off,
 				  const uint32_t* s2o, uint32_t n, uint32_t cap, int hshift, int2* out,
@@ -261,17 +262,20 @@ struct PairTables {
 // d2max / list_rc (optional): the displacement track of the list's build and
 // its list radius. With them, rows that lie deeper inside the box than
 // list_rc + 2 * sqrt(*d2max) (plus a safety band) take no minimum image.
-// row_far / split (optional, with d2max): the far entries at the end of each
-// row and the distance beyond which all of them were at the build (0: unknown).
-// They are left out of a launch while the displacements since the build cannot
-// have brought one within reach of the tables.
+// row_back / split (optional, with d2max): rows of far entries followed by
+// row_back near ones, and the distance beyond which all the far ones were at
+// the build (0: not so). They are left out of a launch while the displacements
+// since the build cannot have brought one within reach of the tables.
 void pair_forces(const float4* sorted_pos, const uint32_t* nbr, const uint32_t* row_len,
 				 uint32_t n, uint32_t cap, int lanes_per_row, const PairTables& t, const Box& box,
 				 float cutoff_sq, int get_energy, float4* force_sorted, double* energy_virial,
 				 cudaStream_t st, const unsigned int* d2max = nullptr, float list_rc = 0.0f,
-				 const uint32_t* row_far = nullptr, float split = 0.0f);
-// Where a build for these tables splits its rows near / far (0: it does not).
+				 const uint32_t* row_back = nullptr, float split = 0.0f);
+// Where a build for these tables parts its rows near / far (0: it does not), and
+// whether the far part then is what a step mostly leaves out, so that the rows
+// keep the near part, the short one, behind it (the join moves that).
 float row_split(const PairTables& t, const Box& box, float rc_list, float cutoff);
+inline bool split_ends_early(float split, float cutoff) { return split > 0.0f && split < 0.8f * cutoff; }
 // Host: per-type-pair lookup constants and per-bin force / (U0, dU) arrays of
 // a set of tabulated pair tables; returns the total number of bins.
 size_t pair_table_arrays(int num_types, const uint32_t* term_matrix, int num_tables,
@@ -294,13 +298,13 @@ struct FastTableBufs {
 			 const std::vector<float2>& be, PairTables& t);
 };
 // Batched replicas: row i's box is boxes[sorted_keys[i] >> sys_shift]; moved,
-// row_far and split as d2max, row_far and split above, moved per system.
+// row_back and split as d2max, row_back and split above, moved per system.
 void pair_forces_systems(const float4* sorted_pos, const uint32_t* nbr, const uint32_t* row_len,
 						 uint32_t n, uint32_t cap, int lanes_per_row, const PairTables& t,
 						 const Box* boxes, const uint32_t* sorted_keys, int sys_shift,
 						 bool all_periodic, float cutoff_sq, int get_energy, float4* force_sorted,
 						 double* ev, cudaStream_t st, const unsigned int* moved,
-						 const uint32_t* row_far, float split, float longest_edge);
+						 const uint32_t* row_back, float split, float longest_edge);
 void scatter_add_forces(const float4* force_sorted, const uint32_t* s2o, uint32_t n,
 						float4* force_energy, int get_energy, cudaStream_t st);
 // Exhaustive device check of sqrt_rn_nr against __fsqrt_rn on [2^-60,

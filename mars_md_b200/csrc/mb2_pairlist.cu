@@ -221,15 +221,15 @@ __global__ void __launch_bounds__(256) export_kernel(const uint32_t* __restrict_
 }
 
 // After a storing walk: each slice's far entries joined to its near ones.
-__global__ void __launch_bounds__(256) join_far_kernel(uint32_t* __restrict__ nbr,
+__global__ void __launch_bounds__(256) join_back_kernel(uint32_t* __restrict__ nbr,
 													   const uint32_t* __restrict__ row_len,
-													   const uint32_t* __restrict__ row_far,
+													   const uint32_t* __restrict__ row_back,
 													   uint32_t n, uint32_t cap, int hshift) {
 	const uint32_t slice = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
 	const uint32_t slices = (n + (1u << hshift) - 1u) >> hshift;
 	if (slice >= slices) return;  // whole warp
 	const uint32_t i = (slice << hshift) + (threadIdx.x & ((1u << hshift) - 1u));
-	join_far_slice(nbr, i < n ? row_len[i] : 0u, i < n ? row_far[i] : 0u, slice, cap, hshift);
+	join_back_slice(nbr, i < n ? row_len[i] : 0u, i < n ? row_back[i] : 0u, slice, cap, hshift);
 }
 
 // DisplacementKernel::min_image (AdaptiveKernels.h:56-65). Both inputs are
@@ -331,25 +331,25 @@ void build_walk(const float4* sorted_pos, const uint32_t* keys, const uint32_t* 
 				const uint32_t* begin, const uint32_t* end, const StencilEntry* stencil,
 				int num_stencil, const WalkGrid& wg, uint32_t n, const Box& box,
 				const Exclusions& ex, uint32_t* nbr, uint32_t cap, int hshift, uint32_t* row_len,
-				uint32_t* row_far, const unsigned long long* outside, unsigned long long* stats,
+				uint32_t* row_back, const unsigned long long* outside, unsigned long long* stats,
 				cudaStream_t st) {
 	MB2_CUDA(cudaMemsetAsync(stats, 0, 2 * sizeof(unsigned long long), st));
 	if (n == 0) return;
 	const bool excl = ex.offsets != nullptr || ex.rigid_body_id != nullptr;
 	const WalkArrays w{sorted_pos, s2o, begin,  end,    stencil, num_stencil,
-					   nbr,        cap, hshift, row_len, row_far};
+					   nbr,        cap, hshift, row_len, row_back};
 	const uint32_t rows = walk_rows(n);
 	auto kern = excl ? build_walk_kernel<true> : build_walk_kernel<false>;
 	MB2_LAUNCH kern<<<(n + 8 * rows - 1) / (8 * rows), 256, 0, st>>>(keys, w, wg, n, box, ex, rows,
 																	 outside, stats);
 }
 
-void join_far(uint32_t* nbr, const uint32_t* row_len, const uint32_t* row_far, uint32_t n,
+void join_back(uint32_t* nbr, const uint32_t* row_len, const uint32_t* row_back, uint32_t n,
 			  uint32_t cap, int hshift, cudaStream_t st) {
 	if (n == 0) return;
 	const uint32_t slices = (n + (1u << hshift) - 1u) >> hshift;
 	const uint32_t blocks = (slices + 7u) / 8u;  // 8 warps (slices) per block
-	MB2_LAUNCH join_far_kernel<<<blocks, 256, 0, st>>>(nbr, row_len, row_far, n, cap, hshift);
+	MB2_LAUNCH join_back_kernel<<<blocks, 256, 0, st>>>(nbr, row_len, row_back, n, cap, hshift);
 }
 
 void export_pairs(const uint32_t* nbr, const uint32_t* row_len, const uint32_t* row_off,

@@ -46,7 +46,7 @@ struct WalkArrays {
 	uint32_t cap;
 	int hshift;
 	uint32_t* row_len;
-	uint32_t* row_far;
+	uint32_t* row_back;
 };
 
 // nearest image of x (a multiple of l away): x - l rint(x / l), one rounding;
@@ -79,8 +79,8 @@ __device__ __forceinline__ float nearest(float x, float l, float inv, float* k) 
 // outside the box (exact_all) take the exact test throughout.
 //
 // A row's hits are appended with two ballots: near entries (within split2)
-// from the front of its slots, far ones from the back; join_far_slice then
-// moves the far ones behind the near ones. Entries past cap are only counted
+// from the front of its slots, far ones from the back, or (near_last) the other
+// way round; join_back_slice then moves the back part behind the front part. Entries past cap are only counted
 // (the host then grows the list and walks again). Returns the rows' total and
 // longest lengths in *total and *longest (the same in every lane).
 template <bool kExcl>
@@ -131,7 +131,7 @@ __device__ __forceinline__ void walk_run(const WalkArrays& w, const WalkGrid& wg
 #pragma unroll
 	for (int a = 0; a < 3; ++a)
 		per_row = per_row || (box.periodic[a] && len[a] <= 2.0f * (rc + half[a] + wg.eps[a]));
-	uint32_t row_len = 0, row_far = 0;  // of row `lane`
+	uint32_t row_len = 0, row_back = 0;  // of row `lane`
 	uint32_t queued = 0;
 	const bool split = wg.split2 < INFINITY;
 
@@ -160,24 +160,24 @@ __device__ __forceinline__ void walk_run(const WalkArrays& w, const WalkGrid& wg
 				const int4 e = sh.excl[r];
 				hit = !is_excluded(ex, bj, e.x, e.y, e.z);
 			}
-			const bool near = !split || d2 <= wg.split2;
-			const uint32_t nm = __ballot_sync(0xFFFFFFFFu, hit && near);
-			const uint32_t fm = __ballot_sync(0xFFFFFFFFu, hit && !near);
+			const bool front = !split || (d2 <= wg.split2) != (wg.near_last != 0);
+			const uint32_t nm = __ballot_sync(0xFFFFFFFFu, hit && front);
+			const uint32_t fm = __ballot_sync(0xFFFFFFFFu, hit && !front);
 			if ((nm | fm) == 0u) continue;
 			const uint32_t all = __shfl_sync(0xFFFFFFFFu, row_len, r);
-			const uint32_t far = __shfl_sync(0xFFFFFFFFu, row_far, r);
+			const uint32_t back = __shfl_sync(0xFFFFFFFFu, row_back, r);
 			if (hit) {
 				const uint32_t place = all + static_cast<uint32_t>(__popc((nm | fm) & lt));
 				const uint32_t slot =
-					near ? all - far + static_cast<uint32_t>(__popc(nm & lt))
-						 : w.cap - 1u - (far + static_cast<uint32_t>(__popc(fm & lt)));
+					front ? all - back + static_cast<uint32_t>(__popc(nm & lt))
+						  : w.cap - 1u - (back + static_cast<uint32_t>(__popc(fm & lt)));
 				const uint32_t flip = bj < __float_as_int(row.w) ? kOrientBit : 0u;
 				if (place < w.cap)
 					w.nbr[sh.base[r] + (static_cast<unsigned long long>(slot) << w.hshift)] = j | flip;
 			}
 			if (static_cast<int>(lane) == r) {
 				row_len += static_cast<uint32_t>(__popc(nm | fm));
-				row_far += static_cast<uint32_t>(__popc(fm));
+				row_back += static_cast<uint32_t>(__popc(fm));
 			}
 		}
 	};
@@ -265,35 +265,37 @@ __device__ __forceinline__ void walk_run(const WalkArrays& w, const WalkGrid& wg
 	__syncwarp();
 	if (lane < static_cast<uint32_t>(nr)) {
 		w.row_len[rb + lane] = row_len;
-		w.row_far[rb + lane] = row_far;
+		w.row_back[rb + lane] = row_back;
 	}
 	*total_out = __reduce_add_sync(0xFFFFFFFFu, row_len);
 	*longest_out = __reduce_max_sync(0xFFFFFFFFu, row_len);
 }
 
-// Moves a slice's far entries (stored backwards from the end of each row's cap
-// slots) to follow its near entries, so that a row is one contiguous run: near
-// entries in candidate order, then the far ones. One warp per slice of H rows;
-// len, far: of row (lane mod H). Lane l copies entries l / H, l / H + 32 / H,
-// ... of that row, so each load and store instruction touches neighbouring
-// words. Destinations precede sources (near + far <= cap) and every batch is
-// loaded before it is stored, so the in-place copy is safe.
-__device__ __forceinline__ void join_far_slice(uint32_t* __restrict__ nbr, uint32_t len, uint32_t far,
-											   uint32_t slice, uint32_t cap, int hshift) {
+// Moves the back entries of a slice's rows (stored backwards from the end of
+// each row's cap slots) to follow the front ones, so that a row is one
+// contiguous run, each part in candidate order but the back one reversed. One
+// warp per slice of H rows; len, back: of row (lane mod H). Lane l copies
+// entries l / H, l / H + 32 / H, ... of that row, so each load and store
+// instruction touches neighbouring words. Destinations precede sources (front +
+// back <= cap) and every batch is loaded before it is stored, so the in-place
+// copy is safe.
+__device__ __forceinline__ void join_back_slice(uint32_t* __restrict__ nbr, uint32_t len,
+												uint32_t back, uint32_t slice, uint32_t cap,
+												int hshift) {
 	const uint32_t lane = threadIdx.x & 31u;
 	const uint32_t h = 1u << hshift;
 	const uint32_t r = lane & (h - 1u), kk = lane >> hshift, step = 32u >> hshift;
-	const uint32_t near = len - far;
-	uint32_t most = far;
+	const uint32_t front = len - back;
+	uint32_t most = back;
 #pragma unroll
 	for (int o = 16; o > 0; o >>= 1) most = max(most, __shfl_xor_sync(0xFFFFFFFFu, most, o));
 	uint32_t* base = nbr + static_cast<size_t>(slice) * cap * h + r;
 	for (uint32_t k0 = 0; k0 < most; k0 += step) {
 		const uint32_t k = k0 + kk;
 		uint32_t v = 0u;
-		if (k < far) v = base[static_cast<size_t>(cap - far + k) * h];
+		if (k < back) v = base[static_cast<size_t>(cap - back + k) * h];
 		__syncwarp();
-		if (k < far) base[static_cast<size_t>(near + k) * h] = v;
+		if (k < back) base[static_cast<size_t>(front + k) * h] = v;
 		__syncwarp();
 	}
 }
