@@ -121,7 +121,7 @@ void remap_indices(int* idx, size_t count, const uint32_t* inv, uint32_t n, cuda
 size_t sort_work_words(uint32_t n);
 void radix_sort_pairs_into(uint32_t* keys, uint32_t* vals, uint32_t n, uint32_t* keys_alt,
 						   uint32_t* vals_alt, uint32_t* work, cudaStream_t st,
-						   uint32_t* error = nullptr);
+						   uint32_t* report = nullptr);
 // noalloc.cu: the same sort over the library's static scratch (no allocation).
 void radix_sort_pairs_static(uint32_t* keys, uint32_t* vals, uint32_t n, cudaStream_t st);
 

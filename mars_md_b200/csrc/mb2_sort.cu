@@ -78,24 +78,31 @@ __global__ void __launch_bounds__(kSortThreads) radix_hist_kernel(const uint32_t
 }
 
 // One pass: tile -> its place in the output. hist: this pass's 256 digit
-// counts; status[tile][256]: look-back words; ticket: zero at the start; error: set when an earlier tile's counts never came (the tile
-// then writes nothing).
+// counts; status[tile][256]: look-back words; ticket: zero at the start; error
+// (and report, where given): set when an earlier tile's counts never came. The
+// tile then writes nothing, nor do tiles that start after it, in this pass and the
+// next ones: a pass never reads slots that the one before it left unwritten.
 template <int kItems>
 __global__ void __launch_bounds__(kSortThreads) radix_pass_kernel(
 	const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in, uint32_t n,
 	int pass, const uint32_t* __restrict__ hist, unsigned long long* status, uint32_t* ticket,
-	uint32_t* error, uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out) {
+	uint32_t* error, uint32_t* report, uint32_t* __restrict__ keys_out,
+	uint32_t* __restrict__ vals_out) {
 	__shared__ uint32_t warp_count[kSortWarps][256];
 	__shared__ uint32_t warp_tot[2][kSortWarps];
-	__shared__ uint32_t tile_sh;
+	__shared__ uint32_t tile_sh, stop_sh;
 	__shared__ uint32_t to_global[256];  // output slot of digit d less its slot in the tile
 	__shared__ uint32_t sorted_key[kSortThreads * kItems], sorted_val[kSortThreads * kItems];
 	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, d = threadIdx.x;
 	const int shift = 8 * pass;
 	const unsigned long long own = 2ull * pass + 1ull, all = own + 1ull;
-	if (threadIdx.x == 0) tile_sh = atomicAdd(ticket, 1u);
+	if (threadIdx.x == 0) {
+		stop_sh = *static_cast<volatile uint32_t*>(error);
+		tile_sh = atomicAdd(ticket, 1u);
+	}
 	for (int w = 0; w < kSortWarps; ++w) warp_count[w][d] = 0;
 	__syncthreads();
+	if (stop_sh != 0u) return;
 	const uint32_t tile = tile_sh;
 	const uint32_t base = (tile * kSortThreads + warp * 32) * kItems + lane;
 	uint32_t key[kItems], val[kItems], rank[kItems];
@@ -195,8 +202,10 @@ __global__ void __launch_bounds__(kSortThreads) radix_pass_kernel(
 				}
 			}
 		}
-		if (failed) *static_cast<volatile uint32_t*>(error) = 1u;
-		else *row = (all << kTagShift) | (prefix + count);
+		if (failed) {
+			*static_cast<volatile uint32_t*>(error) = 1u;
+			if (report) *static_cast<volatile uint32_t*>(report) = 1u;
+		} else *row = (all << kTagShift) | (prefix + count);
 	}
 	to_global[d] = first + static_cast<uint32_t>(prefix) - tfirst;
 	failed = __syncthreads_or(failed);
@@ -326,7 +335,7 @@ size_t sort_work_words(uint32_t n) {
 }
 
 void radix_sort_pairs_into(uint32_t* keys, uint32_t* vals, uint32_t n, uint32_t* keys_alt,
-						   uint32_t* vals_alt, uint32_t* work, cudaStream_t st, uint32_t* error) {
+						   uint32_t* vals_alt, uint32_t* work, cudaStream_t st, uint32_t* report) {
 	if (n <= 1) return;
 	if (n <= kRankSortMax) {
 		const size_t smem = static_cast<size_t>((n + 3u) / 4u) * sizeof(uint4);
@@ -338,7 +347,7 @@ void radix_sort_pairs_into(uint32_t* keys, uint32_t* vals, uint32_t n, uint32_t*
 	}
 	const uint32_t tiles = sort_tiles(n);
 	uint32_t* tickets = work + 4 * 256;
-	if (!error) error = tickets + 4;
+	uint32_t* error = tickets + 4;
 	unsigned long long* status = reinterpret_cast<unsigned long long*>(work + kSortHeadWords);
 	MB2_CUDA(cudaMemsetAsync(work, 0, sort_work_words(n) * sizeof(uint32_t), st));
 	MB2_LAUNCH radix_hist_kernel<<<std::min(tiles, 592u), kSortThreads, 0, st>>>(keys, n, work);
@@ -347,7 +356,7 @@ void radix_sort_pairs_into(uint32_t* keys, uint32_t* vals, uint32_t n, uint32_t*
 										   : radix_pass_kernel<kLargeItems>;
 	for (int pass = 0; pass < 4; ++pass) {
 		MB2_LAUNCH pass_kernel<<<tiles, kSortThreads, 0, st>>>(
-			ks, vs, n, pass, work + 256 * pass, status, tickets + pass, error, kd, vd);
+			ks, vs, n, pass, work + 256 * pass, status, tickets + pass, error, report, kd, vd);
 		std::swap(ks, kd);
 		std::swap(vs, vd);
 	}
