@@ -273,8 +273,7 @@ void sort_particles(mb2_context* ctx, const float4* pos, const int* type_ids, ui
 	ctx->inv.ensure(n);
 	ctx->sorted_pos.ensure(n);
 	morton_encode(pos, n, bmin, bmax, ctx->keys.ptr, ctx->s2o.ptr, st);
-	radix_sort_pairs(ctx->scratch, ctx->keys.ptr, ctx->s2o.ptr, n, st);
-	inverse_and_gather(ctx->s2o.ptr, n, pos, ctx->inv.ptr, nullptr, st);
+	radix_sort_pairs(ctx->scratch, ctx->keys.ptr, ctx->s2o.ptr, n, st, ctx->inv.ptr);
 	pack_sorted_positions(pos, type_ids, ctx->s2o.ptr, n, ctx->sorted_pos.ptr, st, odd, &ctx->box);
 }
 
@@ -697,17 +696,15 @@ int mb2_sort_morton(mb2_context* ctx, const float* pos4, uint32_t n, const float
 		require(n == 0 || pos4, MB2_ERR_ARG, "mb2_sort_morton: null positions");
 		const cudaStream_t st = S(stream);
 		const float4* pos = reinterpret_cast<const float4*>(pos4);
+		// Sorted in the caller's arrays where it gives them (the context's state
+		// is of no use after this call).
 		ctx->keys.ensure(n);
 		ctx->s2o.ensure(n);
-		ctx->inv.ensure(n);
-		morton_encode(pos, n, bmin, bmax, ctx->keys.ptr, ctx->s2o.ptr, st);
-		radix_sort_pairs(ctx->scratch, ctx->keys.ptr, ctx->s2o.ptr, n, st);
-		inverse_and_gather(ctx->s2o.ptr, n, pos, ctx->inv.ptr,
-						   reinterpret_cast<float4*>(sorted_pos4_out), st);
-		const size_t b = static_cast<size_t>(n) * sizeof(uint32_t);
-		if (keys_out) MB2_CUDA(cudaMemcpyAsync(keys_out, ctx->keys.ptr, b, cudaMemcpyDeviceToDevice, st));
-		if (s2o_out) MB2_CUDA(cudaMemcpyAsync(s2o_out, ctx->s2o.ptr, b, cudaMemcpyDeviceToDevice, st));
-		if (inverse_out) MB2_CUDA(cudaMemcpyAsync(inverse_out, ctx->inv.ptr, b, cudaMemcpyDeviceToDevice, st));
+		uint32_t* keys = keys_out ? keys_out : ctx->keys.ptr;
+		uint32_t* s2o = s2o_out ? s2o_out : ctx->s2o.ptr;
+		morton_encode(pos, n, bmin, bmax, keys, s2o, st);
+		radix_sort_pairs(ctx->scratch, keys, s2o, n, st, inverse_out);
+		if (sorted_pos4_out) permute_gather(pos, s2o, n, 16, sorted_pos4_out, st);
 		ctx->built = false;  // the sort state no longer matches a pairlist
 	});
 }
@@ -1093,9 +1090,7 @@ int mb2_reorder_begin(mb2_context* ctx, const float* pos4, uint32_t n, void* str
 		ctx->ro_inv.ensure(n);
 		morton_encode(reinterpret_cast<const float4*>(pos4), n, bmin, bmax, ctx->ro_keys.ptr,
 					  ctx->ro_s2o.ptr, st);
-		radix_sort_pairs(ctx->scratch, ctx->ro_keys.ptr, ctx->ro_s2o.ptr, n, st);
-		inverse_and_gather(ctx->ro_s2o.ptr, n, reinterpret_cast<const float4*>(pos4),
-						   ctx->ro_inv.ptr, nullptr, st);
+		radix_sort_pairs(ctx->scratch, ctx->ro_keys.ptr, ctx->ro_s2o.ptr, n, st, ctx->ro_inv.ptr);
 		ctx->ro_n = n;
 		ctx->built = false;  // every stored particle index changes: rebuild before use
 		ctx->win.valid = false;

@@ -102,14 +102,16 @@ __global__ void __launch_bounds__(256) batch_compact_kernel(
 __global__ void __launch_bounds__(256) batch_scatter_sorted_kernel(
 	const uint32_t* __restrict__ ckeys, const uint32_t* __restrict__ cidx, uint32_t m,
 	const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ cstart,
-	uint32_t* __restrict__ keys, uint32_t* __restrict__ s2o) {
+	uint32_t* __restrict__ keys, uint32_t* __restrict__ s2o, uint32_t* __restrict__ inv) {
 	const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
 	if (k >= m) return;
 	const uint32_t key = ckeys[k];
 	const uint32_t s = key >> kSysShift;
 	const uint32_t g = offsets[s] + (k - cstart[s]);
+	const uint32_t o = cidx[k];
 	keys[g] = key;
-	s2o[g] = cidx[k];
+	s2o[g] = o;
+	inv[o] = g;
 }
 
 // Row statistics of the whole list: stats[0] += entries, stats[1] = the
@@ -540,14 +542,13 @@ void batch_build(mb2_batch* b, const float4* pos, const int* type_ids, float rc,
 		if (m)
 			MB2_LAUNCH batch_scatter_sorted_kernel<<<(m + 255) / 256, 256, 0, st>>>(
 				b->ckeys.ptr, b->cidx.ptr, m, b->offsets_d.ptr, b->cstart.ptr, b->keys.ptr,
-				b->s2o.ptr);
+				b->s2o.ptr, b->inv.ptr);
 	} else {
 		if (n)
 			MB2_LAUNCH batch_encode_kernel<<<(n + 255) / 256, 256, 0, st>>>(
 				pos, b->sys_of.ptr, b->boxes.ptr, n, b->keys.ptr, b->s2o.ptr, b->outside.ptr);
-		radix_sort_pairs(b->scratch, b->keys.ptr, b->s2o.ptr, n, st);
+		radix_sort_pairs(b->scratch, b->keys.ptr, b->s2o.ptr, n, st, b->inv.ptr);
 	}
-	inverse_and_gather(b->s2o.ptr, n, pos, b->inv.ptr, nullptr, st);
 	pack_sorted_positions(pos, type_ids, b->s2o.ptr, n, b->sorted_pos.ptr, st);
 	b->cell_begin.ensure(b->total_cells);
 	b->cell_end.ensure(b->total_cells);

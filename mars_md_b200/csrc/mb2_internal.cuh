@@ -107,9 +107,10 @@ struct StencilEntry {
 // sort.cu
 void morton_encode(const float4* pos, uint32_t n, const float* bmin, const float* bmax,
 				   uint32_t* keys, uint32_t* idx, cudaStream_t st);
-void radix_sort_pairs(Scratch& s, uint32_t* keys, uint32_t* vals, uint32_t n, cudaStream_t st);
-void inverse_and_gather(const uint32_t* s2o, uint32_t n, const float4* pos, uint32_t* inv,
-						float4* sorted_pos, cudaStream_t st);
+// place_of (optional; the values are then 0 .. n - 1): the inverse of the
+// permutation, place_of[value] = sorted slot, left by the last pass.
+void radix_sort_pairs(Scratch& s, uint32_t* keys, uint32_t* vals, uint32_t n, cudaStream_t st,
+					  uint32_t* place_of = nullptr);
 // out[s] = in[s2o[s]] for elements of 4 or 16 bytes.
 void permute_gather(const void* in, const uint32_t* s2o, uint32_t n, int elem_bytes, void* out,
 					cudaStream_t st);
@@ -121,7 +122,7 @@ void remap_indices(int* idx, size_t count, const uint32_t* inv, uint32_t n, cuda
 size_t sort_work_words(uint32_t n);
 void radix_sort_pairs_into(uint32_t* keys, uint32_t* vals, uint32_t n, uint32_t* keys_alt,
 						   uint32_t* vals_alt, uint32_t* work, cudaStream_t st,
-						   uint32_t* report = nullptr);
+						   uint32_t* report = nullptr, uint32_t* place_of = nullptr);
 // noalloc.cu: the same sort over the library's static scratch (no allocation).
 void radix_sort_pairs_static(uint32_t* keys, uint32_t* vals, uint32_t n, cudaStream_t st);
 

@@ -82,12 +82,14 @@ __global__ void __launch_bounds__(kSortThreads) radix_hist_kernel(const uint32_t
 // (and report, where given): set when an earlier tile's counts never came. The
 // tile then writes nothing, nor do tiles that start after it, in this pass and the
 // next ones: a pass never reads slots that the one before it left unwritten.
+// place_of (the last pass of a sort whose values are 0 .. n - 1):
+// place_of[value] = output slot, the inverse of the permutation.
 template <int kItems>
 __global__ void __launch_bounds__(kSortThreads) radix_pass_kernel(
 	const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in, uint32_t n,
 	int pass, const uint32_t* __restrict__ hist, unsigned long long* status, uint32_t* ticket,
 	uint32_t* error, uint32_t* report, uint32_t* __restrict__ keys_out,
-	uint32_t* __restrict__ vals_out) {
+	uint32_t* __restrict__ vals_out, uint32_t* __restrict__ place_of) {
 	__shared__ uint32_t warp_count[kSortWarps][256];
 	__shared__ uint32_t warp_tot[2][kSortWarps];
 	__shared__ uint32_t tile_sh, stop_sh;
@@ -219,22 +221,12 @@ __global__ void __launch_bounds__(kSortThreads) radix_pass_kernel(
 		if (slot < here) {
 			const uint32_t out_key = sorted_key[slot];
 			const uint32_t dst = to_global[(out_key >> shift) & 255u] + slot;
+			const uint32_t out_val = sorted_val[slot];
 			keys_out[dst] = out_key;
-			vals_out[dst] = sorted_val[slot];
+			vals_out[dst] = out_val;
+			if (place_of) place_of[out_val] = dst;
 		}
 	}
-}
-
-__global__ void __launch_bounds__(256) inverse_gather_kernel(const uint32_t* __restrict__ s2o,
-															 uint32_t n,
-															 const float4* __restrict__ pos,
-															 uint32_t* __restrict__ inv,
-															 float4* __restrict__ sorted_pos) {
-	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-	if (i >= n) return;
-	const uint32_t o = s2o[i];
-	if (inv && o < n) inv[o] = i;
-	if (sorted_pos) sorted_pos[i] = pos[o];
 }
 
 // out[s] = in[s2o[s]] for 4- or 16-byte elements (DeviceParticle::permute).
@@ -311,11 +303,14 @@ __global__ void __launch_bounds__(256) rank_sort_kernel(const uint32_t* __restri
 __global__ void __launch_bounds__(256) copy_pairs_kernel(const uint32_t* __restrict__ keys_in,
 														 const uint32_t* __restrict__ vals_in,
 														 uint32_t n, uint32_t* __restrict__ keys,
-														 uint32_t* __restrict__ vals) {
+														 uint32_t* __restrict__ vals,
+														 uint32_t* __restrict__ place_of) {
 	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
 	if (i >= n) return;
+	const uint32_t v = vals_in[i];
 	keys[i] = keys_in[i];
-	vals[i] = vals_in[i];
+	vals[i] = v;
+	if (place_of) place_of[v] = i;
 }
 
 uint32_t sort_tiles(uint32_t n) {
@@ -335,14 +330,19 @@ size_t sort_work_words(uint32_t n) {
 }
 
 void radix_sort_pairs_into(uint32_t* keys, uint32_t* vals, uint32_t n, uint32_t* keys_alt,
-						   uint32_t* vals_alt, uint32_t* work, cudaStream_t st, uint32_t* report) {
-	if (n <= 1) return;
+						   uint32_t* vals_alt, uint32_t* work, cudaStream_t st, uint32_t* report,
+						   uint32_t* place_of) {
+	if (n == 0) return;
+	if (n == 1) {
+		if (place_of) MB2_CUDA(cudaMemsetAsync(place_of, 0, sizeof(uint32_t), st));
+		return;
+	}
 	if (n <= kRankSortMax) {
 		const size_t smem = static_cast<size_t>((n + 3u) / 4u) * sizeof(uint4);
 		MB2_LAUNCH rank_sort_kernel<<<(n + 31) / 32, 256, smem, st>>>(keys, vals, n, keys_alt,
 																	  vals_alt);
 		MB2_LAUNCH copy_pairs_kernel<<<(n + 255) / 256, 256, 0, st>>>(keys_alt, vals_alt, n, keys,
-																	  vals);
+																	  vals, place_of);
 		return;
 	}
 	const uint32_t tiles = sort_tiles(n);
@@ -356,17 +356,20 @@ void radix_sort_pairs_into(uint32_t* keys, uint32_t* vals, uint32_t n, uint32_t*
 										   : radix_pass_kernel<kLargeItems>;
 	for (int pass = 0; pass < 4; ++pass) {
 		MB2_LAUNCH pass_kernel<<<tiles, kSortThreads, 0, st>>>(
-			ks, vs, n, pass, work + 256 * pass, status, tickets + pass, error, report, kd, vd);
+			ks, vs, n, pass, work + 256 * pass, status, tickets + pass, error, report, kd, vd,
+			pass == 3 ? place_of : nullptr);
 		std::swap(ks, kd);
 		std::swap(vs, vd);
 	}
 	// Four passes: the sorted data is back in the caller's buffers.
 }
 
-void radix_sort_pairs(Scratch& s, uint32_t* keys, uint32_t* vals, uint32_t n, cudaStream_t st) {
-	if (n <= 1) return;
+void radix_sort_pairs(Scratch& s, uint32_t* keys, uint32_t* vals, uint32_t n, cudaStream_t st,
+					  uint32_t* place_of) {
+	if (n == 0) return;
 	s.ensure_sort(n, sort_work_words(n));
-	radix_sort_pairs_into(keys, vals, n, s.keys_alt.ptr, s.vals_alt.ptr, s.work.ptr, st, s.sort_error);
+	radix_sort_pairs_into(keys, vals, n, s.keys_alt.ptr, s.vals_alt.ptr, s.work.ptr, st, s.sort_error,
+						  place_of);
 }
 
 void morton_encode(const float4* pos, uint32_t n, const float* bmin, const float* bmax,
@@ -377,12 +380,6 @@ void morton_encode(const float4* pos, uint32_t n, const float* bmin, const float
 							   fmaxf(bmax[2] - bmin[2], 1e-6f));
 	if (n == 0) return;
 	MB2_LAUNCH morton_encode_kernel<<<(n + 255) / 256, 256, 0, st>>>(pos, n, lo, range, keys, idx);
-}
-
-void inverse_and_gather(const uint32_t* s2o, uint32_t n, const float4* pos, uint32_t* inv,
-						float4* sorted_pos, cudaStream_t st) {
-	if (n == 0) return;
-	MB2_LAUNCH inverse_gather_kernel<<<(n + 255) / 256, 256, 0, st>>>(s2o, n, pos, inv, sorted_pos);
 }
 
 void permute_gather(const void* in, const uint32_t* s2o, uint32_t n, int elem_bytes, void* out,

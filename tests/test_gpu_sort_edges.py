@@ -26,3 +26,17 @@ def test_sort_is_the_stable_sort(ctx_factory, n, bits):
     order = np.argsort(keys_np, kind="stable")
     assert np.array_equal(keys.cpu().numpy().view(np.uint32), keys_np[order])
     assert np.array_equal(vals.cpu().numpy(), vals_np[order])
+
+
+@pytest.mark.parametrize("n", [1, 2, 8192, 8193, 262144, 262145])
+def test_morton_sort_leaves_the_inverse(ctx_factory, n):
+    rng = np.random.default_rng(n)
+    pos = torch.from_numpy(rng.uniform(0.0, 50.0, (n, 4)).astype(np.float32)).cuda()
+    pos[n // 3:n // 2] = pos[0]   # one key many times: the sort is stable
+    keys, s2o, inv, sp = (t.cpu().numpy() for t in ctx_factory(n).sort_morton(
+        pos, [0.0, 0.0, 0.0], [50.0, 50.0, 50.0]))
+    keys = keys.view(np.uint32)
+    assert np.array_equal(np.sort(s2o), np.arange(n))
+    assert np.array_equal(inv[s2o], np.arange(n))
+    assert np.array_equal(sp, pos.cpu().numpy()[s2o])
+    assert np.all((keys[1:] > keys[:-1]) | ((keys[1:] == keys[:-1]) & (s2o[1:] > s2o[:-1])))
