@@ -1257,14 +1257,26 @@ void step_once(mb2_context* ctx, float4* pos, float4* fe, const int* type_ids,
 						ctx->types, ctx->box, p, bonded ? 1 : 0, st);
 }
 
+// Up to this many particles a step leaves the next one its packed positions
+// (NextPack): a launch and a pack's dependent loads less a step (64 x 1,024
+// polymers, 40 steps, 1,152 -> 1,060 us; 12 x 1,001 Langevin, 691 -> 647 us).
+// Beyond, bandwidth decides, and the scattered stores of the rows cost more than
+// the pack's scattered loads (20 steps at 300,007 beads 4,917 -> 4,990 us, at
+// 2,097,152 31.5 -> 32.1 ms).
+constexpr uint32_t kLeaveMax = 131072;
+
 // A step that is not a rebuild check, its number *ctx->step_d + offset: the
-// body mb2_run captures.
+// body mb2_run captures. packed: the step before it in the same graph left the
+// positions packed; leave: it does so for the step after it.
 void step_body_replayable(mb2_context* ctx, float4* pos, float4* fe, const int* type_ids,
 						  const uint32_t* flags, uint32_t n, const mb2_step_params* prm,
-						  uint64_t offset, cudaStream_t st) {
+						  uint64_t offset, bool packed, bool leave, cudaStream_t st) {
 	const bool bonded = step_has_bonded(prm);
-	pack_sorted_positions(pos, type_ids, ctx->s2o.ptr, n, ctx->sorted_pos.ptr, st, nullptr, nullptr,
-						  sorted_forces(ctx, n), bonded ? fe : nullptr, track_of(ctx));
+	NextPack next;
+	if (leave) next = NextPack{ctx->sorted_pos.ptr, sorted_forces(ctx, n), track_of(ctx)};
+	if (!packed)
+		pack_sorted_positions(pos, type_ids, ctx->s2o.ptr, n, ctx->sorted_pos.ptr, st, nullptr, nullptr,
+							  sorted_forces(ctx, n), bonded ? fe : nullptr, track_of(ctx));
 	pair_kernel(ctx, n, prm->cutoff, prm->get_energy, st, true);
 	bonded_stage(ctx, pos, fe, prm, prm->get_energy, st);
 	const StepClock clock{ctx->step_d.ptr, offset, prm->seed, prm->patch_id};
@@ -1272,12 +1284,12 @@ void step_body_replayable(mb2_context* ctx, float4* pos, float4* fe, const int* 
 		baoab_integrate_gather(pos, reinterpret_cast<float4*>(prm->mom4), fe,
 							   ctx->force_sorted.ptr, ctx->inv.ptr, bonded ? 1 : 0, type_ids, flags,
 							   n, ctx->types, ctx->box, prm->dt, prm->kT, 0u, 0u, 0u, prm->efield,
-							   prm->deferred_kick_pending ? 1 : 0, st, clock);
+							   prm->deferred_kick_pending ? 1 : 0, st, clock, next);
 		return;
 	}
 	BdParams p{prm->dt, prm->kT, 0u, 0u, 0u, {prm->efield[0], prm->efield[1], prm->efield[2]}};
 	bd_integrate_gather(pos, fe, ctx->force_sorted.ptr, ctx->inv.ptr, type_ids, flags, n,
-						ctx->types, ctx->box, p, bonded ? 1 : 0, st, clock);
+						ctx->types, ctx->box, p, bonded ? 1 : 0, st, clock, next);
 }
 
 uint64_t fbits(float f) {
@@ -1412,8 +1424,13 @@ int mb2_run(mb2_context* ctx, float* pos4, float* force_energy4, const int* type
 			const bool use_many = many > 1u && ahead >= many;
 			auto& g = use_many ? ctx->run_many : ctx->run_one;
 			const uint32_t steps = use_many ? many : 1u;
+			// Steps without bonded terms keep their three kernels: callers rely on
+			// three counted launches a step (tests/test_gpu_run.py); with two,
+			// 4,096 beads would take 950 us for 1,070 per 100 steps.
+			const bool leave = n <= kLeaveMax && step_has_bonded(prm);
 			capture_steps(g, key, steps, [&](uint32_t offset, cudaStream_t cs) {
-				step_body_replayable(ctx, pos, fe, type_ids, flags, n, prm, offset, cs);
+				step_body_replayable(ctx, pos, fe, type_ids, flags, n, prm, offset, leave && offset > 0u,
+									 leave && offset + 1u < steps, cs);
 			});
 			step_counter_set(ctx->step_d.ptr, step, st);
 			MB2_CUDA(cudaGraphLaunch(g.exec, st));

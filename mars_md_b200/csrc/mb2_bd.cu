@@ -213,6 +213,23 @@ __device__ __forceinline__ uint64_t mix_seed(uint64_t seed, uint64_t patch, uint
 	return (seed * 0x9E3779B97F4A7C15ULL) ^ (patch << 32) ^ (step * 0xBF58476D1CE4E5B9ULL);
 }
 
+// The tracked word so far, read by a warp's first lane ahead of its other loads.
+__device__ __forceinline__ unsigned int seen_of(const DisplacementTrack& t) {
+	return t.d2max && (threadIdx.x & 31) == 0
+			   ? *reinterpret_cast<volatile unsigned int*>(t.d2max) : 0u;
+}
+
+// Particle (row of the list's order, new position p) for the step after
+// (NextPack). All of a warp's `lanes` call it together.
+__device__ __forceinline__ void leave_next(const NextPack& next, uint32_t row, float4 p, int type,
+										   unsigned int seen, unsigned int lanes) {
+	next.forces[row] = make_float4(0.f, 0.f, 0.f, 0.f);
+	if (next.track.d2max)
+		raise_track(next.track, tracked_d2(next.track, p, next.track.ref_sorted[row]), seen, lanes);
+	p.w = __int_as_float(type);
+	next.sorted_pos[row] = p;
+}
+
 // Fused-step variant: the pair force is gathered from the Z-ordered
 // accumulator through the inverse permutation (random reads, coalesced
 // writes), added to what the bonded kernels left in ForceEnergy when any ran
@@ -224,12 +241,13 @@ __device__ __forceinline__ uint64_t mix_seed(uint64_t seed, uint64_t patch, uint
 // the wait for the force kernels (its base is set by a launch before the
 // graph, so it is readable by then). kGrids false (no grid loaded): without the grid
 // code the kernel takes fewer registers and more warps fit on an SM.
-template <bool kGrids>
+// kNext: see NextPack; the force is then read through next.forces, and cleared.
+template <bool kGrids, bool kNext>
 __global__ void __launch_bounds__(256) bd_gather_kernel(
 	float4* __restrict__ pos, float4* __restrict__ fe, const float4* __restrict__ fs,
 	const uint32_t* __restrict__ inv, const int* __restrict__ type_ids,
 	const uint32_t* __restrict__ flags, uint32_t n, TypeTable ty, Box box, BdParams bp,
-	int read_fe, StepClock clock) {
+	int read_fe, StepClock clock, NextPack next) {
 	chain_begin();
 	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
 	if (clock.ptr) {
@@ -239,8 +257,11 @@ __global__ void __launch_bounds__(256) bd_gather_kernel(
 	}
 	const float3 xi = bd_noise(bp.base_seed, bp.base_ctr + i, bp.step);
 	chain_wait();
+	const unsigned int seen = kNext ? seen_of(next.track) : 0u;
+	const unsigned int lanes = kNext ? __ballot_sync(0xFFFFFFFFu, i < n) : 0u;
 	if (i >= n) return;
-	float4 f = fs[inv[i]];
+	const uint32_t row = inv[i];
+	float4 f = kNext ? next.forces[row] : fs[row];
 	if (read_fe) {
 		const float4 ext = fe[i];
 		f.x = __fadd_rn(ext.x, f.x);
@@ -248,17 +269,22 @@ __global__ void __launch_bounds__(256) bd_gather_kernel(
 		f.z = __fadd_rn(ext.z, f.z);
 		f.w = __fadd_rn(ext.w, f.w);
 	}
-	if (flags && (flags[i] & kFlagRbAttached)) {
+	const bool attached = flags && (flags[i] & kFlagRbAttached);
+	if (!kNext && attached) {
 		fe[i] = f;
 		return;
 	}
-	const float4 p = pos[i];
+	float4 p = pos[i];
 	const int type = type_ids[i];
-	const float4 pmf = position_force<kGrids>(ty, type, p.x, p.y, p.z, bp.efield);
-	if (pmf.w != 0.0f) f.w = __fadd_rn(f.w, pmf.w);
-	fe[i] = f;
-	pos[i] = bd_update(p, __fadd_rn(f.x, pmf.x), __fadd_rn(f.y, pmf.y), __fadd_rn(f.z, pmf.z),
-					   ty.diffusion[type], xi, box, bp);
+	if (!attached) {
+		const float4 pmf = position_force<kGrids>(ty, type, p.x, p.y, p.z, bp.efield);
+		if (pmf.w != 0.0f) f.w = __fadd_rn(f.w, pmf.w);
+		p = bd_update(p, __fadd_rn(f.x, pmf.x), __fadd_rn(f.y, pmf.y), __fadd_rn(f.z, pmf.z),
+					  ty.diffusion[type], xi, box, bp);
+		pos[i] = p;
+	}
+	fe[i] = kNext && read_fe ? make_float4(0.f, 0.f, 0.f, 0.f) : f;
+	if (kNext) leave_next(next, row, p, type, seen, lanes);
 }
 
 // FORCE_CONVERSION_FACTOR, SQRT_CAL_TO_JOULE (src/Constants.h:30,34) and the
@@ -279,13 +305,13 @@ __device__ __forceinline__ float half_kick(float m, float f, float h) {
 // accumulator through the inverse permutation, plus what the bonded kernels
 // left in ForceEnergy when any ran (read_fe), and ForceEnergy receives the
 // sum as the reference leaves it.
-template <bool kGather>
+template <bool kGather, bool kNext>
 __global__ void __launch_bounds__(256) baoab_kernel(
 	float4* __restrict__ pos, float4* __restrict__ mom, float4* __restrict__ fe,
 	const float4* __restrict__ fs, const uint32_t* __restrict__ inv, int read_fe,
 	const int* __restrict__ type_ids, const uint32_t* __restrict__ flags, uint32_t n,
 	TypeTable ty, Box box, float dt, float kT, uint32_t step, uint64_t seed, uint32_t base_ctr,
-	float3 efield, int pending, StepClock clock) {
+	float3 efield, int pending, StepClock clock, NextPack next) {
 	chain_begin();
 	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
 	if (clock.ptr) {  // as bd_gather_kernel
@@ -295,11 +321,14 @@ __global__ void __launch_bounds__(256) baoab_kernel(
 	}
 	const float3 xi = bd_noise(seed, base_ctr + i, step, kBaoabStream);
 	chain_wait();
+	const unsigned int seen = kNext ? seen_of(next.track) : 0u;
+	const unsigned int lanes = kNext ? __ballot_sync(0xFFFFFFFFu, i < n) : 0u;
 	if (i >= n) return;
+	const uint32_t row = kGather ? inv[i] : 0u;
 	float4 p = pos[i];
 	float4 f;
 	if (kGather) {
-		f = fs[inv[i]];
+		f = kNext ? next.forces[row] : fs[row];
 		if (read_fe) {
 			const float4 ext = fe[i];
 			f.x = __fadd_rn(ext.x, f.x);
@@ -320,45 +349,49 @@ __global__ void __launch_bounds__(256) baoab_kernel(
 		f.w = __fadd_rn(f.w, pmf.w);
 		if (!kGather) fe[i] = f;
 	}
-	if (kGather) fe[i] = f;
-	if (flags && (flags[i] & kFlagRbAttached)) return;
-	float4 m = mom[i];
-	const float h = __fmul_rn(0.5f, dt);
-	if (pending) {
-		m.x = half_kick(m.x, f.x, h);
+	if (kGather) fe[i] = kNext && read_fe ? make_float4(0.f, 0.f, 0.f, 0.f) : f;
+	const bool attached = flags && (flags[i] & kFlagRbAttached);
+	if (!kNext && attached) return;
+	if (!attached) {
+		float4 m = mom[i];
+		const float h = __fmul_rn(0.5f, dt);
+		if (pending) {
+			m.x = half_kick(m.x, f.x, h);
+			m.y = half_kick(m.y, f.y, h);
+			m.z = half_kick(m.z, f.z, h);
+		}
+		m.x = half_kick(m.x, f.x, h);  // B
 		m.y = half_kick(m.y, f.y, h);
 		m.z = half_kick(m.z, f.z, h);
+		const float ms = ty.mass[type];
+		const float inv_m = __fdiv_rn(1.0f, ms);
+		auto drift = [&](float x, float mv) {
+			return __fadd_rn(x, __fmul_rn(__fmul_rn(__fmul_rn(h, mv), inv_m), 10000.0f));
+		};
+		p.x = drift(p.x, m.x);  // A
+		p.y = drift(p.y, m.y);
+		p.z = drift(p.z, m.z);
+		const float4 g = ty.damping[type];
+		auto ou = [&](float mv, float gamma, float r) {  // O
+			const float c = expf(__fmul_rn(-gamma, dt));
+			const float ns = __fmul_rn(
+				__fsqrt_rn(__fmul_rn(__fmul_rn(kT, ms), __fsub_rn(1.0f, __fmul_rn(c, c)))),
+				kSqrtCalToJoule);
+			return __fadd_rn(__fmul_rn(c, mv), __fmul_rn(ns, r));
+		};
+		m.x = ou(m.x, g.x, xi.x);
+		m.y = ou(m.y, g.y, xi.y);
+		m.z = ou(m.z, g.z, xi.z);
+		p.x = drift(p.x, m.x);  // A
+		p.y = drift(p.y, m.y);
+		p.z = drift(p.z, m.z);
+		if (box.periodic[0]) p.x = wrap_scalar(p.x, box.origin[0], box.size[0], box.inv[0]);
+		if (box.periodic[1]) p.y = wrap_scalar(p.y, box.origin[1], box.size[1], box.inv[1]);
+		if (box.periodic[2]) p.z = wrap_scalar(p.z, box.origin[2], box.size[2], box.inv[2]);
+		pos[i] = p;
+		mom[i] = m;
 	}
-	m.x = half_kick(m.x, f.x, h);  // B
-	m.y = half_kick(m.y, f.y, h);
-	m.z = half_kick(m.z, f.z, h);
-	const float ms = ty.mass[type];
-	const float inv_m = __fdiv_rn(1.0f, ms);
-	auto drift = [&](float x, float mv) {
-		return __fadd_rn(x, __fmul_rn(__fmul_rn(__fmul_rn(h, mv), inv_m), 10000.0f));
-	};
-	p.x = drift(p.x, m.x);  // A
-	p.y = drift(p.y, m.y);
-	p.z = drift(p.z, m.z);
-	const float4 g = ty.damping[type];
-	auto ou = [&](float mv, float gamma, float r) {  // O
-		const float c = expf(__fmul_rn(-gamma, dt));
-		const float ns = __fmul_rn(
-			__fsqrt_rn(__fmul_rn(__fmul_rn(kT, ms), __fsub_rn(1.0f, __fmul_rn(c, c)))),
-			kSqrtCalToJoule);
-		return __fadd_rn(__fmul_rn(c, mv), __fmul_rn(ns, r));
-	};
-	m.x = ou(m.x, g.x, xi.x);
-	m.y = ou(m.y, g.y, xi.y);
-	m.z = ou(m.z, g.z, xi.z);
-	p.x = drift(p.x, m.x);  // A
-	p.y = drift(p.y, m.y);
-	p.z = drift(p.z, m.z);
-	if (box.periodic[0]) p.x = wrap_scalar(p.x, box.origin[0], box.size[0], box.inv[0]);
-	if (box.periodic[1]) p.y = wrap_scalar(p.y, box.origin[1], box.size[1], box.inv[1]);
-	if (box.periodic[2]) p.z = wrap_scalar(p.z, box.origin[2], box.size[2], box.inv[2]);
-	pos[i] = p;
-	mom[i] = m;
+	if (kNext) leave_next(next, row, p, type, seen, lanes);
 }
 
 __global__ void __launch_bounds__(256) baoab_last_kernel(float4* __restrict__ mom,
@@ -440,12 +473,15 @@ uint32_t integrate_threads(uint32_t n) { return n <= 148u * 256u ? 64u : 256u; }
 void bd_integrate_gather(float4* pos, float4* fe, const float4* force_sorted, const uint32_t* inv,
 						 const int* type_ids, const uint32_t* flags, uint32_t n,
 						 const TypeTable& types, const Box& box, const BdParams& p, int read_fe,
-						 cudaStream_t st, const StepClock& clock) {
+						 cudaStream_t st, const StepClock& clock, const NextPack& next) {
 	if (n == 0) return;
-	auto kern = types.num_grids == 0 ? bd_gather_kernel<false> : bd_gather_kernel<true>;
+	auto kern = next.sorted_pos
+					? (types.num_grids == 0 ? bd_gather_kernel<false, true> : bd_gather_kernel<true, true>)
+					: (types.num_grids == 0 ? bd_gather_kernel<false, false>
+											: bd_gather_kernel<true, false>);
 	const uint32_t threads = integrate_threads(n);
 	launch_chained(kern, (n + threads - 1) / threads, threads, 0, st, pos, fe, force_sorted, inv,
-				   type_ids, flags, n, types, box, p, read_fe, clock);
+				   type_ids, flags, n, types, box, p, read_fe, clock, next);
 }
 
 void baoab_integrate(float4* pos, float4* mom, float4* fe, const int* type_ids,
@@ -453,9 +489,9 @@ void baoab_integrate(float4* pos, float4* mom, float4* fe, const int* type_ids,
 					 float dt, float kT, uint32_t step, uint64_t base_seed, uint32_t base_ctr,
 					 const float* efield, int pending, cudaStream_t st) {
 	if (n == 0) return;
-	MB2_LAUNCH baoab_kernel<false><<<(n + 255) / 256, 256, 0, st>>>(
+	MB2_LAUNCH baoab_kernel<false, false><<<(n + 255) / 256, 256, 0, st>>>(
 		pos, mom, fe, nullptr, nullptr, 0, type_ids, flags, n, types, box, dt, kT, step, base_seed,
-		base_ctr, make_float3(efield[0], efield[1], efield[2]), pending, StepClock{});
+		base_ctr, make_float3(efield[0], efield[1], efield[2]), pending, StepClock{}, NextPack{});
 }
 
 void baoab_integrate_gather(float4* pos, float4* mom, float4* fe, const float4* force_sorted,
@@ -463,13 +499,14 @@ void baoab_integrate_gather(float4* pos, float4* mom, float4* fe, const float4* 
 							const uint32_t* flags, uint32_t n, const TypeTable& types,
 							const Box& box, float dt, float kT, uint32_t step, uint64_t base_seed,
 							uint32_t base_ctr, const float* efield, int pending, cudaStream_t st,
-							const StepClock& clock) {
+							const StepClock& clock, const NextPack& next) {
 	if (n == 0) return;
 	const uint32_t threads = integrate_threads(n);
-	launch_chained(baoab_kernel<true>, (n + threads - 1) / threads, threads, 0, st, pos, mom, fe,
+	auto kern = next.sorted_pos ? baoab_kernel<true, true> : baoab_kernel<true, false>;
+	launch_chained(kern, (n + threads - 1) / threads, threads, 0, st, pos, mom, fe,
 				   force_sorted, inv, read_fe, type_ids, flags, n, types, box, dt, kT, step,
 				   base_seed, base_ctr, make_float3(efield[0], efield[1], efield[2]), pending,
-				   clock);
+				   clock, next);
 }
 
 void baoab_last_update(float4* mom, const float4* fe, const uint32_t* flags, uint32_t n,

@@ -205,6 +205,48 @@ struct DisplacementTrack {
 };
 DisplacementTrack displacement_track(const Box& box, const float4* ref_sorted,
 									 unsigned int* d2max);
+#ifdef __CUDACC__
+// DisplacementKernel::min_image (AdaptiveKernels.h:56-65). Both inputs are
+// wrapped, so one step suffices; the loops are capped so that a non-finite or
+// unwrapped input can never keep a thread spinning.
+__device__ __forceinline__ float min_image(float d, float l) {
+	if (l <= 0.0f) return d;
+	const float h = 0.5f * l;
+	for (int it = 0; it < 8 && d > h; ++it) d = __fsub_rn(d, l);
+	for (int it = 0; it < 8 && d < -h; ++it) d = __fadd_rn(d, l);
+	return d;
+}
+// The squared displacement of p from its position r at the build.
+__device__ __forceinline__ float tracked_d2(const DisplacementTrack& t, const float4& p,
+											const float4& r) {
+	const float d2 = len2(min_image(__fsub_rn(p.x, r.x), t.len[0]),
+						  min_image(__fsub_rn(p.y, r.y), t.len[1]),
+						  min_image(__fsub_rn(p.z, r.z), t.len[2]));
+	const float c[3] = {p.x, p.y, p.z};
+	bool inside = d2 <= 3.402823466e38f;  // false for NaN and infinity
+#pragma unroll
+	for (int a = 0; a < 3; ++a)
+		inside = inside && (t.len[a] == 0.0f || (c[a] >= t.lo[a] && c[a] <= t.hi[a]));
+	return inside ? d2 : INFINITY;
+}
+// Raises the word to the largest d2 of a warp's `lanes`, which all call this.
+// Non-negative floats order like their bit patterns; the word only grows between
+// builds, so most warps find nothing to raise above what was `seen`.
+__device__ __forceinline__ void raise_track(const DisplacementTrack& t, float d2,
+											unsigned int seen, unsigned int lanes) {
+	const unsigned int bits = __reduce_max_sync(lanes, __float_as_uint(d2));
+	if ((threadIdx.x & 31) == 0 && bits > seen) atomicMax(t.d2max, bits);
+}
+#endif
+// What an integrate leaves for the step after it in place of that step's pack: the
+// new positions in the list's order, the pair-force accumulator cleared (each
+// particle's as it is read) and the displacement tracked; ForceEnergy, where
+// bonded terms add to it, zero instead of this step's. Off: sorted_pos == nullptr.
+struct NextPack {
+	float4* sorted_pos = nullptr;
+	float4* forces = nullptr;
+	DisplacementTrack track;
+};
 // odd (optional, with box): odd[0] incremented once per particle with a NaN or
 // infinite coordinate, odd[2] set when one lies more than half a box outside a
 // periodic axis.
@@ -380,7 +422,8 @@ struct StepClock {
 void bd_integrate_gather(float4* pos, float4* fe, const float4* force_sorted, const uint32_t* inv,
 						 const int* type_ids, const uint32_t* flags, uint32_t n,
 						 const TypeTable& types, const Box& box, const BdParams& p, int read_fe,
-						 cudaStream_t st, const StepClock& clock = StepClock{});
+						 cudaStream_t st, const StepClock& clock = StepClock{},
+						 const NextPack& next = NextPack{});
 // Langevin BAOAB (Integrator/BAOAB.h): with grids, ForceEnergy += position
 // force for every particle; `pending` applies the deferred closing half-kick
 // first; then B-A-O-A and wrap. Noise key (seed, base_ctr + i, step, stream 0x1356914).
@@ -395,7 +438,7 @@ void baoab_integrate_gather(float4* pos, float4* mom, float4* fe, const float4* 
 							const uint32_t* flags, uint32_t n, const TypeTable& types,
 							const Box& box, float dt, float kT, uint32_t step, uint64_t base_seed,
 							uint32_t base_ctr, const float* efield, int pending, cudaStream_t st,
-							const StepClock& clock = StepClock{});
+							const StepClock& clock = StepClock{}, const NextPack& next = NextPack{});
 // BAOAB_LastUpdate: mom += 0.5 dt F (closing half-kick) for non-frozen particles.
 void baoab_last_update(float4* mom, const float4* fe, const uint32_t* flags, uint32_t n,
 					   float dt, cudaStream_t st);

