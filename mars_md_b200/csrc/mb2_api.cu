@@ -108,7 +108,7 @@ struct mb2_context {
 		mb2_step_params prm{};
 		const int* type_ids = nullptr;
 	} win;
-	DevBuf<float4> ckpt, states, wpos, wfe, lam, mu, mu_sorted, tan, tan_sorted;
+	DevBuf<float4> ckpt, states, wfe, lam, mu, mu_sorted, tan, tan_sorted;
 	DevBuf<double4> adj_tan, adj_tan_sorted;  // FP64 tangent accumulators of the reverse sweep
 	float4* record_states = nullptr;  // caller's buffer for the states a reverse sweep differentiates
 	uint64_t record_cap = 0;          // its capacity in float4 rows
@@ -597,25 +597,39 @@ bool step_has_bonded(const mb2_step_params* prm) {
 		   prm->num_restraints != 0;
 }
 
+// Up to this many particles a step leaves the next one its packed positions
+// (NextPack): a launch and a pack's dependent loads less a step (64 x 1,024
+// polymers, 40 steps, 1,152 -> 1,060 us; 12 x 1,001 Langevin, 691 -> 647 us).
+// Beyond, bandwidth decides, and the scattered stores of the rows cost more than
+// the pack's scattered loads (20 steps at 300,007 beads 4,917 -> 4,990 us, at
+// 2,097,152 31.5 -> 32.1 ms).
+constexpr uint32_t kLeaveMax = 131072;
+
 // One step of the window without the rebuild decision (the segment's list
-// was built at its first step): the mb2_step sequence otherwise.
-void window_step(mb2_context* ctx, float4* pos, float4* fe, const int* type_ids, uint32_t n,
-				 uint64_t step, const mb2_step_params* prm, cudaStream_t st) {
+// was built at its first step): the mb2_step sequence otherwise, from the
+// positions `from` to `to` (the same array: in place). packed, leave: the step
+// before left the positions packed, this one does so for the next (NextPack).
+void window_step(mb2_context* ctx, const float4* from, float4* to, float4* fe, const int* type_ids,
+				 uint32_t n, uint64_t step, bool packed, bool leave, const mb2_step_params* prm,
+				 cudaStream_t st) {
 	const bool bonded = prm->num_bonds != 0 || prm->num_angles != 0;
-	pack_sorted_positions(pos, type_ids, ctx->s2o.ptr, n, ctx->sorted_pos.ptr, st, nullptr, nullptr,
-						  sorted_forces(ctx, n), bonded ? fe : nullptr, track_of(ctx));
+	NextPack next;
+	if (leave) next = NextPack{ctx->sorted_pos.ptr, sorted_forces(ctx, n), track_of(ctx)};
+	if (!packed)
+		pack_sorted_positions(from, type_ids, ctx->s2o.ptr, n, ctx->sorted_pos.ptr, st, nullptr, nullptr,
+							  sorted_forces(ctx, n), bonded ? fe : nullptr, track_of(ctx));
 	pair_kernel(ctx, n, prm->cutoff, 0, st, true);
 	if (bonded)
 		bond_angle_forces(reinterpret_cast<const int2*>(prm->bonds2), prm->bond_table_idx,
 						  prm->num_bonds, ctx->bonded_tables[0].ptr,
 						  reinterpret_cast<const int4*>(prm->angles4), prm->angle_table_idx,
-						  prm->num_angles, ctx->bonded_tables[1].ptr, pos, fe, ctx->box, 0,
+						  prm->num_angles, ctx->bonded_tables[1].ptr, from, fe, ctx->box, 0,
 						  ctx->energy.ptr + 2, ctx->energy.ptr + 3, st);
 	BdParams p{prm->dt, prm->kT, static_cast<uint32_t>(step),
 			   mb2_bd_seed(prm->seed, prm->patch_id, step), 0u,
 			   {prm->efield[0], prm->efield[1], prm->efield[2]}};
-	bd_integrate_gather(pos, fe, ctx->force_sorted.ptr, ctx->inv.ptr, type_ids, nullptr, n,
-						ctx->types, ctx->box, p, bonded ? 1 : 0, st);
+	bd_integrate_gather(from, to, fe, ctx->force_sorted.ptr, ctx->inv.ptr, type_ids, nullptr, n,
+						ctx->types, ctx->box, p, bonded ? 1 : 0, st, StepClock{}, next);
 }
 
 void copy4(float4* dst, const float4* src, uint32_t n, cudaStream_t st) {
@@ -1253,17 +1267,9 @@ void step_once(mb2_context* ctx, float4* pos, float4* fe, const int* type_ids,
 	BdParams p{prm->dt, prm->kT, static_cast<uint32_t>(step),
 			   mb2_bd_seed(prm->seed, prm->patch_id, step), 0u,
 			   {prm->efield[0], prm->efield[1], prm->efield[2]}};
-	bd_integrate_gather(pos, fe, ctx->force_sorted.ptr, ctx->inv.ptr, type_ids, flags, n,
+	bd_integrate_gather(pos, pos, fe, ctx->force_sorted.ptr, ctx->inv.ptr, type_ids, flags, n,
 						ctx->types, ctx->box, p, bonded ? 1 : 0, st);
 }
-
-// Up to this many particles a step leaves the next one its packed positions
-// (NextPack): a launch and a pack's dependent loads less a step (64 x 1,024
-// polymers, 40 steps, 1,152 -> 1,060 us; 12 x 1,001 Langevin, 691 -> 647 us).
-// Beyond, bandwidth decides, and the scattered stores of the rows cost more than
-// the pack's scattered loads (20 steps at 300,007 beads 4,917 -> 4,990 us, at
-// 2,097,152 31.5 -> 32.1 ms).
-constexpr uint32_t kLeaveMax = 131072;
 
 // A step that is not a rebuild check, its number *ctx->step_d + offset: the
 // body mb2_run captures. packed: the step before it in the same graph left the
@@ -1288,7 +1294,7 @@ void step_body_replayable(mb2_context* ctx, float4* pos, float4* fe, const int* 
 		return;
 	}
 	BdParams p{prm->dt, prm->kT, 0u, 0u, 0u, {prm->efield[0], prm->efield[1], prm->efield[2]}};
-	bd_integrate_gather(pos, fe, ctx->force_sorted.ptr, ctx->inv.ptr, type_ids, flags, n,
+	bd_integrate_gather(pos, pos, fe, ctx->force_sorted.ptr, ctx->inv.ptr, type_ids, flags, n,
 						ctx->types, ctx->box, p, bonded ? 1 : 0, st, clock, next);
 }
 
@@ -1462,6 +1468,7 @@ int mb2_window_forward(mb2_context* ctx, float* pos4, float* force_energy4, cons
 		float4* pos = reinterpret_cast<float4*>(pos4);
 		float4* fe = reinterpret_cast<float4*>(force_energy4);
 		const uint32_t segs = (num_steps + checkpoint_every - 1) / checkpoint_every;
+		const bool leave = n <= kLeaveMax;
 		ctx->ckpt.ensure(static_cast<size_t>(std::max<uint32_t>(segs, 1)) * n);
 		for (uint32_t sgi = 0; sgi < segs; ++sgi) {
 			const uint32_t k0 = sgi * checkpoint_every;
@@ -1469,7 +1476,8 @@ int mb2_window_forward(mb2_context* ctx, float* pos4, float* force_energy4, cons
 			copy4(ctx->ckpt.ptr + static_cast<size_t>(sgi) * n, pos, n, st);
 			build(ctx, pos, type_ids, n, prm->pairlist_cutoff, prm->cutoff, st, true);
 			for (uint32_t k = k0; k < k1; ++k)
-				window_step(ctx, pos, fe, type_ids, n, first_step + k, prm, st);
+				window_step(ctx, pos, pos, fe, type_ids, n, first_step + k, leave && k > k0,
+							leave && k + 1 < k1, prm, st);
 		}
 		ctx->win.valid = true;
 		ctx->win.n = n;
@@ -1513,12 +1521,13 @@ int mb2_window_backward(mb2_context* ctx, const float* grad_final4, float* grad_
 		const cudaStream_t st = S(stream);
 		const uint32_t n = w.n, C = w.every;
 		const uint32_t segs = (w.num_steps + C - 1) / C;
+		const bool leave = n <= kLeaveMax;
 		require(!ctx->record_states ||
 					ctx->record_cap >= static_cast<uint64_t>(w.num_steps) * n,
 				MB2_ERR_CAPACITY,
 				"mb2_window_backward: the recorded-states buffer holds fewer than steps x n rows");
 		ctx->states.ensure(static_cast<size_t>(C) * n);
-		for (auto* b : {&ctx->wpos, &ctx->wfe, &ctx->lam, &ctx->mu, &ctx->mu_sorted})
+		for (auto* b : {&ctx->wfe, &ctx->lam, &ctx->mu, &ctx->mu_sorted})
 			b->ensure(n);
 		ctx->adj_tan.ensure(n);
 		ctx->adj_tan_sorted.ensure(n);
@@ -1552,14 +1561,14 @@ int mb2_window_backward(mb2_context* ctx, const float* grad_final4, float* grad_
 			const uint32_t k0 = sgi * C;
 			const uint32_t k1 = std::min(w.num_steps, k0 + C);
 			// Recompute the segment from its checkpoint, keeping every state.
-			copy4(ctx->wpos.ptr, ctx->ckpt.ptr + static_cast<size_t>(sgi) * n, n, st);
-			build(ctx, ctx->wpos.ptr, w.type_ids, n, prm->pairlist_cutoff, prm->cutoff, st, true);
-			for (uint32_t k = k0; k < k1; ++k) {
-				copy4(ctx->states.ptr + static_cast<size_t>(k - k0) * n, ctx->wpos.ptr, n, st);
-				if (k + 1 < k1)
-					window_step(ctx, ctx->wpos.ptr, ctx->wfe.ptr, w.type_ids, n, w.first_step + k,
-								prm, st);
-			}
+			// (Each step writes the next state; copies between them would also part
+			// the chained launches.)
+			float4* x = ctx->states.ptr;
+			copy4(x, ctx->ckpt.ptr + static_cast<size_t>(sgi) * n, n, st);
+			build(ctx, x, w.type_ids, n, prm->pairlist_cutoff, prm->cutoff, st, true);
+			for (uint32_t k = k0; k + 1 < k1; ++k, x += n)
+				window_step(ctx, x, x + n, ctx->wfe.ptr, w.type_ids, n, w.first_step + k,
+							leave && k > k0, leave && k + 2 < k1, prm, st);
 			if (ctx->record_states)
 				MB2_CUDA(cudaMemcpyAsync(ctx->record_states + static_cast<size_t>(k0) * n,
 										 ctx->states.ptr,

@@ -244,7 +244,7 @@ __device__ __forceinline__ void leave_next(const NextPack& next, uint32_t row, f
 // kNext: see NextPack; the force is then read through next.forces, and cleared.
 template <bool kGrids, bool kNext>
 __global__ void __launch_bounds__(256) bd_gather_kernel(
-	float4* __restrict__ pos, float4* __restrict__ fe, const float4* __restrict__ fs,
+	const float4* from, float4* pos, float4* __restrict__ fe, const float4* __restrict__ fs,
 	const uint32_t* __restrict__ inv, const int* __restrict__ type_ids,
 	const uint32_t* __restrict__ flags, uint32_t n, TypeTable ty, Box box, BdParams bp,
 	int read_fe, StepClock clock, NextPack next) {
@@ -274,7 +274,7 @@ __global__ void __launch_bounds__(256) bd_gather_kernel(
 		fe[i] = f;
 		return;
 	}
-	float4 p = pos[i];
+	float4 p = from[i];
 	const int type = type_ids[i];
 	if (!attached) {
 		const float4 pmf = position_force<kGrids>(ty, type, p.x, p.y, p.z, bp.efield);
@@ -470,8 +470,8 @@ namespace {
 uint32_t integrate_threads(uint32_t n) { return n <= 148u * 256u ? 64u : 256u; }
 }  // namespace
 
-void bd_integrate_gather(float4* pos, float4* fe, const float4* force_sorted, const uint32_t* inv,
-						 const int* type_ids, const uint32_t* flags, uint32_t n,
+void bd_integrate_gather(const float4* from, float4* pos, float4* fe, const float4* force_sorted,
+						 const uint32_t* inv, const int* type_ids, const uint32_t* flags, uint32_t n,
 						 const TypeTable& types, const Box& box, const BdParams& p, int read_fe,
 						 cudaStream_t st, const StepClock& clock, const NextPack& next) {
 	if (n == 0) return;
@@ -480,8 +480,8 @@ void bd_integrate_gather(float4* pos, float4* fe, const float4* force_sorted, co
 					: (types.num_grids == 0 ? bd_gather_kernel<false, false>
 											: bd_gather_kernel<true, false>);
 	const uint32_t threads = integrate_threads(n);
-	launch_chained(kern, (n + threads - 1) / threads, threads, 0, st, pos, fe, force_sorted, inv,
-				   type_ids, flags, n, types, box, p, read_fe, clock, next);
+	launch_chained(kern, (n + threads - 1) / threads, threads, 0, st, from, pos, fe, force_sorted,
+				   inv, type_ids, flags, n, types, box, p, read_fe, clock, next);
 }
 
 void baoab_integrate(float4* pos, float4* mom, float4* fe, const int* type_ids,

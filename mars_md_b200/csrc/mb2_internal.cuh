@@ -409,7 +409,8 @@ struct BdParams {
 };
 void bd_integrate(float4* pos, float4* fe, const int* type_ids, const uint32_t* flags, uint32_t n,
 				  const TypeTable& types, const Box& box, const BdParams& p, cudaStream_t st);
-// The fused step's integrate: force = force_sorted[inv[i]] (+ fe[i] if read_fe).
+// The fused step's integrate: force = force_sorted[inv[i]] (+ fe[i] if read_fe),
+// from the positions `from` to pos (the same array: in place).
 // clock.ptr non-null: the step number is *clock.ptr + clock.offset at run time
 // (a replayed graph, whose base a step_counter_set launched before it sets) and
 // the Philox key is mixed on the device from seed and patch_id; p.step and
@@ -419,8 +420,8 @@ struct StepClock {
 	unsigned long long offset = 0;
 	uint64_t seed = 0, patch_id = 0;
 };
-void bd_integrate_gather(float4* pos, float4* fe, const float4* force_sorted, const uint32_t* inv,
-						 const int* type_ids, const uint32_t* flags, uint32_t n,
+void bd_integrate_gather(const float4* from, float4* pos, float4* fe, const float4* force_sorted,
+						 const uint32_t* inv, const int* type_ids, const uint32_t* flags, uint32_t n,
 						 const TypeTable& types, const Box& box, const BdParams& p, int read_fe,
 						 cudaStream_t st, const StepClock& clock = StepClock{},
 						 const NextPack& next = NextPack{});
