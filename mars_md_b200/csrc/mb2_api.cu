@@ -267,14 +267,15 @@ void morton_domain(mb2_context* ctx, const float4* pos, uint32_t n, cudaStream_t
 
 void sort_particles(mb2_context* ctx, const float4* pos, const int* type_ids, uint32_t n,
 					const float* bmin, const float* bmax, cudaStream_t st,
-					unsigned long long* odd) {
+					unsigned long long* odd, const DisplacementTrack& track) {
 	ctx->keys.ensure(n);
 	ctx->s2o.ensure(n);
 	ctx->inv.ensure(n);
 	ctx->sorted_pos.ensure(n);
 	morton_encode(pos, n, bmin, bmax, ctx->keys.ptr, ctx->s2o.ptr, st);
 	radix_sort_pairs(ctx->scratch, ctx->keys.ptr, ctx->s2o.ptr, n, st, ctx->inv.ptr);
-	pack_sorted_positions(pos, type_ids, ctx->s2o.ptr, n, ctx->sorted_pos.ptr, st, odd, &ctx->box);
+	pack_sorted_positions(pos, type_ids, ctx->s2o.ptr, n, ctx->sorted_pos.ptr, st, odd, &ctx->box,
+						  nullptr, nullptr, track);
 }
 
 // cutoff: the interaction cutoff the list will serve. When it lies in
@@ -300,7 +301,28 @@ void build(mb2_context* ctx, const float4* pos, const int* type_ids, uint32_t n,
 	ctx->stats.ensure(kBuildStats);
 	MB2_CUDA(cudaMemsetAsync(ctx->stats.ptr + 2, 0, (kBuildStats - 2) * sizeof(unsigned long long), st));
 	ctx->scratch.sort_error = reinterpret_cast<uint32_t*>(ctx->stats.ptr + 3);
-	sort_particles(ctx, pos, type_ids, n, bmin, bmax, st, ctx->stats.ptr + 2);
+	const float split = row_split(ctx->pt, ctx->box, rc_list, cutoff);
+	const bool near_last = split_ends_early(split, cutoff);
+	// Rows whose far entries are mostly not read (ends_early) count as their
+	// near part, unless the caller's kernels read all of them (the adjoint's).
+	// Below some 16,000 particles a step is launches and latency: a 4,096-bead
+	// run lost 12 % to the tracking pack, 12,012 beads were level and 65,536
+	// gained 12 %.
+	const bool ends_early = near_last && n > 16384u;
+	// The displacement since this build is tracked where it saves the pair
+	// kernel the rows' far part, and above kSmallN particles, where the inner
+	// rows save it 2.6 % at 2,097,152 beads (on a 65,536-bead step the pack's
+	// extra read and reduction cost more for those alone, 1-2 us). The word
+	// starts at zero, or at infinity where this pack meets a particle outside
+	// the box: the step that builds packs no more before its pair kernel.
+	const bool tracked = n > kSmallN || ends_early;
+	DisplacementTrack start;
+	if (tracked) {
+		ctx->d2max.ensure(1);
+		MB2_CUDA(cudaMemsetAsync(ctx->d2max.ptr, 0, sizeof(unsigned int), st));
+		start = displacement_track(ctx->box, nullptr, ctx->d2max.ptr);
+	}
+	sort_particles(ctx, pos, type_ids, n, bmin, bmax, st, ctx->stats.ptr + 2, start);
 
 	const float rc2 = rc_list * rc_list;
 	if (!ctx->grid_valid || ctx->grid_rc != rc_list || ctx->grid_n != n ||
@@ -330,9 +352,8 @@ void build(mb2_context* ctx, const float4* pos, const int* type_ids, uint32_t n,
 	wg.m = g.m;
 	wg.shift = g.shift;
 	wg.rc2 = rc2;
-	const float split = row_split(ctx->pt, ctx->box, rc_list, cutoff);
 	wg.split2 = split > 0.0f ? split * split : INFINITY;
-	wg.near_last = split_ends_early(split, cutoff) ? 1 : 0;
+	wg.near_last = near_last ? 1 : 0;
 	// Coordinates the walk's cheap distances round: the box, or on an open axis
 	// the particles' extent.
 	Box around = ctx->box;
@@ -371,12 +392,6 @@ void build(mb2_context* ctx, const float4* pos, const int* type_ids, uint32_t n,
 	// step than 8 or 4 at 4,096 (21.3 against 23.3 us), 32,768 (54.9 / 58.5)
 	// and 65,536 beads (polymers, 52.9 / 55.5); at 2,097,152 beads 8 lanes are
 	// the fastest.
-	// Rows whose far entries are mostly not read (ends_early) count as their
-	// near part, unless the caller's kernels read all of them (the adjoint's).
-	// Below some 16,000 particles a step is launches and latency: a 4,096-bead
-	// run lost 12 % to the tracking pack, 12,012 beads were level and 65,536
-	// gained 12 %.
-	const bool ends_early = wg.near_last && n > 16384u;
 	auto choose_lanes = [&](double mean) {
 		if (ctx->lanes_request) return ctx->lanes_request;
 		if (ends_early && !whole_rows) {
@@ -422,20 +437,14 @@ void build(mb2_context* ctx, const float4* pos, const int* type_ids, uint32_t n,
 	ctx->ref_pos.ensure(n);
 	MB2_CUDA(cudaMemcpyAsync(ctx->ref_pos.ptr, pos, static_cast<size_t>(n) * sizeof(float4),
 							 cudaMemcpyDeviceToDevice, st));
-	// and, in Z order, the origin of the displacement the packs track: where
-	// it saves the pair kernel the rows' far part, and above kSmallN
-	// particles, where the inner rows save it 2.6 % at 2,097,152 beads (on a
-	// 65,536-bead step the pack's extra read and reduction cost more for
-	// those alone, 1-2 us).
+	// and, in Z order, the origin of the displacement the packs track.
 	ctx->track_rc = 0.0f;
-	ctx->split = wg.near_last ? split : 0.0f;
-	if (n > kSmallN || ends_early) {
+	ctx->split = near_last ? split : 0.0f;
+	if (tracked) {
 		ctx->ref_sorted.ensure(n);
-		ctx->d2max.ensure(1);
 		MB2_CUDA(cudaMemcpyAsync(ctx->ref_sorted.ptr, ctx->sorted_pos.ptr,
 								 static_cast<size_t>(n) * sizeof(float4), cudaMemcpyDeviceToDevice,
 								 st));
-		MB2_CUDA(cudaMemsetAsync(ctx->d2max.ptr, 0, sizeof(unsigned int), st));
 		ctx->track_rc = rc_list;
 	}
 	ctx->num_pairs = stats.first;

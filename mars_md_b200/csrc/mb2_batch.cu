@@ -151,11 +151,13 @@ __global__ void __launch_bounds__(256) batch_row_stats_kernel(const uint32_t* __
 }
 
 // The list-build snapshot of the rebuilt systems' positions (flags null:
-// every system), from which their displacements are measured.
+// every system), from which their displacements are measured: zero so far, or
+// without bound when the build met a particle far outside its box (*outside).
 __global__ void __launch_bounds__(256) batch_snapshot_kernel(const float4* __restrict__ pos,
 															 const uint32_t* __restrict__ sys_of,
 															 const uint32_t* __restrict__ offsets,
 															 const uint32_t* __restrict__ flags,
+															 const uint32_t* __restrict__ outside,
 															 uint32_t n, float4* __restrict__ ref,
 															 unsigned int* __restrict__ moved) {
 	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -163,7 +165,7 @@ __global__ void __launch_bounds__(256) batch_snapshot_kernel(const float4* __res
 	const uint32_t s = sys_of[i];
 	if (flags && !flags[s]) return;
 	ref[i] = pos[i];
-	if (i == offsets[s]) moved[s] = 0u;
+	if (i == offsets[s]) moved[s] = *outside ? 0x7F800000u : 0u;
 }
 
 // The step's pack: Z-ordered positions, the pair-force accumulator cleared,
@@ -624,7 +626,8 @@ void batch_build(mb2_batch* b, const float4* pos, const int* type_ids, float rc,
 	b->moved.ensure(b->num_systems);
 	if (n)
 		MB2_LAUNCH batch_snapshot_kernel<<<(n + 255) / 256, 256, 0, st>>>(
-			pos, b->sys_of.ptr, b->offsets_d.ptr, dflags, n, b->ref_pos.ptr, b->moved.ptr);
+			pos, b->sys_of.ptr, b->offsets_d.ptr, dflags, b->outside.ptr, n, b->ref_pos.ptr,
+			b->moved.ptr);
 	b->num_pairs = stats.first;
 	b->built = true;
 	b->system_rebuilds += rebuilt;

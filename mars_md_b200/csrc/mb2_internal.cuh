@@ -193,7 +193,8 @@ void max_displacement_sq(const float4* cur, const float4* prev, uint32_t n, cons
 // kept by the step's pack: d2max (a device word) holds its square as float
 // bits, raised with atomicMax and cleared at each build; +inf when a position
 // is not finite or lies outside a periodic axis of the box by more than
-// kTrackBand. ref_sorted: the Z-ordered positions the list was built from.
+// kTrackBand. ref_sorted: the Z-ordered positions the list was built from (null
+// in the build's own pack: nothing has moved yet).
 // d2max == nullptr: not tracked.
 constexpr float kTrackBand = 0.5f;
 struct DisplacementTrack {

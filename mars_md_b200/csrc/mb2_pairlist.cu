@@ -284,9 +284,7 @@ __global__ void __launch_bounds__(256) pack_kernel(const float4* __restrict__ po
 				p.z < far_lo.z || p.z > far_hi.z)
 				odd[2] = 1ull;
 		}
-		if (track.d2max) {
-			d2 = tracked_d2(track, p, track.ref_sorted[s]);
-		}
+		if (track.d2max) d2 = tracked_d2(track, p, track.ref_sorted ? track.ref_sorted[s] : p);
 		p.w = __int_as_float(type_ids ? type_ids[o] : 0);
 		sorted_pos[s] = p;
 	}
