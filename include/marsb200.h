@@ -196,6 +196,13 @@ MB2_API int mb2_pair_distance_window(float cutoff, float* d2_lo, float* d2_hi);
  * (0 when the kernels' root is the IEEE one). Synchronises. */
 MB2_API int mb2_selftest_sqrt(mb2_context* ctx, uint64_t* mismatches);
 
+/* mb2_radix_sort_pairs with the number of times that a tile of its passes asks
+ * for the earlier tiles' digit counts before it counts the keys before it itself
+ * (0: at once): the result is the same sort for every value. inverse_out (may be
+ * NULL; the values are then 0 .. n - 1): inverse_out[value] = sorted slot. */
+MB2_API int mb2_selftest_sort_polls(mb2_context* ctx, uint32_t* keys, uint32_t* vals, uint32_t n,
+									uint32_t max_polls, uint32_t* inverse_out, void* stream);
+
 /* FP64 reductions of the last force calls made with get_energy: pair energy,
  * pair virial (sum of r . f), bond energy, angle energy. Synchronises.
  * New on this path: the reference sums per-particle floats on the host

@@ -18,7 +18,7 @@ unsigned long long g_launches = 0;
 // restraint energy.
 constexpr int kEnergySlots = 6;
 // Words of a build's statistics (see build).
-constexpr int kBuildStats = 6;
+constexpr int kBuildStats = 4;
 
 struct mb2_context {
 	int device = 0;
@@ -296,11 +296,10 @@ void build(mb2_context* ctx, const float4* pos, const int* type_ids, uint32_t n,
 	for (int a = 0; a < 3; ++a) extent[a] = bmax[a] - bmin[a];
 	// stats: [0] pairs, [1] longest row (both set by each walk), [2] particles
 	// with a non-finite coordinate (counted while packing, read with the
-	// walk's statistics, so no extra synchronisation), [3] set by a sort that
-	// gave up waiting, [4] set when a particle lies far outside the box.
+	// walk's statistics, so no extra synchronisation), [3] set when a particle
+	// lies far outside the box.
 	ctx->stats.ensure(kBuildStats);
 	MB2_CUDA(cudaMemsetAsync(ctx->stats.ptr + 2, 0, (kBuildStats - 2) * sizeof(unsigned long long), st));
-	ctx->scratch.sort_error = reinterpret_cast<uint32_t*>(ctx->stats.ptr + 3);
 	const float split = row_split(ctx->pt, ctx->box, rc_list, cutoff);
 	const bool near_last = split_ends_early(split, cutoff);
 	// Rows whose far entries are mostly not read (ends_early) count as their
@@ -372,12 +371,11 @@ void build(mb2_context* ctx, const float4* pos, const int* type_ids, uint32_t n,
 		const int hshift = __builtin_ctz(32 / ctx->lanes);
 		build_walk(ctx->sorted_pos.ptr, ctx->keys.ptr, ctx->s2o.ptr, ctx->cell_begin.ptr,
 				   ctx->cell_end.ptr, ctx->stencil.ptr, g.num_stencil, wg, n, ctx->box, ctx->excl,
-				   ctx->nbr.ptr, cap, hshift, ctx->row_len.ptr, ctx->row_back.ptr, ctx->stats.ptr + 4,
+				   ctx->nbr.ptr, cap, hshift, ctx->row_len.ptr, ctx->row_back.ptr, ctx->stats.ptr + 3,
 				   ctx->stats.ptr, st);
-		MB2_CUDA(cudaMemcpyAsync(ctx->pinned, ctx->stats.ptr, 4 * sizeof(uint64_t),
+		MB2_CUDA(cudaMemcpyAsync(ctx->pinned, ctx->stats.ptr, 3 * sizeof(uint64_t),
 								 cudaMemcpyDeviceToHost, st));
 		MB2_CUDA(cudaStreamSynchronize(st));
-		require(ctx->pinned[3] == 0, MB2_ERR_CUDA, "mb2_build_pairlist: the sort did not finish");
 		// The walk runs on such particles without harm (cell indices come from
 		// the clamped Morton keys, and a NaN fails every distance test), but
 		// the list is not the reference's meaning of one: refuse it.
@@ -737,6 +735,14 @@ int mb2_radix_sort_pairs(mb2_context* ctx, uint32_t* keys, uint32_t* vals, uint3
 	return guarded(ctx, [&] {
 		require(n == 0 || (keys && vals), MB2_ERR_ARG, "mb2_radix_sort_pairs: null argument");
 		radix_sort_pairs(ctx->scratch, keys, vals, n, S(stream));
+	});
+}
+
+int mb2_selftest_sort_polls(mb2_context* ctx, uint32_t* keys, uint32_t* vals, uint32_t n,
+							uint32_t max_polls, uint32_t* inverse_out, void* stream) {
+	return guarded(ctx, [&] {
+		require(n == 0 || (keys && vals), MB2_ERR_ARG, "mb2_selftest_sort_polls: null argument");
+		radix_sort_pairs(ctx->scratch, keys, vals, n, S(stream), inverse_out, max_polls);
 	});
 }
 

@@ -90,7 +90,6 @@ struct DevBuf {
 // Context-owned scratch for sorting and scanning.
 struct Scratch {
 	DevBuf<uint32_t> keys_alt, vals_alt, work, scan_blocks;
-	uint32_t* sort_error = nullptr;  // set by a sort that gave up (null: only in its work)
 	void ensure_sort(size_t n, size_t work_words) {
 		keys_alt.ensure(n);
 		vals_alt.ensure(n);
@@ -108,9 +107,12 @@ struct StencilEntry {
 void morton_encode(const float4* pos, uint32_t n, const float* bmin, const float* bmax,
 				   uint32_t* keys, uint32_t* idx, cudaStream_t st);
 // place_of (optional; the values are then 0 .. n - 1): the inverse of the
-// permutation, place_of[value] = sorted slot, left by the last pass.
+// permutation, place_of[value] = sorted slot, left by the last pass. max_polls:
+// how often a tile asks for the earlier ones' counts (a second or so by default)
+// before it counts the elements before it itself.
+constexpr uint32_t kMaxPolls = 1u << 20;
 void radix_sort_pairs(Scratch& s, uint32_t* keys, uint32_t* vals, uint32_t n, cudaStream_t st,
-					  uint32_t* place_of = nullptr);
+					  uint32_t* place_of = nullptr, uint32_t max_polls = kMaxPolls);
 // out[s] = in[s2o[s]] for elements of 4 or 16 bytes.
 void permute_gather(const void* in, const uint32_t* s2o, uint32_t n, int elem_bytes, void* out,
 					cudaStream_t st);
@@ -122,7 +124,7 @@ void remap_indices(int* idx, size_t count, const uint32_t* inv, uint32_t n, cuda
 size_t sort_work_words(uint32_t n);
 void radix_sort_pairs_into(uint32_t* keys, uint32_t* vals, uint32_t n, uint32_t* keys_alt,
 						   uint32_t* vals_alt, uint32_t* work, cudaStream_t st,
-						   uint32_t* report = nullptr, uint32_t* place_of = nullptr);
+						   uint32_t* place_of = nullptr, uint32_t max_polls = kMaxPolls);
 // noalloc.cu: the same sort over the library's static scratch (no allocation).
 void radix_sort_pairs_static(uint32_t* keys, uint32_t* vals, uint32_t n, cudaStream_t st);
 
@@ -249,7 +251,7 @@ struct NextPack {
 	DisplacementTrack track;
 };
 // odd (optional, with box): odd[0] incremented once per particle with a NaN or
-// infinite coordinate, odd[2] set when one lies more than half a box outside a
+// infinite coordinate, odd[1] set when one lies more than half a box outside a
 // periodic axis.
 // clear_a / clear_b (may be null): float4[n] arrays zeroed by the same launch.
 // track (optional): raises track.d2max to this step's largest displacement.

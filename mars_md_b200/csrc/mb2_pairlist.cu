@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(256) pack_kernel(const float4* __restrict__ po
 			if (!(isfinite(p.x) && isfinite(p.y) && isfinite(p.z))) atomicAdd(odd, 1ull);
 			if (p.x < far_lo.x || p.x > far_hi.x || p.y < far_lo.y || p.y > far_hi.y ||
 				p.z < far_lo.z || p.z > far_hi.z)
-				odd[2] = 1ull;
+				odd[1] = 1ull;
 		}
 		if (track.d2max) d2 = tracked_d2(track, p, track.ref_sorted ? track.ref_sorted[s] : p);
 		p.w = __int_as_float(type_ids ? type_ids[o] : 0);

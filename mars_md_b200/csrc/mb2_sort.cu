@@ -34,8 +34,6 @@ constexpr int kSortWarps = kSortThreads / 32;
 constexpr int kSmallItems = 4;
 constexpr int kLargeItems = 16;
 constexpr uint32_t kSmallTileMaxN = 1u << 18;
-// Polls of an earlier tile's counts (some seconds) after which a tile gives up.
-constexpr uint32_t kMaxPolls = 1u << 24;
 
 // Look-back word: a tag in the top four bits (2 pass + 1: the tile's own
 // count, 2 pass + 2: the count of all tiles up to and including it; anything
@@ -78,33 +76,30 @@ __global__ void __launch_bounds__(kSortThreads) radix_hist_kernel(const uint32_t
 }
 
 // One pass: tile -> its place in the output. hist: this pass's 256 digit
-// counts; status[tile][256]: look-back words; ticket: zero at the start; error
-// (and report, where given): set when an earlier tile's counts never came. The
-// tile then writes nothing, nor do tiles that start after it, in this pass and the
-// next ones: a pass never reads slots that the one before it left unwritten.
-// place_of (the last pass of a sort whose values are 0 .. n - 1):
-// place_of[value] = output slot, the inverse of the permutation.
+// counts; status[tile][256]: look-back words; ticket: zero at the start. The
+// tickets promise that every earlier tile publishes its counts; should they not
+// come within max_polls all the same (0: not waited for at all), the tile counts
+// the keys before it itself, which takes no other tile: the wait is bounded and
+// the result is the sort either way. place_of (the last pass of a sort whose
+// values are 0 .. n - 1): place_of[value] = output slot, the inverse of the
+// permutation.
 template <int kItems>
 __global__ void __launch_bounds__(kSortThreads) radix_pass_kernel(
 	const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in, uint32_t n,
 	int pass, const uint32_t* __restrict__ hist, unsigned long long* status, uint32_t* ticket,
-	uint32_t* error, uint32_t* report, uint32_t* __restrict__ keys_out,
-	uint32_t* __restrict__ vals_out, uint32_t* __restrict__ place_of) {
+	uint32_t max_polls, uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out,
+	uint32_t* __restrict__ place_of) {
 	__shared__ uint32_t warp_count[kSortWarps][256];
 	__shared__ uint32_t warp_tot[2][kSortWarps];
-	__shared__ uint32_t tile_sh, stop_sh;
+	__shared__ uint32_t tile_sh;
 	__shared__ uint32_t to_global[256];  // output slot of digit d less its slot in the tile
 	__shared__ uint32_t sorted_key[kSortThreads * kItems], sorted_val[kSortThreads * kItems];
 	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, d = threadIdx.x;
 	const int shift = 8 * pass;
 	const unsigned long long own = 2ull * pass + 1ull, all = own + 1ull;
-	if (threadIdx.x == 0) {
-		stop_sh = *static_cast<volatile uint32_t*>(error);
-		tile_sh = atomicAdd(ticket, 1u);
-	}
+	if (threadIdx.x == 0) tile_sh = atomicAdd(ticket, 1u);
 	for (int w = 0; w < kSortWarps; ++w) warp_count[w][d] = 0;
 	__syncthreads();
-	if (stop_sh != 0u) return;
 	const uint32_t tile = tile_sh;
 	const uint32_t base = (tile * kSortThreads + warp * 32) * kItems + lane;
 	uint32_t key[kItems], val[kItems], rank[kItems];
@@ -173,13 +168,14 @@ __global__ void __launch_bounds__(kSortThreads) radix_pass_kernel(
 	}
 	// Counts of the tiles before this one, eight words in flight at a time.
 	unsigned long long prefix = 0;
-	bool failed = false;
+	bool alone = false;  // not told within max_polls
 	if (tile > 0) {
 		constexpr int kBatch = 8;
 		int64_t t = static_cast<int64_t>(tile) - 1;
 		uint32_t polls = 0;
 		bool done = false;
-		while (!done) {
+		alone = max_polls == 0u;
+		while (!done && !alone) {
 			unsigned long long v[kBatch];
 #pragma unroll
 			for (int q = 0; q < kBatch; ++q)
@@ -196,24 +192,24 @@ __global__ void __launch_bounds__(kSortThreads) radix_pass_kernel(
 				}
 			}
 			t -= used;
-			if (!done && used == 0) {
-				if (++polls > kMaxPolls ||
-					((polls & 1023u) == 0u && *static_cast<volatile uint32_t*>(error) != 0u)) {
-					failed = true;
-					break;
-				}
-			}
+			if (!done && used == 0 && ++polls >= max_polls) alone = true;
 		}
-		if (failed) {
-			*static_cast<volatile uint32_t*>(error) = 1u;
-			if (report) *static_cast<volatile uint32_t*>(report) = 1u;
-		} else *row = (all << kTagShift) | (prefix + count);
+		if (!alone) *row = (all << kTagShift) | (prefix + count);
 	}
 	to_global[d] = first + static_cast<uint32_t>(prefix) - tfirst;
-	failed = __syncthreads_or(failed);
-	if (failed) return;
-	// Written in tile order, so that a digit's elements are neighbouring stores.
 	const uint32_t start = tile * (kSortThreads * kItems);
+	if (__syncthreads_or(alone)) {
+		warp_count[0][d] = 0u;
+		__syncthreads();
+		for (uint32_t i = threadIdx.x; i < start; i += kSortThreads)
+			atomicAdd(&warp_count[0][(keys_in[i] >> shift) & 255u], 1u);
+		__syncthreads();
+		prefix = warp_count[0][d];
+		*row = (all << kTagShift) | (prefix + count);
+		to_global[d] = first + static_cast<uint32_t>(prefix) - tfirst;
+		__syncthreads();
+	}
+	// Written in tile order, so that a digit's elements are neighbouring stores.
 	const uint32_t here = min(static_cast<uint32_t>(kSortThreads * kItems), n - start);
 #pragma unroll
 	for (int k = 0; k < kItems; ++k) {
@@ -320,7 +316,7 @@ uint32_t sort_tiles(uint32_t n) {
 }
 
 // Words before the look-back rows: the four histograms, a ticket for each
-// pass, the error word.
+// pass.
 constexpr size_t kSortHeadWords = 4 * 256 + 8;
 
 }  // namespace
@@ -331,8 +327,8 @@ size_t sort_work_words(uint32_t n) {
 }
 
 void radix_sort_pairs_into(uint32_t* keys, uint32_t* vals, uint32_t n, uint32_t* keys_alt,
-						   uint32_t* vals_alt, uint32_t* work, cudaStream_t st, uint32_t* report,
-						   uint32_t* place_of) {
+						   uint32_t* vals_alt, uint32_t* work, cudaStream_t st, uint32_t* place_of,
+						   uint32_t max_polls) {
 	if (n == 0) return;
 	if (n == 1) {
 		if (place_of) MB2_CUDA(cudaMemsetAsync(place_of, 0, sizeof(uint32_t), st));
@@ -348,7 +344,6 @@ void radix_sort_pairs_into(uint32_t* keys, uint32_t* vals, uint32_t n, uint32_t*
 	}
 	const uint32_t tiles = sort_tiles(n);
 	uint32_t* tickets = work + 4 * 256;
-	uint32_t* error = tickets + 4;
 	unsigned long long* status = reinterpret_cast<unsigned long long*>(work + kSortHeadWords);
 	MB2_CUDA(cudaMemsetAsync(work, 0, sort_work_words(n) * sizeof(uint32_t), st));
 	MB2_LAUNCH radix_hist_kernel<<<std::min(tiles, 592u), kSortThreads, 0, st>>>(keys, n, work);
@@ -357,7 +352,7 @@ void radix_sort_pairs_into(uint32_t* keys, uint32_t* vals, uint32_t n, uint32_t*
 										   : radix_pass_kernel<kLargeItems>;
 	for (int pass = 0; pass < 4; ++pass) {
 		MB2_LAUNCH pass_kernel<<<tiles, kSortThreads, 0, st>>>(
-			ks, vs, n, pass, work + 256 * pass, status, tickets + pass, error, report, kd, vd,
+			ks, vs, n, pass, work + 256 * pass, status, tickets + pass, max_polls, kd, vd,
 			pass == 3 ? place_of : nullptr);
 		std::swap(ks, kd);
 		std::swap(vs, vd);
@@ -366,11 +361,11 @@ void radix_sort_pairs_into(uint32_t* keys, uint32_t* vals, uint32_t n, uint32_t*
 }
 
 void radix_sort_pairs(Scratch& s, uint32_t* keys, uint32_t* vals, uint32_t n, cudaStream_t st,
-					  uint32_t* place_of) {
+					  uint32_t* place_of, uint32_t max_polls) {
 	if (n == 0) return;
 	s.ensure_sort(n, sort_work_words(n));
-	radix_sort_pairs_into(keys, vals, n, s.keys_alt.ptr, s.vals_alt.ptr, s.work.ptr, st, s.sort_error,
-						  place_of);
+	radix_sort_pairs_into(keys, vals, n, s.keys_alt.ptr, s.vals_alt.ptr, s.work.ptr, st, place_of,
+						  max_polls);
 }
 
 void morton_encode(const float4* pos, uint32_t n, const float* bmin, const float* bmax,

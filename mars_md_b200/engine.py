@@ -205,6 +205,11 @@ class Context:
         self.check(self.lib.mb2_radix_sort_pairs(self.h, _p(keys), _p(vals), keys.shape[0],
                                                  _stream(stream)))
 
+    def selftest_sort_polls(self, keys, vals, max_polls, inverse=None, stream=None):
+        """radix_sort_pairs with a limit of its own on the polls of a tile's look-back."""
+        self.check(self.lib.mb2_selftest_sort_polls(self.h, _p(keys), _p(vals), keys.shape[0],
+                                                    int(max_polls), _p(inverse), _stream(stream)))
+
     def radix_sort_pairs_static(self, keys, vals, stream=None):
         """Same sort over the library's static scratch: allocates no device memory
         (n <= MB2_SORT_STATIC_MAX; concurrent calls on one device race)."""

@@ -40,3 +40,21 @@ def test_morton_sort_leaves_the_inverse(ctx_factory, n):
     assert np.array_equal(inv[s2o], np.arange(n))
     assert np.array_equal(sp, pos.cpu().numpy()[s2o])
     assert np.all((keys[1:] > keys[:-1]) | ((keys[1:] == keys[:-1]) & (s2o[1:] > s2o[:-1])))
+
+
+@pytest.mark.parametrize("polls", [0, 1, 3])
+@pytest.mark.parametrize("n", [8193, 9217, 262145, 300001])
+@pytest.mark.parametrize("bits", [3, 32])
+def test_sort_without_the_earlier_tiles_counts(ctx_factory, n, bits, polls):
+    """Tiles that are not told the counts before them in time count them
+    themselves: none waits (0 polls), or some do and some do not."""
+    rng = np.random.default_rng(n + bits)
+    keys_np = rng.integers(0, 1 << bits, n, dtype=np.uint64).astype(np.uint32)
+    keys = torch.from_numpy(keys_np.view(np.int32).copy()).cuda()
+    vals = torch.arange(n, dtype=torch.int32, device="cuda")
+    inv = torch.full((n,), -1, dtype=torch.int32, device="cuda")
+    ctx_factory(n).selftest_sort_polls(keys, vals, polls, inv)
+    order = np.argsort(keys_np, kind="stable")
+    assert np.array_equal(keys.cpu().numpy().view(np.uint32), keys_np[order])
+    assert np.array_equal(vals.cpu().numpy(), order)
+    assert np.array_equal(inv.cpu().numpy()[order], np.arange(n))
