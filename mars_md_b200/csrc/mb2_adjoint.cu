@@ -62,23 +62,22 @@ __device__ __forceinline__ void add_d3(double* t, double x, double y, double z) 
 
 // mu = (D / kT * dt) * lambda per type and axis, in original and sorted order;
 // the step's tangent accumulators cleared.
-__global__ void __launch_bounds__(256) adj_mu_kernel(const float4* __restrict__ lam,
+__global__ void __launch_bounds__(256) adj_mu_kernel(const float4* lam,
 													 const int* __restrict__ type_ids,
 													 const float4* __restrict__ diffusion,
 													 const uint32_t* __restrict__ inv, uint32_t n,
-													 float dt_over_kT, float4* __restrict__ mu,
-													 float4* __restrict__ mu_sorted,
-													 double4* __restrict__ tan,
-													 double4* __restrict__ tan_sorted) {
+													 float dt_over_kT, float4* mu,
+													 float4* mu_sorted, double4* tan,
+													 double4* tan_sorted) {
 	chain_begin();
 	chain_wait();
 	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
 	if (i >= n) return;
+	const float4 d = diffusion[type_ids[i]];
+	const float4 l = lam[i];
 	// The tangent accumulators of this step start at zero.
 	tan[i] = make_double4(0.0, 0.0, 0.0, 0.0);
 	tan_sorted[i] = make_double4(0.0, 0.0, 0.0, 0.0);
-	const float4 d = diffusion[type_ids[i]];
-	const float4 l = lam[i];
 	const float4 m = make_float4(d.x * dt_over_kT * l.x, d.y * dt_over_kT * l.y,
 								 d.z * dt_over_kT * l.z, 0.0f);
 	mu[i] = m;
@@ -96,11 +95,11 @@ __device__ __forceinline__ void flush_bins(const double* sg, double* g, uint32_t
 // over the grid). tan_sorted accumulates J mu in sorted order.
 template <int G, bool kAllPeriodic>
 __global__ void __launch_bounds__(256) adj_pair_kernel(
-	const float4* __restrict__ sorted_pos, const float4* __restrict__ mu_sorted,
-	const uint32_t* __restrict__ nbr, const uint32_t* __restrict__ row_len, uint32_t n,
-	uint32_t cap, int T, const PairTableRef* __restrict__ refs_g,
-	const float* __restrict__ force_g, uint32_t total_bins, Box box, float cutoff_sq,
-	double* tan_sorted, double* __restrict__ grad_bins) {
+	const float4* sorted_pos, const float4* mu_sorted, const uint32_t* __restrict__ nbr,
+	const uint32_t* __restrict__ row_len, uint32_t n, uint32_t cap, int T,
+	const PairTableRef* __restrict__ refs_g, const float* __restrict__ force_g,
+	uint32_t total_bins, Box box, float cutoff_sq, double* tan_sorted,
+	double* __restrict__ grad_bins) {
 	constexpr int H = 32 / G;
 	chain_begin();
 	extern __shared__ double sg[];
@@ -124,10 +123,22 @@ __global__ void __launch_bounds__(256) adj_pair_kernel(
 		const uint32_t cnt = valid ? row_len[i] : 0u;
 		const uint32_t* col = nbr + (static_cast<size_t>(i / H) * cap) * H + (i % H);
 		double tx = 0.0, ty = 0.0, tz = 0.0;
+		// The next pair's position is read ahead of this one's atomics, which
+		// plain loads do not pass.
+		uint32_t e_next = 0;
+		float4 p_next = make_float4(0.f, 0.f, 0.f, 0.f);
+		if (static_cast<uint32_t>(sub) < cnt) {
+			e_next = __ldg(col + static_cast<size_t>(sub) * H);
+			p_next = sorted_pos[e_next & ~kOrientBit];
+		}
 		for (uint32_t t = sub; t < cnt; t += G) {
-			const uint32_t e = __ldg(col + static_cast<size_t>(t) * H);
+			const uint32_t e = e_next;
 			const uint32_t j = e & ~kOrientBit;
-			const float4 pj = sorted_pos[j];
+			const float4 pj = p_next;
+			if (t + G < cnt) {
+				e_next = __ldg(col + static_cast<size_t>(t + G) * H);
+				p_next = sorted_pos[e_next & ~kOrientBit];
+			}
 			// Distance, cutoff test and table bin exactly as the forward pair
 			// kernel decides them (the pair oriented as the reference orients
 			// it, reference rounding), so the derivative is that of the map
@@ -185,10 +196,9 @@ __global__ void __launch_bounds__(256) adj_pair_kernel(
 // bond-table gradient accumulated in shared memory and flushed at its end.
 __device__ __forceinline__ void adj_bonds(
 	uint32_t block, uint32_t nblocks, const int2* __restrict__ bonds,
-	const int* __restrict__ table_idx, uint32_t nb, const float4* __restrict__ pos,
-	const float4* __restrict__ mu, const Table* __restrict__ tables,
-	const float* __restrict__ values_base, uint32_t total_bins, const Box& box, double* tan,
-	double* __restrict__ grad_bins, double* sg) {
+	const int* __restrict__ table_idx, uint32_t nb, const float4* pos, const float4* mu,
+	const Table* __restrict__ tables, const float* __restrict__ values_base, uint32_t total_bins,
+	const Box& box, double* tan, double* __restrict__ grad_bins, double* sg) {
 	for (uint32_t k = threadIdx.x; k < total_bins; k += blockDim.x) sg[k] = 0.0;
 	__syncthreads();
 	for (uint32_t b = block * blockDim.x + threadIdx.x; b < nb; b += nblocks * blockDim.x) {
@@ -225,8 +235,8 @@ __device__ __forceinline__ void adj_bonds(
 // Angle term: tangent of the AngleGeometry force along mu (dual numbers).
 __device__ __forceinline__ void adj_angle(
 	uint32_t q, const int4* __restrict__ angles, const int* __restrict__ table_idx, uint32_t na,
-	const float4* __restrict__ pos, const float4* __restrict__ mu, const Table* __restrict__ tables,
-	const Box& box, double* tan) {
+	const float4* pos, const float4* mu, const Table* __restrict__ tables, const Box& box,
+	double* tan) {
 	if (q >= na) return;
 	const int4 a = angles[q];
 	const float4 pi = pos[a.x], pj = pos[a.y], pk = pos[a.z];
@@ -293,7 +303,7 @@ __global__ void __launch_bounds__(256) adj_bond_angle_kernel(
 	uint32_t nb, const Table* __restrict__ bond_tables, const float* __restrict__ values_base,
 	uint32_t total_bins, double* __restrict__ grad_bins, const int4* __restrict__ angles,
 	const int* __restrict__ angle_idx, uint32_t na, const Table* __restrict__ angle_tables,
-	const float4* __restrict__ pos, const float4* __restrict__ mu, Box box, double* tan) {
+	const float4* pos, const float4* mu, Box box, double* tan) {
 	chain_begin();
 	chain_wait();
 	extern __shared__ double sg[];
@@ -306,9 +316,8 @@ __global__ void __launch_bounds__(256) adj_bond_angle_kernel(
 }
 
 // lambda += tan (original order) + tan_sorted (gathered through inv).
-__global__ void __launch_bounds__(256) adj_combine_kernel(float4* __restrict__ lam,
-														  const double4* __restrict__ tan,
-														  const double4* __restrict__ tan_sorted,
+__global__ void __launch_bounds__(256) adj_combine_kernel(float4* lam, const double4* tan,
+														  const double4* tan_sorted,
 														  const uint32_t* __restrict__ inv,
 														  uint32_t n) {
 	chain_begin();

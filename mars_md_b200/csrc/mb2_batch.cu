@@ -176,10 +176,9 @@ __global__ void __launch_bounds__(256) batch_snapshot_kernel(const float4* __res
 // particle than without, against the rows' far part that the pair kernel then
 // need not read (see set_far).
 __global__ void __launch_bounds__(256) batch_pack_kernel(
-	const float4* __restrict__ pos, const int* __restrict__ type_ids,
-	const uint32_t* __restrict__ s2o, const uint32_t* __restrict__ keys,
-	const Box* __restrict__ boxes, const float4* __restrict__ ref, uint32_t n,
-	float4* __restrict__ sorted_pos, float4* __restrict__ clear, unsigned int* moved) {
+	const float4* pos, const int* __restrict__ type_ids, const uint32_t* __restrict__ s2o,
+	const uint32_t* __restrict__ keys, const Box* __restrict__ boxes, const float4* ref,
+	uint32_t n, float4* sorted_pos, float4* clear, unsigned int* moved) {
 	chain_begin();
 	chain_wait();
 	const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;

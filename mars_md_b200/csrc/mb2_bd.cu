@@ -244,7 +244,7 @@ __device__ __forceinline__ void leave_next(const NextPack& next, uint32_t row, f
 // kNext: see NextPack; the force is then read through next.forces, and cleared.
 template <bool kGrids, bool kNext>
 __global__ void __launch_bounds__(256) bd_gather_kernel(
-	const float4* from, float4* pos, float4* __restrict__ fe, const float4* __restrict__ fs,
+	const float4* from, float4* pos, float4* fe, const float4* fs,
 	const uint32_t* __restrict__ inv, const int* __restrict__ type_ids,
 	const uint32_t* __restrict__ flags, uint32_t n, TypeTable ty, Box box, BdParams bp,
 	int read_fe, StepClock clock, NextPack next) {
@@ -307,8 +307,8 @@ __device__ __forceinline__ float half_kick(float m, float f, float h) {
 // sum as the reference leaves it.
 template <bool kGather, bool kNext>
 __global__ void __launch_bounds__(256) baoab_kernel(
-	float4* __restrict__ pos, float4* __restrict__ mom, float4* __restrict__ fe,
-	const float4* __restrict__ fs, const uint32_t* __restrict__ inv, int read_fe,
+	float4* pos, float4* mom, float4* fe, const float4* fs,
+	const uint32_t* __restrict__ inv, int read_fe,
 	const int* __restrict__ type_ids, const uint32_t* __restrict__ flags, uint32_t n,
 	TypeTable ty, Box box, float dt, float kT, uint32_t step, uint64_t seed, uint32_t base_ctr,
 	float3 efield, int pending, StepClock clock, NextPack next) {
@@ -416,11 +416,10 @@ __global__ void __launch_bounds__(256) baoab_last_kernel(float4* __restrict__ mo
 // captured graph can be replayed step after step. kGrids as bd_gather_kernel.
 template <bool kGrids>
 __global__ void __launch_bounds__(256) bd_systems_kernel(
-	float4* __restrict__ pos, float4* __restrict__ fe, const float4* __restrict__ fs,
-	const uint32_t* __restrict__ inv, const int* __restrict__ type_ids,
-	const uint32_t* __restrict__ sys_of, const uint32_t* __restrict__ offsets,
-	const Box* __restrict__ boxes, uint32_t n, TypeTable ty, float dt, float kT, uint64_t seed,
-	uint64_t patch_id, const unsigned long long* __restrict__ step_ptr) {
+	float4* pos, float4* fe, const float4* fs, const uint32_t* __restrict__ inv,
+	const int* __restrict__ type_ids, const uint32_t* __restrict__ sys_of,
+	const uint32_t* __restrict__ offsets, const Box* __restrict__ boxes, uint32_t n, TypeTable ty,
+	float dt, float kT, uint64_t seed, uint64_t patch_id, const unsigned long long* step_ptr) {
 	chain_begin();
 	chain_wait();
 	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;

@@ -345,7 +345,7 @@ struct OneBox {
 	float margin;
 	__device__ __forceinline__ const Box& row(uint32_t) const { return b; }
 	// The largest squared displacement since the list's build (float bits).
-	__device__ __forceinline__ unsigned int moved(uint32_t) const { return __ldg(d2max); }
+	__device__ __forceinline__ unsigned int moved(uint32_t) const { return *d2max; }
 };
 // Added to the list radius in the inner-row test: covers kTrackBand and the
 // rounding of the displacement and of the walk's radius test.
@@ -354,10 +354,10 @@ struct SystemBoxes {
 	const Box* __restrict__ boxes;
 	const uint32_t* __restrict__ keys;
 	int sys_shift;
-	const unsigned int* __restrict__ d2sys;  // per system (may be null)
+	const unsigned int* d2sys;  // per system (may be null)
 	__device__ __forceinline__ Box row(uint32_t i) const { return boxes[keys[i] >> sys_shift]; }
 	__device__ __forceinline__ unsigned int moved(uint32_t i) const {
-		return __ldg(d2sys + (keys[i] >> sys_shift));
+		return d2sys[keys[i] >> sys_shift];
 	}
 };
 
@@ -372,7 +372,7 @@ constexpr int pair_min_blocks() {
 template <int G, bool kEnergy, bool kAllPeriodic, bool kTerms, class BoxSrc>
 __global__ void __launch_bounds__(
 	256, pair_min_blocks<kEnergy, kTerms, std::is_same<BoxSrc, OneBox>::value>()) pair_force_kernel(
-	const float4* __restrict__ sorted_pos, const uint32_t* __restrict__ nbr,
+	const float4* sorted_pos, const uint32_t* __restrict__ nbr,
 	const uint32_t* __restrict__ row_len, uint32_t n, uint32_t cap, int T,
 	const PairTableRef* __restrict__ refs_g, const float* __restrict__ force_g,
 	const float2* __restrict__ energy_g, uint32_t total_bins,
@@ -480,7 +480,7 @@ constexpr int fast_min_blocks() {
 template <int G, bool kEnergy, bool kDirect, bool kFar, class BoxSrc>
 __global__ void __launch_bounds__(256, fast_min_blocks<kEnergy, std::is_same<BoxSrc, OneBox>::value>())
 	fast_pair_kernel(
-	const float4* __restrict__ sorted_pos, const uint32_t* __restrict__ nbr,
+	const float4* sorted_pos, const uint32_t* __restrict__ nbr,
 	const uint32_t* __restrict__ row_len, uint32_t n, uint32_t cap, FastArgs fa, BoxSrc boxes,
 	float4* force, double* __restrict__ ev) {
 	constexpr int H = 32 / G;
@@ -586,7 +586,7 @@ __global__ void __launch_bounds__(256, fast_min_blocks<kEnergy, std::is_same<Box
 	bool inner = false;
 	if constexpr (std::is_same<BoxSrc, OneBox>::value) {
 		if (boxes.d2max != nullptr) {
-			const float m = boxes.margin + 2.0f * sqrtf(__uint_as_float(__ldg(boxes.d2max)));
+			const float m = boxes.margin + 2.0f * sqrtf(__uint_as_float(*boxes.d2max));
 			const float c[3] = {pi.x, pi.y, pi.z};
 			inner = true;
 #pragma unroll
@@ -640,7 +640,7 @@ __device__ __forceinline__ float calc_distance(const Box& box, const float4& fro
 // the reference's forms[] check skips it.
 __device__ __forceinline__ double bond_term(uint32_t k, const int2* __restrict__ bonds,
 											const int* __restrict__ table_idx, uint32_t nb,
-											const float4* __restrict__ pos, float4* fe,
+											const float4* pos, float4* fe,
 											const Table* __restrict__ tables, const Box& box,
 											int get_energy) {
 	double e_acc = 0.0;
@@ -678,7 +678,7 @@ __global__ void __launch_bounds__(256) bond_kernel(const int2* __restrict__ bond
 // Angle tables wrap (src/Interactions/DeviceBondedInteraction.h:234).
 __device__ __forceinline__ double angle_term(uint32_t k, const int4* __restrict__ angles,
 											 const int* __restrict__ table_idx, uint32_t na,
-											 const float4* __restrict__ pos, float4* fe,
+											 const float4* pos, float4* fe,
 											 const Table* __restrict__ tables, const Box& box,
 											 int get_energy) {
 	double e_acc = 0.0;
@@ -743,7 +743,7 @@ __global__ void __launch_bounds__(256) bond_angle_kernel(
 	const int2* __restrict__ bonds, const int* __restrict__ bond_idx, uint32_t nb,
 	const Table* __restrict__ bond_tables, const int4* __restrict__ angles,
 	const int* __restrict__ angle_idx, uint32_t na, const Table* __restrict__ angle_tables,
-	const float4* __restrict__ pos, float4* fe, Box box, int get_energy, double* bond_energy,
+	const float4* pos, float4* fe, Box box, int get_energy, double* bond_energy,
 	double* angle_energy) {
 	chain_begin();
 	chain_wait();

@@ -52,8 +52,15 @@ void launch_chained(void (*kernel)(P...), uint32_t blocks, uint32_t threads, siz
 // First thing in every kernel that launch_chained launches: lets the next
 // kernel of the chain be scheduled, then waits until the kernels before this
 // one have ended and their writes are visible (nothing to wait for in an
-// ordinary launch). Each kernel of a chain waits before it touches memory, so
-// a kernel's end implies the end of all before it.
+// ordinary launch). Each kernel of a chain waits before it writes anything, so
+// a kernel's end implies the end of all before it. Before the wait a kernel reads
+// only what no kernel of a chain writes: the tables (set by synchronous copies)
+// and the step clock (set by an ordinary launch ahead of the graph that reads it).
+// Whatever a chained kernel writes (positions, their packed copies, force sums,
+// momenta, the displacement words, the adjoint's vectors) is read after the wait
+// and through plain pointers: __ldg and const __restrict__ promise that memory
+// does not change while the kernel is resident, and it is resident before the
+// writer has ended.
 __device__ __forceinline__ void chain_begin() { asm volatile("griddepcontrol.launch_dependents;"); }
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

@@ -255,14 +255,11 @@ __global__ void __launch_bounds__(256) displacement_kernel(const float4* __restr
 	if ((threadIdx.x & 31) == 0 && bits > seen) atomicMax(out, bits);
 }
 
-__global__ void __launch_bounds__(256) pack_kernel(const float4* __restrict__ pos,
-												   const int* __restrict__ type_ids,
-												   const uint32_t* __restrict__ s2o, uint32_t n,
-												   float4* __restrict__ sorted_pos,
-												   unsigned long long* odd, float3 far_lo,
-												   float3 far_hi, float4* __restrict__ clear_a,
-												   float4* __restrict__ clear_b,
-												   DisplacementTrack track) {
+__global__ void __launch_bounds__(256) pack_kernel(const float4* pos, const int* type_ids,
+												   const uint32_t* s2o, uint32_t n,
+												   float4* sorted_pos, unsigned long long* odd,
+												   float3 far_lo, float3 far_hi, float4* clear_a,
+												   float4* clear_b, DisplacementTrack track) {
 	chain_begin();
 	chain_wait();
 	const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -272,20 +269,23 @@ __global__ void __launch_bounds__(256) pack_kernel(const float4* __restrict__ po
 								  : 0u;
 	float d2 = 0.0f;
 	if (s < n) {
+		const uint32_t o = s2o[s];
+		float4 p = pos[o];
+		const int type = type_ids ? type_ids[o] : 0;
+		float4 ref = p;
+		if (track.ref_sorted) ref = track.ref_sorted[s];
 		// Accumulators of the step that follows, cleared here instead of by
 		// separate memsets (one launch less each on short steps).
 		if (clear_a) clear_a[s] = make_float4(0.f, 0.f, 0.f, 0.f);
 		if (clear_b) clear_b[s] = make_float4(0.f, 0.f, 0.f, 0.f);
-		const uint32_t o = s2o[s];
-		float4 p = pos[o];
 		if (odd) {
 			if (!(isfinite(p.x) && isfinite(p.y) && isfinite(p.z))) atomicAdd(odd, 1ull);
 			if (p.x < far_lo.x || p.x > far_hi.x || p.y < far_lo.y || p.y > far_hi.y ||
 				p.z < far_lo.z || p.z > far_hi.z)
 				odd[1] = 1ull;
 		}
-		if (track.d2max) d2 = tracked_d2(track, p, track.ref_sorted ? track.ref_sorted[s] : p);
-		p.w = __int_as_float(type_ids ? type_ids[o] : 0);
+		if (track.d2max) d2 = tracked_d2(track, p, ref);
+		p.w = __int_as_float(type);
 		sorted_pos[s] = p;
 	}
 	if (track.d2max) {
