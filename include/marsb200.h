@@ -193,7 +193,9 @@ MB2_API int mb2_pair_distance_window(float cutoff, float* d2_lo, float* d2_hi);
 /* Exhaustive device check of the pair kernels' correctly rounded square root
  * (one Newton-Raphson step on the hardware estimate) against the CUDA
  * intrinsic __fsqrt_rn on every float in [2^-60, FLT_MAX]: the mismatch count
- * (0 when the kernels' root is the IEEE one). Synchronises. */
+ * (0 when the kernels' root is the IEEE one); and the root and reciprocal of the
+ * pair kernel for uniform tables against __fsqrt_rn and __frcp_rn likewise.
+ * Synchronises. */
 MB2_API int mb2_selftest_sqrt(mb2_context* ctx, uint64_t* mismatches);
 
 /* mb2_radix_sort_pairs with the number of times that a tile of its passes asks

@@ -75,6 +75,21 @@ __device__ __forceinline__ float sqrt_rn_nr(float a) {
 	return __fmaf_rn(__fmaf_rn(-g, g, a), h, g);
 }
 
+// The same root (the estimate flushing subnormals, which the range does not
+// reach) and its correctly rounded reciprocal, again an estimate and one
+// correction by Markstein's method. An estimate of its own (PTX rcp.approx), not
+// 1/sqrt(a) once more: corrected once from that, 188 of the floats in [2^-60,
+// FLT_MAX] gave a reciprocal an ulp off, and corrected twice those whose root's
+// significand is all ones still did. mb2_selftest_sqrt checks both on every one.
+__device__ __forceinline__ void sqrt_and_inverse(float a, float& root, float& inverse) {
+	float y, z;
+	asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(a));
+	const float g = __fmul_rn(a, y);
+	root = __fmaf_rn(__fmaf_rn(-g, g, a), __fmul_rn(0.5f, y), g);
+	asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(z) : "f"(root));
+	inverse = __fmaf_rn(z, __fmaf_rn(-root, z, 1.0f), z);
+}
+
 // The reference's pair test as a window on the squared distance d2: it skips
 // a pair when dist = RN(sqrt(d2)) < 1e-6 or RN(dist * dist) > cutoff_sq
 // (cutoff_sq > 0). Both sides are monotone in d2, so the test is d2 < lo or

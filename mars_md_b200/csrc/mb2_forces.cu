@@ -451,10 +451,10 @@ __global__ void __launch_bounds__(
 // pair takes fewer instructions to it (the general kernel is bound by issuing
 // them, 76 thread instructions a pair and 82 % issue active at 2,097,152
 // beads, with the L1's data pipe at 80 % close behind):
-//  * one hardware 1 / sqrt (PTX rsqrt.approx) serves the root and the
-//    reciprocal, each by one Newton-Raphson correction (Markstein, see
-//    sqrt_rn_nr): root and reciprocal are the correctly rounded ones, but for
-//    one reciprocal in some 10^7 that is an ulp off;
+//  * the root and its reciprocal are a hardware estimate and one Newton-Raphson
+//    correction each (sqrt_and_inverse), the correctly rounded ones on every
+//    float (one estimate for both, which was not, took 0.5 % less of a 20-step
+//    run: 31.92 ms for 32.09 at 2,097,152 beads, 4.907 for 4.924 at 300,007);
 //  * the bin comes from one addition rounded down, with the first bin of the
 //    row's types in the addend, and is read at (type pair) * stride + bin: no
 //    conversion, no clamp, no lookup of the table;
@@ -523,11 +523,8 @@ __global__ void __launch_bounds__(256, fast_min_blocks<kEnergy, std::is_same<Box
 		const float2 sq = __fmul2_rn(dxy, dxy);
 		const float d2 = __fadd_rn(__fadd_rn(sq.x, sq.y), __fmul_rn(dz, dz));
 		if (d2 > fa.loose) return;
-		float y;
-		asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d2));
-		const float g = __fmul_rn(d2, y);
-		const float dist = __fmaf_rn(__fmaf_rn(-g, g, d2), __fmul_rn(0.5f, y), g);
-		const float inv = __fmaf_rn(y, __fmaf_rn(-dist, y, 1.0f), y);
+		float dist, inv;
+		sqrt_and_inverse(d2, dist, inv);
 		const float w = __fmul_rn(__fsub_rn(dist, fa.start), fa.step_inv);
 		const float t = __fadd_rd(w, magic);
 		uint32_t home = __float_as_uint(t);
@@ -1232,8 +1229,8 @@ void pair_forces_systems(const float4* sorted_pos, const uint32_t* nbr, const ui
 
 namespace {
 
-// Every float with bit pattern in [lo, hi]: sqrt_rn_nr against __fsqrt_rn,
-// mismatches counted.
+// Every float with bit pattern in [lo, hi]: sqrt_rn_nr and sqrt_and_inverse
+// against __fsqrt_rn and __frcp_rn, floats with a mismatch counted.
 __global__ void __launch_bounds__(256) sqrt_check_kernel(uint32_t lo, uint32_t hi,
 														unsigned long long* bad) {
 	const uint64_t count = static_cast<uint64_t>(hi) - lo + 1;
@@ -1241,7 +1238,12 @@ __global__ void __launch_bounds__(256) sqrt_check_kernel(uint32_t lo, uint32_t h
 	for (uint64_t k = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; k < count;
 		 k += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
 		const float a = __uint_as_float(lo + static_cast<uint32_t>(k));
-		mine += __float_as_uint(__fsqrt_rn(a)) != __float_as_uint(sqrt_rn_nr(a));
+		const float want = __fsqrt_rn(a);
+		float root, inverse;
+		sqrt_and_inverse(a, root, inverse);
+		mine += __float_as_uint(want) != __float_as_uint(sqrt_rn_nr(a)) ||
+				__float_as_uint(want) != __float_as_uint(root) ||
+				__float_as_uint(__frcp_rn(want)) != __float_as_uint(inverse);
 	}
 	if (mine) atomicAdd(bad, mine);
 }

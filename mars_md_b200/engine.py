@@ -338,8 +338,8 @@ class Context:
                                                   mom.shape[0], float(dt), _stream(stream)))
 
     def selftest_sqrt(self) -> int:
-        """Mismatches of the pair kernels' square root against __fsqrt_rn over
-        every float in [2^-60, FLT_MAX] (0 expected)."""
+        """Mismatches of the pair kernels' square root and reciprocal against
+        __fsqrt_rn and __frcp_rn over every float in [2^-60, FLT_MAX] (0 expected)."""
         a = C.c_uint64(0)
         self.check(self.lib.mb2_selftest_sqrt(self.h, C.byref(a)))
         return a.value

@@ -1,6 +1,7 @@
 """The pair kernels' square root (one Newton-Raphson step on the hardware
-estimate, Markstein's method) is the IEEE round-to-nearest one on every
-float in [2^-60, FLT_MAX]: checked against CUDA's __fsqrt_rn on the device,
+estimate, Markstein's method), and the root and its reciprocal of the kernel for
+uniform tables, are the IEEE round-to-nearest ones on every float in [2^-60,
+FLT_MAX]: checked against CUDA's __fsqrt_rn and __frcp_rn on the device,
 exhaustively."""
 import pytest
 
