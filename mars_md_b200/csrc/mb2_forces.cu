@@ -877,7 +877,9 @@ FastArgs fast_args(const PairTables& t, float cutoff_sq, int get_energy) {
 	fa.start = u.start;
 	fa.step_inv = u.step_inv;
 	const DistWindow win = dist_window(cutoff_sq);
-	const double end = (get_energy ? t.reach_energy : t.reach_force) * (1.0 + 1e-6);
+	// (the rounding of the coordinate distance - start is a few 2^-24 of that sum)
+	const double reach = get_energy ? t.reach_energy : t.reach_force;
+	const double end = reach + 1e-6 * (reach + std::max(0.0, -static_cast<double>(u.start)));
 	fa.loose = std::min(win.hi, static_cast<float>(end * end * (1.0 + 1e-6)));
 	fa.lo = win.lo;
 	const double close = std::max(1e-5, u.start > 0.0f ? u.start * (1.0 + 1e-6) : 0.0);

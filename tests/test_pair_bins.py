@@ -12,7 +12,8 @@ f = np.float32
 @pytest.mark.parametrize("first", [0, 200, 400 * 15, 32000])
 @pytest.mark.parametrize("start,step_inv,last,end", [
     (0.0, 10.0, 199, 4.5), (0.0, 13.333333, 399, 29.925), (0.05, 10.0, 99, 9.95),
-    (3.0, 25.0, 300, 15.0), (-1.0, 8.0, 120, 14.0)])
+    (3.0, 25.0, 300, 15.0), (-1.0, 8.0, 120, 14.0),
+    (-541.27612, 6.8795, 3829, 0.349)])
 def test_sum_rounded_down_holds_the_references_bin(first, start, step_inv, last, end):
     rng = np.random.default_rng(7)
     start, step_inv = f(start), f(step_inv)
@@ -21,7 +22,7 @@ def test_sum_rounded_down_holds_the_references_bin(first, start, step_inv, last,
     near = edges[:, None] * (1.0 + rng.uniform(-1, 1, (1, 64)) * 10.0 ** rng.uniform(-8, -2, (1, 64)))
     d = np.concatenate([rng.uniform(0, end, 200000), near.ravel(), 10.0 ** rng.uniform(-5, -1, 20000),
                         [1e-6, 1.1e-5, 0.25 / float(step_inv), end]]).astype(f)
-    reach = end * (1 + 1e-6)                                    # fast_args: loose
+    reach = end + 1e-6 * (end + max(0.0, -float(start)))       # fast_args: loose
     close = max(1e-5, float(start) * (1 + 1e-6))                # fast_args: close2
     d = d[(d <= f(reach * (1 + 1e-6))) & (d >= f(close * (1 + 1e-6)))]
     w = ((d - start).astype(f) * step_inv).astype(f)
