@@ -173,10 +173,19 @@ __device__ __forceinline__ void analytic_terms(uint32_t terms, const PairTermRef
 	}
 }
 
-// The table references of one row's type.
+// The table references of one row's type: the full 16-byte reference per j
+// type, or (kUniform) the shared start, step inverse and last bin with the
+// offset, one shared-memory word, per j type.
+template <bool kUniform>
 struct TableRow {
 	const PairTableRef* row;
-	__device__ __forceinline__ PairTableRef operator()(int tj) const { return row[tj]; }
+	PairTableRef u;
+	__device__ __forceinline__ PairTableRef operator()(int tj) const {
+		if (!kUniform) return row[tj];
+		PairTableRef t = u;
+		t.offset = row[tj].offset;
+		return t;
+	}
 };
 
 // r = wrap_diff(pos[second] - pos[first]) as the reference rounds it: sgn is -1
@@ -367,14 +376,21 @@ constexpr int pair_min_blocks() {
 	return !kOneBox ? 6 : (kTerms ? 3 : (kEnergy ? 5 : 8));
 }
 
-// The general pair kernel: tables of different starts or bin widths, and the
-// analytical terms. Every pair in the reference's own operations.
-template <int G, bool kEnergy, bool kAllPeriodic, bool kTerms, class BoxSrc>
+// The general pair kernel: tables of different starts or bin widths, open axes,
+// and the analytical terms. Every pair in the reference's own operations.
+// kUniform (tables of one start, bin width and length, on open axes mostly;
+// fast_pair_kernel has the periodic boxes): one word a lookup in place of a
+// 16-byte reference, 231 -> 217 us a launch at 300,007 beads with one open axis.
+// The shorter minimum image of rows inside the box is fast_pair_kernel's alone:
+// here its second loop costs what it saves (230 us without, 235 with it at
+// 300,007 beads with tables of two bin widths, 1,008 and 1,009 at 1,500,000), and
+// with analytical terms more (487 and 572).
+template <int G, bool kEnergy, bool kAllPeriodic, bool kTerms, bool kUniform, class BoxSrc>
 __global__ void __launch_bounds__(
 	256, pair_min_blocks<kEnergy, kTerms, std::is_same<BoxSrc, OneBox>::value>()) pair_force_kernel(
 	const float4* sorted_pos, const uint32_t* __restrict__ nbr,
 	const uint32_t* __restrict__ row_len, uint32_t n, uint32_t cap, int T,
-	const PairTableRef* __restrict__ refs_g, const float* __restrict__ force_g,
+	const PairTableRef* __restrict__ refs_g, PairTableRef uref, const float* __restrict__ force_g,
 	const float2* __restrict__ energy_g, uint32_t total_bins,
 	const PairTermRef* __restrict__ terms_g, PairSolvent sv, BoxSrc boxes, DistWindow win,
 	float4* force, double* __restrict__ ev) {
@@ -410,7 +426,7 @@ __global__ void __launch_bounds__(
 	const bool valid = i < n;
 	const Box& box = boxes.row(valid ? i : 0u);
 	const float4 pi = valid ? sorted_pos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-	const TableRow trow{refs + (valid ? type_of(pi) : 0) * T};
+	const TableRow<kUniform> trow{refs + (valid ? type_of(pi) : 0) * T, uref};
 	const PairTermRef* arow = kTerms ? terms_g + (valid ? type_of(pi) : 0) * T : nullptr;
 	const uint32_t cnt = valid ? row_len[i] : 0u;
 	// Entry k of row i: ((i / H) * cap + k) * H + i % H.
@@ -925,13 +941,13 @@ void launch_fast(const float4* sorted_pos, const uint32_t* nbr, const uint32_t* 
 				   ev);
 }
 
-template <int G, bool kEnergy, bool kAllPeriodic, bool kTerms, class BoxSrc>
+template <int G, bool kEnergy, bool kAllPeriodic, bool kTerms, class BoxSrc, bool kUniform = false>
 void launch_pair(const float4* sorted_pos, const uint32_t* nbr, const uint32_t* row_len,
 				 uint32_t n, uint32_t cap, const PairTables& t, const BoxSrc& boxes,
 				 float cutoff_sq, float4* force_sorted, double* ev, cudaStream_t st) {
 	const uint32_t rows = 256 / G;
 	const uint32_t blocks = (n + rows - 1) / rows;
-	auto kern = pair_force_kernel<G, kEnergy, kAllPeriodic, kTerms, BoxSrc>;
+	auto kern = pair_force_kernel<G, kEnergy, kAllPeriodic, kTerms, kUniform, BoxSrc>;
 	constexpr bool kStage = !std::is_same<BoxSrc, OneBox>::value;
 	const size_t smem =
 		static_cast<size_t>(t.num_types * t.num_types) * sizeof(PairTableRef) +
@@ -942,8 +958,8 @@ void launch_pair(const float4* sorted_pos, const uint32_t* nbr, const uint32_t* 
 		MB2_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
 									  static_cast<int>(smem)));
 	launch_chained(kern, blocks, 256u, smem, st, sorted_pos, nbr, row_len, n, cap, t.num_types,
-				   t.refs, t.bin_force, t.bin_energy, t.total_bins, t.terms, t.solvent, boxes,
-				   dist_window(cutoff_sq), force_sorted, ev);
+				   t.refs, t.uniform_ref, t.bin_force, t.bin_energy, t.total_bins, t.terms, t.solvent,
+				   boxes, dist_window(cutoff_sq), force_sorted, ev);
 }
 
 template <int G, bool kEnergy, class BoxSrc>
@@ -960,6 +976,11 @@ void launch_pair_e(const float4* sorted_pos, const uint32_t* nbr, const uint32_t
 		if (t.terms) {
 			if (all_periodic) launch_pair<G, kEnergy, true, true>(sorted_pos, nbr, row_len, n, cap, t, boxes, cutoff_sq, force_sorted, ev, st);
 			else launch_pair<G, kEnergy, false, true>(sorted_pos, nbr, row_len, n, cap, t, boxes, cutoff_sq, force_sorted, ev, st);
+			return;
+		}
+		if (t.fast_force) {  // uniform tables
+			if (all_periodic) launch_pair<G, kEnergy, true, false, BoxSrc, true>(sorted_pos, nbr, row_len, n, cap, t, boxes, cutoff_sq, force_sorted, ev, st);
+			else launch_pair<G, kEnergy, false, false, BoxSrc, true>(sorted_pos, nbr, row_len, n, cap, t, boxes, cutoff_sq, force_sorted, ev, st);
 			return;
 		}
 	}
