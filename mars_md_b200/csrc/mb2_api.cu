@@ -308,13 +308,15 @@ void build(mb2_context* ctx, const float4* pos, const int* type_ids, uint32_t n,
 	// run lost 12 % to the tracking pack, 12,012 beads were level and 65,536
 	// gained 12 %.
 	const bool ends_early = near_last && n > 16384u;
-	// The displacement since this build is tracked where it saves the pair
-	// kernel the rows' far part, and above kSmallN particles, where the inner
-	// rows save it 2.6 % at 2,097,152 beads (on a 65,536-bead step the pack's
-	// extra read and reduction cost more for those alone, 1-2 us). The word
+	// The displacement since this build is tracked for the pair kernel of uniform
+	// tables in periodic boxes: where it saves it the rows' far part, and above
+	// kSmallN particles, where the inner rows save it 2.6 % at 2,097,152 beads (on
+	// a 65,536-bead step the pack's extra read and reduction cost more for those
+	// alone, 1-2 us). For the other kernels, which do not ask, it would cost a
+	// 20-step run of 300,007 beads 60 us of 4,270. The word
 	// starts at zero, or at infinity where this pack meets a particle outside
 	// the box: the step that builds packs no more before its pair kernel.
-	const bool tracked = n > kSmallN || ends_early;
+	const bool tracked = ends_early || (n > kSmallN && displacement_asked(ctx->pt, ctx->box));
 	DisplacementTrack start;
 	if (tracked) {
 		ctx->d2max.ensure(1);

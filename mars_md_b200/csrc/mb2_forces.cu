@@ -1199,6 +1199,10 @@ void FastTableBufs::set(const std::vector<PairTableRef>& refs, const std::vector
 	t.fast_energy = energy.ptr;
 }
 
+bool displacement_asked(const PairTables& t, const Box& box) {
+	return box.periodic[0] && box.periodic[1] && box.periodic[2] && t.fast_force && !t.terms;
+}
+
 // Rows put the pairs that are likely to come within reach of the tables before
 // the next rebuild first and the rest after them, so that in a row's tail a
 // whole warp's pairs are beyond it, or are not read at all (set_far). The split
@@ -1212,9 +1216,7 @@ void FastTableBufs::set(const std::vector<PairTableRef>& refs, const std::vector
 float row_split(const PairTables& t, const Box& box, float rc_list, float cutoff) {
 	if (!(cutoff > 0.0f && cutoff < rc_list)) return 0.0f;
 	const float skin = rc_list - cutoff, wide = cutoff + 0.25f * skin;
-	const bool fast = box.periodic[0] && box.periodic[1] && box.periodic[2] && t.fast_force &&
-					  !t.terms;
-	return fast ? std::min(wide, t.reach_force + 1.5f * skin) : wide;
+	return displacement_asked(t, box) ? std::min(wide, t.reach_force + 1.5f * skin) : wide;
 }
 
 void pair_forces(const float4* sorted_pos, const uint32_t* nbr, const uint32_t* row_len,

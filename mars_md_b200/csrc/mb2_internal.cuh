@@ -324,6 +324,9 @@ void pair_forces(const float4* sorted_pos, const uint32_t* nbr, const uint32_t* 
 				 float cutoff_sq, int get_energy, float4* force_sorted, double* energy_virial,
 				 cudaStream_t st, const unsigned int* d2max = nullptr, float list_rc = 0.0f,
 				 const uint32_t* row_back = nullptr, float split = 0.0f);
+// Whether launches for these tables and box take the pair kernel that asks for the
+// displacement since the build.
+bool displacement_asked(const PairTables& t, const Box& box);
 // Where a build for these tables parts its rows near / far (0: it does not), and
 // whether the far part then is what a step mostly leaves out, so that the rows
 // keep the near part, the short one, behind it (the join moves that).
