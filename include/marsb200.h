@@ -385,8 +385,8 @@ MB2_API int mb2_step(mb2_context* ctx, float* pos4, float* force_energy4, const 
  * Langevin, are replayed from CUDA graphs (the whole interval between two
  * checks as one where the call has it all), the step number read from a device
  * word, so that small systems are not bound by launch overhead; a graph is
- * captured on first use and again whenever a pointer, size or parameter it
- * bakes in changes. Rebuild checks and steps while per-stage profiling is on
+ * captured on second use, and again whenever a pointer, size or parameter it
+ * bakes in has changed for two uses. Rebuild checks and steps while per-stage profiling is on
  * run as mb2_step. */
 MB2_API int mb2_run(mb2_context* ctx, float* pos4, float* force_energy4, const int* type_ids,
             const uint32_t* flags, uint32_t n, uint64_t first_step, uint32_t num_steps,

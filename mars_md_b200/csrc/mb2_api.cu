@@ -119,10 +119,11 @@ struct mb2_context {
 	bool profiling = false;
 	// mb2_run: the replayed graphs of the step bodies between rebuild checks,
 	// one of a single step and one of all the steps of an interval, the values
-	// each bakes in, its kernel launches, and the device step counter.
+	// each bakes in, those last met without a graph, its kernel launches, and the
+	// device step counter.
 	struct RunGraph {
 		cudaGraphExec_t exec = nullptr;
-		std::vector<uint64_t> key;
+		std::vector<uint64_t> key, seen;
 		unsigned long long launches = 0;
 	} run_one, run_many;
 	DevBuf<unsigned long long> step_d;
@@ -1288,12 +1289,14 @@ void step_once(mb2_context* ctx, float4* pos, float4* fe, const int* type_ids,
 						ctx->types, ctx->box, p, bonded ? 1 : 0, st);
 }
 
-// A step that is not a rebuild check, its number *ctx->step_d + offset: the
-// body mb2_run captures. packed: the step before it in the same graph left the
-// positions packed; leave: it does so for the step after it.
+// A step that is not a rebuild check, its number by the clock (in a graph) or
+// `step`: the body mb2_run captures, or launches as it is. packed: the step before
+// it in the same interval left the positions packed; leave: it does so for the
+// step after it.
 void step_body_replayable(mb2_context* ctx, float4* pos, float4* fe, const int* type_ids,
 						  const uint32_t* flags, uint32_t n, const mb2_step_params* prm,
-						  uint64_t offset, bool packed, bool leave, cudaStream_t st) {
+						  uint64_t step, const StepClock& clock, bool packed, bool leave,
+						  cudaStream_t st) {
 	const bool bonded = step_has_bonded(prm);
 	NextPack next;
 	if (leave) next = NextPack{ctx->sorted_pos.ptr, sorted_forces(ctx, n), track_of(ctx)};
@@ -1302,15 +1305,17 @@ void step_body_replayable(mb2_context* ctx, float4* pos, float4* fe, const int* 
 							  sorted_forces(ctx, n), bonded ? fe : nullptr, track_of(ctx));
 	pair_kernel(ctx, n, prm->cutoff, prm->get_energy, st, true);
 	bonded_stage(ctx, pos, fe, prm, prm->get_energy, st);
-	const StepClock clock{ctx->step_d.ptr, offset, prm->seed, prm->patch_id};
+	const uint64_t seed = mb2_bd_seed(prm->seed, prm->patch_id, step);
 	if (prm->integrator == 1) {
 		baoab_integrate_gather(pos, reinterpret_cast<float4*>(prm->mom4), fe,
 							   ctx->force_sorted.ptr, ctx->inv.ptr, bonded ? 1 : 0, type_ids, flags,
-							   n, ctx->types, ctx->box, prm->dt, prm->kT, 0u, 0u, 0u, prm->efield,
+							   n, ctx->types, ctx->box, prm->dt, prm->kT,
+							   static_cast<uint32_t>(step), seed, 0u, prm->efield,
 							   prm->deferred_kick_pending ? 1 : 0, st, clock, next);
 		return;
 	}
-	BdParams p{prm->dt, prm->kT, 0u, 0u, 0u, {prm->efield[0], prm->efield[1], prm->efield[2]}};
+	BdParams p{prm->dt, prm->kT, static_cast<uint32_t>(step), seed, 0u,
+			   {prm->efield[0], prm->efield[1], prm->efield[2]}};
 	bd_integrate_gather(pos, pos, fe, ctx->force_sorted.ptr, ctx->inv.ptr, type_ids, flags, n,
 						ctx->types, ctx->box, p, bonded ? 1 : 0, st, clock, next);
 }
@@ -1362,11 +1367,18 @@ std::vector<uint64_t> run_graph_key(const mb2_context* ctx, const float4* pos, c
 	return k;
 }
 
-// Captures `steps` step bodies into g unless it already holds them for this key.
+// Whether g holds `steps` step bodies for this key: captured when the key comes
+// the second time in a row without a graph. The first time, which for buffers that
+// change with every call is every time, a capture (0.2 ms for the 19 steps of an
+// interval) would cost more than it saves.
 template <class Body>
-void capture_steps(mb2_context::RunGraph& g, std::vector<uint64_t> key, uint32_t steps, Body body) {
+bool steps_captured(mb2_context::RunGraph& g, std::vector<uint64_t> key, uint32_t steps, Body body) {
 	key.push_back(steps);
-	if (g.exec && key == g.key) return;
+	if (g.exec && key == g.key) return true;
+	if (key != g.seen) {
+		g.seen = std::move(key);
+		return false;
+	}
 	if (g.exec) {
 		MB2_CUDA(cudaGraphExecDestroy(g.exec));
 		g.exec = nullptr;
@@ -1398,6 +1410,7 @@ void capture_steps(mb2_context::RunGraph& g, std::vector<uint64_t> key, uint32_t
 	cudaGraphDestroy(graph);
 	MB2_CUDA(ei);
 	g.key = std::move(key);
+	return true;
 }
 
 }  // namespace
@@ -1426,7 +1439,8 @@ int mb2_run(mb2_context* ctx, float* pos4, float* force_energy4, const int* type
 		// every step while per-stage profiling is on) run as mb2_step does. The
 		// steps from one check to the next are one graph where the call has them
 		// all (up to kRunSteps of them), so that no launch gap is left between
-		// them; what is left over is replayed step by step.
+		// them; what is left over is replayed step by step. Steps met for the first
+		// time are launched as they are, chained like the graphs' (steps_captured).
 		constexpr uint32_t kRunSteps = 32;
 		const uint32_t period = prm->rebuild_period;
 		const bool replayable = period != 0 && n > 0;
@@ -1451,13 +1465,20 @@ int mb2_run(mb2_context* ctx, float* pos4, float* force_energy4, const int* type
 			// three counted launches a step (tests/test_gpu_run.py); with two,
 			// 4,096 beads would take 950 us for 1,070 per 100 steps.
 			const bool leave = n <= kLeaveMax && step_has_bonded(prm);
-			capture_steps(g, key, steps, [&](uint32_t offset, cudaStream_t cs) {
-				step_body_replayable(ctx, pos, fe, type_ids, flags, n, prm, offset, leave && offset > 0u,
-									 leave && offset + 1u < steps, cs);
+			auto body = [&](uint32_t q, uint64_t at, const StepClock& clock, cudaStream_t on) {
+				step_body_replayable(ctx, pos, fe, type_ids, flags, n, prm, at, clock, leave && q > 0u,
+									 leave && q + 1u < steps, on);
+			};
+			const bool replay = steps_captured(g, key, steps, [&](uint32_t q, cudaStream_t cs) {
+				body(q, 0, StepClock{ctx->step_d.ptr, q, prm->seed, prm->patch_id}, cs);
 			});
-			step_counter_set(ctx->step_d.ptr, step, st);
-			MB2_CUDA(cudaGraphLaunch(g.exec, st));
-			g_launches += g.launches;
+			if (replay) {
+				step_counter_set(ctx->step_d.ptr, step, st);
+				MB2_CUDA(cudaGraphLaunch(g.exec, st));
+				g_launches += g.launches;
+			} else {
+				for (uint32_t q = 0; q < steps; ++q) body(q, step + q, StepClock{}, st);
+			}
 			k += steps;
 		}
 	});

@@ -45,6 +45,69 @@ def test_run_matches_steps(ctx_factory, langevin, first, lengths):
         assert (m <= 1e-3).mean() >= 0.99
 
 
+@pytest.mark.parametrize("period,steps", [(34, 70), (65, 140), (100, 130), (2, 9)])
+def test_run_over_intervals_of_other_lengths(ctx_factory, period, steps):
+    """Rebuild checks further apart than the longest graph (32 steps), whose
+    intervals are one graph and single steps or several graphs, and every other
+    step."""
+    w = W.plain_bd(n=2500, box=170.0)
+    got = []
+    for by_run in (True, False):
+        ctx = ctx_factory(w.n)
+        dev = setup_workload(ctx, w)
+        prm = step_params(w)
+        prm.rebuild_period = period
+        if by_run:
+            ctx.run(dev["pos"], dev["fe"], dev["type"], None, 1, steps, prm)
+        else:
+            for s in range(1, steps + 1):
+                ctx.step(dev["pos"], dev["fe"], dev["type"], None, s, prm)
+        got.append(dev["pos"].cpu().numpy()[:, :3])
+    d = np.abs(got[0] - got[1])
+    d = np.minimum(d, w.box_size[0] - d).max(axis=1)
+    assert (d <= 1e-4).mean() >= 0.99 and d.max() <= 0.1, float(d.max())
+
+
+@pytest.mark.parametrize("langevin", [False, True])
+def test_run_with_other_buffers_every_call(ctx_factory, langevin):
+    """Buffers met once are stepped without a graph, buffers that come back with
+    one: every call here has another ForceEnergy than the call before, then two
+    have the same."""
+    w = W.polymers(n_chains=3, beads=257, box=300.0, with_grid=False)
+    # (checks every five steps, so that few steps pass all the cases: over many the
+    # order of the float sums would part the two, as above)
+    lengths, which = [5, 5, 2, 3, 5, 5, 5], [0, 1, 0, 1, 0, 0, 0]
+    got = []
+    for by_run in (True, False):
+        ctx = ctx_factory(w.n)
+        dev = setup_workload(ctx, w)
+        fes = [dev["fe"], torch.zeros_like(dev["fe"])]
+        prm = step_params(w, bonds=dev["bonds"], bond_idx=dev["bond_idx"], angles=dev["angles"],
+                          angle_idx=dev["angle_idx"])
+        prm.rebuild_period = 5
+        if langevin:
+            t = len(w.diffusion)
+            ctx.set_langevin_types([150.0] * t, [[2e4] * 3] * t)
+            g = torch.Generator(device="cuda").manual_seed(3)
+            dev["mom"] = torch.randn((w.n, 4), device="cuda", generator=g) * 19.0
+            prm.integrator, prm.mom4, prm.deferred_kick_pending = 1, dev["mom"].data_ptr(), 1
+        s = 1
+        for k, b in zip(lengths, which):
+            if by_run:
+                ctx.run(dev["pos"], fes[b], dev["type"], None, s, k, prm)
+            else:
+                for q in range(k):
+                    ctx.step(dev["pos"], fes[b], dev["type"], None, s + q, prm)
+            s += k
+        got.append((dev["pos"].cpu().numpy()[:, :3], [f.cpu().numpy()[:, :3] for f in fes]))
+    d = np.abs(got[0][0] - got[1][0])
+    d = np.minimum(d, w.box_size[0] - d).max(axis=1)
+    assert (d <= 1e-4).mean() >= 0.99 and d.max() <= 0.1, float(d.max())
+    for a, b in zip(got[0][1], got[1][1]):
+        f = np.abs(a - b).max(axis=1)
+        assert (f <= 1e-2 * np.maximum(1.0, np.abs(b).max(axis=1))).mean() >= 0.99
+
+
 @pytest.mark.parametrize("beads,chains,langevin,grid", [(33, 1, False, False), (257, 3, True, False),
                                                         (1024, 17, False, True)])
 def test_steps_in_one_graph_hand_over(ctx_factory, beads, chains, langevin, grid):
