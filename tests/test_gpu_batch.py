@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 import torch
 
-from conftest import box_of
+from conftest import box_of, force_errors, tableset
 from mars_md_b200 import _lib, workloads as W
 from mars_md_b200.engine import Context, setup_batch, setup_workload, step_params
 
@@ -234,5 +234,84 @@ def test_batch_rejects_boxes_smaller_than_twice_the_list_radius():
     try:
         with pytest.raises(_lib.MB2Error):
             b.build(dev["pos"], dev["type"], 25.0)
+    finally:
+        b.close()
+
+
+def test_far_entries_with_systems_on_both_sides_of_the_limit(oracle):
+    """The tables end at a sixth of the cutoff, so a batch's rows are split and a
+    system's far entries are left out while its own displacement since its build
+    allows it: here, in one launch, a system that has hardly moved, one just
+    inside the limit and one beyond it, whose far entries hold pairs that have
+    come within reach. Forces against the oracle's over the list."""
+    ws = W.batched(seed=SEED, systems=3, nmin=2500, nmax=4000)
+    b, dev = setup_batch(ws)
+    try:
+        prm = step_params(ws[0], seed=SEED)
+        prm.rebuild_period = 1000
+        b.step(dev["pos"], dev["fe"], dev["type"], 1, prm)   # lists built from ws[s].pos
+        split, reach = 12.0, 4.5   # 1.5 skins beyond the tables' last force at 4.5 A
+        rng = np.random.default_rng(5)
+        pos = []
+        for w, moved in zip(ws, (0.5, 3.6, 5.0)):
+            u = rng.normal(size=(w.n, 3))
+            u *= moved / np.linalg.norm(u, axis=1, keepdims=True)
+            p = w.pos.copy()
+            p[:, :3] = np.mod(p[:, :3] + u, w.box_size[0]).astype(np.float32)
+            pos.append(p)
+        dev["pos"].copy_(torch.from_numpy(np.concatenate(pos)))
+        b.step(dev["pos"], dev["fe"], dev["type"], 2, prm)
+        assert b.rebuild_schedule()[1] == 1
+        fe = dev["fe"].cpu().numpy()
+        per = _split_pairs(b.export_pairs().cpu().numpy().astype(np.int64), b.offsets)
+        for s, w in enumerate(ws):
+            pairs = np.ascontiguousarray(per[s].astype(np.int32))
+            L = w.box_size[0]
+
+            def dist(p):
+                d = p[pairs[:, 1], :3].astype(np.float64) - p[pairs[:, 0], :3]
+                return np.linalg.norm(d - L * np.rint(d / L), axis=1)
+            came = ((dist(w.pos) > split) & (dist(pos[s]) < reach - 0.1)).sum()
+            assert (came > 0) == (s == 2)
+            tags = oracle.resolve_tags(pairs, w.type_ids, w.term_matrix, w.num_types)
+            _, f64, fabs = oracle.pair_forces(pairs, pos[s], tags, tableset(w), box_of(w),
+                                              np.float32(w.cutoff) ** 2)
+            scaled, plain = force_errors(fe[b.offsets[s]:b.offsets[s + 1]], f64, fabs)
+            assert scaled <= 1e-5, (s, scaled, plain)
+    finally:
+        b.close()
+
+
+def test_partial_rebuilds_of_a_fast_system_beside_a_slow_one():
+    """Two systems of one batch, checked at every step, one whose beads diffuse ten
+    times as fast: it is rebuilt again and again beside the other's kept rows (split
+    near / far). Against each system run alone."""
+    ws = W.batched(seed=SEED, systems=2, nmin=1500, nmax=3000)
+    for s, w in enumerate(ws):
+        w.num_types, w.type_ids = 2, np.full(w.n, s, np.int32)
+        w.term_matrix = np.repeat(w.term_matrix, 4)
+        w.charge = np.zeros(2, np.float32)
+        w.diffusion = np.array([[15.0] * 3, [150.0] * 3], np.float32)
+    steps = 12
+
+    def prm_for(w, s):
+        p = step_params(w, seed=SEED + s)
+        p.rebuild_period = 1
+        return p
+
+    plain = _plain_trajectories(ws, prm_for, steps)
+    b, dev = setup_batch(ws)
+    try:
+        prm = prm_for(ws[0], 0)
+        b.run(dev["pos"], dev["fe"], dev["type"], 1, steps, prm)
+        torch.cuda.synchronize()
+        builds, systems = b.rebuild_schedule()[1], b.system_rebuilds()
+        assert builds >= 3 and systems == builds + 1   # both at first, then one of them
+        pos = dev["pos"].cpu().numpy()
+        for s, w in enumerate(ws):
+            d = _periodic_diff(pos[b.offsets[s]:b.offsets[s + 1], :3], plain[s][0][:, :3],
+                               w.box_size[0]).max(axis=1)
+            # (the sums' order moves a pair over a bin edge now and then)
+            assert (d <= 1e-4).mean() >= 0.99 and d.max() <= 0.1, (s, float(d.max()))
     finally:
         b.close()

@@ -65,9 +65,8 @@ def test_radix_sort_large_sortedness(ctx_factory):
 
 @pytest.mark.parametrize("n", [2, 3, 1000, 4097, 8192, 8193, 20000])
 def test_radix_sort_small_stable(ctx_factory, n):
-    """Up to 8,192 pairs one CTA sorts (a bitonic network over key and
-    position), above that the radix passes: both must give a host stable
-    argsort's permutation, here with many equal keys (16 distinct values) and
+    """Up to 8,192 pairs each element counts those that precede it, above that
+    the radix passes: both must give a host stable argsort's permutation, here with many equal keys (16 distinct values) and
     payloads that are not in ascending order, on both sides of the switch."""
     rng = np.random.default_rng(n)
     keys_np = rng.integers(0, 16, n).astype(np.uint32) * np.uint32(0x10001001)

@@ -69,22 +69,27 @@ def _wrap_reference(x, l):
 
 @pytest.mark.parametrize("l", [1015.9, 127.0, 253.98427, 600.0, 33.3])
 def test_inner_row_minimum_image(l):
-    """The pair kernel's rows inside the box (every neighbour's difference in
-    [-l/2, l/2)) take x, or RN(RN(x + l) - l) for a set sign bit, in place of
-    the reference's floor sequence: the same float on every such x, signed
-    zeros and tiny magnitudes included (+l/2 itself is outside the rows'
-    bound and is the one value where the two differ)."""
+    """The rows inside the box of the pair kernel for uniform tables (every
+    neighbour's difference in [-l/2, l/2)) take RN(RN(x + m) - m) in place of the
+    reference's floor sequence, with m = fma(min(max(x 2^126, 0), 1), -l, l): 0 for
+    x > 0, l otherwise. The same float on every such x, signed zeros and tiny
+    magnitudes down to the smallest normal included (+l/2 itself is outside the
+    rows' bound and is the one value where the two differ)."""
     f = np.float32
     l = f(l)
     half = f(0.5) * l
     rng = np.random.default_rng(7)
+    tiny = np.finfo(f).tiny
     x = np.concatenate([
         rng.uniform(-half, half, 1_000_000).astype(f),
         (rng.uniform(-1, 1, 100_000) * 1e-3).astype(f),
         (rng.uniform(-1, 1, 100_000) * 1e-30).astype(f),
-        np.array([0.0, -0.0, -half, np.nextafter(half, f(0)), -np.nextafter(half, f(0))], f)])
-    w = ((x + l).astype(f) + (-l)).astype(f)
-    inner = np.where(x.view(np.int32) < 0, w, x).astype(f)
+        np.array([0.0, -0.0, tiny, -half, np.nextafter(half, f(0)), -np.nextafter(half, f(0))], f)])
+    with np.errstate(over="ignore"):
+        up = np.clip(x * f(2.0 ** 126), f(0), f(1)).astype(f)   # saturating: -0 and below give 0
+    m = (l - up * l).astype(f)                                  # exact: up is 0 or 1
+    assert np.all((up == 0) | (up == 1))
+    inner = ((x + m).astype(f) - m).astype(f)
     ref = _wrap_reference(x, l)
     assert np.array_equal(inner.view(np.uint32), ref.view(np.uint32))
     assert _wrap_reference(np.array([half], f), l)[0] != half  # the excluded end
