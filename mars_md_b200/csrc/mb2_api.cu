@@ -722,8 +722,8 @@ int mb2_sort_morton(mb2_context* ctx, const float* pos4, uint32_t n, const float
 		const float4* pos = reinterpret_cast<const float4*>(pos4);
 		// Sorted in the caller's arrays where it gives them (the context's state
 		// is of no use after this call).
-		ctx->keys.ensure(n);
-		ctx->s2o.ensure(n);
+		if (!keys_out) ctx->keys.ensure(n);
+		if (!s2o_out) ctx->s2o.ensure(n);
 		uint32_t* keys = keys_out ? keys_out : ctx->keys.ptr;
 		uint32_t* s2o = s2o_out ? s2o_out : ctx->s2o.ptr;
 		morton_encode(pos, n, bmin, bmax, keys, s2o, st);
@@ -1461,9 +1461,9 @@ int mb2_run(mb2_context* ctx, float* pos4, float* force_energy4, const int* type
 			const bool use_many = many > 1u && ahead >= many;
 			auto& g = use_many ? ctx->run_many : ctx->run_one;
 			const uint32_t steps = use_many ? many : 1u;
-			// Steps without bonded terms keep their three kernels: callers rely on
-			// three counted launches a step (tests/test_gpu_run.py); with two,
-			// 4,096 beads would take 950 us for 1,070 per 100 steps.
+			// Steps without bonded terms keep the pack as a launch of their own, so that
+			// mb2_launch_count goes up by three a step as it does for mb2_step; handed
+			// over, 100 steps of 4,096 beads would take 950 us for 1,070.
 			const bool leave = n <= kLeaveMax && step_has_bonded(prm);
 			auto body = [&](uint32_t q, uint64_t at, const StepClock& clock, cudaStream_t on) {
 				step_body_replayable(ctx, pos, fe, type_ids, flags, n, prm, at, clock, leave && q > 0u,

@@ -7,7 +7,9 @@
 // +f on the second, half the energy to each. Each pair's float result is
 // rounded exactly as the reference rounds it (explicit _rn intrinsics, the
 // same orientation via bit 31 of the list entry); only the order in which
-// the per-particle sums accumulate differs.
+// the per-particle sums accumulate differs. (Two corners aside: beads three and
+// more box edges apart, see oriented_image; and a distance of exactly 1e-6f,
+// which the reference keeps but gives no direction.)
 //
 // Table lookup (TabulatedPotential::compute, TabulatedPotential.h:19-52) is
 // precomputed per bin: bin_force[k] = -(U[k+1] - U[k]) * step_inv rounded as
@@ -192,7 +194,9 @@ struct TableRow {
 // when the pair is stored second to first (pi - pj is exactly -(pj - pi) in
 // round-to-nearest, so the multiply is the flip, on the FMA pipe). npi =
 // (-pi.x, -pi.y). kInner: the caller knows that every component lies in
-// [-l/2, l/2] of an all-periodic box.
+// [-l/2, l/2] of an all-periodic box. The packed multiply and add of the image
+// (x and y) come out as one operation rounded once, however they are written; that
+// is the reference's two roundings wherever image * l is exact, up to two images.
 template <bool kAllPeriodic, bool kInner>
 __device__ __forceinline__ void oriented_image(const float4& pi, const float2& npi,
 											   const float4& pj, float sgn, const Box& box,
@@ -463,10 +467,10 @@ __global__ void __launch_bounds__(
 }
 
 // Pair forces through tables of one start and bin width. The list, its layout,
-// the sums and every pair's value, bit for bit, are the general kernel's; a
-// pair takes fewer instructions to it (the general kernel is bound by issuing
-// them, 76 thread instructions a pair and 82 % issue active at 2,097,152
-// beads, with the L1's data pipe at 80 % close behind):
+// the sums and every pair's value, bit for bit, are the general kernel's, which
+// is bound by issue (82 % of the slots) and the L1's data pipe (80 %) together;
+// fewer of a pair's instructions are lookups and conversions here (1,048,576
+// beads, under the profiler: 618 us a launch for 642):
 //  * the root and its reciprocal are a hardware estimate and one Newton-Raphson
 //    correction each (sqrt_and_inverse), the correctly rounded ones on every
 //    float (one estimate for both, which was not, took 0.5 % less of a 20-step
@@ -486,9 +490,10 @@ __global__ void __launch_bounds__(
 // flight together spill 60 bytes there and at 40 registers lose the warps
 // (run of 20 steps at 2,097,152 beads, with a first form of this arithmetic:
 // 32.5 ms with the general kernel, 37.1 and 34.7 ms for those two, 31.0 ms
-// pipelined). What bounds it is then the L1's data pipe (81 % of its
-// wavefronts, half of them the j-forces' reductions) with issue (78 %) close
-// behind; the tables in shared memory instead of L1 took 34.5 ms.
+// pipelined). What bounds it is issue (83 % of the slots, 3.04 warp instructions a
+// stored pair) with the L1's data pipe behind (74 %: 128 M wavefronts, and the
+// j-forces' reductions touch 79 M sectors); the tables in shared memory instead of
+// L1 took 34.5 ms a run of 20 steps at 2,097,152.
 template <bool kEnergy, bool kOneBox>
 constexpr int fast_min_blocks() {
 	return kEnergy ? 5 : (kOneBox ? 8 : 6);

@@ -160,7 +160,13 @@ struct CellGrid {
 constexpr uint32_t kSmallN = 131072;
 // Rows a warp walks when a list is built (at most kWalkRows): as many as share
 // the finding of candidates well, fewer where the GPU would be left short of
-// warps.
+// warps. One storing walk in us at 1 / 2 / 4 / 8 rows, short lists (radius 25,
+// 0.0005 beads a cubic Angstrom) and long ones (35, 0.002): at 8,000 beads 17 / 15 /
+// 17 / 24 and 60 / 62 / 71 / 101; 12,288 24 / 23 / 22 / 27 and 80 / 83 / 91 / 125;
+// 20,000 41 / 33 / 30 / 34 and 110 / 101 / 97 / 127; 32,768 72 / 59 / 45 / 41 and 201 /
+// 174 / 139 / 157; 65,536 100 / 70 / 51 / 45 and 333 / 255 / 204 / 188; 300,007 349 /
+// 241 / 171 / 144 and 1,450 / 1,121 / 834 / 709. The lines lie where the two lists are
+// about even, or one gains what the other loses.
 inline uint32_t walk_rows(uint32_t n) {
 	return n >= 65536u ? 8u : (n >= 32768u ? 4u : (n >= 12288u ? 2u : 1u));
 }

@@ -13,12 +13,13 @@
 // particles are a contiguous run of the sorted array. The stencil is every
 // cell whose box-to-box distance from the home cell can be within rc (a
 // pruned sphere, not the reference's (2r+1)^3 cube), at the cell level chosen
-// per run to minimise candidates plus per-cell cost. One warp owns one
-// group of 32 consecutive sorted particles and walks, in lockstep, the cells
-// within rc of the group's cell bounding box, testing one candidate per
-// step against all of them. The test is a cheap minimum-image distance; only candidates
-// inside a rounding band around rc (sized from the float ulp of the box)
-// take the exact reference computation.
+// per run to minimise the walk's cost (choose_cell_grid). A warp owns up to 8
+// consecutive sorted particles (walk_rows) and walks them in runs of one cell: its
+// lanes find and load 32 candidates of the cell's stencil at a time, drop those
+// too far from the run's coordinate box, and test the rest, one a lane, against
+// every row of the run (walk_run). The test is a cheap minimum-image distance; only
+// candidates inside a rounding band around rc (sized from the float ulp of the
+// box) take the exact reference computation.
 //
 // Storage. A half list in sliced ELL form: rows of H consecutive particles
 // form a slice; entry k of row i sits at ((i / H) * cap + k) * H + i % H, so
